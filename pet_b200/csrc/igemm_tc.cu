@@ -45,6 +45,11 @@ constexpr int kMathTf32x3 = 3, kMathTf32x1 = 1, kMathBf16x3 = 16;
 constexpr int kAHalfBytes = kTileM * 128; // one 128 x 32 operand tile
 constexpr int kThreads = 352;   // warps: 0 B producer, 1 MMA, 2 raw producer, 3-6 and 7-10 two transform/epilogue sets
 constexpr int kProfSlots = 24; // tuning counters per CTA (see IgemmParams::prof)
+#ifdef PETB200_TUNE
+constexpr bool kTune = true; // a build of its own: the counters cost instructions in every role's inner loop
+#else
+constexpr bool kTune = false;
+#endif
 constexpr int kMaxNB = 6;
 constexpr int kMaxNR = 6;
 
@@ -89,7 +94,7 @@ struct IgemmParams {
     const float *res; // optional residual, laid out like y: y = act(sum + bias + res)
     float *y;
     int *status;
-    long long *prof; // optional per-CTA counters (kProfSlots per CTA), for tuning only
+    long long *prof; // optional per-CTA counters (kProfSlots per CTA), filled by builds with -DPETB200_TUNE only
     int pp;          // persistent "ping-pong" mode: the grid's x extent is smaller than the number of pixel tiles (mtiles); a CTA
                      // walks tiles blockIdx.x, + gridDim.x, ...; the two transform sets take alternate TILES (each set produces
                      // every A stage of its tile and then stores it) and the accumulators alternate between two TMEM
@@ -608,6 +613,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_bhi,
         const __grid_constant__ CUtensorMap tmap_blo, const IgemmParams P) {
     extern __shared__ uint8_t smem_raw[];
+    long long *const prof = kTune ? P.prof : nullptr;
     // 1024-byte alignment for the swizzled operand tiles
     uint8_t *smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
     const SmemLayout L = smem_layout(P, A_TMEM);
@@ -636,8 +642,8 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
     constexpr int KE = BF ? 64 : 32;              // K elements per stage
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     long long *prof_cta = nullptr; // wall-clock marks of this CTA (entry, prologue done, epilogue done, exit), tuning only
-    if (P.prof && threadIdx.x == 96) {
-        prof_cta = P.prof + ((size_t)(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * kProfSlots;
+    if (prof && threadIdx.x == 96) {
+        prof_cta = prof + ((size_t)(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * kProfSlots;
         prof_cta[8] = (long long)ptx::globaltimer_ns();
     }
     const int ntile = blockIdx.y / P.ksplit;
@@ -861,225 +867,160 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
         const uint64_t bdesc0 = ptx::smem_desc_k128(ptx::smem_u32(sB));
         const uint64_t adesc0 = A_TMEM ? 0ull : ptx::smem_desc_k128(ptx::smem_u32(sA));
         const uint32_t b_half16 = b_half >> 4;
-        uint32_t tmem_acc = tmem_base, tmem_small = tmem_base + (uint32_t)P.BN; // main and cross-term accumulators of the tile
-        uint32_t accumulate = 0;
-        int sa = 0, sb = 0, prev_sa = -1, prev_sb = -1;
-        uint32_t pa = 0, pb = 0;
+        // What this loop costs besides its MMAs decides the kernel's rate: the tensor pipe needs 770 / 385 / 240 cycles for the
+        // eight MMAs of a stage at BN = 128 / 64 / 32, a wait on a complete mbarrier 110-130, a vote 41, elect 35.  So: ring
+        // positions as running values, the next stage's barriers polled before this stage's MMAs are issued, one elected
+        // block per stage, nothing else on the common path.  A wait that gives up sets the CTA's abort flag, after which
+        // every later wait returns at once: the loop then simply runs out.  (12 K stages at BN = 32, m128 n2304 k768:
+        // 11.8 -> 10.0 us; BN = 64 persistent, 64-channel 3x3 at batch 64: 117 -> 97 us; BN = 128: unchanged, the operand
+        // warps are the bound there.)
         long long t_wa = 0, t_wb = 0, t_wf = 0;
-        const long long t_begin = P.prof ? clock64() : 0;
-        bool ok = true, ready_next = false;
-        const int FLm = PP ? 0 : P.fl;
-        int gpos = 0, gidx = 0; // position of the stage inside its flush group, index of the group
+        const long long t_begin = prof ? clock64() : 0;
+        const uint32_t BNu = (uint32_t)P.BN, a_col0 = tmem_base + (uint32_t)P.a_col;
+        const int NA = P.NA, NB = P.NB;
+        uint32_t tmem_acc = tmem_base, tmem_small = tmem_base + BNu; // main and cross-term accumulators of the tile
+        uint32_t sa = 0, sb = 0, pa = 0, pb = 0;
+        bool ok = true;
+        const int FLm = (PP || !SPLIT) ? 0 : P.fl;
+        int gpos = 0; // position of the stage inside its flush group
+        uint32_t gpar = 0; // parity of the group's drain
+        bool ready = false; // the current stage has been seen complete
         bool cross_prepaid = false; // the current stage's cross-term MMAs were issued ahead, during the previous stage
         // Ping-pong mode: each transform set fills its own half of the A ring (slots 2*set, 2*set + 1, alternately), so every
         // slot's barriers see one producer in order; bit i of `apar` is the parity of slot i's next completed fill.
         uint32_t apar = 0;
-        for (int tl = 0; tl < ntl && ok; ++tl) {
-        if (PP) {
-            // accumulators alternate between two TMEM regions; before reusing one, its previous tile must have been read out
-            tmem_acc = tmem_base + (uint32_t)((tl & 1) * 2 * P.BN);
-            tmem_small = tmem_acc + (uint32_t)P.BN;
-            if (tl >= 2) {
-                ok = ptx::mbar_wait(acc_empty + (tl & 1), (uint32_t)(((tl >> 1) - 1) & 1), abort_flag);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok)
-                    break;
-                ptx::tc_fence_after();
-            }
-            accumulate = 0;
-            ready_next = false;
-            prev_sa = -1;
-        }
-        for (int ks = 0; ks < KS; ++ks) {
+        for (int tl = 0; tl < ntl; ++tl) {
             if (PP) {
-                sa = (tl & 1) * 2 + (ks & 1);
-                pa = (apar >> sa) & 1u;
-            }
-            if (!ready_next) { // not already seen complete by the poll issued in the shadow of the previous stage's MMAs
-                if (P.prof) {
-                    const long long q0c = clock64();
-                    ok = ptx::mbar_wait(a_full + sa, pa, abort_flag);
-                    const long long q1c = clock64();
-                    ok = ok && ptx::mbar_wait(b_full + sb, pb, abort_flag);
-                    t_wa += q1c - q0c;
-                    t_wb += clock64() - q1c;
-                } else {
-                    ok = ptx::mbar_wait(a_full + sa, pa, abort_flag) && ptx::mbar_wait(b_full + sb, pb, abort_flag);
-                }
-                ok = __all_sync(0xffffffffu, ok);
-            }
-            if (!ok)
-                break;
-            ptx::tc_fence_after();
-            const uint64_t bhi = bdesc0 + (uint64_t)((uint32_t)sb * 2u * b_half16);
-            const uint32_t ahi_t = tmem_base + (uint32_t)P.a_col + (uint32_t)sa * 64u, alo_t = ahi_t + 32u;
-            const uint64_t ahi_s = adesc0 + (uint64_t)((uint32_t)sa * 2u * (kAHalfBytes >> 4));
-            const uint64_t alo_s = ahi_s + (kAHalfBytes >> 4);
-            // next stage's ring positions, polled (non-blocking) while this stage's last MMAs are still queued
-            int nsa = sa + 1, nsb = sb + 1;
-            uint32_t npa = pa, npb = pb;
-            if (nsa == P.NA) {
-                nsa = 0;
-                npa ^= 1u;
-            }
-            if (PP) { // the next stage of this tile sits in the set's other slot
-                nsa = (tl & 1) * 2 + ((ks + 1) & 1);
-                npa = (apar >> nsa) & 1u;
-                apar ^= 1u << sa;
-            }
-            if (nsb == P.NB) {
-                nsb = 0;
-                npb ^= 1u;
-            }
-            // one K=8 step.  The cross terms have their own accumulator: the tensor core truncates (rounds toward zero) its
-            // accumulator after every MMA, a bias proportional to the accumulator's magnitude; keeping the small terms
-            // away from the big sum removes most of those truncations from it.
-            auto issue_step = [&](int kk) {
-                const uint32_t acc_kk = kk == 0 ? accumulate : 1u;
-                if (SPLIT) {
-                    if (A_TMEM)
-                        mma_ts(tmem_acc, ahi_t + kk * 8, bhi + 2 * kk, idesc_wide, acc_kk);
-                    else
-                        ptx::mma_tf32_ss(tmem_acc, ahi_s + 2 * kk, bhi + 2 * kk, idesc_wide, acc_kk);
-                } else {
-                    mma_ts(tmem_acc, ahi_t + kk * 8, bhi + 2 * kk, idesc, acc_kk); // single TF32 pass
-                }
-                if (kk == 0 && prev_sa >= 0) { // release the previous stage once this stage's first MMA is queued
-                    ptx::mma_commit(a_empty + prev_sa);
-                    ptx::mma_commit(b_empty + prev_sb);
-                }
-                if (SPLIT) {
-                    if (A_TMEM)
-                        mma_ts(tmem_small, alo_t + kk * 8, bhi + 2 * kk, idesc, 1u);
-                    else
-                        ptx::mma_tf32_ss(tmem_small, alo_s + 2 * kk, bhi + 2 * kk, idesc, 1u);
-                }
-            };
-            // First stage of a new flush group: the main accumulator restarts from zero, but only after the transform warps
-            // have drained the previous group's sum.  The stage's eight cross-term MMAs do not touch the main accumulator
-            // and are issued first, so the tensor pipe has work while the drain is in flight.
-            auto issue_main_only = [&](int kk) {
-                mma_ts(tmem_acc, ahi_t + kk * 8, bhi + 2 * kk, idesc, 1u);
-                if (kk == 0 && prev_sa >= 0) {
-                    ptx::mma_commit(a_empty + prev_sa);
-                    ptx::mma_commit(b_empty + prev_sb);
-                }
-            };
-            const bool group_start = SPLIT && FLm > 0 && ks > 0 && gpos == 0; // (no division: this warp's loop is latency bound)
-            const bool prepaid_now = cross_prepaid;
-            cross_prepaid = false;
-            if (group_start) {
-                const uint64_t blo = bhi + b_half16;
-                if (ptx::elect_one()) {
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        mma_ts(tmem_small, ahi_t + kk * 8, blo + 2 * kk, idesc, 1u);
-                        if (kk == 0 && prev_sa >= 0) {
-                            ptx::mma_commit(a_empty + prev_sa);
-                            ptx::mma_commit(b_empty + prev_sb);
-                        }
-                        mma_ts(tmem_small, alo_t + kk * 8, bhi + 2 * kk, idesc, 1u);
-                    }
-                }
-                __syncwarp();
-                // ... and, if the stage after this one is already there, its eight cross-term MMAs as well: 2 x 8 MMAs of
-                // cover for the drain (that stage then only issues its four main MMAs)
-                bool pre = (ks + 1 < KS) && FLm >= 2 && ptx::mbar_test_wait(a_full + nsa, npa) && ptx::mbar_test_wait(b_full + nsb, npb);
-                pre = __all_sync(0xffffffffu, pre);
-                if (pre) {
+                // accumulators alternate between two TMEM regions; before reusing one, its previous tile must have been read out
+                tmem_acc = tmem_base + (uint32_t)(tl & 1) * 2u * BNu;
+                tmem_small = tmem_acc + BNu;
+                if (tl >= 2) {
+                    ok = ptx::mbar_wait(acc_empty + (tl & 1), (uint32_t)(((tl >> 1) - 1) & 1), abort_flag) && ok;
+                    __syncwarp();
                     ptx::tc_fence_after();
-                    const uint64_t nbhi = bdesc0 + (uint64_t)((uint32_t)nsb * 2u * b_half16), nblo = nbhi + b_half16;
-                    const uint32_t nahi = tmem_base + (uint32_t)P.a_col + (uint32_t)nsa * 64u, nalo = nahi + 32u;
+                }
+            }
+            for (int ks = 0; ks < KS; ++ks) {
+                if (PP) {
+                    sa = (uint32_t)((tl & 1) * 2 + (ks & 1));
+                    pa = (apar >> sa) & 1u;
+                    apar ^= 1u << sa;
+                }
+                if (!ready) {
+                    const long long q0 = prof ? clock64() : 0;
+                    ok = ptx::mbar_wait(a_full + sa, pa, abort_flag) && ok;
+                    const long long q1 = prof ? clock64() : 0;
+                    ok = ptx::mbar_wait(b_full + sb, pb, abort_flag) && ok;
+                    if (prof)
+                        t_wa += q1 - q0, t_wb += clock64() - q1;
+                    __syncwarp();
+                }
+                ptx::tc_fence_after();
+                const uint64_t bhi = bdesc0 + (uint64_t)(sb * 2u * b_half16);
+                const uint32_t ahi_t = a_col0 + sa * 64u, alo_t = ahi_t + 32u;
+                const uint64_t ahi_s = adesc0 + (uint64_t)(sa * 2u * (kAHalfBytes >> 4)), alo_s = ahi_s + (kAHalfBytes >> 4);
+                uint32_t nsa = sa + 1, nsb = sb + 1, npa = pa, npb = pb; // the next stage's ring positions
+                if (nsa == (uint32_t)NA)
+                    nsa = 0, npa ^= 1u;
+                if (nsb == (uint32_t)NB)
+                    nsb = 0, npb ^= 1u;
+                if (PP) { // the next stage of this tile sits in the set's other slot
+                    nsa = (uint32_t)((tl & 1) * 2 + ((ks + 1) & 1));
+                    npa = (apar >> nsa) & 1u;
+                }
+                // Is the next stage there?  Asked before this stage's MMAs and read after them: the answer (about 100 cycles on
+                // a busy shared-memory port) travels while they are being issued.
+                const bool next_a = ptx::mbar_test_wait(a_full + nsa, npa), next_b = ptx::mbar_test_wait(b_full + nsb, npb);
+                const bool group_start = FLm > 0 && gpos == 0 && ks > 0;
+                if (group_start) {
+                    // First stage of a new flush group: the main accumulator restarts from zero, but only after the transform
+                    // warps have drained the previous group's sum.  The stage's eight cross-term MMAs do not touch the main
+                    // accumulator and are issued first, so the tensor pipe has work while the drain is in flight ...
+                    const uint64_t blo = bhi + b_half16;
                     if (ptx::elect_one()) {
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk) {
-                            mma_ts(tmem_small, nahi + kk * 8, nblo + 2 * kk, idesc, 1u);
-                            mma_ts(tmem_small, nalo + kk * 8, nbhi + 2 * kk, idesc, 1u);
+                            mma_ts(tmem_small, ahi_t + kk * 8, blo + 2 * kk, idesc, 1u);
+                            mma_ts(tmem_small, alo_t + kk * 8, bhi + 2 * kk, idesc, 1u);
                         }
                     }
                     __syncwarp();
-                    cross_prepaid = true;
-                }
-                const long long qf0 = P.prof ? clock64() : 0;
-                ok = ptx::mbar_wait(flushed, (uint32_t)((gidx - 1) & 1), abort_flag);
-                if (P.prof)
-                    t_wf += clock64() - qf0;
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok)
-                    break;
-                ptx::tc_fence_after();
-                if (ptx::elect_one()) {
+                    // ... and, if the stage after this one is already there, its eight cross-term MMAs as well: 2 x 8 MMAs of
+                    // cover for the drain (that stage then only issues its four main MMAs)
+                    const bool pre = __all_sync(0xffffffffu, next_a && next_b) && ks + 1 < KS && FLm >= 2;
+                    if (pre) {
+                        ptx::tc_fence_after();
+                        const uint64_t nbhi = bdesc0 + (uint64_t)(nsb * 2u * b_half16), nblo = nbhi + b_half16;
+                        const uint32_t nahi = a_col0 + nsa * 64u, nalo = nahi + 32u;
+                        if (ptx::elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < 3; ++kk)
-                        mma_ts(tmem_acc, ahi_t + kk * 8, bhi + 2 * kk, idesc, kk == 0 ? 0u : 1u);
-                }
-                __syncwarp();
-            } else if (prepaid_now) { // the cross terms of this stage were issued with the previous stage's
-                if (ptx::elect_one()) {
+                            for (int kk = 0; kk < 4; ++kk) {
+                                mma_ts(tmem_small, nahi + kk * 8, nblo + 2 * kk, idesc, 1u);
+                                mma_ts(tmem_small, nalo + kk * 8, nbhi + 2 * kk, idesc, 1u);
+                            }
+                        }
+                        __syncwarp();
+                    }
+                    const long long q2 = prof ? clock64() : 0;
+                    ok = ptx::mbar_wait(flushed, gpar, abort_flag) && ok;
+                    t_wf += prof ? clock64() - q2 : 0;
+                    gpar ^= 1u;
+                    __syncwarp();
+                    ptx::tc_fence_after();
+                    if (ptx::elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < 3; ++kk)
-                        issue_main_only(kk);
-                }
-                __syncwarp();
-            } else {
-                if (ptx::elect_one()) {
+                        for (int kk = 0; kk < 4; ++kk)
+                            mma_ts(tmem_acc, ahi_t + kk * 8, bhi + 2 * kk, idesc, kk == 0 ? 0u : 1u);
+                        ptx::mma_commit(a_empty + sa);
+                        ptx::mma_commit(b_empty + sb);
+                    }
+                    cross_prepaid = pre;
+                } else if (cross_prepaid) { // the cross terms of this stage were issued with the previous stage's
+                    cross_prepaid = false;
+                    if (ptx::elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < 3; ++kk)
-                        issue_step(kk);
-                }
-                __syncwarp();
-            }
-            ready_next = (ks + 1 < KS) && ptx::mbar_test_wait(a_full + nsa, npa) && ptx::mbar_test_wait(b_full + nsb, npb);
-            ready_next = __all_sync(0xffffffffu, ready_next);
-            const bool group_end = SPLIT && FLm > 0 && gpos == FLm - 1 && ks + 1 < KS;
-            if (++gpos == FLm)
-                gpos = 0, ++gidx;
-            if (ptx::elect_one()) {
-                if (group_start)
-                    mma_ts(tmem_acc, ahi_t + 24, bhi + 6, idesc, 1u);
-                else if (prepaid_now)
-                    issue_main_only(3);
-                else
-                    issue_step(3);
-                if (group_end) // fires once every MMA of the group has completed
-                    ptx::mma_commit(acc_ready);
-            }
-            __syncwarp();
-            accumulate = 1u;
-            if (ready_next) {
-                // MMA-bound: the release of this stage rides behind the next stage's first MMA (nothing to wait for)
-                prev_sa = sa;
-                prev_sb = sb;
-            } else {
-                // transform-bound: the next stage is not there yet, and its producers may be waiting for this slot
-                if (ptx::elect_one()) {
+                        for (int kk = 0; kk < 4; ++kk)
+                            mma_ts(tmem_acc, ahi_t + kk * 8, bhi + 2 * kk, idesc, 1u);
+                        ptx::mma_commit(a_empty + sa);
+                        ptx::mma_commit(b_empty + sb);
+                    }
+                } else if (ptx::elect_one()) {
+                    // The cross terms have their own accumulator: the tensor core truncates (rounds toward zero) its
+                    // accumulator after every MMA, a bias proportional to the accumulator's magnitude; keeping the small
+                    // terms away from the big sum removes most of those truncations from it.
+                    const uint32_t acc0 = ks > 0 ? 1u : 0u;
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk) {
+                        if (!SPLIT) { // single TF32 pass
+                            mma_ts(tmem_acc, ahi_t + kk * 8, bhi + 2 * kk, idesc, kk == 0 ? acc0 : 1u);
+                        } else if (A_TMEM) {
+                            mma_ts(tmem_acc, ahi_t + kk * 8, bhi + 2 * kk, idesc_wide, kk == 0 ? acc0 : 1u);
+                            mma_ts(tmem_small, alo_t + kk * 8, bhi + 2 * kk, idesc, 1u);
+                        } else {
+                            ptx::mma_tf32_ss(tmem_acc, ahi_s + 2 * kk, bhi + 2 * kk, idesc_wide, kk == 0 ? acc0 : 1u);
+                            ptx::mma_tf32_ss(tmem_small, alo_s + 2 * kk, bhi + 2 * kk, idesc, 1u);
+                        }
+                    }
                     ptx::mma_commit(a_empty + sa);
                     ptx::mma_commit(b_empty + sb);
                 }
                 __syncwarp();
-                prev_sa = -1;
+                if (FLm > 0 && ++gpos == FLm) {
+                    gpos = 0;
+                    if (ks + 1 < KS && ptx::elect_one()) // fires once every MMA of the group has completed
+                        ptx::mma_commit(acc_ready);
+                    __syncwarp();
+                }
+                ready = __all_sync(0xffffffffu, next_a && next_b) && ks + 1 < KS;
+                sa = nsa, sb = nsb, pa = npa, pb = npb;
             }
-            sa = nsa;
-            sb = nsb;
-            pa = npa;
-            pb = npb;
-        }
-        if (ptx::elect_one()) {
-            if (ok && prev_sa >= 0) {
-                ptx::mma_commit(a_empty + prev_sa);
-                ptx::mma_commit(b_empty + prev_sb);
-            }
-            if (ok)
+            if (ok && ptx::elect_one())
                 ptx::mma_commit((PP && (tl & 1)) ? acc_full1 : acc_full);
+            __syncwarp();
         }
-        __syncwarp();
-        }
-        if (lane == 0 && P.prof) {
-            long long *pr = P.prof + ((size_t)(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * kProfSlots;
-            pr[0] = t_wa;
-            pr[1] = t_wb;
-            pr[2] = clock64() - t_begin;
-            pr[16] = t_wf;
+        if (prof && lane == 0) {
+            long long *pr = prof + ((size_t)(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * kProfSlots;
+            pr[0] = t_wa, pr[1] = t_wb, pr[2] = clock64() - t_begin, pr[16] = t_wf;
         }
     } else {
         // ---------------- transform + epilogue: two sets of four warps (3..6 and 7..10) ----------------
@@ -1090,13 +1031,13 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
         const int p = quarter * 32 + lane;    // pixel row inside the tile
         bool alive = true;
         long long t_we = 0, t_wr = 0, t_g = 0, t_st = 0, t_dw = 0, t_dd = 0, t_loop = 0, t_epi0 = 0;
-        const long long t_begin = P.prof ? clock64() : 0;
+        const long long t_begin = prof ? clock64() : 0;
         const bool reg_total = !PP && SPLIT && A_TMEM && P.fl > 0 && P.fl_regs != 0; // (ping-pong plans never flush)
         const int FL = (!PP && SPLIT && A_TMEM && !reg_total) ? P.fl : 0;
         // Register-total mode: set 1 only drains (a function of its own: its 128 totals per thread want the whole register file)
         if (reg_total && tset == 1)
             alive = drain_only_set(tmem_base + ((uint32_t)(quarter * 32) << 16), (KS + P.fl - 1) / P.fl, acc_ready, acc_full, flushed,
-                                   abort_flag, lane, P.prof ? &t_dw : nullptr, P.prof ? &t_dd : nullptr);
+                                   abort_flag, lane, prof ? &t_dw : nullptr, prof ? &t_dd : nullptr);
         // Ping-pong mode: this set takes every second TILE of the CTA (set 0 the even ones) and produces all of its stages;
         // otherwise there is one tile and the sets take alternate stages of it.
         // Ping-pong mode: parities of this set's two A slots (free at first), and how many raw chunks of the CTA (all tiles,
@@ -1220,10 +1161,10 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
         const int fcol0 = tset == 0 ? 0 : ((P.BN / 32 + 1) / 2) * 32, fcol1 = tset == 0 ? ((P.BN / 32 + 1) / 2) * 32 : P.BN;
         int fg = 0; // next group this warp has to drain
         auto drain_group = [&](int g, bool wait_mma, bool signal) -> bool {
-            const long long cd0 = P.prof ? clock64() : 0;
+            const long long cd0 = prof ? clock64() : 0;
             if (wait_mma && !ptx::mbar_wait(acc_ready, (uint32_t)(g & 1), abort_flag))
                 return false;
-            const long long cd1 = P.prof ? clock64() : 0;
+            const long long cd1 = prof ? clock64() : 0;
             ptx::tc_fence_after();
             const uint32_t tq = tmem_base + ((uint32_t)(quarter * 32) << 16);
             for (int cc = fcol0; cc < fcol1; cc += 32) {
@@ -1244,7 +1185,7 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
             __syncwarp();
             if (signal && lane == 0)
                 ptx::mbar_arrive(flushed);
-            if (P.prof) {
+            if (prof) {
                 t_dw += cd1 - cd0;
                 t_dd += clock64() - cd1;
             }
@@ -1260,11 +1201,11 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
         int sa = PP ? 2 * tset : st;
         uint32_t pa = PP ? (own_apar & 1u) : 1u;
         for (int ch = 0; ch < ((reg_total && tset == 1) ? 0 : c1 - c0) && alive; ++ch, st -= P.spc) {
-            const long long cr0 = P.prof ? clock64() : 0;
+            const long long cr0 = prof ? clock64() : 0;
             const bool band_gather = BAND == 2; // no raw tiles: the operands come from global memory
             if (!band_gather)
                 alive = ptx::mbar_wait(raw_full + rb, prw, abort_flag); // also by a set without a stage in this chunk
-            if (P.prof)
+            if (prof)
                 t_wr += clock64() - cr0;
             const float *raw = reinterpret_cast<const float *>(sRaw + (size_t)rb * P.raw_bytes) + base_p;
             for (; st < P.spc && alive; st += sstep, gs += sstep) {
@@ -1281,9 +1222,9 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                     break;
                 const int4 *ko = reinterpret_cast<const int4 *>(sKoff + st * KE);
                 if (!A_TMEM) {
-                    const long long ce0 = P.prof ? clock64() : 0;
+                    const long long ce0 = prof ? clock64() : 0;
                     alive = ptx::mbar_wait(a_empty + sa, pa, abort_flag);
-                    if (P.prof)
+                    if (prof)
                         t_we += clock64() - ce0;
                     if (!alive)
                         break;
@@ -1294,7 +1235,7 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                     // on top of its slots in the ring.
                     uint32_t hi[32], lo[32];
                     const uint8_t *krow = sRaw + (size_t)rb * P.raw_bytes + (size_t)p * 128;
-                    const long long cg0 = P.prof ? clock64() : 0;
+                    const long long cg0 = prof ? clock64() : 0;
                     if (BAND == 2) {
                         // stage (c0 + ch) of the tile covers keys k0 .. k0 + 31 of the row tile's window; this set's next stage
                         // (two on) is fetched while this one is split and written
@@ -1324,15 +1265,15 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                         gather_split<kGatherFlat, PASSES>(ko, raw, krow, p, tmask, 0, true, zero_word, hi, lo);
                     else
                         gather_split<kGatherTable, PASSES>(ko, raw, krow, p, tmask, 0, false, zero_word, hi, lo);
-                    const long long ce0 = P.prof ? clock64() : 0;
+                    const long long ce0 = prof ? clock64() : 0;
                     alive = ptx::mbar_wait(a_empty + sa, pa, abort_flag);
                     if (!alive)
                         break;
                     ptx::tc_fence_after();
                     const uint32_t t = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)P.a_col + (uint32_t)sa * 64u;
                     ptx::tmem_st_32x32(t, hi);
-                    const long long cg1 = P.prof ? clock64() : 0;
-                    if (P.prof) {
+                    const long long cg1 = prof ? clock64() : 0;
+                    if (prof) {
                         t_we += cg1 - ce0;
                         t_g -= cg1 - ce0; // the gather time below is measured up to cg1
                     }
@@ -1340,7 +1281,7 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                         ptx::tmem_st_32x32(t + 32u, lo);
                     ptx::tmem_st_wait();
                     ptx::tc_fence_before();
-                    if (P.prof) {
+                    if (prof) {
                         t_g += cg1 - cg0;
                         t_st += clock64() - cg1;
                     }
@@ -1391,7 +1332,7 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
             }
         }
         // ---------------- epilogue ----------------
-        t_loop = P.prof ? clock64() - t_begin : 0;
+        t_loop = prof ? clock64() - t_begin : 0;
         if (PP) // the next tile's fills (the other set's): their loads only wait for buffers this tile has already released
             observe_until(min((tl + 2) * (c1 - c0), ntl * (c1 - c0)));
         // Addresses and store mode first: the MMA warp is still working through the last stages, so this costs nothing.
@@ -1440,7 +1381,7 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
             ptx::named_bar_sync(1, 256);
             ptx::tc_fence_after();
         }
-        t_epi0 = P.prof ? clock64() : 0;
+        t_epi0 = prof ? clock64() : 0;
         if (alive) {
             ptx::tc_fence_after();
 #define PETB200_EPI(ACT_)                                                                                              \
@@ -1464,8 +1405,8 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
         } // tiles of this set
         if (PP)
             observe_until(ntl * (c1 - c0)); // fills of tiles after this set's last one
-        if (P.prof && threadIdx.x == 96) { // lane 0 of warp 3 (transform set 0)
-            long long *pr = P.prof + ((size_t)(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * kProfSlots;
+        if (prof && threadIdx.x == 96) { // lane 0 of warp 3 (transform set 0)
+            long long *pr = prof + ((size_t)(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * kProfSlots;
             pr[3] = t_we;
             pr[4] = t_wr;
             pr[5] = t_loop;

@@ -59,6 +59,8 @@ __device__ unsigned long long g_mbar_wait_limit_ns = 2000000000ull;
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
     if (mbar_try_wait(bar, parity))
         return true;
+    if (*abort_flag)
+        return false;
     uint64_t t0 = globaltimer_ns();
     uint32_t spins = 0;
     while (!mbar_try_wait(bar, parity)) {
