@@ -13,17 +13,23 @@ import torch
 from . import lib as L
 
 
+# The calls below sit in front of kernels of a few microseconds: plain integers instead of ctypes objects (every entry point
+# declares its argument types), and the stream handle without a torch.cuda.Stream object around it.
+_current_device, _raw_stream = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
+
+
 def _ptr(t):
-    return C.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 def _stream():
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return _raw_stream(_current_device())
 
 
 def _f32(t):
-    assert t.is_cuda and t.dtype == torch.float32, "device fp32 tensors only"
+    assert t.is_cuda and t.dtype is torch.float32, "device fp32 tensors only"
     return t.contiguous()
+
 
 
 def perm_spec(after):
@@ -104,7 +110,7 @@ class Context:
     def conv2d_run(self, plan, x, bias=None, out=None, residual=None):
         """y = act(conv(x) + bias [+ residual]); residual (shaped like y) folds a following Add into the epilogue."""
         x = _f32(x)
-        y = out if out is not None else torch.empty(plan.out_shape, device=x.device, dtype=torch.float32)
+        y = out if out is not None else x.new_empty(plan.out_shape)
         b = _ptr(_f32(bias) if bias is not None else None)
         if residual is not None:
             if tuple(residual.shape) != tuple(plan.out_shape):
@@ -150,7 +156,7 @@ class Context:
             plan = self._plans[key] = self.conv3d_plan(x.shape, w.shape, pad, stride, dil, bias is not None, act, algo)
         plan._w = _f32(w)
         self.check(self.lib.petb200_conv3d_set_weights(plan.h, _ptr(plan._w), _stream()))
-        y = torch.empty(plan.out_shape, device=x.device, dtype=torch.float32)
+        y = x.new_empty(plan.out_shape)
         if residual is not None:
             self.check(self.lib.petb200_conv_run_residual(plan.h, _ptr(_f32(x)), _ptr(bias), _ptr(_f32(residual)), _ptr(y), _stream()))
         else:
@@ -179,7 +185,7 @@ class Context:
         if w is not None:
             plan._w = _f32(w)
             self.check(self.lib.petb200_convtrans_set_weights(plan.h, _ptr(plan._w), _stream()))
-        y = torch.empty(plan.out_shape, device=x.device, dtype=torch.float32)
+        y = x.new_empty(plan.out_shape)
         self.check(self.lib.petb200_convtrans_run(plan.h, _ptr(_f32(x)), _ptr(_f32(bias) if bias is not None else None),
                                                   _ptr(y), _stream()))
         return y
@@ -249,7 +255,7 @@ class Context:
         self.check(self.lib.petb200_matmul_set_weights(plan.h, _ptr(plan._b), _stream()))
 
     def matmul_run(self, plan, a, b, bias=None, out=None, residual=None):
-        c = out if out is not None else torch.empty(plan.out_shape, device=a.device, dtype=torch.float32)
+        c = out if out is not None else a.new_empty(plan.out_shape)
         if residual is not None:
             if tuple(residual.shape) != tuple(plan.out_shape):
                 raise L.PetError(L.ERR_INVALID, "residual must have the shape of the output")
