@@ -24,6 +24,10 @@ int tc_matmul_native_a(void *h);
 void tc_matmul_destroy(void *h);
 int tc_matmul_pack_b(void *h, const float *b, cudaStream_t s);
 int tc_matmul_run(void *h, const float *a_t, const float *bias, const float *res, float *cmat, cudaStream_t s);
+// implemented in gemv.cu
+constexpr int kGemvRows = 8;
+int gemv_run(petb200_ctx *ctx, const float *a, const float *b, const float *bias, const float *res, float *c, int bs, int m, int n, int k,
+             int transA, int transB, int act, cudaStream_t s);
 
 // -------------------------------------------------------------------------------------------------------------
 // CUDA-core kernels (exact fp32 products, sequential accumulation in the reference's loop order cc,tt,rr,ss)
@@ -103,122 +107,6 @@ __global__ void __launch_bounds__(256) k_matmul_simt(const float *__restrict__ a
         if (res)
             acc += __ldg(res + i);
         c[i] = apply_act(acc, act);
-    }
-}
-
-// Matrix-vector shapes (m <= 8 rows of A, e.g. a classifier head at batch 1): the 128-row tensor-core tile would be
-// almost empty, and the work is one pass over B.  A block owns 32 columns of C for all rows; exact fp32 FMA.
-//   B as [k][n]: lanes = columns (coalesced rows of B), the 8 warps split K and are added up through shared memory.
-//   B as [n][k]: a warp owns 4 columns, lanes split K (coalesced rows of B), lanes are added up by shuffles.
-constexpr int kGemvRows = 8, kGemvWarps = 16, kGemvKTile = 768;
-__global__ void __launch_bounds__(kGemvWarps * 32) k_gemv_small_m(const float *__restrict__ a, const float *__restrict__ b,
-                                                                 const float *__restrict__ bias, const float *__restrict__ res,
-                                                                 float *__restrict__ c, int m, int n, int k, int transA, int transB,
-                                                                 int act) {
-    pdl_prologue();
-    __shared__ float sa[kGemvRows][kGemvKTile];        // a K tile of A, row r at sa[r]
-    __shared__ float red[kGemvWarps][kGemvRows][33];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, bb = blockIdx.y;
-    const float *ab = a + (long long)bb * m * k, *bm = b + (long long)bb * k * n;
-    float acc[kGemvRows];
-#pragma unroll
-    for (int r = 0; r < kGemvRows; ++r)
-        acc[r] = 0.f;
-    const int col0 = blockIdx.x * 32;
-    for (int kt = 0; kt < k; kt += kGemvKTile) {
-        const int kn = min(kGemvKTile, k - kt);
-        __syncthreads(); // the previous tile has been consumed
-        for (int i = threadIdx.x; i < m * kn; i += kGemvWarps * 32) {
-            int r, kk;
-            if (transA) // A is [k][m]: consecutive threads read consecutive addresses
-                kk = i / m, r = i - kk * m;
-            else
-                r = i / kn, kk = i - r * kn;
-            sa[r][kk] = __ldg(transA ? ab + (long long)(kt + kk) * m + r : ab + (long long)r * k + kt + kk);
-        }
-        __syncthreads();
-        if (!transB) {
-            // B as [k][n]: lanes = columns (coalesced rows of B), the warps split the tile's K range
-            const int col = col0 + lane;
-            const int kbeg = kn * warp / kGemvWarps, kend = kn * (warp + 1) / kGemvWarps;
-            for (int k0 = kbeg; k0 < kend; k0 += 16) {
-                float bv[16]; // sixteen rows of B in flight per lane
-#pragma unroll
-                for (int u = 0; u < 16; ++u)
-                    bv[u] = (k0 + u < kend && col < n) ? __ldg(bm + (long long)(kt + k0 + u) * n + col) : 0.f;
-#pragma unroll
-                for (int u = 0; u < 16; ++u) {
-                    const int kk = min(k0 + u, kend - 1); // rows past the end carry bv = 0
-#pragma unroll
-                    for (int r = 0; r < kGemvRows; ++r)
-                        acc[r] = fmaf(sa[r][kk], bv[u], acc[r]);
-                }
-            }
-        } else {
-            // B as [n][k]: a warp owns columns warp and warp + 16 of the block, lanes split K (coalesced rows of B);
-            // two accumulator sets would be needed to keep both: process the tile column by column instead
-            for (int cc = 0; cc < 2; ++cc) {
-                const int col = col0 + warp + cc * kGemvWarps;
-                if (col >= n)
-                    break;
-                float part[kGemvRows];
-#pragma unroll
-                for (int r = 0; r < kGemvRows; ++r)
-                    part[r] = 0.f;
-                for (int k0 = lane; k0 < kn; k0 += 8 * 32) {
-                    float bv[8];
-#pragma unroll
-                    for (int u = 0; u < 8; ++u)
-                        bv[u] = k0 + 32 * u < kn ? __ldg(bm + (long long)col * k + kt + k0 + 32 * u) : 0.f;
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        const int kk = min(k0 + 32 * u, kn - 1);
-#pragma unroll
-                        for (int r = 0; r < kGemvRows; ++r)
-                            part[r] = fmaf(sa[r][kk], bv[u], part[r]);
-                    }
-                }
-                // per-column partial sums of this K tile go through shared memory, slot [cc*16 + warp... ] is this column
-#pragma unroll
-                for (int r = 0; r < kGemvRows; ++r) {
-                    float v = part[r];
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1)
-                        v += __shfl_xor_sync(0xffffffffu, v, o);
-                    if (lane == 0)
-                        red[cc][r][warp] = (kt == 0 ? 0.f : red[cc][r][warp]) + v;
-                }
-            }
-        }
-    }
-    if (!transB) {
-#pragma unroll
-        for (int r = 0; r < kGemvRows; ++r)
-            red[warp][r][lane] = acc[r];
-    }
-    __syncthreads();
-    // thread (warp = row, lane = column) finishes one output
-    if (warp < m) {
-        const int r = warp;
-        float v = 0.f;
-        int col;
-        if (!transB) {
-            col = col0 + lane;
-#pragma unroll
-            for (int w = 0; w < kGemvWarps; ++w) // K slices in order
-                v += red[w][r][lane];
-        } else {
-            col = col0 + (lane & 15) + (lane >> 4) * kGemvWarps;
-            v = red[lane >> 4][r][lane & 15];
-        }
-        if (col < n) {
-            if (bias)
-                v += __ldg(bias + col);
-            const long long co = ((long long)bb * m + r) * n + col;
-            if (res)
-                v += __ldg(res + co);
-            c[co] = apply_act(v, act);
-        }
     }
 }
 
@@ -554,11 +442,8 @@ int matmul_run(petb200_plan *plan, const float *a, const float *b, const float *
         }
         return tc_matmul_run(pl->tc, at, pl->has_bias ? bias : nullptr, res, c, s);
     }
-    if (pl->gemv) {
-        launch_pdl(k_gemv_small_m, dim3((unsigned)((pl->n + 31) / 32), (unsigned)pl->bs), kGemvWarps * 32, 0, s, 
-            a, b, pl->has_bias ? bias : nullptr, res, c, pl->m, pl->n, pl->k, pl->transA, pl->transB, pl->act);
-        return launched(ctx, "k_gemv_small_m");
-    }
+    if (pl->gemv)
+        return gemv_run(ctx, a, b, pl->has_bias ? bias : nullptr, res, c, pl->bs, pl->m, pl->n, pl->k, pl->transA, pl->transB, pl->act, s);
     long long total = (long long)pl->bs * pl->m * pl->n;
     launch_pdl(k_matmul_simt, grid_for(ctx, total, 256), 256, 0, s, a, b, pl->has_bias ? bias : nullptr, res, c, pl->bs, pl->m, pl->n, pl->k,
                                                             pl->transA, pl->transB, pl->act);

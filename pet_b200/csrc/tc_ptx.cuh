@@ -107,6 +107,11 @@ __device__ __forceinline__ void st_shared_f32(uint32_t cta_addr, float v) {
 __device__ __forceinline__ void st_dsmem_f32(uint32_t cluster_addr, float v) {
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_addr), "f"(v) : "memory");
 }
+__device__ __forceinline__ float ld_dsmem_f32(uint32_t cluster_addr) {
+    float v;
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_addr) : "memory");
+    return v;
+}
 
 // ---- 4-byte asynchronous copies (for sources TMA cannot address) ---------------------------------------------------
 // Copies 4 bytes, or writes 4 zero bytes without reading the source when `valid` is false (the zeros are then tracked
