@@ -21,8 +21,8 @@
 // or 128-bit per thread (row-major matmul output).
 //
 // Variants (template parameters): 3xTF32 (default), one TF32 pass, error-compensated bf16 (64 K elements per stage, K = 16 per
-// MMA); persistent "ping-pong" tiles for narrow filter tiles (a CTA walks several pixel tiles, the transform sets take
-// alternate tiles, accumulators alternate between two TMEM regions).  Long K ranges drain the main accumulator into a
+// MMA); persistent tiles (a CTA walks several pixel tiles, the transform sets run on into the next tile while the drain warps
+// store the last one).  Long K ranges drain the main accumulator into a
 // running total every few stages (the tensor core truncates its fp32 accumulator after every MMA).
 // Split-K: the ksplit CTAs of one output tile form a thread-block cluster and exchange their partial sums through
 // distributed shared memory (pushes into the owner's landing area, one cluster barrier, reduction in rank order).
@@ -34,6 +34,7 @@
 #include <array>
 #include <cstdlib>
 #include <map>
+#include <type_traits>
 
 namespace petb200 {
 
@@ -43,7 +44,21 @@ constexpr int kStageK = 32;               // 32-bit words per K stage = one 128-
 // error-compensated bf16 (hi/lo bf16 halves, three products, K = 16 per instruction: half the MMAs of 3xTF32 per K)
 constexpr int kMathTf32x3 = 3, kMathTf32x1 = 1, kMathBf16x3 = 16;
 constexpr int kAHalfBytes = kTileM * 128; // one 128 x 32 operand tile
-constexpr int kThreads = 352;   // warps: 0 B producer, 1 MMA, 2 raw producer, 3-6 and 7-10 two transform/epilogue sets
+// Warps: 0 filter producer, 1 MMA, 2 raw producer (3 idle); 4-7 and 8-11 the two transform sets; 12-15 the drain warps.  Each
+// group of four covers the four lane quarters of TMEM.
+constexpr int kThreads = 512, kSetWarp = 4, kDrainWarp = 12;
+constexpr int kNA = 4; // A stages in TMEM: a transform set owns slots `set` and `set + 2`
+// Kernel modes.  Single: one tile per CTA.  Persistent: a CTA walks several tiles, the transform sets run on into the next tile
+// while the drain warps store the last one; with BN <= 64 and no accumulator flush (narrow) accumulators alternate between two
+// TMEM regions, otherwise (wide) the drain warps take the sums of the one region into registers and hand it back first.
+enum { kSingle = 0, kNarrow = 1, kWide = 2 };
+// Registers per thread of the four warp groups (512 in sum, what the block is launched with): drain warps that keep a row of 128
+// sums need 184 or more; in single-tile mode the transform sets also run the epilogue.
+template <int PP> struct Regs {
+    static constexpr int control = PP == kSingle ? 56 : 72, set = PP == kSingle ? 136 : (PP == kNarrow ? 144 : 120),
+                         drain = PP == kSingle ? 184 : (PP == kNarrow ? 152 : 200);
+    static_assert(control + 2 * set + drain <= 512, "more registers than the block was launched with: setmaxnreg would wait forever");
+};
 constexpr int kProfSlots = 24; // tuning counters per CTA (see IgemmParams::prof)
 #ifdef PETB200_TUNE
 constexpr bool kTune = true; // a build of its own: the counters cost instructions in every role's inner loop
@@ -53,7 +68,24 @@ constexpr bool kTune = false;
 constexpr int kMaxNB = 6;
 constexpr int kMaxNR = 6;
 
+// Division by a number fixed when the plan is made: q = (umulhi(n, m) + n) >> s for 0 <= n < 2^31.  Tile coordinates take half a
+// dozen divisions in each of four roles; as generic divisions they are more instructions per tile than a K stage, and the
+// persistent kernel's roles together then overflow the SM's instruction cache.
+struct FastDiv {
+    uint32_t d, m, s;
+    void set(int div) {
+        d = (uint32_t)(div > 0 ? div : 1);
+        for (s = 0; (1ull << s) < d; ++s) {
+        }
+        m = (uint32_t)(((1ull << 32) * ((1ull << s) - d)) / d + 1);
+    }
+#ifdef __CUDACC__
+    __device__ __forceinline__ int div(int n) const { return (int)((__umulhi((uint32_t)n, m) + (uint32_t)n) >> s); }
+#endif
+};
+
 struct IgemmParams {
+    FastDiv by_ntiles, by_mtiles, by_tpi, by_pw, by_od, by_own, by_ohn, by_row_tiles; // (made by set_divisors)
     int Pw, units;          // pixels of one output plane (one image, one depth slice); number of such planes
     int OD, OH, OW;         // full output extents (for addressing y)
     int ohn, own, oh0, ow0; // output window actually computed (ohn*own = Pw)
@@ -68,14 +100,10 @@ struct IgemmParams {
     int tpi, ipt;           // otherwise: tiles per plane (plane larger than a tile) or whole planes per tile
     int ksplit;             // K is split over this many CTAs, launched as one thread-block cluster (2, 4, 8 or 16); partial
                             // tiles are added up through distributed shared memory
-    int NA, NB, NR;         // ring depths: A stages, B stages, raw activation buffers
+    int NB, NR;             // ring depths: B stages, raw activation buffers
     int fl;                 // 3xTF32 only: every `fl` K stages the main accumulator is drained into a running total that
                             // is summed with round-to-nearest adds (0: never).  The tensor core truncates its accumulator
                             // after every MMA; restarting it keeps the truncated partial sums short and small
-    int a_col;              // first TMEM column of the A-operand ring (TS variants)
-    int fl_regs;            // 128-wide tiles: the running total lives in the registers of the second transform set, whose
-                            // warps then do nothing but drain (the first set produces every A stage); narrower tiles
-                            // keep the total in TMEM columns [2*BN,3*BN) and both sets drain between their stages
     int a_kmajor;           // matmul with row-major A: the raw tile is [128 rows][32 k], 128B-swizzled, one per K stage
     int m_rows;             // a_kmajor: rows of A per batch entry
     int raw_bytes;          // bytes of one raw buffer (128-aligned)
@@ -83,8 +111,7 @@ struct IgemmParams {
                             // dense and unpadded, fetched as a 2-D box [flat_rows][flat_w] of the contiguous run; padding
                             // becomes a per-pixel mask over the filter taps (<= 32 taps)
     int flat_w, flat_rows;
-    int cstride;            // BC % 32 == 0, or BC 16 / 8: floats between consecutive channels of the raw tile (else 0: table)
-    int gruns;              // runs (filter taps) per 32-wide K stage in that mode: 1, 2 (BC 16) or 4 (BC 8)
+    int cstride;            // BC % 8 == 0: floats between consecutive channels of the raw tile (else 0: table)
     int T3[3], dil[3];      // filter extents and dilations (flat only: for the tap mask)
     int xD, xH, xW;         // input extents (flat only)
     long long ys_n, ys_f, ys_p;
@@ -95,31 +122,26 @@ struct IgemmParams {
     float *y;
     int *status;
     long long *prof; // optional per-CTA counters (kProfSlots per CTA), filled by builds with -DPETB200_TUNE only
-    int pp;          // persistent "ping-pong" mode: the grid's x extent is smaller than the number of pixel tiles (mtiles); a CTA
-                     // walks tiles blockIdx.x, + gridDim.x, ...; the two transform sets take alternate TILES (each set produces
-                     // every A stage of its tile and then stores it) and the accumulators alternate between two TMEM
-                     // regions, so one tile's epilogue and the next tile's start-up hide behind the MMAs of the other
-    int mtiles;      // pixel tiles along x
+    int pp;          // persistent mode: a one-dimensional grid of at most one CTA per SM walks all output tiles, CTA i tiles i,
+                     // i + gridDim.x, ...
+    int tiles, ntiles, mtiles; // persistent mode: all tiles, filter tiles (they vary fastest), pixel tiles
+    int band_g2;     // the banded product is G2BMM (host side)
     int band_w;      // > 0: banded product y[b,i,j] = q[b,i,:] . k[b,i+j-w,:] (row-major A = q, "filters" = the keys of the window
-                     // [128*tile - w, 128*tile + 127 + w] of the tile's rows, blockIdx.y = 64-key piece of that window); the
+                     // [128*tile - w, 128*tile + 127 + w] of the tile's rows, the filter tile being a 64-key piece of that window); the
                      // epilogue stores the band entries of each row at their skewed positions, zero where the key is outside [0,n)
+    long long band_words; // GBMML: words of the whole band
     const float *band_p; // non-null: GBMML y[b,i,c] = sum_j p[b,i,j] * v[b,i+j-w,c]: the A operand is the band p [bs][n][2w+1] read
-                     // straight from global memory by the transform threads (row i of the tile meets key k through p[i][k-i+w]),
+                     // row by row with asynchronous copies (row i of the tile meets key k through p[i][k-i+w]),
                      // the "filters" are v's columns with the keys as K (window of the tile's rows, start rounded down to 4)
-    int band_nt;     // banded product: 64-key pieces per row tile; the x tile index runs over (row tile, piece) pairs, piece fastest,
-                     // so that the cheap pieces at the band's edges are spread over all CTAs
-    int epi_direct;  // tuning: store the epilogue straight from registers (no transposition through shared memory)
     int starve;      // test hook: the filter producer announces more bytes than it loads, so the stage never completes
 };
 
 struct SmemLayout {
-    uint32_t a_off, b_off, raw_off, koff_off, split_off, stage_off, bar_off, total;
+    uint32_t b_off, raw_off, koff_off, split_off, stage_off, bar_off, total;
 };
-__host__ __device__ inline SmemLayout smem_layout(const IgemmParams &P, bool a_tmem) {
+__host__ __device__ inline SmemLayout smem_layout(const IgemmParams &P) {
     SmemLayout L;
     uint32_t o = 0;
-    L.a_off = o;
-    o += a_tmem ? 0 : (uint32_t)P.NA * 2 * kAHalfBytes;
     L.b_off = o;
     o += (uint32_t)P.NB * 2 * (uint32_t)P.BN * 128;
     L.raw_off = o;
@@ -130,24 +152,17 @@ __host__ __device__ inline SmemLayout smem_layout(const IgemmParams &P, bool a_t
     // own region: peers push into it while this CTA may still be in its main loop.
     L.split_off = (o + 127) & ~127u;
     o = L.split_off + (P.ksplit > 1 ? 512u * (uint32_t)P.BN + 1024u : 0u); // + each tile row's offset in y (-1: none)
-    // ping-pong mode: the epilogue's 32x32 transposition blocks need their own room (the B ring is never idle), one per warp
+    // persistent mode: the drain warps' 32x32 transposition blocks need their own room (the B ring is never idle)
     L.stage_off = (o + 127) & ~127u;
-    // (GBMML's operand fetch, which is not in ping-pong mode, keeps two blocks per warp: one stage in flight)
-    o = L.stage_off + (P.pp ? 8u * 4096u : ((P.a_kmajor && P.band_w > 0) ? 16u * 4096u : 0u));
+    o = L.stage_off + (P.pp ? 4u * 4096u : 0u);
     L.bar_off = (o + 15) & ~15u;
     L.total = L.bar_off + 384;
     return L;
 }
 
-// Which rows of an output plane the pixels [q_lo, q_hi] of that plane touch (all of them when a tile holds several
-// whole planes); shared by the raw producer, the transform threads and the host-side box sizing.
-__host__ __device__ inline void tile_rows(const IgemmParams &P, int q_lo, int q_hi, bool whole, int &yl_lo, int &yl_hi) {
-    yl_lo = 0;
-    yl_hi = P.ohn - 1;
-    if (whole)
-        return;
-    yl_lo = q_lo / P.own;
-    yl_hi = q_hi / P.own;
+static void set_divisors(IgemmParams &P) {
+    P.by_ntiles.set(P.ntiles), P.by_mtiles.set(P.mtiles), P.by_tpi.set(P.tpi), P.by_pw.set(P.Pw);
+    P.by_od.set(P.OD), P.by_own.set(P.own), P.by_ohn.set(P.ohn), P.by_row_tiles.set(P.row_tiles);
 }
 
 template <int ACT> __device__ __forceinline__ float act_fn(float v) {
@@ -361,120 +376,137 @@ __device__ __forceinline__ void epilogue_banded(uint32_t tacc, uint32_t tcross, 
     }
 }
 
-// One K stage of one tile row: fetch the stage's operands (32, or 64 for bf16) and split them into hi/lo parts — TF32:
-// hi = top 19 bits, lo = x - hi, one value per word; bf16: hi = bf16(x), lo = bf16(x - hi), two values per word, the
-// lower K index in the low half; a single pass rounds instead.  Where the operands come from:
-//   kGatherTable   im2col through the offset table of the stage (entry < 0: no such element);
-//   kGatherFlat    the same for unpadded whole-plane raw tiles: entries carry the filter tap in bits 24..30 and `tmask`
-//                  tells which taps fall inside the input for this pixel;
-//   kGatherStride  the stage is RUNS runs of consecutive channels, each of ONE tap, so the operands of a run sit
-//                  `cstride` floats apart from the run's first table entry - no table reads, no per-element tests;
-//   kGatherKMajor  matmul with row-major A: row p of the 128B-swizzled [128][32] tile (two tiles for a 64-wide stage).
-enum { kGatherTable = 0, kGatherFlat = 1, kGatherStride = 2, kGatherKMajor = 3 };
-template <int MODE, int PASSES, int RUNS = 1>
-__device__ __forceinline__ void gather_split(const int4 *ko, const float *raw, const uint8_t *krow, int p, uint32_t tmask,
-                                             int cstride, bool flat, const float *zero_word, uint32_t (&hi)[32],
-                                             uint32_t (&lo)[32]) {
-    constexpr bool BF = PASSES == kMathBf16x3;
-    constexpr int KE = BF ? 64 : 32;  // operands per stage
-    constexpr int kRun = KE / RUNS;   // channels per run
-    const float *q[RUNS];
-    int cs[RUNS];
+// Operands of one tile row, eight 32-bit words at a time (a K stage is four such pieces: 32 TF32 values, or 64 bf16 in pairs),
+// split into hi/lo parts — TF32: hi = top 19 bits, lo = x - hi, one value per word; bf16: hi = bf16(x), lo = bf16(x - hi), two
+// values per word, the lower K index in the low half; a single pass rounds instead.
+// (A stage is 200 to 300 instructions that every transform warp fetches again for every stage — the SM quarter's first-level
+// instruction cache does not hold them — at about five cycles each, which is what bounds narrow tiles.  As a rolled loop of
+// eight elements it was no faster: the branches and the shorter runs of independent loads cost what the fetches did.)
+template <int PASSES> __device__ __forceinline__ void split_words(const float *v, uint32_t *hi, uint32_t *lo) {
+    if (PASSES == kMathBf16x3) {
 #pragma unroll
-    for (int r = 0; r < RUNS; ++r) {
-        q[r] = raw;
-        cs[r] = cstride;
-        if (MODE == kGatherStride) {
-            const int o0 = ko[r * (kRun / 4)].x; // first table entry of the run
-            // past the end of the chunk's K range, or a tap outside the input for this pixel: read zeros
-            const bool off = o0 < 0 || (flat && !((tmask >> (o0 >> 24)) & 1u));
-            q[r] = off ? zero_word : raw + (flat ? (o0 & 0xffffff) : o0);
-            cs[r] = off ? 0 : cstride;
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t h = ptx::pack_bf16x2(v[2 * i], v[2 * i + 1]);
+            hi[i] = h;
+            lo[i] = ptx::pack_bf16x2(v[2 * i] - __uint_as_float(h << 16), v[2 * i + 1] - __uint_as_float(h & 0xffff0000u));
         }
-    }
+    } else {
 #pragma unroll
-    for (int c4 = 0; c4 < KE / 4; ++c4) {
-        float v[4];
-        if (MODE == kGatherKMajor) { // 16-byte chunk c of row p sits at c ^ (p & 7); the second tile follows the first
-            const float4 t4 = *reinterpret_cast<const float4 *>(krow + (c4 >> 3) * kAHalfBytes + (((c4 & 7) ^ (p & 7)) << 4));
-            v[0] = t4.x, v[1] = t4.y, v[2] = t4.z, v[3] = t4.w;
-        } else if (MODE == kGatherStride) {
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-                v[i] = q[(4 * c4 + i) / kRun][((4 * c4 + i) % kRun) * cs[(4 * c4 + i) / kRun]];
-        } else {
-            const int4 o4 = ko[c4];
-            const int o[4] = {o4.x, o4.y, o4.z, o4.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                if (MODE == kGatherFlat)
-                    v[i] = (o[i] >= 0 && ((tmask >> (o[i] >> 24)) & 1u)) ? raw[o[i] & 0xffffff] : 0.f;
-                else
-                    v[i] = raw[o[i]]; // plain table mode has no negative entries
-            }
-        }
-        if (BF) {
-#pragma unroll
-            for (int i = 0; i < 4; i += 2) {
-                const uint32_t h = ptx::pack_bf16x2(v[i], v[i + 1]);
-                hi[2 * c4 + i / 2] = h;
-                lo[2 * c4 + i / 2] = ptx::pack_bf16x2(v[i] - __uint_as_float(h << 16), v[i + 1] - __uint_as_float(h & 0xffff0000u));
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                if (PASSES == kMathTf32x3) {
-                    hi[4 * c4 + i] = __float_as_uint(v[i]) & 0xffffe000u;
-                    lo[4 * c4 + i] = __float_as_uint(v[i] - __uint_as_float(hi[4 * c4 + i]));
-                } else { // single pass: round to nearest TF32 instead of letting the tensor core truncate
-                    hi[4 * c4 + i] = ptx::cvt_rna_tf32(v[i]);
-                }
+        for (int i = 0; i < 8; ++i) {
+            if (PASSES == kMathTf32x3) {
+                hi[i] = __float_as_uint(v[i]) & 0xffffe000u;
+                lo[i] = __float_as_uint(v[i] - __uint_as_float(hi[i]));
+            } else { // single pass: round to nearest TF32 instead of letting the tensor core truncate
+                hi[i] = ptx::cvt_rna_tf32(v[i]);
             }
         }
     }
 }
 
-// GBMML's operand fetch: one K stage = keys k0 .. k0 + 31; row i of the tile meets key k through the band entry p[i][k - i + w].
-// The 32 entries of a row are contiguous in global memory but every row starts elsewhere, so the warp fetches them row by
-// row (lane = key: one coalesced 128-byte read per row; entries outside the band, the row range or the sequence count as
-// zero) into an XOR-swizzled 32 x 32 block of shared memory, from which each thread then takes its own row.  The fetch is
-// asynchronous (cp.async, zero-filling what does not exist): band_issue starts the copies of a stage and closes a group,
-// band_take waits for the group and splits; the caller keeps one stage in flight while it works on the one before.
-__device__ __forceinline__ void band_issue(const float *pb /*band of this batch entry*/, int n, int w, int i0 /*first row of the warp*/, int k0,
-                                           float *stage, int lane) {
-    const int bw = 2 * w + 1, key = k0 + lane;
-    const bool key_ok = key >= 0 && key < n;
-    const float *src = pb + (long long)i0 * bw + (key - i0 + w); // row r: src + r * (bw - 1)
-    const uint32_t dst = ptx::smem_u32(stage);
+// Eight consecutive K elements of one tile row.  Where they come from:
+//   kGatherTable   im2col through the offset table of the stage (`ko`: the eight entries);
+//   kGatherFlat    the same for unpadded whole-plane raw tiles: entries < 0 mean no such element, the filter tap sits in bits
+//                  24..30 and `tmask` tells which taps fall inside the input for this pixel;
+//   kGatherStride  chunks of a multiple of eight channels: the eight are consecutive channels of ONE tap, `cstride` floats
+//                  apart from the first one's table entry - one table read, no per-element tests (kGatherPlain: chunks of a
+//                  multiple of 32 channels, one read per stage);
+//   kGatherKMajor  matmul with row-major A: half of a 128-byte row piece of the swizzled [128][32] tile (`krow`, 16-byte chunks
+//                  c and c + 1).
+enum { kGatherTable = 0, kGatherFlat = 1, kGatherStride = 2, kGatherPlain = 3, kGatherKMajor = 4, kGatherBand = 5 };
+template <int MODE>
+__device__ __forceinline__ void gather8(const int *ko, const float *raw, const uint8_t *krow, int c, int p, uint32_t tmask, int cstride, bool flat,
+                                        const float *zero_word, float *v) {
+    if (MODE == kGatherKMajor) { // 16-byte chunk c of row p sits at c ^ (p & 7)
+        const float4 a = *reinterpret_cast<const float4 *>(krow + ((c ^ (p & 7)) << 4)), b = *reinterpret_cast<const float4 *>(krow + (((c + 1) ^ (p & 7)) << 4));
+        v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w, v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+    } else if (MODE == kGatherStride) {
+        const int o0 = *ko;
+        // past the end of the chunk's K range, or a tap outside the input for this pixel: read zeros
+        const bool off = o0 < 0 || (flat && !((tmask >> (o0 >> 24)) & 1u));
+        const float *q = off ? zero_word : raw + (flat ? (o0 & 0xffffff) : o0);
+        const int cs = off ? 0 : cstride;
 #pragma unroll
-    for (int r = 0; r < 32; ++r, src += bw - 1) {
-        const int j = key - (i0 + r) + w;
-        const bool ok = key_ok && i0 + r < n && j >= 0 && j < bw;
-        // 4 bytes per lane; a source size of 0 writes zeros and reads nothing (the address is then a harmless valid one)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + (uint32_t)(r * 32 + (lane ^ r)) * 4u), "l"(ok ? src : pb),
-                     "r"(ok ? 4 : 0)
-                     : "memory");
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-}
-template <int PASSES>
-__device__ __forceinline__ void band_take(const float *stage, bool newer_in_flight, int lane, uint32_t (&hi)[32], uint32_t (&lo)[32]) {
-    if (newer_in_flight)
-        asm volatile("cp.async.wait_group 1;" ::: "memory"); // all but the newest group: this stage has landed
-    else
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncwarp(); // every lane's copies
+        for (int i = 0; i < 8; ++i)
+            v[i] = q[i * cs];
+    } else {
+        const int4 a = *reinterpret_cast<const int4 *>(ko), b = *reinterpret_cast<const int4 *>(ko + 4);
+        const int o[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-    for (int e = 0; e < 32; ++e) {
-        const float x = stage[lane * 32 + (e ^ lane)];
-        if (PASSES == kMathTf32x3) {
-            hi[e] = __float_as_uint(x) & 0xffffe000u;
-            lo[e] = __float_as_uint(x - __uint_as_float(hi[e]));
-        } else {
-            hi[e] = ptx::cvt_rna_tf32(x);
+        for (int i = 0; i < 8; ++i) {
+            if (MODE == kGatherFlat)
+                v[i] = (o[i] >= 0 && ((tmask >> (o[i] >> 24)) & 1u)) ? raw[o[i] & 0xffffff] : 0.f;
+            else
+                v[i] = raw[o[i]]; // plain table mode has no negative entries
         }
     }
-    __syncwarp(); // the block may be overwritten by a later stage's copies
+}
+
+// GBMML's operand: row i of the tile meets key k through the band entry p[i][k - i + w].  A chunk is the entries of 64 keys (two K
+// stages) for the tile's 128 rows.  A row's entries are contiguous, but rows are 2w + 1 words apart (odd), so each starts
+// somewhere else in its first 16 bytes: the transform warps fetch 16-byte pieces from the boundary below (16 lanes per row,
+// asynchronous copies, up to three chunks ahead), rows sit kBandPitch words apart in shared memory (16-byte reads of eight
+// neighbouring rows then hit different banks), and the thread that owns a row shifts its values into place while it reads
+// them.  What lies outside the band, the rows or the sequence counts as zero, whatever the memory holds.  (At n = 10000,
+// w = 1000 one 4-byte copy per entry took 66 us: 64 copies and reads with their own addresses and tests per thread and stage,
+// which overran the instruction cache as well; a bulk copy per row took 93 us, about 53 cycles of the copy engine each.)
+constexpr int kBandStages = 2, kBandKeys = kBandStages * kStageK, kBandPitch = kBandKeys + 4;
+// Word of the whole band at which row i's entry for key k0 sits (k0 a multiple of 4), and its place in its 16 bytes.
+__device__ __forceinline__ long long band_word(const IgemmParams &P, int zb, int i, int k0) {
+    return ((long long)zb * P.m_rows + i) * (2 * P.band_w + 1) + (k0 - i + P.band_w);
+}
+// One chunk, transform warp `wi` of eight: rows 2 * wi + (lane >> 4), + 16, ..  Sixteen rows on, a row's chunk starts exactly 32w
+// words further, so inside the band (all but the first and last chunks of a row tile) the copies need no tests and one
+// addition each.  Every lane arrives on `bar` when its copies have landed.
+__device__ __forceinline__ void band_copy(const IgemmParams &P, int zb, int i0, int k0, int wi, int lane, uint32_t raw_addr, uint64_t *bar) {
+    const int bw = 2 * P.band_w + 1, rows = min(kTileM, P.m_rows - i0), off0 = k0 - i0 + P.band_w;
+    const long long row0 = ((long long)zb * P.m_rows + i0) * bw; // first entry of the tile's first row
+    const float *base = P.band_p + (row0 & ~3ll);                // word offsets below are relative to this
+    const int in0 = (int)(row0 & 3), p0 = 2 * wi + (lane >> 4), c = 4 * (lane & 15);
+    const int a0 = (in0 + p0 * bw + off0 - p0) & ~3; // the first row's first word
+    uint32_t dst = raw_addr + (uint32_t)(p0 * kBandPitch + c) * 4u;
+    // the 17th pieces: one of this warp's sixteen rows per lane
+    const int p17 = 2 * wi + (lane & 1) + 16 * ((lane & 15) >> 1);
+    const int a17 = ((in0 + p17 * bw + off0 - p17) & ~3) + kBandKeys;
+    const uint32_t dst17 = raw_addr + (uint32_t)(p17 * kBandPitch + kBandKeys) * 4u;
+    if (rows == kTileM && off0 - (kTileM - 1) >= 0 && off0 + kBandPitch + 3 <= bw) {
+        const float *src = base + (a0 + c);
+#pragma unroll
+        for (int r = 0; r < 8; ++r, src += 32 * P.band_w, dst += 16 * kBandPitch * 4)
+            ptx::cp_async_16(dst, src);
+        if (lane < 16)
+            ptx::cp_async_16(dst17, base + a17);
+    } else {
+        const int end = (int)min(P.band_words / 4 * 4 - (row0 & ~3ll), 1ll << 30);
+        // 16-byte pieces that hold entries of the row (the last, incomplete one of the whole band is left out: with w >= 3 its
+        // keys lie past the sequence)
+        auto exists = [&](int p, int a) {
+            const int row = in0 + p * bw;
+            return p < rows && a >= (row & ~3) && a < min((row + bw + 3) & ~3, end);
+        };
+#pragma unroll 2
+        for (int r = 0; r < 8; ++r, dst += 16 * kBandPitch * 4)
+            if (exists(p0 + 16 * r, a0 + c + r * 32 * P.band_w))
+                ptx::cp_async_16(dst, base + (a0 + c + r * 32 * P.band_w));
+        if (lane < 16 && exists(p17, a17))
+            ptx::cp_async_16(dst17, base + a17);
+    }
+    ptx::cp_async_mbar_arrive_noinc(bar);
+}
+// Eight of a row's operands: `src` is their place in shared memory, `shift` the row's place in its first 16 bytes, [lo_e, hi_e)
+// the elements that exist.
+__device__ __forceinline__ void band_take8(const float *src, int shift, int lo_e, int hi_e, float *v) {
+    float q[12];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const float4 t = *reinterpret_cast<const float4 *>(src + 4 * c);
+        q[4 * c] = t.x, q[4 * c + 1] = t.y, q[4 * c + 2] = t.z, q[4 * c + 3] = t.w;
+    }
+#pragma unroll
+    for (int e = 0; e < 11; ++e)
+        q[e] = (shift & 1) ? q[e + 1] : q[e];
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+        v[e] = e >= lo_e && e < hi_e ? ((shift & 2) ? q[e + 2] : q[e]) : 0.f;
 }
 
 // Split-K reduction inside a thread-block cluster.  The ksplit CTAs of one output tile form a cluster; CTA `rank` owns
@@ -553,62 +585,191 @@ __device__ __forceinline__ void cluster_reduce_store(const float *stage, int ksp
     }
 }
 
-// Register-total flush mode, transform set 1: its threads keep the 128 columns of their tile row in registers, add the main
-// accumulator of every completed group of K stages to them (round-to-nearest adds, in group order), and at the end write
-// total + last group back over the main accumulator, which the epilogue of both sets then reads as if nothing had happened.
-// Returns false if a wait gave up.
-__device__ __noinline__ bool drain_only_set(uint32_t tq /*TMEM address of this warp's lane quarter, column 0*/, int groups,
-                                            uint64_t *acc_ready, uint64_t *acc_full, uint64_t *flushed, volatile int *abort_flag,
-                                            int lane, long long *t_wait, long long *t_work) {
-    float racc[128];
+// Drain warps: a thread keeps the BN sums of its tile row in registers.  add_main: sums (+)= main accumulator; with the cross
+// terms on top for the last (or only) group of a tile: hi*hi sum + (lo*hi + hi*lo) sum, one rounded fp32 add.
+template <bool CROSS>
+__device__ __forceinline__ void drain_add(float (&racc)[128], uint32_t tmain, uint32_t tcross, int BN, bool first) {
 #pragma unroll
-    for (int j = 0; j < 128; ++j)
-        racc[j] = 0.f;
-    for (int g = 0; g < groups; ++g) {
-        const bool last = g == groups - 1;
-        const long long cd0 = t_wait ? clock64() : 0;
-        if (!(last ? ptx::mbar_wait(acc_full, 0u, abort_flag) : ptx::mbar_wait(acc_ready, (uint32_t)(g & 1), abort_flag)))
-            return false;
-        const long long cd1 = t_wait ? clock64() : 0;
-        ptx::tc_fence_after();
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            uint32_t v0[16], v1[16];
-            ptx::tmem_ld_32x16(tq + (uint32_t)(b * 32), v0);
-            ptx::tmem_ld_32x16(tq + (uint32_t)(b * 32 + 16), v1);
+    for (int b = 0; b < 8; ++b) {
+        if (b * 16 < BN) {
+            uint32_t v[16], c[16];
+            ptx::tmem_ld_32x16(tmain + (uint32_t)(b * 16), v);
+            if (CROSS)
+                ptx::tmem_ld_32x16(tcross + (uint32_t)(b * 16), c);
             ptx::tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-                racc[b * 32 + j] += __uint_as_float(v0[j]);
-                racc[b * 32 + 16 + j] += __uint_as_float(v1[j]);
+                float x = __uint_as_float(v[j]);
+                if (!first)
+                    x = racc[b * 16 + j] + x;
+                racc[b * 16 + j] = CROSS ? x + __uint_as_float(c[j]) : x;
             }
-            if (last) {
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    v0[j] = __float_as_uint(racc[b * 32 + j]);
-                    v1[j] = __float_as_uint(racc[b * 32 + 16 + j]);
-                }
-                ptx::tmem_st_32x16(tq + (uint32_t)(b * 32), v0);
-                ptx::tmem_st_32x16(tq + (uint32_t)(b * 32 + 16), v1);
-            }
-        }
-        if (last)
-            ptx::tmem_st_wait();
-        ptx::tc_fence_before();
-        __syncwarp();
-        if (!last && lane == 0)
-            ptx::mbar_arrive(flushed);
-        if (t_wait) {
-            *t_wait += cd1 - cd0;
-            *t_work += clock64() - cd1;
         }
     }
-    return true;
+}
+
+__device__ __forceinline__ void act4(float4 &v, int act) {
+    if (act == PETB200_ACT_NONE)
+        return;
+    if (act == PETB200_ACT_RELU) {
+        v.x = fmaxf(v.x, 0.f), v.y = fmaxf(v.y, 0.f), v.z = fmaxf(v.z, 0.f), v.w = fmaxf(v.w, 0.f);
+        return;
+    }
+    v.x = apply_act(v.x, act), v.y = apply_act(v.y, act), v.z = apply_act(v.z, act), v.w = apply_act(v.w, act);
+}
+
+// Persistent mode: one 32-column block of a warp's 32 tile rows, sums in r (thread = row), to y through the warp's 4 KB block of
+// shared memory, so that every store instruction writes whole 16-byte pieces of consecutive addresses.
+//   kStorePixels  y's pixels are contiguous (NCHW): a lane stores four pixels of one filter;
+//   kStoreFilters y's filters are contiguous (row-major matmul, channels last): a lane stores four filters of one row;
+//   kStoreAny     anything else: a thread stores its own row, one element at a time.
+// The drain warps store a tile while the tensor core works on the next, which at 64 filters and few K stages lasts only two to
+// four thousand cycles, and a taken branch costs them 70 to 250 (see the MMA issuer): the common activations go out in
+// straight-line code, eight predicated loads and stores in flight; bias, residual and activation are applied on the way out,
+// once per 16 bytes.  (As a loop with tests per store a tile of 16 valid pixels took 15000 cycles.)
+enum { kStorePixels = 0, kStoreFilters = 1, kStoreAny = 2 };
+struct StoreJob {
+    float *y;                // filter 0 of the group
+    const float *bias, *res; // the same, or null
+    long long ys_f, y_off, y_off0; // this row, the warp's first row
+    int mode, Fg, act, nvalid, lane;
+    bool valid;
+};
+template <bool RES>
+__device__ __forceinline__ void store_pixels(const StoreJob &J, const float *stage, int f0) { // four pixels that are all valid per lane
+    const int px = (J.lane & 7) * 4, cq = J.lane >> 3, fmax = px + 4 <= J.nvalid ? J.Fg - f0 - cq : 0; // filters left from this lane's first one
+    const long long off = J.y_off0 + (long long)(f0 + cq) * J.ys_f + px, step = 4 * J.ys_f;
+    float4 v[8];
+    if (RES) {
+        const float *rs = J.res + off;
+#pragma unroll
+        for (int i = 0; i < 8; ++i, rs += step)
+            v[i] = 4 * i < fmax ? __ldg(reinterpret_cast<const float4 *>(rs)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    float b[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        b[i] = J.bias != nullptr && 4 * i < fmax ? __ldg(J.bias + f0 + cq + 4 * i) : 0.f;
+    float *dst = J.y + off;
+#pragma unroll
+    for (int i = 0; i < 8; ++i, dst += step) {
+        float4 q = *reinterpret_cast<const float4 *>(stage + (cq + 4 * i) * 32 + px);
+        if (J.bias != nullptr)
+            q.x += b[i], q.y += b[i], q.z += b[i], q.w += b[i];
+        if (RES) // y = act(sum + bias + residual): the residual's four pixels sit where y's will
+            q.x += v[i].x, q.y += v[i].y, q.z += v[i].z, q.w += v[i].w;
+        if (J.act == PETB200_ACT_RELU)
+            q.x = fmaxf(q.x, 0.f), q.y = fmaxf(q.y, 0.f), q.z = fmaxf(q.z, 0.f), q.w = fmaxf(q.w, 0.f);
+        if (4 * i < fmax)
+            *reinterpret_cast<float4 *>(dst) = q;
+    }
+}
+__device__ __forceinline__ void store_block(const StoreJob &J, const float *r /*32 sums*/, float *stage, int f0) {
+    const int lane = J.lane;
+    if (J.mode == kStorePixels && J.nvalid == 0)
+        return;
+    __syncwarp(); // the previous block has been read
+    if (J.mode == kStoreFilters) {
+        // row r of the block at [r][32], 16-byte chunk c at c ^ (r & 7): conflict-free both ways
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+            *reinterpret_cast<float4 *>(stage + lane * 32 + ((c ^ (lane & 7)) << 2)) = make_float4(r[4 * c], r[4 * c + 1], r[4 * c + 2], r[4 * c + 3]);
+        __syncwarp();
+        const int c = lane & 7, f = f0 + 4 * c;
+        const bool live = f < J.Fg; // (Fg % 4 == 0 in this mode)
+        float4 bv = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (J.bias != nullptr && live)
+            bv = make_float4(__ldg(J.bias + f), __ldg(J.bias + f + 1), __ldg(J.bias + f + 2), __ldg(J.bias + f + 3));
+        const long long yo = J.valid ? J.y_off : -1;
+        if (J.act <= PETB200_ACT_RELU) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int row = 4 * i + (lane >> 3);
+                const long long off = __shfl_sync(0xffffffffu, yo, row);
+                const bool go = off >= 0 && live;
+                float4 v = *reinterpret_cast<const float4 *>(stage + row * 32 + ((c ^ (row & 7)) << 2));
+                if (J.bias != nullptr)
+                    v.x += bv.x, v.y += bv.y, v.z += bv.z, v.w += bv.w;
+                if (J.res != nullptr && go) {
+                    const float4 q = __ldg(reinterpret_cast<const float4 *>(J.res + off + f));
+                    v.x += q.x, v.y += q.y, v.z += q.z, v.w += q.w;
+                }
+                if (J.act == PETB200_ACT_RELU)
+                    v.x = fmaxf(v.x, 0.f), v.y = fmaxf(v.y, 0.f), v.z = fmaxf(v.z, 0.f), v.w = fmaxf(v.w, 0.f);
+                if (go)
+                    *reinterpret_cast<float4 *>(J.y + off + f) = v;
+            }
+            return;
+        }
+#pragma unroll 1
+        for (int i = 0; i < 8; ++i) {
+            const int row = 4 * i + (lane >> 3);
+            const long long off = __shfl_sync(0xffffffffu, yo, row);
+            if (off >= 0 && live) {
+                float4 v = *reinterpret_cast<const float4 *>(stage + row * 32 + ((c ^ (row & 7)) << 2));
+                if (J.bias != nullptr)
+                    v.x += bv.x, v.y += bv.y, v.z += bv.z, v.w += bv.w;
+                if (J.res != nullptr) {
+                    const float4 q = __ldg(reinterpret_cast<const float4 *>(J.res + off + f));
+                    v.x += q.x, v.y += q.y, v.z += q.z, v.w += q.w;
+                }
+                act4(v, J.act);
+                *reinterpret_cast<float4 *>(J.y + off + f) = v;
+            }
+        }
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+        stage[j * 32 + lane] = r[j];
+    __syncwarp();
+    if (J.mode == kStorePixels && J.act <= PETB200_ACT_RELU) {
+        if (J.res != nullptr)
+            store_pixels<true>(J, stage, f0);
+        else
+            store_pixels<false>(J, stage, f0);
+        if ((J.nvalid & 3) == 0 || lane < (J.nvalid & ~3)) // (only the last one to three pixels of a ragged window are left)
+            return;
+    }
+    if (J.mode == kStorePixels && J.act > PETB200_ACT_RELU) {
+        const int px = (lane & 7) * 4, cq = lane >> 3;
+        const int fmax = px + 4 <= J.nvalid ? J.Fg - f0 - cq : 0;
+        const long long off = J.y_off0 + (long long)(f0 + cq) * J.ys_f + px;
+#pragma unroll 1
+        for (int i = 0; 4 * i < fmax && i < 8; ++i) {
+            const long long o = off + (long long)(4 * i) * J.ys_f;
+            float4 v = *reinterpret_cast<const float4 *>(stage + (cq + 4 * i) * 32 + px);
+            if (J.bias != nullptr) {
+                const float bf = __ldg(J.bias + f0 + cq + 4 * i);
+                v.x += bf, v.y += bf, v.z += bf, v.w += bf;
+            }
+            if (J.res != nullptr) {
+                const float4 q = __ldg(reinterpret_cast<const float4 *>(J.res + o));
+                v.x += q.x, v.y += q.y, v.z += q.z, v.w += q.w;
+            }
+            act4(v, J.act);
+            *reinterpret_cast<float4 *>(J.y + o) = v;
+        }
+        if ((J.nvalid & 3) == 0 || lane < (J.nvalid & ~3))
+            return;
+    }
+    if (J.valid) {
+#pragma unroll 1
+        for (int j = 0; j < 32 && f0 + j < J.Fg; ++j) { // one element at a time: this lane's own row
+            float v = stage[j * 32 + lane];
+            const long long o = J.y_off + (long long)(f0 + j) * J.ys_f;
+            if (J.bias != nullptr)
+                v += __ldg(J.bias + f0 + j);
+            if (J.res != nullptr)
+                v += __ldg(J.res + o);
+            J.y[o] = apply_act(v, J.act);
+        }
+    }
 }
 
 // BAND: 0 ordinary operands; 1 G2BMM (banded epilogue, key windows per tile; persistent row-major mode only); 2 GBMML (A operand
 // gathered from the band in global memory; row-major mode only).  Kernels of their own, so that the others carry none of it.
-template <bool A_TMEM, bool A_KMAJOR, int PASSES, bool PP = false, int BAND = 0>
+template <bool A_KMAJOR, int PASSES, int PP = kSingle, int BAND = 0>
 __global__ void __launch_bounds__(kThreads, 1)
 k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_bhi,
         const __grid_constant__ CUtensorMap tmap_blo, const IgemmParams P) {
@@ -616,8 +777,7 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
     long long *const prof = kTune ? P.prof : nullptr;
     // 1024-byte alignment for the swizzled operand tiles
     uint8_t *smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
-    const SmemLayout L = smem_layout(P, A_TMEM);
-    uint8_t *sA = smem + L.a_off;
+    const SmemLayout L = smem_layout(P);
     uint8_t *sB = smem + L.b_off;
     uint8_t *sRaw = smem + L.raw_off;
     int *sKoff = reinterpret_cast<int *>(smem + L.koff_off);
@@ -633,46 +793,47 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
     volatile int *abort_flag = reinterpret_cast<volatile int *>(acc_full + 2);
     float *zero_word = reinterpret_cast<float *>(acc_full + 3); // holds 0.0f: what a masked-off filter tap reads
     uint64_t *acc_ready = acc_full + 4; // a group of `fl` K stages has been accumulated: the main accumulator may be drained
-    uint64_t *flushed = acc_full + 5;   // all eight transform warps have drained it: the MMA warp may restart it
-    uint64_t *acc_full1 = acc_full + 6; // ping-pong mode: the second accumulator region is complete
-    uint64_t *acc_empty = acc_full + 7; // [2]: the owning transform set has read accumulator region 0 / 1 out
+    uint64_t *flushed = acc_full + 5;   // the four drain warps have drained it: the MMA warp may restart it
+    uint64_t *acc_full1 = acc_full + 6; // persistent mode: the second accumulator region is complete
+    uint64_t *acc_empty = acc_full + 7; // [2]: the drain warps have read accumulator region 0 / 1 out
 
     constexpr bool SPLIT = PASSES != kMathTf32x1; // hi/lo operands, two accumulators
     constexpr bool BF = PASSES == kMathBf16x3;
     constexpr int KE = BF ? 64 : 32;              // K elements per stage
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     long long *prof_cta = nullptr; // wall-clock marks of this CTA (entry, prologue done, epilogue done, exit), tuning only
-    if (prof && threadIdx.x == 96) {
+    if (prof && threadIdx.x == kSetWarp * 32) {
         prof_cta = prof + ((size_t)(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * kProfSlots;
         prof_cta[8] = (long long)ptx::globaltimer_ns();
     }
-    const int ntile = blockIdx.y / P.ksplit;
-    const int ksp = blockIdx.y - ntile * P.ksplit;
-    const int zb = blockIdx.z;
+    int ntile = PP ? 0 : (int)blockIdx.y / P.ksplit; // (persistent mode: set per tile by set_tile)
+    const int ksp = PP ? 0 : (int)blockIdx.y - ntile * P.ksplit;
+    int zb = PP ? 0 : (int)blockIdx.z;
     const uint32_t b_half = (uint32_t)P.BN * 128u;
-    // TMEM columns: [0,BN) accumulator of the hi*hi products, [BN,2*BN) accumulator of the two small cross terms,
-    // [2*BN,3*BN) the running total of drained main accumulators (P.fl > 0), [P.a_col,512) the A stages of the TS variant
-    const uint32_t tmem_cols = A_TMEM ? 512u : 256u;
+    // TMEM columns: [0,BN) accumulator of the hi*hi products, [BN,2*BN) accumulator of the two small cross terms (persistent
+    // narrow tiles: a second such pair behind them), [256,512) the A stages
+    constexpr uint32_t kTmemCols = 512, kACol = 256;
+    constexpr bool two_regions = PP == kNarrow;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kMaxNR; ++i) {
-            ptx::mbar_init(raw_full + i, 1);
-            ptx::mbar_init(raw_empty + i, P.fl_regs ? 4 : 8);
+            ptx::mbar_init(raw_full + i, BAND == 2 ? 256 : 1); // (GBMML: every transform thread)
+            ptx::mbar_init(raw_empty + i, 8);
         }
         for (int i = 0; i < kMaxNB; ++i) {
             ptx::mbar_init(b_full + i, 1);
             ptx::mbar_init(b_empty + i, 1);
         }
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < kNA; ++i) {
             ptx::mbar_init(a_full + i, 4);
             ptx::mbar_init(a_empty + i, 1);
         }
         ptx::mbar_init(acc_full, 1);
         ptx::mbar_init(acc_ready, 1);
-        ptx::mbar_init(flushed, P.fl_regs ? 4 : 8);
+        ptx::mbar_init(flushed, 4);
         ptx::mbar_init(acc_full1, 1);
-        ptx::mbar_init(acc_empty, BAND == 1 ? 8 : 4); // (G2BMM: both sets read every tile out)
-        ptx::mbar_init(acc_empty + 1, BAND == 1 ? 8 : 4);
+        ptx::mbar_init(acc_empty, 4);
+        ptx::mbar_init(acc_empty + 1, 4);
         *abort_flag = 0;
         *zero_word = 0.f;
         ptx::fence_mbar_init();
@@ -683,7 +844,7 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
     for (int i = threadIdx.x; i < P.spc * KE; i += kThreads)
         sKoff[i] = P.koff[i];
     if (warp == 2) {
-        ptx::tmem_alloc(tmem_slot, tmem_cols);
+        ptx::tmem_alloc(tmem_slot, kTmemCols);
         ptx::tmem_relinquish();
     }
     ptx::tc_fence_before();
@@ -698,37 +859,37 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
         prof_cta[9] = (long long)ptx::globaltimer_ns();
 
     // Tile origin in the input: first image, depth slice, row and (16-byte aligned) column of the raw box.  `bx` is the
-    // pixel-tile index: blockIdx.x, or in ping-pong mode every gridDim.x-th tile from there.
+    // pixel-tile index: blockIdx.x, or in persistent mode every gridDim.x-th tile from there.
     int bx = (int)blockIdx.x;
-    const int ntl = PP ? (P.mtiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 1; // tiles of this CTA
+    const int ntl = PP ? (P.tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 1; // tiles of this CTA
     int n_lo = 0, q0 = 0, unit0 = 0, z_start = 0, y_start = 0, x_start = 0, w_zl = 0, w_yl = 0, w_tx = 0;
-    int nt_cur = ntile; // filter tile of the current pixel tile (differs per tile only for banded products)
     auto set_tile = [&](int tile) {
         bx = tile;
-        if (BAND == 1) {
-            bx = tile / P.band_nt;
-            nt_cur = tile - bx * P.band_nt;
+        if (PP) {
+            const int m = P.by_ntiles.div(tile);
+            ntile = tile - m * P.ntiles;
+            zb = P.by_mtiles.div(m);
+            bx = m - zb * P.mtiles;
         }
         n_lo = 0, q0 = 0, unit0 = 0, w_zl = 0, w_yl = 0, w_tx = 0;
         if (A_KMAJOR) {
             z_start = y_start = x_start = 0; // the tile is rows [bx*128, +128) of A[zb]
         } else if (P.wide) {
-            const int row = bx / P.row_tiles;
+            const int row = P.by_row_tiles.div(bx), plane = P.by_ohn.div(row);
             w_tx = bx - row * P.row_tiles;
-            n_lo = row / (P.OD * P.ohn);
-            w_zl = (row / P.ohn) % P.OD;
-            w_yl = row % P.ohn;
+            w_yl = row - plane * P.ohn;
+            n_lo = P.by_od.div(plane);
+            w_zl = plane - n_lo * P.OD;
             z_start = w_zl * P.sd - P.pd;
             y_start = (P.oh0 + w_yl) * P.sh - P.ph;
             const int xs = (P.ow0 + w_tx * kTileM) * P.sw - P.pw;
             x_start = (xs >= 0) ? (xs & ~3) : -(((-xs) + 3) & ~3);
         } else {
-            const int tu = bx / P.tpi;
+            const int tu = P.by_tpi.div(bx);
             q0 = (bx - tu * P.tpi) * kTileM;
             unit0 = tu * P.ipt;
-            n_lo = unit0 / P.OD;
-            int yl_lo, yl_hi;
-            tile_rows(P, q0, min(q0 + kTileM, P.Pw) - 1, P.ipt > 1, yl_lo, yl_hi);
+            n_lo = P.by_od.div(unit0);
+            const int yl_lo = P.ipt > 1 ? 0 : P.by_own.div(q0); // first output row of the tile
             z_start = (unit0 - n_lo * P.OD) * P.sd - P.pd;
             y_start = (P.oh0 + yl_lo) * P.sh - P.ph;
             x_start = P.x0;
@@ -758,15 +919,15 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
         } else {
             int ul = 0, q = q0 + p;
             if (P.ipt > 1) {
-                ul = p / P.Pw;
+                ul = P.by_pw.div(p);
                 q = p - ul * P.Pw;
             }
             const int unit = unit0 + ul;
             valid = (ul < P.ipt) && (unit < P.units) && (q < P.Pw);
             if (valid) {
-                const int n = unit / P.OD;
+                const int n = P.by_od.div(unit);
                 const int zl = unit - n * P.OD;
-                const int yl = q / P.own;
+                const int yl = P.by_own.div(q);
                 const int xl = q - yl * P.own;
                 const int oh = P.oh0 + yl, ow = P.ow0 + xl;
                 base_p = (((n - n_lo) * P.BC * P.RD + (zl * P.sd - P.pd - z_start)) * P.RH + (oh * P.sh - P.ph - y_start)) * P.RW +
@@ -776,50 +937,63 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
             }
         }
     };
+    // May runs of pixels be stored 16 bytes at a time?  Pixel-contiguous NCHW output, full-width rows (no column window), one
+    // plane per tile, 16-byte aligned runs (of y and of the residual, which is laid out like y).
+    auto pixel_runs = [&]() {
+        const long long plane_elems = (long long)P.OD * P.OH * P.OW;
+        return P.ys_p == 1 && P.ipt == 1 && P.own == P.OW && P.ow0 == 0 && (plane_elems & 3) == 0 && (P.ys_n & 3) == 0 &&
+               ((P.OH * P.OW) & 3) == 0 && (!P.wide || (P.OW & 3) == 0) && (P.ys_f & 3) == 0 && ((P.oh0 * P.OW) & 3) == 0 &&
+               ((reinterpret_cast<uintptr_t>(P.y) | reinterpret_cast<uintptr_t>(P.res)) & 15) == 0;
+    };
     // split-K: this CTA reduces the channel chunks [c0, c1)
     const int c0 = (int)((long long)ksp * P.nchunks / P.ksplit), c1 = (int)((long long)(ksp + 1) * P.nchunks / P.ksplit);
     const int KS = (c1 - c0) * P.spc;
 
+    if (warp < kSetWarp)
+        ptx::reg_dealloc<Regs<PP>::control>();
     if (warp == 0) {
         // ---------------- packed-weight producer (one thread) ----------------
         if (lane == 0) {
-            int row0 = zb * P.Fg + ntile * P.BN;
             int sb = 0;
             uint32_t pb = 1; // first pass over the ring: every slot is free
-            for (int ks = 0; ks < KS * ntl; ++ks) { // the same KS filter tiles for every pixel tile of this CTA
-                if (!ptx::mbar_wait(b_empty + sb, pb, abort_flag))
-                    break;
-                uint8_t *dst = sB + (size_t)sb * 2 * b_half;
-                ptx::mbar_expect_tx(b_full + sb, (SPLIT ? 2u : 1u) * b_half + (P.starve ? 64u : 0u));
-                const int kst = ntl > 1 ? ks % KS : ks;
-                int kx = (c0 * P.spc + kst) * KE; // first K element of the stage
+            bool go = true;
+            for (int tl = 0; tl < ntl && go; ++tl) {
+                if (PP)
+                    set_tile((int)blockIdx.x + tl * (int)gridDim.x);
+                int row0 = zb * P.Fg + ntile * P.BN;
+                int kx = c0 * P.spc * KE; // first K element of the stage
                 if (BAND == 2) // the key window of the row tile, start rounded down to a multiple of 4
-                    kx += (((int)blockIdx.x * kTileM - P.band_w) & ~3);
-                if (BAND == 1) { // the key window moves with the row tile (rows before the tensor or past it read as zero / are masked)
-                    const int tile = (int)blockIdx.x + (ks / KS) * (int)gridDim.x, rt = tile / P.band_nt;
-                    row0 = zb * P.m_rows + rt * kTileM - P.band_w + (tile - rt * P.band_nt) * P.BN;
-                }
-                ptx::tma_load_2d(dst, &tmap_bhi, b_full + sb, kx, row0);
-                if (SPLIT)
-                    ptx::tma_load_2d(dst + b_half, &tmap_blo, b_full + sb, kx, row0);
-                if (++sb == P.NB) {
-                    sb = 0;
-                    pb ^= 1u;
+                    kx += (bx * kTileM - P.band_w) & ~3;
+                if (BAND == 1) // the key window moves with the row tile (rows before the tensor or past it read as zero / are masked)
+                    row0 = zb * P.m_rows + bx * kTileM - P.band_w + ntile * P.BN;
+                for (int ks = 0; ks < KS; ++ks, kx += KE) {
+                    if (!ptx::mbar_wait(b_empty + sb, pb, abort_flag)) {
+                        go = false;
+                        break;
+                    }
+                    uint8_t *dst = sB + (size_t)sb * 2 * b_half;
+                    ptx::mbar_expect_tx(b_full + sb, (SPLIT ? 2u : 1u) * b_half + (P.starve ? 64u : 0u));
+                    ptx::tma_load_2d(dst, &tmap_bhi, b_full + sb, kx, row0);
+                    if (SPLIT)
+                        ptx::tma_load_2d(dst + b_half, &tmap_blo, b_full + sb, kx, row0);
+                    if (++sb == P.NB) {
+                        sb = 0;
+                        pb ^= 1u;
+                    }
                 }
             }
         }
     } else if (warp == 2) {
         // ---------------- raw activation producer ----------------
-        const int c_base = P.z_is_batch ? 0 : zb * P.cpg;
-        if (lane == 0) {
+        if (BAND != 2 && lane == 0) { // (GBMML's transform warps fetch their operand themselves)
             const uint32_t bytes = (uint32_t)P.RN * P.BC * P.RD * P.RH * P.RW * 4u;
             int rb = 0;
             uint32_t pr = 1; // first pass over the ring: every buffer is free
             bool go = true;
-            for (int tl = 0; tl < ntl && go && !(BAND == 2); ++tl) { // (GBMML reads its A operand from global memory)
+            for (int tl = 0; tl < ntl && go; ++tl) {
             if (tl > 0)
                 set_tile((int)blockIdx.x + tl * (int)gridDim.x);
-            const int n_start = P.z_is_batch ? zb : n_lo;
+            const int n_start = P.z_is_batch ? zb : n_lo, c_base = P.z_is_batch ? 0 : zb * P.cpg;
             for (int ch = 0; ch < c1 - c0; ++ch) {
                 if (!ptx::mbar_wait(raw_empty + rb, pr, abort_flag)) {
                     go = false;
@@ -847,586 +1021,564 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
             }
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        // The whole warp runs this loop with uniform control flow and only the tcgen05 instructions sit under
-        // elect_one: descriptors and TMEM addresses then live in uniform registers.  (With the loop confined to one
-        // lane the same instruction stream was issue-bound: 94 instead of 64 cycles per 128x128x8 MMA.)
+        // ---------------- MMA issuer (one thread) ----------------
         // 3xTF32 with two MMAs per K=8 step instead of three: the hi and lo filter tiles of a stage are adjacent in shared
         // memory, i.e. one K-major tile of 2*BN rows, so  A_hi x [B_hi ; B_lo]  is ONE MMA of width 2*BN whose result columns
         // [0,BN) are the main accumulator and [BN,2BN) the accumulator of the cross terms; A_lo x B_hi then adds to the
-        // latter.  Same tensor-pipe work, a third fewer instructions from the warp that every stage waits for.
-        const uint32_t idesc = BF ? ptx::idesc_bf16(kTileM, P.BN) : ptx::idesc_tf32(kTileM, P.BN);
-        const uint32_t idesc_wide = BF ? ptx::idesc_bf16(kTileM, 2 * P.BN) : ptx::idesc_tf32(kTileM, 2 * P.BN);
-        // A from TMEM; per instruction K = 8 TF32 values or 16 bf16 values, either way 8 columns of A and 32 bytes of a B row
-        auto mma_ts = [](uint32_t d, uint32_t a, uint64_t b, uint32_t id, uint32_t acc) {
-            if (BF)
-                ptx::mma_bf16_ts(d, a, b, id, acc);
-            else
-                ptx::mma_tf32_ts(d, a, b, id, acc);
-        };
-        const uint64_t bdesc0 = ptx::smem_desc_k128(ptx::smem_u32(sB));
-        const uint64_t adesc0 = A_TMEM ? 0ull : ptx::smem_desc_k128(ptx::smem_u32(sA));
-        const uint32_t b_half16 = b_half >> 4;
-        // What this loop costs besides its MMAs decides the kernel's rate: the tensor pipe needs 770 / 385 / 240 cycles for the
-        // eight MMAs of a stage at BN = 128 / 64 / 32, a wait on a complete mbarrier 110-130, a vote 41, elect 35.  So: ring
-        // positions as running values, the next stage's barriers polled before this stage's MMAs are issued, one elected
-        // block per stage, nothing else on the common path.  A wait that gives up sets the CTA's abort flag, after which
-        // every later wait returns at once: the loop then simply runs out.  (12 K stages at BN = 32, m128 n2304 k768:
-        // 11.8 -> 10.0 us; BN = 64 persistent, 64-channel 3x3 at batch 64: 117 -> 97 us; BN = 128: unchanged, the operand
-        // warps are the bound there.)
-        long long t_wa = 0, t_wb = 0, t_wf = 0;
-        const long long t_begin = prof ? clock64() : 0;
-        const uint32_t BNu = (uint32_t)P.BN, a_col0 = tmem_base + (uint32_t)P.a_col;
-        const int NA = P.NA, NB = P.NB;
-        uint32_t tmem_acc = tmem_base, tmem_small = tmem_base + BNu; // main and cross-term accumulators of the tile
-        uint32_t sa = 0, sb = 0, pa = 0, pb = 0;
-        bool ok = true;
-        const int FLm = (PP || !SPLIT) ? 0 : P.fl;
-        int gpos = 0; // position of the stage inside its flush group
-        uint32_t gpar = 0; // parity of the group's drain
-        bool ready = false; // the current stage has been seen complete
-        bool cross_prepaid = false; // the current stage's cross-term MMAs were issued ahead, during the previous stage
-        // Ping-pong mode: each transform set fills its own half of the A ring (slots 2*set, 2*set + 1, alternately), so every
-        // slot's barriers see one producer in order; bit i of `apar` is the parity of slot i's next completed fill.
-        uint32_t apar = 0;
-        for (int tl = 0; tl < ntl; ++tl) {
-            if (PP) {
-                // accumulators alternate between two TMEM regions; before reusing one, its previous tile must have been read out
-                tmem_acc = tmem_base + (uint32_t)(tl & 1) * 2u * BNu;
-                tmem_small = tmem_acc + BNu;
-                if (tl >= 2) {
-                    ok = ptx::mbar_wait(acc_empty + (tl & 1), (uint32_t)(((tl >> 1) - 1) & 1), abort_flag) && ok;
-                    __syncwarp();
-                    ptx::tc_fence_after();
-                }
-            }
-            for (int ks = 0; ks < KS; ++ks) {
-                if (PP) {
-                    sa = (uint32_t)((tl & 1) * 2 + (ks & 1));
-                    pa = (apar >> sa) & 1u;
-                    apar ^= 1u << sa;
-                }
-                if (!ready) {
+        // latter.  Same tensor-pipe work, a third fewer instructions from the thread that every stage waits for.
+        // What this loop does besides its MMAs decides the kernel's rate: the tensor pipe needs 770 / 385 / 240 cycles for the
+        // eight MMAs of a stage at BN = 128 / 64 / 32 and queues only two or three instructions, while a wait on a complete
+        // mbarrier takes 110-130 cycles, a vote 41, elect 35, a warp barrier 23 — and a taken branch 70 to 250, because the
+        // warps of an SM quarter share an instruction cache that the transform warps' unrolled code keeps flushing.  So: one
+        // thread, ring positions as running values, the next stage's barriers polled before this stage's MMAs are issued,
+        // and a plain stage that is one short straight line; everything rare (waits, group starts) sits outside it.
+        // A wait that gives up cuts the loops short (their bounds are running values), so that the common path has no test for
+        // it; nothing is issued or committed after it: releasing a filter slot whose bytes never came would let its producer
+        // arrive once more on a phase that expects no further arrival, which is a fault.
+        if (ptx::elect_one()) {
+            const uint32_t idesc = BF ? ptx::idesc_bf16(kTileM, P.BN) : ptx::idesc_tf32(kTileM, P.BN);
+            const uint32_t idesc_wide = BF ? ptx::idesc_bf16(kTileM, 2 * P.BN) : ptx::idesc_tf32(kTileM, 2 * P.BN);
+            // A from TMEM; per instruction K = 8 TF32 values or 16 bf16 values, either way 8 columns of A and 32 bytes of a B row
+            auto mma_ts = [](uint32_t d, uint32_t a, uint64_t b, uint32_t id, uint32_t acc) {
+                if (BF)
+                    ptx::mma_bf16_ts(d, a, b, id, acc);
+                else
+                    ptx::mma_tf32_ts(d, a, b, id, acc);
+            };
+            const uint64_t bdesc0 = ptx::smem_desc_k128(ptx::smem_u32(sB));
+            const uint32_t b_half16 = b_half >> 4;
+            long long t_wa = 0, t_wf = 0;
+            const long long t_begin = prof ? clock64() : 0;
+            const uint32_t BNu = (uint32_t)P.BN, a_col0 = tmem_base + kACol, NB = (uint32_t)P.NB;
+            uint32_t tmem_acc = tmem_base, tmem_small = tmem_base + BNu; // main and cross-term accumulators of the tile
+            int tiles_left = ntl, stages_end = KS, left = 0; // tiles, end of the tile's K stages, stages left in the flush group
+            bool ok = true;
+            auto give_up = [&]() {
+                ok = false;
+                tiles_left = stages_end = left = 0;
+            };
+            bool ready = false, next_ready = false; // the current / the next stage has been seen complete
+            // Ring positions: slot, parity, and what they select.
+            uint32_t sa = 0, sb = 0, pa = 0, pb = 0;
+            uint64_t bhi = bdesc0;
+            auto wait_stage = [&]() {
+                if (__builtin_expect(!ready, 0)) {
                     const long long q0 = prof ? clock64() : 0;
-                    ok = ptx::mbar_wait(a_full + sa, pa, abort_flag) && ok;
-                    const long long q1 = prof ? clock64() : 0;
-                    ok = ptx::mbar_wait(b_full + sb, pb, abort_flag) && ok;
-                    if (prof)
-                        t_wa += q1 - q0, t_wb += clock64() - q1;
-                    __syncwarp();
+                    if (!ptx::mbar_wait(a_full + sa, pa, abort_flag) || !ptx::mbar_wait(b_full + sb, pb, abort_flag)) {
+                        give_up();
+                        return false;
+                    }
+                    t_wa += prof ? clock64() - q0 : 0;
                 }
                 ptx::tc_fence_after();
-                const uint64_t bhi = bdesc0 + (uint64_t)(sb * 2u * b_half16);
+                return true;
+            };
+            struct Pos {
+                uint32_t sa, sb, pa, pb;
+            };
+            auto next_pos = [&]() {
+                Pos n{sa + 1, sb + 1, pa, pb};
+                if (n.sa == (uint32_t)kNA)
+                    n.sa = 0, n.pa ^= 1u;
+                if (n.sb == NB)
+                    n.sb = 0, n.pb ^= 1u;
+                return n;
+            };
+            auto finish_stage = [&](const Pos &n) { // release the stage's slots, go on to the next
+                ptx::mma_commit(a_empty + sa);
+                ptx::mma_commit(b_empty + sb);
+                sa = n.sa, sb = n.sb, pa = n.pa, pb = n.pb;
+                bhi = bdesc0 + (uint64_t)(sb * 2u * b_half16);
+                ready = next_ready;
+            };
+            // One K stage.  The cross terms have their own accumulator: the tensor core truncates (rounds toward zero) its
+            // accumulator after every MMA, a bias proportional to the accumulator's magnitude; keeping the small terms away
+            // from the big sum removes most of those truncations from it.
+            auto plain_stage = [&](uint32_t acc0) {
+                if (!wait_stage())
+                    return;
+                const Pos n = next_pos();
+                // Is the next stage there?  Asked before this stage's MMAs and read after them: the answer travels while they
+                // are being issued.
+                const bool next_a = ptx::mbar_test_wait(a_full + n.sa, n.pa), next_b = ptx::mbar_test_wait(b_full + n.sb, n.pb);
                 const uint32_t ahi_t = a_col0 + sa * 64u, alo_t = ahi_t + 32u;
-                const uint64_t ahi_s = adesc0 + (uint64_t)(sa * 2u * (kAHalfBytes >> 4)), alo_s = ahi_s + (kAHalfBytes >> 4);
-                uint32_t nsa = sa + 1, nsb = sb + 1, npa = pa, npb = pb; // the next stage's ring positions
-                if (nsa == (uint32_t)NA)
-                    nsa = 0, npa ^= 1u;
-                if (nsb == (uint32_t)NB)
-                    nsb = 0, npb ^= 1u;
-                if (PP) { // the next stage of this tile sits in the set's other slot
-                    nsa = (uint32_t)((tl & 1) * 2 + ((ks + 1) & 1));
-                    npa = (apar >> nsa) & 1u;
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk) {
+                    mma_ts(tmem_acc, ahi_t + kk * 8, bhi + 2 * kk, SPLIT ? idesc_wide : idesc, kk == 0 ? acc0 : 1u);
+                    if (SPLIT)
+                        mma_ts(tmem_small, alo_t + kk * 8, bhi + 2 * kk, idesc, 1u);
                 }
-                // Is the next stage there?  Asked before this stage's MMAs and read after them: the answer (about 100 cycles on
-                // a busy shared-memory port) travels while they are being issued.
-                const bool next_a = ptx::mbar_test_wait(a_full + nsa, npa), next_b = ptx::mbar_test_wait(b_full + nsb, npb);
-                const bool group_start = FLm > 0 && gpos == 0 && ks > 0;
-                if (group_start) {
-                    // First stage of a new flush group: the main accumulator restarts from zero, but only after the transform
-                    // warps have drained the previous group's sum.  The stage's eight cross-term MMAs do not touch the main
-                    // accumulator and are issued first, so the tensor pipe has work while the drain is in flight ...
-                    const uint64_t blo = bhi + b_half16;
-                    if (ptx::elect_one()) {
+                next_ready = next_a && next_b;
+                finish_stage(n);
+            };
+            auto cross_terms = [&](const uint32_t slot_a, const uint64_t hi) { // of one stage: eight MMAs that leave the main accumulator alone
+                const uint32_t ahi_t = a_col0 + slot_a * 64u;
 #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk) {
-                            mma_ts(tmem_small, ahi_t + kk * 8, blo + 2 * kk, idesc, 1u);
-                            mma_ts(tmem_small, alo_t + kk * 8, bhi + 2 * kk, idesc, 1u);
+                for (int kk = 0; kk < 4; ++kk) {
+                    mma_ts(tmem_small, ahi_t + kk * 8, hi + b_half16 + 2 * kk, idesc, 1u);
+                    mma_ts(tmem_small, ahi_t + 32u + kk * 8, hi + 2 * kk, idesc, 1u);
+                }
+            };
+            auto main_terms = [&](uint32_t acc0) {
+                const uint32_t ahi_t = a_col0 + sa * 64u;
+#pragma unroll
+                for (int kk = 0; kk < 4; ++kk)
+                    mma_ts(tmem_acc, ahi_t + kk * 8, bhi + 2 * kk, idesc, kk == 0 ? acc0 : 1u);
+            };
+            uint32_t gpar = 0; // parity of the flush group's drain
+            // First stage(s) of a new flush group: the main accumulator restarts from zero, but only after the drain warps have
+            // taken the previous group's sum.  The stage's eight cross-term MMAs do not touch the main accumulator and are
+            // issued first, so the tensor pipe has work while the drain is in flight; if the stage after it is already there
+            // (and belongs to the group), its eight as well.
+            auto group_start = [&]() {
+                if (!wait_stage())
+                    return;
+                const Pos n = next_pos();
+                cross_terms(sa, bhi);
+                next_ready = ptx::mbar_test_wait(a_full + n.sa, n.pa) && ptx::mbar_test_wait(b_full + n.sb, n.pb);
+                const bool two = next_ready && left >= 2;
+                if (two) {
+                    ptx::tc_fence_after();
+                    cross_terms(n.sa, bdesc0 + (uint64_t)(n.sb * 2u * b_half16));
+                }
+                const long long q2 = prof ? clock64() : 0;
+                if (!ptx::mbar_wait(flushed, gpar, abort_flag)) {
+                    give_up();
+                    return;
+                }
+                t_wf += prof ? clock64() - q2 : 0;
+                gpar ^= 1u;
+                ptx::tc_fence_after();
+                main_terms(0u);
+                finish_stage(n);
+                --left;
+                if (!two)
+                    return;
+                const Pos n2 = next_pos();
+                next_ready = ptx::mbar_test_wait(a_full + n2.sa, n2.pa) && ptx::mbar_test_wait(b_full + n2.sb, n2.pb);
+                main_terms(1u);
+                finish_stage(n2);
+                --left;
+            };
+            const int FLm = (PP == kNarrow || !SPLIT || P.fl == 0) ? KS : P.fl; // stages per flush group
+            for (int tl = 0; tl < tiles_left; ++tl) {
+                if (PP) {
+                    // before an accumulator region is reused, its previous tile must have been read out
+                    const int reg = two_regions ? (tl & 1) : 0, use = two_regions ? (tl >> 1) : tl; // the use-th tile of region reg
+                    tmem_acc = tmem_base + (uint32_t)reg * 2u * BNu;
+                    tmem_small = tmem_acc + BNu;
+                    if (use >= 1) {
+                        const long long q3 = prof ? clock64() : 0;
+                        if (!ptx::mbar_wait(acc_empty + reg, (uint32_t)((use - 1) & 1), abort_flag)) {
+                            give_up();
+                            break;
                         }
-                    }
-                    __syncwarp();
-                    // ... and, if the stage after this one is already there, its eight cross-term MMAs as well: 2 x 8 MMAs of
-                    // cover for the drain (that stage then only issues its four main MMAs)
-                    const bool pre = __all_sync(0xffffffffu, next_a && next_b) && ks + 1 < KS && FLm >= 2;
-                    if (pre) {
+                        t_wf += prof ? clock64() - q3 : 0;
                         ptx::tc_fence_after();
-                        const uint64_t nbhi = bdesc0 + (uint64_t)(nsb * 2u * b_half16), nblo = nbhi + b_half16;
-                        const uint32_t nahi = a_col0 + nsa * 64u, nalo = nahi + 32u;
-                        if (ptx::elect_one()) {
-#pragma unroll
-                            for (int kk = 0; kk < 4; ++kk) {
-                                mma_ts(tmem_small, nahi + kk * 8, nblo + 2 * kk, idesc, 1u);
-                                mma_ts(tmem_small, nalo + kk * 8, nbhi + 2 * kk, idesc, 1u);
+                    }
+                }
+                for (int g0 = 0; g0 < stages_end; g0 += FLm) {
+                    left = min(FLm, KS - g0);
+                    if (PP != kNarrow && g0 > 0)
+                        group_start();
+                    uint32_t acc0 = g0 > 0 ? 1u : 0u;
+#pragma unroll 1
+                    for (; left > 0; --left, acc0 = 1u)
+                        plain_stage(acc0);
+                    if (PP != kNarrow && g0 + FLm < stages_end) // fires once every MMA of the group has completed
+                        ptx::mma_commit(acc_ready);
+                }
+                if (ok)
+                    ptx::mma_commit((two_regions && (tl & 1)) ? acc_full1 : acc_full);
+            }
+            if (prof) {
+                long long *pr = prof + ((size_t)(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * kProfSlots;
+                pr[0] = t_wa, pr[2] = clock64() - t_begin, pr[16] = t_wf;
+            }
+        }
+        __syncwarp();
+    } else if (warp >= kSetWarp && warp < kDrainWarp) {
+        // ---------------- transform: two sets of four warps taking alternate K stages (and the epilogue of a single tile) --------
+        // The per-stage chain  wait -> gather -> tcgen05.st -> wait::st -> arrive  is latency bound (about 750 cycles: 110-130
+        // for a wait, 270-310 from the first tcgen05.st to the arrive); two sets halve the time between stages.
+        if (PP == kWide)
+            ptx::reg_dealloc<Regs<PP>::set>();
+        else
+            ptx::reg_alloc<Regs<PP>::set>();
+        const int tset = (warp - kSetWarp) >> 2; // 0 or 1
+        const int quarter = warp & 3;            // TMEM lane quarter this warp may access
+        const int p = quarter * 32 + lane;       // pixel row inside the tile
+        bool alive = true;
+        long long t_we = 0, t_wr = 0, t_g = 0, t_st = 0;
+        const long long t_begin = prof ? clock64() : 0;
+        const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16);
+        // This set's stages are number tset, tset + 2, ... of the CTA (all tiles in a row): `st` is the next one's index inside
+        // the current chunk, `sa` / `pa` its A slot and the parity to wait for (first pass over the ring: every slot is free).
+        int st = tset, rb = 0;
+        uint32_t sa = (uint32_t)tset, pa = 1u, prw = 0;
+        bool valid = false;
+        long long y_off = 0;
+        // The whole loop is instantiated per kind of gather, so that a stage is short and straight.
+        auto transform = [&](auto mode_c) {
+            constexpr int MODE = decltype(mode_c)::value;
+            const bool flat = MODE == kGatherFlat || ((MODE == kGatherStride || MODE == kGatherPlain) && P.flat != 0);
+            bool raw_ok = true; // this lane has not given up on a raw tile (the warp agrees on it where it asks for an A slot)
+            int fetched = 0, frb = 0; // GBMML: chunks asked for, ring slot of the next and the parity that says it is free
+            uint32_t fpr = 0;
+            const int nfetch = ntl * (c1 - c0);
+            for (int tl = 0; tl < ntl && alive; ++tl) {
+                set_tile((int)blockIdx.x + tl * (int)gridDim.x);
+                int base_p;
+                pixel_geom(p, valid, base_p, y_off);
+                if (P.ksplit > 1 && tset == 0)
+                    sYoff[p] = valid ? y_off : -1; // read by the split-K reduction, after the cluster barrier
+                uint32_t tmask = 0;
+                if (MODE < kGatherKMajor && flat && valid) { // which filter taps of this pixel lie inside the (unpadded) input
+                    int ul = 0, q = q0 + p;
+                    if (P.ipt > 1) {
+                        ul = P.by_pw.div(p);
+                        q = p - ul * P.Pw;
+                    }
+                    const int zl = unit0 + ul - P.by_od.div(unit0 + ul) * P.OD, yl = P.by_own.div(q), xl = q - yl * P.own;
+                    const int z0 = zl * P.sd - P.pd, y0 = (P.oh0 + yl) * P.sh - P.ph, x0 = (P.ow0 + xl) * P.sw - P.pw;
+                    int tap = 0;
+                    for (int t = 0; t < P.T3[0]; ++t)
+                        for (int r = 0; r < P.T3[1]; ++r)
+                            for (int sx = 0; sx < P.T3[2]; ++sx, ++tap) {
+                                const int z = z0 + t * P.dil[0], y = y0 + r * P.dil[1], x = x0 + sx * P.dil[2];
+                                if (z >= 0 && z < P.xD && y >= 0 && y < P.xH && x >= 0 && x < P.xW)
+                                    tmask |= 1u << tap;
+                            }
+                }
+                for (int ch = 0; ch < c1 - c0 && alive; ++ch, st -= P.spc) {
+                    if constexpr (MODE == kGatherBand) { // keep NR - 1 chunks in flight
+                        for (; fetched < nfetch && fetched < tl * (c1 - c0) + ch + P.NR && alive; ++fetched) {
+                            if (fetched >= P.NR) {
+                                alive = ptx::mbar_wait_warp(raw_empty + frb, fpr, abort_flag); // (its previous chunk has been read by all)
+                            }
+                            const int ft = fetched / (c1 - c0), fm = PP ? P.by_ntiles.div((int)blockIdx.x + ft * (int)gridDim.x) : 0;
+                            const int fz = PP ? P.by_mtiles.div(fm) : zb, fx = PP ? fm - fz * P.mtiles : bx;
+                            band_copy(P, fz, fx * kTileM, ((fx * kTileM - P.band_w) & ~3) + (fetched - ft * (c1 - c0)) * kBandKeys, warp - kSetWarp,
+                                      lane, ptx::smem_u32(sRaw + (size_t)frb * P.raw_bytes), raw_full + frb);
+                            if (++frb == P.NR) {
+                                frb = 0;
+                                fpr ^= fetched >= P.NR ? 1u : 0u;
                             }
                         }
-                        __syncwarp();
+                        if (!alive)
+                            break;
                     }
-                    const long long q2 = prof ? clock64() : 0;
-                    ok = ptx::mbar_wait(flushed, gpar, abort_flag) && ok;
-                    t_wf += prof ? clock64() - q2 : 0;
-                    gpar ^= 1u;
-                    __syncwarp();
-                    ptx::tc_fence_after();
-                    if (ptx::elect_one()) {
+                    const long long cr0 = prof ? clock64() : 0;
+                    raw_ok = ptx::mbar_wait(raw_full + rb, prw, abort_flag) && raw_ok; // also by a set without a stage in this chunk
+                    if (prof)
+                        t_wr += clock64() - cr0;
+                    const float *raw = reinterpret_cast<const float *>(sRaw + (size_t)rb * P.raw_bytes) + base_p;
+                    for (; st < P.spc && alive; st += 2) {
+                        const int *ko = sKoff + st * KE;
+                        // Is the slot free?  Asked before the gather, read after it.
+                        const bool slot_free = ptx::mbar_test_wait(a_empty + sa, pa);
+                        // The operands are gathered and split into registers BEFORE the wait for the stage's slot in tensor
+                        // memory: when the slot frees, only the two tcgen05.st remain, so a set is one stage ahead in
+                        // registers on top of its slots in the ring.  (Announcing a stage only after the next one's gather,
+                        // to hide the 200 to 250 cycles of the stores, was 8 % slower: the MMA thread starts later.)
+                        uint32_t hi[32], lo[32];
+                        const long long cg0 = prof ? clock64() : 0;
+                        if constexpr (MODE == kGatherBand) {
+                            const int i = bx * kTileM + p, k0 = ((bx * kTileM - P.band_w) & ~3) + ((c0 + ch) * kBandStages + st) * kStageK;
+                            const int j0 = k0 - i + P.band_w; // band column of the stage's first key
+                            const float *brow = reinterpret_cast<const float *>(sRaw + (size_t)rb * P.raw_bytes) + p * kBandPitch + st * kStageK;
+                            const int shift = (int)(band_word(P, zb, i, k0) & 3), lo_e = max(-j0, -k0);
+                            const int hi_e = i < P.m_rows ? min(2 * P.band_w + 1 - j0, P.m_rows - k0) : 0;
 #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk)
-                            mma_ts(tmem_acc, ahi_t + kk * 8, bhi + 2 * kk, idesc, kk == 0 ? 0u : 1u);
-                        ptx::mma_commit(a_empty + sa);
-                        ptx::mma_commit(b_empty + sb);
-                    }
-                    cross_prepaid = pre;
-                } else if (cross_prepaid) { // the cross terms of this stage were issued with the previous stage's
-                    cross_prepaid = false;
-                    if (ptx::elect_one()) {
-#pragma unroll
-                        for (int kk = 0; kk < 4; ++kk)
-                            mma_ts(tmem_acc, ahi_t + kk * 8, bhi + 2 * kk, idesc, 1u);
-                        ptx::mma_commit(a_empty + sa);
-                        ptx::mma_commit(b_empty + sb);
-                    }
-                } else if (ptx::elect_one()) {
-                    // The cross terms have their own accumulator: the tensor core truncates (rounds toward zero) its
-                    // accumulator after every MMA, a bias proportional to the accumulator's magnitude; keeping the small
-                    // terms away from the big sum removes most of those truncations from it.
-                    const uint32_t acc0 = ks > 0 ? 1u : 0u;
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) {
-                        if (!SPLIT) { // single TF32 pass
-                            mma_ts(tmem_acc, ahi_t + kk * 8, bhi + 2 * kk, idesc, kk == 0 ? acc0 : 1u);
-                        } else if (A_TMEM) {
-                            mma_ts(tmem_acc, ahi_t + kk * 8, bhi + 2 * kk, idesc_wide, kk == 0 ? acc0 : 1u);
-                            mma_ts(tmem_small, alo_t + kk * 8, bhi + 2 * kk, idesc, 1u);
+                            for (int c = 0; c < 4; ++c) {
+                                float v[8];
+                                band_take8(brow + 8 * c, shift, lo_e - 8 * c, hi_e - 8 * c, v);
+                                split_words<PASSES>(v, hi + 8 * c, lo + 8 * c);
+                            }
                         } else {
-                            ptx::mma_tf32_ss(tmem_acc, ahi_s + 2 * kk, bhi + 2 * kk, idesc_wide, kk == 0 ? acc0 : 1u);
-                            ptx::mma_tf32_ss(tmem_small, alo_s + 2 * kk, bhi + 2 * kk, idesc, 1u);
+                            const uint8_t *krow = sRaw + (size_t)rb * P.raw_bytes + (size_t)p * 128;
+                            const float *q = raw; // kGatherPlain: first element of the run
+                            int cs = P.cstride;
+                            if constexpr (MODE == kGatherPlain) {
+                                const int o0 = *ko;
+                                const bool off = o0 < 0 || (flat && !((tmask >> (o0 >> 24)) & 1u));
+                                q = off ? zero_word : raw + (flat ? (o0 & 0xffffff) : o0);
+                                cs = off ? 0 : cs;
+                            }
+#pragma unroll
+                            for (int c = 0; c < 4; ++c) {
+                                float v[BF ? 16 : 8];
+#pragma unroll
+                                for (int h = 0; h < (BF ? 2 : 1); ++h) { // (bf16: the second tile of a row-major stage follows the first)
+                                    const int e = BF ? 2 * c + h : c;     // group of eight K elements
+                                    if constexpr (MODE == kGatherPlain) {
+                                        if (BF && e == 4) { // (64 elements: two runs of 32)
+                                            const int o0 = ko[32];
+                                            const bool off = o0 < 0 || (flat && !((tmask >> (o0 >> 24)) & 1u));
+                                            q = off ? zero_word : raw + (flat ? (o0 & 0xffffff) : o0);
+                                            cs = off ? 0 : P.cstride;
+                                        }
+#pragma unroll
+                                        for (int i = 0; i < 8; ++i)
+                                            v[8 * h + i] = q[(8 * (BF ? e & 3 : e) + i) * cs];
+                                    } else {
+                                        gather8<MODE>(ko + 8 * e, raw, krow + (e >> 2) * kAHalfBytes, 2 * (e & 3), p, tmask, P.cstride, flat, zero_word, v + 8 * h);
+                                    }
+                                }
+                                split_words<PASSES>(v, hi + 8 * c, lo + 8 * c);
+                            }
                         }
+                        const long long ce0 = prof ? clock64() : 0;
+                        if (__builtin_expect(!__all_sync(0xffffffffu, slot_free && raw_ok), 0)) {
+                            raw_ok = __all_sync(0xffffffffu, raw_ok) != 0;
+                            alive = raw_ok && ptx::mbar_wait_warp(a_empty + sa, pa, abort_flag);
+                            if (!alive)
+                                break;
+                        }
+                        ptx::tc_fence_after();
+                        const long long cg1 = prof ? clock64() : 0;
+                        const uint32_t t = t_row + kACol + sa * 64u;
+                        ptx::tmem_st_32x32(t, hi);
+                        if (SPLIT)
+                            ptx::tmem_st_32x32(t + 32u, lo);
+                        ptx::tmem_st_wait();
+                        ptx::tc_fence_before();
+                        if (prof)
+                            t_we += cg1 - ce0, t_g += ce0 - cg0, t_st += clock64() - cg1;
+                        __syncwarp();
+                        if (lane == 0)
+                            ptx::mbar_arrive(a_full + sa);
+                        sa ^= 2u;
+                        pa ^= (sa & 2u) ? 0u : 1u; // back at the set's first slot: the ring's next pass
                     }
-                    ptx::mma_commit(a_empty + sa);
-                    ptx::mma_commit(b_empty + sb);
-                }
-                __syncwarp();
-                if (FLm > 0 && ++gpos == FLm) {
-                    gpos = 0;
-                    if (ks + 1 < KS && ptx::elect_one()) // fires once every MMA of the group has completed
-                        ptx::mma_commit(acc_ready);
                     __syncwarp();
-                }
-                ready = __all_sync(0xffffffffu, next_a && next_b) && ks + 1 < KS;
-                sa = nsa, sb = nsb, pa = npa, pb = npb;
-            }
-            if (ok && ptx::elect_one())
-                ptx::mma_commit((PP && (tl & 1)) ? acc_full1 : acc_full);
-            __syncwarp();
-        }
-        if (prof && lane == 0) {
-            long long *pr = prof + ((size_t)(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * kProfSlots;
-            pr[0] = t_wa, pr[1] = t_wb, pr[2] = clock64() - t_begin, pr[16] = t_wf;
-        }
-    } else {
-        // ---------------- transform + epilogue: two sets of four warps (3..6 and 7..10) ----------------
-        // The per-stage chain  wait -> gather -> tcgen05.st -> wait::st -> arrive  is latency bound (~600 cycles);
-        // two sets taking alternate K stages double the rate at which A stages are produced.
-        const int tset = (warp - 3) >> 2;     // 0 or 1
-        const int quarter = warp & 3;         // TMEM lane quarter this warp may access
-        const int p = quarter * 32 + lane;    // pixel row inside the tile
-        bool alive = true;
-        long long t_we = 0, t_wr = 0, t_g = 0, t_st = 0, t_dw = 0, t_dd = 0, t_loop = 0, t_epi0 = 0;
-        const long long t_begin = prof ? clock64() : 0;
-        const bool reg_total = !PP && SPLIT && A_TMEM && P.fl > 0 && P.fl_regs != 0; // (ping-pong plans never flush)
-        const int FL = (!PP && SPLIT && A_TMEM && !reg_total) ? P.fl : 0;
-        // Register-total mode: set 1 only drains (a function of its own: its 128 totals per thread want the whole register file)
-        if (reg_total && tset == 1)
-            alive = drain_only_set(tmem_base + ((uint32_t)(quarter * 32) << 16), (KS + P.fl - 1) / P.fl, acc_ready, acc_full, flushed,
-                                   abort_flag, lane, prof ? &t_dw : nullptr, prof ? &t_dd : nullptr);
-        // Ping-pong mode: this set takes every second TILE of the CTA (set 0 the even ones) and produces all of its stages;
-        // otherwise there is one tile and the sets take alternate stages of it.
-        // Ping-pong mode: parities of this set's two A slots (free at first), and how many raw chunks of the CTA (all tiles,
-        // in load order) this set has seen complete.  The raw ring is shared by both sets and a parity wait cannot tell a fill
-        // from the one two fills earlier, so BOTH sets wait for every fill in order and release it: a set does that for the
-        // other set's tiles (which it does not read) in the pauses of its own work.
-        uint32_t own_apar = 3u;
-        int rseen = 0;
-        auto observe_until = [&](int limit) {
-            for (; rseen < limit && alive; ++rseen) {
-                alive = ptx::mbar_wait(raw_full + rseen % P.NR, (uint32_t)((rseen / P.NR) & 1), abort_flag);
-                __syncwarp();
-                if (lane == 0 && alive)
-                    ptx::mbar_arrive(raw_empty + rseen % P.NR);
-            }
-        };
-        if (BAND == 1) {
-            // G2BMM: a tile is two K stages and 32 KB of skewed stores, so the epilogue is the long part: both sets store half
-            // of EVERY tile (32 of its 64 key columns each), and the set that owns tile t + 2's operands produces them right
-            // after its half of tile t, i.e. while the MMA warp is on tile t + 1.
-            const int nch = c1 - c0;
-            auto produce = [&](int tl) {
-                observe_until(tl * nch); // fills of the other set's tiles
-                if (!alive)
-                    return;
-                rseen += nch;
-                const int chunk0 = tl * nch;
-                int rb = chunk0 % P.NR, sa = 2 * tset;
-                uint32_t prw = (uint32_t)((chunk0 / P.NR) & 1);
-                for (int ch = 0; ch < nch && alive; ++ch) {
-                    alive = ptx::mbar_wait(raw_full + rb, prw, abort_flag);
-                    if (!alive)
-                        break;
-                    uint32_t hi[32], lo[32];
-                    gather_split<kGatherKMajor, PASSES>(nullptr, nullptr, sRaw + (size_t)rb * P.raw_bytes + (size_t)p * 128, p, 0u, 0, false,
-                                                        zero_word, hi, lo);
-                    alive = ptx::mbar_wait(a_empty + sa, (own_apar >> (sa & 1)) & 1u, abort_flag);
-                    if (!alive)
-                        break;
-                    ptx::tc_fence_after();
-                    const uint32_t t = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)P.a_col + (uint32_t)sa * 64u;
-                    ptx::tmem_st_32x32(t, hi);
-                    ptx::tmem_st_32x32(t + 32u, lo);
-                    ptx::tmem_st_wait();
-                    ptx::tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) {
-                        ptx::mbar_arrive(a_full + sa);
+                    if (lane == 0 && alive)
                         ptx::mbar_arrive(raw_empty + rb);
-                    }
-                    own_apar ^= 1u << (sa & 1);
-                    sa ^= 1;
                     if (++rb == P.NR) {
                         rb = 0;
                         prw ^= 1u;
                     }
                 }
-            };
-            if (tset < ntl)
-                produce(tset);
-            for (int tl = 0; tl < ntl && alive; ++tl) {
-                alive = ptx::mbar_wait((tl & 1) ? acc_full1 : acc_full, (uint32_t)((tl >> 1) & 1), abort_flag);
-                if (!alive)
-                    break;
-                ptx::tc_fence_after();
-                set_tile((int)blockIdx.x + tl * (int)gridDim.x);
-                const uint32_t tacc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)((tl & 1) * 2 * P.BN);
-                epilogue_banded<PASSES>(tacc, tacc + (uint32_t)P.BN, tset * 32, tset * 32 + 32, nt_cur * P.BN, (warp & 3) * 32, bx, zb, P.m_rows,
-                                        P.band_w, P.y, reinterpret_cast<float *>(smem + L.stage_off) + (warp - 3) * 1024, lane);
-                ptx::tc_fence_before();
-                __syncwarp();
-                if (lane == 0)
-                    ptx::mbar_arrive(acc_empty + (tl & 1));
-                if ((tl & 1) == tset && tl + 2 < ntl)
-                    produce(tl + 2);
             }
-            observe_until(ntl * nch);
-        }
-        if (BAND != 1)
-        for (int tl = PP ? tset : 0; tl < ntl && alive; tl += PP ? 2 : 1) {
-        set_tile((int)blockIdx.x + tl * (int)gridDim.x); // (also for the only tile: nothing of it stays live across the code above)
-        bool valid;
-        int base_p;
-        long long y_off;
-        pixel_geom(p, valid, base_p, y_off);
-        if (P.ksplit > 1 && tset == 0)
-            sYoff[p] = valid ? y_off : -1; // read by the split-K reduction, after the cluster barrier
-        uint32_t tmask = 0;
-        if (!A_KMAJOR && P.flat && valid) { // which filter taps of this pixel lie inside the (unpadded) input
-            int ul = 0, q = q0 + p;
-            if (P.ipt > 1) {
-                ul = p / P.Pw;
-                q = p - ul * P.Pw;
-            }
-            const int zl = (unit0 + ul) % P.OD, yl = q / P.own, xl = q - yl * P.own;
-            const int z0 = zl * P.sd - P.pd, y0 = (P.oh0 + yl) * P.sh - P.ph, x0 = (P.ow0 + xl) * P.sw - P.pw;
-            int tap = 0;
-            for (int t = 0; t < P.T3[0]; ++t)
-                for (int r = 0; r < P.T3[1]; ++r)
-                    for (int sx = 0; sx < P.T3[2]; ++sx, ++tap) {
-                        const int z = z0 + t * P.dil[0], y = y0 + r * P.dil[1], x = x0 + sx * P.dil[2];
-                        if (z >= 0 && z < P.xD && y >= 0 && y < P.xH && x >= 0 && x < P.xW)
-                            tmask |= 1u << tap;
-                    }
-        }
-        if (PP) {
-            observe_until(tl * (c1 - c0)); // fills that belong to the other set's tiles
-            if (!alive)
-                break;
-            rseen += c1 - c0; // this tile's own chunks, waited for and released below
-        }
-        // raw buffer of the tile's first chunk and the parity of its fill
-        const int chunk0 = PP ? tl * (c1 - c0) : 0;
-        int rb = chunk0 % P.NR;
-        uint32_t prw = (uint32_t)((chunk0 / P.NR) & 1);
-        // Accumulator flush (P.fl > 0): the K stages form groups of P.fl; when the MMAs of group g have completed, the
-        // eight transform warps add the main accumulator to the running total in TMEM (round-to-nearest fp32 adds, in
-        // group order) and the MMA warp restarts the main accumulator for group g + 1.  A warp drains the columns its set
-        // stores in the epilogue, of its own lane quarter.
-        const int n_groups = FL > 0 ? (KS + FL - 1) / FL : 1;
-        const int fcol0 = tset == 0 ? 0 : ((P.BN / 32 + 1) / 2) * 32, fcol1 = tset == 0 ? ((P.BN / 32 + 1) / 2) * 32 : P.BN;
-        int fg = 0; // next group this warp has to drain
-        auto drain_group = [&](int g, bool wait_mma, bool signal) -> bool {
-            const long long cd0 = prof ? clock64() : 0;
-            if (wait_mma && !ptx::mbar_wait(acc_ready, (uint32_t)(g & 1), abort_flag))
-                return false;
-            const long long cd1 = prof ? clock64() : 0;
-            ptx::tc_fence_after();
-            const uint32_t tq = tmem_base + ((uint32_t)(quarter * 32) << 16);
-            for (int cc = fcol0; cc < fcol1; cc += 32) {
-                uint32_t mn[32], tt[32];
-                ptx::tmem_ld_32x32(tq + (uint32_t)cc, mn);
-                if (g > 0)
-                    ptx::tmem_ld_32x32(tq + 2u * (uint32_t)P.BN + (uint32_t)cc, tt);
-                ptx::tmem_ld_wait();
-                if (g > 0) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        mn[j] = __float_as_uint(__uint_as_float(tt[j]) + __uint_as_float(mn[j]));
-                }
-                ptx::tmem_st_32x32(tq + 2u * (uint32_t)P.BN + (uint32_t)cc, mn);
-            }
-            ptx::tmem_st_wait();
-            ptx::tc_fence_before();
-            __syncwarp();
-            if (signal && lane == 0)
-                ptx::mbar_arrive(flushed);
-            if (prof) {
-                t_dw += cd1 - cd0;
-                t_dd += clock64() - cd1;
-            }
-            return true;
         };
-        const bool all_stages = reg_total || PP; // this set produces every stage of the tile
-        const int sstep = all_stages ? 1 : 2;  // stages between two stages of one set
-        int gs = all_stages ? 0 : tset; // index of this set's next K stage among the tile's KS stages
-        // This set owns every second K stage (tset, tset + 2, ...) or all of them: `st` is the next one's index inside the
-        // current chunk, `sa`/`pa` its slot of the A ring and the parity to wait for (first pass over the ring: every slot is
-        // free; ping-pong: the tile's first stage follows the tl * KS stages of the earlier tiles).
-        int st = all_stages ? 0 : tset;
-        int sa = PP ? 2 * tset : st;
-        uint32_t pa = PP ? (own_apar & 1u) : 1u;
-        for (int ch = 0; ch < ((reg_total && tset == 1) ? 0 : c1 - c0) && alive; ++ch, st -= P.spc) {
-            const long long cr0 = prof ? clock64() : 0;
-            const bool band_gather = BAND == 2; // no raw tiles: the operands come from global memory
-            if (!band_gather)
-                alive = ptx::mbar_wait(raw_full + rb, prw, abort_flag); // also by a set without a stage in this chunk
-            if (prof)
-                t_wr += clock64() - cr0;
-            const float *raw = reinterpret_cast<const float *>(sRaw + (size_t)rb * P.raw_bytes) + base_p;
-            for (; st < P.spc && alive; st += sstep, gs += sstep) {
-                // Groups that ended before this stage: drain at once if their MMAs are done; otherwise produce one more
-                // stage first (the MMA warp can start on it) and then wait for them.
-                while (fg < n_groups - 1 && gs >= (fg + 1) * FL && alive) {
-                    const bool done = __shfl_sync(0xffffffffu, ptx::mbar_test_wait(acc_ready, (uint32_t)(fg & 1)) ? 1 : 0, 0) != 0;
-                    if (!done && gs < (fg + 1) * FL + 2)
-                        break;
-                    alive = drain_group(fg, !done, true);
-                    ++fg;
+        if constexpr (BAND == 2) {
+            transform(std::integral_constant<int, kGatherBand>());
+            ptx::cp_async_wait_all(); // (nothing may be written to the CTA's shared memory after it is gone)
+        } else if constexpr (A_KMAJOR) {
+            transform(std::integral_constant<int, kGatherKMajor>());
+        } else if (P.cstride && P.BC % kStageK == 0) {
+            transform(std::integral_constant<int, kGatherPlain>());
+        } else if (P.cstride) {
+            transform(std::integral_constant<int, kGatherStride>());
+        } else if (P.flat) {
+            transform(std::integral_constant<int, kGatherFlat>());
+        } else {
+            transform(std::integral_constant<int, kGatherTable>());
+        }
+        const long long t_loop = prof ? clock64() - t_begin : 0;
+        long long t_epi0 = t_loop;
+        if (!PP) {
+            // ---------------- epilogue of the only tile ----------------
+            // Addresses and store mode first: the MMA warp is still working through the last stages, so this costs nothing.
+            const bool vec_ok = (P.ys_f == 1) && ((P.ys_p & 3) == 0) && ((P.ys_n & 3) == 0) && ((P.Fg & 3) == 0) &&
+                                ((reinterpret_cast<uintptr_t>(P.y) & 15) == 0);
+            const int f_tile0 = ntile * P.BN;
+            const long long f_glob0 = P.z_is_batch ? 0 : (long long)zb * P.Fg;
+            float *yp = P.y + y_off + f_glob0 * P.ys_f;
+            const float *bp = (P.has_bias && P.ksplit == 1) ? P.bias + f_glob0 : nullptr;
+            const float *rp = (P.res != nullptr && P.ksplit == 1) ? P.res + y_off + f_glob0 * P.ys_f : nullptr;
+            // split-K: partial sums go to the landing areas of the cluster's CTAs, summed after the role branches
+            const int split_cols = P.BN / P.ksplit, split_shift = 31 - __clz(split_cols);
+            const uint32_t split_addr =
+                P.ksplit > 1 ? ptx::smem_u32(sSplit) + (uint32_t)(((int)ptx::cluster_ctarank() * split_cols) * kTileM + p) * 4u : 0u;
+            float *stage = nullptr;
+            int nvalid_warp = 0;
+            const long long y_off0 = __shfl_sync(0xffffffffu, y_off, 0);
+            float *ybase_warp = yp - y_off + y_off0;
+            const float *rbase_warp = rp != nullptr ? rp - y_off + y_off0 : nullptr;
+            if (pixel_runs() && P.ksplit == 1) {
+                nvalid_warp = __popc(__ballot_sync(0xffffffffu, valid));
+                if (nvalid_warp > 0) // B stages are idle once the accumulator is complete
+                    stage = reinterpret_cast<float *>(sB) + (warp - kSetWarp) * 1024;
+                if ((uint32_t)(warp - kSetWarp + 1) * 4096u > (uint32_t)P.NB * (SPLIT ? 2u : 1u) * b_half)
+                    stage = nullptr; // not enough idle shared memory for this warp's block
+            }
+            // the two sets split the tile's columns (whole 32-column blocks)
+            const int nblk = P.BN / 32, half_blk = (nblk + 1) / 2;
+            const int col0 = tset == 0 ? 0 : half_blk * 32, col1 = tset == 0 ? half_blk * 32 : P.BN;
+            if (alive)
+                alive = ptx::mbar_wait_warp(acc_full, 0u, abort_flag);
+            if (SPLIT && P.fl > 0) // the drain warps have written total + last group over the main accumulator
+                ptx::named_bar_sync(1, 384);
+            t_epi0 = prof ? clock64() : 0;
+            if (alive) {
+                ptx::tc_fence_after();
+#define PETB200_EPI(ACT_)                                                                                              \
+    epilogue_store<ACT_, PASSES>(t_row, t_row + (uint32_t)P.BN, P.BN, f_tile0, P.Fg, valid, bp, rp, yp, P.ys_f, vec_ok, stage, nvalid_warp, \
+                                 ybase_warp, rbase_warp, col0, col1, split_addr, split_shift)
+                switch (P.ksplit > 1 ? PETB200_ACT_NONE : P.act) {
+                case PETB200_ACT_RELU: PETB200_EPI(PETB200_ACT_RELU); break;
+                case PETB200_ACT_SIGMOID: PETB200_EPI(PETB200_ACT_SIGMOID); break;
+                case PETB200_ACT_TANH: PETB200_EPI(PETB200_ACT_TANH); break;
+                case PETB200_ACT_GELU: PETB200_EPI(PETB200_ACT_GELU); break;
+                default: PETB200_EPI(PETB200_ACT_NONE); break;
                 }
+#undef PETB200_EPI
+            }
+        }
+        if (prof_cta) { // lane 0 of the first warp of set 0
+            prof_cta[3] = t_we, prof_cta[4] = t_wr, prof_cta[5] = t_loop, prof_cta[6] = clock64() - t_epi0, prof_cta[7] = t_epi0 - t_begin;
+            prof_cta[10] = (long long)ptx::globaltimer_ns();
+            prof_cta[12] = t_g, prof_cta[13] = t_st;
+        }
+    } else if (warp >= kDrainWarp) {
+        // ---------------- drain warps: running totals of flushed accumulators; persistent mode: the epilogue ----------------
+        ptx::reg_alloc<Regs<PP>::drain>();
+        const int quarter = warp & 3, p = quarter * 32 + lane, FL = SPLIT ? P.fl : 0;
+        const int n_groups = FL > 0 ? (KS + FL - 1) / FL : 1;
+        const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16);
+        bool alive = true;
+        uint32_t gpar = 0; // parity of the next completed group
+        long long t_dw = 0, t_dd = 0, t_acc = 0, t_store = 0;
+        if (BAND == 1) {
+            for (int tl = 0; tl < ntl && alive; ++tl) {
+                set_tile((int)blockIdx.x + tl * (int)gridDim.x);
+                const long long cd0 = prof ? clock64() : 0;
+                alive = ptx::mbar_wait_warp((tl & 1) ? acc_full1 : acc_full, (uint32_t)((tl >> 1) & 1), abort_flag);
                 if (!alive)
                     break;
-                const int4 *ko = reinterpret_cast<const int4 *>(sKoff + st * KE);
-                if (!A_TMEM) {
-                    const long long ce0 = prof ? clock64() : 0;
-                    alive = ptx::mbar_wait(a_empty + sa, pa, abort_flag);
-                    if (prof)
-                        t_we += clock64() - ce0;
-                    if (!alive)
-                        break;
-                }
-                if (A_TMEM) {
-                    // The operands are gathered and split into registers BEFORE the wait for the stage's slot in tensor
-                    // memory: when the slot frees, only the two tcgen05.st remain, so a set is one stage ahead in registers
-                    // on top of its slots in the ring.
-                    uint32_t hi[32], lo[32];
-                    const uint8_t *krow = sRaw + (size_t)rb * P.raw_bytes + (size_t)p * 128;
-                    const long long cg0 = prof ? clock64() : 0;
-                    if (BAND == 2) {
-                        // stage (c0 + ch) of the tile covers keys k0 .. k0 + 31 of the row tile's window; this set's next stage
-                        // (two on) is fetched while this one is split and written
-                        if (PASSES != kMathBf16x3) {
-                            const int k0 = ((bx * kTileM - P.band_w) & ~3) + (c0 + ch) * kStageK, i0w = bx * kTileM + (warp & 3) * 32;
-                            const float *pb = P.band_p + (long long)zb * P.m_rows * (2 * P.band_w + 1);
-                            float *blk = reinterpret_cast<float *>(smem + L.stage_off) + (warp - 3) * 2048; // two blocks per warp
-                            const bool more = ch + sstep < c1 - c0;
-                            if (ch < sstep) // the set's first stage of the tile
-                                band_issue(pb, P.m_rows, P.band_w, i0w, k0, blk + ((ch / sstep) & 1) * 1024, lane);
-                            if (more)
-                                band_issue(pb, P.m_rows, P.band_w, i0w, k0 + sstep * kStageK, blk + ((ch / sstep + 1) & 1) * 1024, lane);
-                            band_take<PASSES>(blk + ((ch / sstep) & 1) * 1024, more, lane, hi, lo);
-                        }
-                    } else if (A_KMAJOR)
-                        gather_split<kGatherKMajor, PASSES>(ko, raw, krow, p, tmask, 0, false, zero_word, hi, lo);
-                    else if (P.cstride) // runs per stage: 1, 2 or 4 of 32 TF32 values; 2, 4 or 8 of 64 bf16 values
-                        if (!BF && P.gruns == 1)
-                            gather_split<kGatherStride, PASSES, 1>(ko, raw, krow, p, tmask, P.cstride, P.flat != 0, zero_word, hi, lo);
-                        else if (P.gruns == 2)
-                            gather_split<kGatherStride, PASSES, 2>(ko, raw, krow, p, tmask, P.cstride, P.flat != 0, zero_word, hi, lo);
-                        else if (!BF || P.gruns == 4)
-                            gather_split<kGatherStride, PASSES, 4>(ko, raw, krow, p, tmask, P.cstride, P.flat != 0, zero_word, hi, lo);
-                        else
-                            gather_split<kGatherStride, PASSES, 8>(ko, raw, krow, p, tmask, P.cstride, P.flat != 0, zero_word, hi, lo);
-                    else if (P.flat)
-                        gather_split<kGatherFlat, PASSES>(ko, raw, krow, p, tmask, 0, true, zero_word, hi, lo);
-                    else
-                        gather_split<kGatherTable, PASSES>(ko, raw, krow, p, tmask, 0, false, zero_word, hi, lo);
-                    const long long ce0 = prof ? clock64() : 0;
-                    alive = ptx::mbar_wait(a_empty + sa, pa, abort_flag);
-                    if (!alive)
-                        break;
-                    ptx::tc_fence_after();
-                    const uint32_t t = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)P.a_col + (uint32_t)sa * 64u;
-                    ptx::tmem_st_32x32(t, hi);
-                    const long long cg1 = prof ? clock64() : 0;
-                    if (prof) {
-                        t_we += cg1 - ce0;
-                        t_g -= cg1 - ce0; // the gather time below is measured up to cg1
-                    }
-                    if (SPLIT)
-                        ptx::tmem_st_32x32(t + 32u, lo);
-                    ptx::tmem_st_wait();
-                    ptx::tc_fence_before();
-                    if (prof) {
-                        t_g += cg1 - cg0;
-                        t_st += clock64() - cg1;
-                    }
-                } else {
-                    uint8_t *rowh = sA + (size_t)sa * 2 * kAHalfBytes + (size_t)p * 128;
-                    uint8_t *rowl = rowh + kAHalfBytes;
-#pragma unroll
-                    for (int c4 = 0; c4 < 8; ++c4) {
-                        const int4 o = ko[c4];
-                        float v0 = o.x >= 0 ? raw[o.x] : 0.f, v1 = o.y >= 0 ? raw[o.y] : 0.f;
-                        float v2 = o.z >= 0 ? raw[o.z] : 0.f, v3 = o.w >= 0 ? raw[o.w] : 0.f;
-                        float4 h, l;
-                        h.x = __uint_as_float(__float_as_uint(v0) & 0xffffe000u);
-                        h.y = __uint_as_float(__float_as_uint(v1) & 0xffffe000u);
-                        h.z = __uint_as_float(__float_as_uint(v2) & 0xffffe000u);
-                        h.w = __uint_as_float(__float_as_uint(v3) & 0xffffe000u);
-                        l.x = v0 - h.x;
-                        l.y = v1 - h.y;
-                        l.z = v2 - h.z;
-                        l.w = v3 - h.w;
-                        const int phys = (c4 ^ (p & 7)) << 4;
-                        *reinterpret_cast<float4 *>(rowh + phys) = h;
-                        *reinterpret_cast<float4 *>(rowl + phys) = l;
-                    }
-                    ptx::fence_proxy_async_smem();
-                }
-                __syncwarp();
-                if (lane == 0)
-                    ptx::mbar_arrive(a_full + sa);
-                if (PP) { // the set's other slot next; a slot's parity flips with every use
-                    own_apar ^= 1u << (sa & 1);
-                    sa ^= 1;
-                    pa = (own_apar >> (sa & 1)) & 1u;
-                } else {
-                    sa += sstep;
-                    if (sa >= P.NA) {
-                        sa -= P.NA;
-                        pa ^= 1u;
-                    }
-                }
-            }
-            __syncwarp();
-            if (lane == 0 && alive && !band_gather)
-                ptx::mbar_arrive(raw_empty + rb);
-            if (++rb == P.NR) {
-                rb = 0;
-                prw ^= 1u;
-            }
-        }
-        // ---------------- epilogue ----------------
-        t_loop = prof ? clock64() - t_begin : 0;
-        if (PP) // the next tile's fills (the other set's): their loads only wait for buffers this tile has already released
-            observe_until(min((tl + 2) * (c1 - c0), ntl * (c1 - c0)));
-        // Addresses and store mode first: the MMA warp is still working through the last stages, so this costs nothing.
-        const bool vec_ok = (P.ys_f == 1) && ((P.ys_p & 3) == 0) && ((P.ys_n & 3) == 0) && ((P.Fg & 3) == 0) &&
-                            ((reinterpret_cast<uintptr_t>(P.y) & 15) == 0);
-        const int f_tile0 = ntile * P.BN;
-        const long long f_glob0 = P.z_is_batch ? 0 : (long long)zb * P.Fg;
-        float *yp = P.y + y_off + f_glob0 * P.ys_f;
-        const float *bp = (P.has_bias && P.ksplit == 1) ? P.bias + f_glob0 : nullptr;
-        const float *rp = (P.res != nullptr && P.ksplit == 1) ? P.res + y_off + f_glob0 * P.ys_f : nullptr;
-        // split-K: partial sums go to the landing areas of the cluster's CTAs, summed after the role branches
-        const int split_cols = P.BN / P.ksplit, split_shift = 31 - __clz(split_cols);
-        const uint32_t split_addr =
-            P.ksplit > 1 ? ptx::smem_u32(sSplit) + (uint32_t)(((int)ptx::cluster_ctarank() * split_cols) * kTileM + p) * 4u : 0u;
-        const uint32_t tacc0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + (PP ? (uint32_t)((tl & 1) * 2 * P.BN) : 0u);
-        const uint32_t tacc = tacc0 + (FL > 0 ? 2u * (uint32_t)P.BN : 0u);
-        const uint32_t tcross = tacc0 + (uint32_t)P.BN;
-        // staged 16-byte stores need: pixel-contiguous NCHW output, full-width rows (no column window), one plane per
-        // tile, 16-byte aligned runs (of y and of the residual, which is laid out like y)
-        float *stage = nullptr;
-        int nvalid_warp = 0;
-        const long long plane_elems = (long long)P.OD * P.OH * P.OW;
-        const long long y_off0 = __shfl_sync(0xffffffffu, y_off, 0);
-        float *ybase_warp = yp - y_off + y_off0;
-        const float *rbase_warp = rp != nullptr ? rp - y_off + y_off0 : nullptr;
-        if (P.ys_p == 1 && P.ipt == 1 && P.own == P.OW && P.ow0 == 0 && (plane_elems & 3) == 0 && (P.ys_n & 3) == 0 &&
-            ((P.OH * P.OW) & 3) == 0 && (!P.wide || (P.OW & 3) == 0) &&
-            (P.ys_f & 3) == 0 && ((P.oh0 * P.OW) & 3) == 0 && P.ksplit == 1 &&
-            (reinterpret_cast<uintptr_t>(P.y) & 15) == 0 && (reinterpret_cast<uintptr_t>(P.res) & 15) == 0 && !P.epi_direct) {
-            nvalid_warp = __popc(__ballot_sync(0xffffffffu, valid));
-            if (nvalid_warp > 0) // B stages are idle once the accumulator is complete; in ping-pong mode they never are
-                stage = reinterpret_cast<float *>(PP ? smem + L.stage_off : sB) + (warp - 3) * 1024;
-            if (!PP && (uint32_t)(warp - 3 + 1) * 4096u > (uint32_t)P.NB * (SPLIT ? 2u : 1u) * b_half)
-                stage = nullptr; // not enough idle shared memory for this warp's block
-        }
-        // the two sets split the tile's columns (whole 32-column blocks)
-        const int nblk = P.BN / 32, half_blk = (nblk + 1) / 2;
-        const int col0 = (PP || tset == 0) ? 0 : half_blk * 32, col1 = (!PP && tset == 0) ? half_blk * 32 : P.BN;
-        for (; fg < n_groups - 1 && alive; ++fg)
-            alive = drain_group(fg, true, true);
-        if (alive)
-            alive = ptx::mbar_wait((PP && (tl & 1)) ? acc_full1 : acc_full, PP ? (uint32_t)((tl >> 1) & 1) : 0u, abort_flag);
-        if (alive && FL > 0) // the last group joins the total; the epilogue then reads the total in place of the accumulator
-            drain_group(n_groups - 1, false, false);
-        if (reg_total) { // set 1 has written total + last group over the main accumulator: both sets meet before reading it
-            ptx::named_bar_sync(1, 256);
-            ptx::tc_fence_after();
-        }
-        t_epi0 = prof ? clock64() : 0;
-        if (alive) {
-            ptx::tc_fence_after();
-#define PETB200_EPI(ACT_)                                                                                              \
-    epilogue_store<ACT_, PASSES>(tacc, tcross, P.BN, f_tile0, P.Fg, valid, bp, rp, yp, P.ys_f, vec_ok, stage, nvalid_warp, \
-                                 ybase_warp, rbase_warp, col0, col1, split_addr, split_shift)
-            switch (P.ksplit > 1 ? PETB200_ACT_NONE : P.act) {
-            case PETB200_ACT_RELU: PETB200_EPI(PETB200_ACT_RELU); break;
-            case PETB200_ACT_SIGMOID: PETB200_EPI(PETB200_ACT_SIGMOID); break;
-            case PETB200_ACT_TANH: PETB200_EPI(PETB200_ACT_TANH); break;
-            case PETB200_ACT_GELU: PETB200_EPI(PETB200_ACT_GELU); break;
-            default: PETB200_EPI(PETB200_ACT_NONE); break;
-            }
-#undef PETB200_EPI
-            if (PP) { // this tile's accumulators are in registers or stored: the MMA warp may reuse the region
+                const long long cd1 = prof ? clock64() : 0;
+                ptx::tc_fence_after();
+                const uint32_t tacc = t_row + (uint32_t)((tl & 1) * 2 * P.BN);
+                epilogue_banded<PASSES>(tacc, tacc + (uint32_t)P.BN, 0, P.BN, ntile * P.BN, quarter * 32, bx, zb, P.m_rows, P.band_w, P.y,
+                                        reinterpret_cast<float *>(smem + L.stage_off) + quarter * 1024, lane);
                 ptx::tc_fence_before();
                 __syncwarp();
                 if (lane == 0)
                     ptx::mbar_arrive(acc_empty + (tl & 1));
+                if (prof)
+                    t_dw += cd1 - cd0, t_dd += clock64() - cd1;
             }
+        } else if (PP || FL > 0) {
+            const bool filters_run = (P.ys_f == 1) && ((P.ys_p & 3) == 0) && ((P.ys_n & 3) == 0) && ((P.Fg & 3) == 0) &&
+                                     (((reinterpret_cast<uintptr_t>(P.y) | reinterpret_cast<uintptr_t>(P.res)) & 15) == 0);
+            const int store_mode = pixel_runs() ? kStorePixels : (filters_run ? kStoreFilters : kStoreAny);
+            float *stage = reinterpret_cast<float *>(smem + L.stage_off) + quarter * 1024;
+            for (int tl = 0; tl < ntl && alive; ++tl) {
+                const int reg = two_regions ? (tl & 1) : 0, use = two_regions ? (tl >> 1) : tl;
+                StoreJob J;
+                if (PP) { // where the tile goes: worked out while its MMAs run
+                    set_tile((int)blockIdx.x + tl * (int)gridDim.x);
+                    int base_p;
+                    pixel_geom(p, J.valid, base_p, J.y_off);
+                    const long long f_glob0 = P.z_is_batch ? 0 : (long long)zb * P.Fg;
+                    J.y = P.y + f_glob0 * P.ys_f;
+                    J.bias = P.has_bias ? P.bias + f_glob0 : nullptr;
+                    J.res = P.res != nullptr ? P.res + f_glob0 * P.ys_f : nullptr;
+                    J.ys_f = P.ys_f, J.mode = store_mode, J.Fg = P.Fg, J.act = P.act, J.lane = lane;
+                    J.nvalid = __popc(__ballot_sync(0xffffffffu, J.valid));
+                    J.y_off0 = __shfl_sync(0xffffffffu, J.y_off, 0);
+                }
+                const uint32_t tmain = t_row + (uint32_t)(reg * 2 * P.BN), tcross = tmain + (uint32_t)P.BN;
+                float racc[PP == kNarrow ? 32 : 128]; // the sums of this thread's tile row (narrow: of the block being stored)
+                auto take_acc_full = [&]() {
+                    const long long c0 = prof ? clock64() : 0;
+                    alive = ptx::mbar_wait_warp(reg ? acc_full1 : acc_full, (uint32_t)(use & 1), abort_flag);
+                    ptx::tc_fence_after();
+                    t_acc += prof ? clock64() - c0 : 0;
+                };
+                auto release = [&]() { // the MMA thread may start the region's next tile
+                    ptx::tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0)
+                        ptx::mbar_arrive(acc_empty + reg);
+                };
+                if constexpr (PP == kNarrow) {
+                    take_acc_full();
+                    if (!alive)
+                        break;
+#pragma unroll 1 // (one copy of the store code: see FastDiv)
+                    for (int c = 0; c < P.BN; c += 32) {
+#pragma unroll
+                        for (int h = 0; h < 32; h += 16) {
+                            uint32_t v[16], x[16];
+                            ptx::tmem_ld_32x16(tmain + (uint32_t)(c + h), v);
+                            if (SPLIT)
+                                ptx::tmem_ld_32x16(tcross + (uint32_t)(c + h), x);
+                            ptx::tmem_ld_wait();
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) // hi*hi sum + (lo*hi + hi*lo) sum, one rounded fp32 add
+                                racc[h + j] = SPLIT ? __uint_as_float(v[j]) + __uint_as_float(x[j]) : __uint_as_float(v[j]);
+                        }
+                        if (c + 32 >= P.BN)
+                            release();
+                        store_block(J, racc, stage, ntile * P.BN + c);
+                    }
+                } else {
+                    // Groups in order, round-to-nearest adds; the MMA thread restarts the main accumulator once a group has been taken.
+                    for (int g = 0; g + 1 < n_groups && alive; ++g, gpar ^= 1u) {
+                        const long long cd0 = prof ? clock64() : 0;
+                        alive = ptx::mbar_wait_warp(acc_ready, gpar, abort_flag);
+                        if (!alive)
+                            break;
+                        const long long cd1 = prof ? clock64() : 0;
+                        ptx::tc_fence_after();
+                        drain_add<false>(racc, tmain, 0u, P.BN, g == 0);
+                        ptx::tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0)
+                            ptx::mbar_arrive(flushed);
+                        if (prof)
+                            t_dw += cd1 - cd0, t_dd += clock64() - cd1;
+                    }
+                    if (alive)
+                        take_acc_full();
+                    if (!alive)
+                        break;
+                    if constexpr (PP == kSingle) { // write the total back over the main accumulator for the transform sets' epilogue
+                        drain_add<false>(racc, tmain, 0u, P.BN, n_groups == 1);
+#pragma unroll
+                        for (int b = 0; b < 8; ++b)
+                            if (b * 16 < P.BN) {
+                                uint32_t v[16];
+#pragma unroll
+                                for (int j = 0; j < 16; ++j)
+                                    v[j] = __float_as_uint(racc[b * 16 + j]);
+                                ptx::tmem_st_32x16(tmain + (uint32_t)(b * 16), v);
+                            }
+                        ptx::tmem_st_wait();
+                        ptx::tc_fence_before();
+                    } else {
+                        drain_add<SPLIT>(racc, tmain, tcross, P.BN, n_groups == 1);
+                        release();
+                        const long long cs0 = prof ? clock64() : 0;
+#pragma unroll 1
+                        for (int c = 0; c < P.BN; c += 32) {
+                            store_block(J, racc, stage, ntile * P.BN + c);
+#pragma unroll
+                            for (int j = 0; j < 96; ++j) // the next block's sums move down
+                                racc[j] = racc[j + 32];
+                        }
+                        t_store += prof ? clock64() - cs0 : 0;
+                    }
+                }
+            }
+            if (!PP && FL > 0) // (also after a wait gave up: the transform sets wait here)
+                ptx::named_bar_sync(1, 384);
         }
-        } // tiles of this set
-        if (PP)
-            observe_until(ntl * (c1 - c0)); // fills of tiles after this set's last one
-        if (prof && threadIdx.x == 96) { // lane 0 of warp 3 (transform set 0)
+        if (prof && threadIdx.x == kDrainWarp * 32) {
             long long *pr = prof + ((size_t)(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * kProfSlots;
-            pr[3] = t_we;
-            pr[4] = t_wr;
-            pr[5] = t_loop;
-            pr[6] = clock64() - t_epi0;
-            pr[7] = t_epi0 - t_begin;
-            pr[10] = (long long)ptx::globaltimer_ns();
-            pr[12] = t_g;
-            pr[13] = t_st;
-            pr[17] = t_dw;
-            pr[18] = t_dd;
+            pr[17] = t_dw, pr[18] = t_dd, pr[19] = t_acc, pr[21] = t_store;
         }
     }
 
     // ---------------- split-K: reduction across the cluster ----------------
     // Every thread of every CTA of the cluster reaches the barrier (all waits above are bounded).
     if (P.ksplit > 1) {
-        if (warp >= 3 && warp < 7) {
+        if (warp >= kSetWarp && warp < kSetWarp + 4) {
             // The bias / residual values the reduction below adds start their way to L1 while the cluster meets.  Set 0's
             // threads do it, for the row each of them wrote into sYoff itself (both halves of the CTA's column slice).
-            const int et = threadIdx.x - 96, cols = P.BN / P.ksplit;
+            const int et = threadIdx.x - kSetWarp * 32, cols = P.BN / P.ksplit;
             const long long y_off = sYoff[et];
             const int f = ntile * P.BN + (int)ptx::cluster_ctarank() * cols;
             const long long f_glob0 = P.z_is_batch ? 0 : (long long)zb * P.Fg;
@@ -1442,8 +1594,8 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
         ptx::cluster_sync_all(); // every CTA's pushes have landed; nothing touches a peer's memory after this
         if (prof_cta)
             prof_cta[14] = (long long)ptx::globaltimer_ns();
-        if (warp >= 3) {
-            const int et = threadIdx.x - 96;
+        if (warp >= kSetWarp && warp < kDrainWarp) {
+            const int et = threadIdx.x - kSetWarp * 32;
             const long long y_off = sYoff[et & (kTileM - 1)];
             if (y_off >= 0 && *abort_flag == 0) {
                 const long long f_glob0 = P.z_is_batch ? 0 : (long long)zb * P.Fg;
@@ -1483,7 +1635,7 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
     ptx::tc_fence_before();
     __syncthreads();
     if (warp == 2)
-        ptx::tmem_dealloc(tmem_base, tmem_cols);
+        ptx::tmem_dealloc(tmem_base, kTmemCols);
     if (prof_cta)
         prof_cta[11] = (long long)ptx::globaltimer_ns();
 }
@@ -1567,10 +1719,11 @@ static int env_int_early(const char *name, int dflt) {
     return v ? atoi(v) : dflt;
 }
 
+typedef void (*KernelFn)(CUtensorMap, CUtensorMap, CUtensorMap, IgemmParams);
+
 struct TcCore {
     petb200_ctx *ctx = nullptr;
     IgemmParams P{};
-    bool a_tmem = false;
     int single_pass = 0;
     int bf16 = 0; // error-compensated bf16 (64 K elements per stage) instead of TF32
     dim3 grid;
@@ -1588,21 +1741,20 @@ struct TcCore {
     long long *prof = nullptr;
     int starve = 0;
 
-    void (*kernel() const)(CUtensorMap, CUtensorMap, CUtensorMap, IgemmParams) {
+    KernelFn kernel() const {
         if (P.a_kmajor && P.band_w > 0) // banded products: G2BMM in persistent mode with its own epilogue, GBMML with its own operand fetch
-            return P.pp ? k_igemm<true, true, kMathTf32x3, true, 1> : k_igemm<true, true, kMathTf32x3, false, 2>;
-        if (P.pp) { // conv plans on the TS variant
-            if (single_pass)
-                return k_igemm<true, false, kMathTf32x1, true>;
-            return bf16 ? k_igemm<true, false, kMathBf16x3, true> : k_igemm<true, false, kMathTf32x3, true>;
-        }
+            return P.band_g2 ? k_igemm<true, kMathTf32x3, kNarrow, 1>
+                             : (!P.pp ? k_igemm<true, kMathTf32x3, kSingle, 2>
+                                      : (P.BN <= 64 && P.fl == 0 ? k_igemm<true, kMathTf32x3, kNarrow, 2> : k_igemm<true, kMathTf32x3, kWide, 2>));
         if (single_pass)
-            return P.a_kmajor ? k_igemm<true, true, kMathTf32x1> : k_igemm<true, false, kMathTf32x1>;
-        if (bf16)
-            return P.a_kmajor ? k_igemm<true, true, kMathBf16x3> : k_igemm<true, false, kMathBf16x3>;
+            return pick<kMathTf32x1>();
+        return bf16 ? pick<kMathBf16x3>() : pick<kMathTf32x3>();
+    }
+    template <int PASSES> KernelFn pick() const {
+        const bool narrow = P.BN <= 64 && P.fl == 0;
         if (P.a_kmajor)
-            return k_igemm<true, true, kMathTf32x3>;
-        return a_tmem ? k_igemm<true, false, kMathTf32x3> : k_igemm<false, false, kMathTf32x3>;
+            return !P.pp ? k_igemm<true, PASSES> : (narrow ? k_igemm<true, PASSES, kNarrow> : k_igemm<true, PASSES, kWide>);
+        return !P.pp ? k_igemm<false, PASSES> : (narrow ? k_igemm<false, PASSES, kNarrow> : k_igemm<false, PASSES, kWide>);
     }
     int encode_x(const float *x) {
         if (x == map_x_ptr)
@@ -1673,6 +1825,7 @@ struct TcCore {
         if (rc)
             return rc;
         IgemmParams p = P;
+        set_divisors(p);
         p.bias = bias;
         p.res = res;
         p.y = y;
@@ -1680,9 +1833,8 @@ struct TcCore {
         p.status = ctx->d_status;
         p.prof = prof;
         p.starve = starve;
-        p.epi_direct = env_int_early("PETB200_TC_EPI_DIRECT", 0);
         p.has_bias = (P.has_bias && bias) ? 1 : 0;
-        void (*kern)(CUtensorMap, CUtensorMap, CUtensorMap, IgemmParams) = kernel();
+        KernelFn kern = kernel();
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = grid;
         cfg.blockDim = dim3(kThreads);
@@ -1750,10 +1902,10 @@ static int cluster_slots(int sm_count, int ks) {
         attr[0].val.clusterDim.x = 1, attr[0].val.clusterDim.y = (unsigned)ks, attr[0].val.clusterDim.z = 1;
         cfg.attrs = attr, cfg.numAttrs = 1;
         int n = 0;
-        (void)cudaFuncSetAttribute(k_igemm<true, false, kMathTf32x3, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        (void)cudaFuncSetAttribute(k_igemm<false, kMathTf32x3>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
         if (ks > 8) // clusters of 16 are beyond the portable size: allowed per function
-            (void)cudaFuncSetAttribute(k_igemm<true, false, kMathTf32x3, false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (cudaOccupancyMaxActiveClusters(&n, k_igemm<true, false, kMathTf32x3, false>, &cfg) != cudaSuccess || n <= 0) {
+            (void)cudaFuncSetAttribute(k_igemm<false, kMathTf32x3>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (cudaOccupancyMaxActiveClusters(&n, k_igemm<false, kMathTf32x3>, &cfg) != cudaSuccess || n <= 0) {
             (void)cudaGetLastError();
             // what B200 was measured to hold; a cluster of 16 is only used where the driver itself says it fits
             n = ks > 8 ? -1 : std::max(1, (sm_count * (ks <= 2 ? 96 : 86) / 100) / ks);
@@ -1799,29 +1951,43 @@ static int choose_ksplit(int sm_count, long long base_ctas, const IgemmParams &P
     return best;
 }
 
-// Accumulator flush period (see IgemmParams::fl) and the TMEM column map that goes with it.  The truncation bias of the
-// tensor core's fp32 accumulator grows with the number of MMAs added into one running sum: K ranges of more than
-// `3 * period` stages per CTA are drained every `period` stages (PETB200_TC_FLUSH in the environment, 0 = never; measured
-// without a flush: 2.4e-4 of the contract's 1e-3 at 18 stages, 3e-4..4e-4 at 36, 2e-3 at 54).  The
-// running total takes BN more TMEM columns; a 128-wide tile then has room for two A stages instead of four.
+// Accumulator flush period (see IgemmParams::fl).  The truncation bias of the tensor core's fp32 accumulator grows with the number
+// of MMAs added into one running sum: K ranges of more than `3 * period` stages per CTA are drained every `period` stages
+// (PETB200_TC_FLUSH in the environment, 0 = never; measured without a flush: 2.4e-4 of the contract's 1e-3 at 18 stages,
+// 3e-4..4e-4 at 36, 2e-3 at 54).
 static void choose_flush(TcCore &core) {
     IgemmParams &P = core.P;
     // (bf16: twice the K per stage and an accuracy class that the split, not the truncation, dominates: half as often)
     const int period = env_int("PETB200_TC_FLUSH", core.bf16 ? 16 : 8);
     const int ks_max = ((P.nchunks + P.ksplit - 1) / P.ksplit) * P.spc;
-    P.fl = (!core.single_pass && core.a_tmem && period > 0 && ks_max > 3 * period) ? period : 0;
-    // register totals make one transform set do all the A stages: only where the gather is the cheap kind (whole 32-channel
-    // stages of one tap, or row-major matmul tiles); slower gathers need both sets and keep the total in TMEM
-    const bool fast_gather = P.a_kmajor || (P.cstride != 0 && P.gruns == (core.bf16 ? 2 : 1));
-    const int regs_env = env_int("PETB200_TC_FLUSH_REGS", -1);
-    P.fl_regs = (P.fl > 0 && P.BN == 128 && (regs_env < 0 ? fast_gather : regs_env != 0)) ? 1 : 0;
-    P.a_col = (P.fl > 0 && P.BN == 128 && !P.fl_regs) ? 384 : 256;
-    if (core.a_tmem)
-        P.NA = (512 - P.a_col) / 64;
+    P.fl = (!core.single_pass && period > 0 && ks_max > 3 * period) ? period : 0;
     if (env_int("PETB200_TC_VERBOSE", 0))
-        fprintf(stderr, "[petb200] igemm plan: BN %d BC %d chunks %d stages/chunk %d ksplit %d flush %d (regs %d) NA %d NB %d NR %d kmajor %d flat %d math %s\n",
-                P.BN, P.BC, P.nchunks, P.spc, P.ksplit, P.fl, P.fl_regs, P.NA, P.NB, P.NR, P.a_kmajor, P.flat,
+        fprintf(stderr, "[petb200] igemm plan: BN %d BC %d chunks %d stages/chunk %d ksplit %d flush %d NB %d NR %d kmajor %d flat %d math %s\n",
+                P.BN, P.BC, P.nchunks, P.spc, P.ksplit, P.fl, P.NB, P.NR, P.a_kmajor, P.flat,
                 core.single_pass ? "1xtf32" : (core.bf16 ? "bf16x3" : "3xtf32"));
+}
+
+// Persistent mode (see IgemmParams::pp) where some SM would otherwise run several CTAs in sequence: the start-up of a CTA (about
+// 3000 cycles to its first MMA) and its epilogue (2000 to 4000) hide behind the MMAs of its neighbour tiles.  Not with a K
+// split (a CTA's tile is then a cluster's).  Sets the grid.
+static void choose_grid(petb200_ctx *ctx, TcCore &core, int mtiles, int ntiles, int gz, size_t budget) {
+    IgemmParams &P = core.P;
+    const long long tiles = (long long)mtiles * ntiles * gz;
+    P.mtiles = mtiles, P.ntiles = ntiles, P.tiles = (int)tiles;
+    P.pp = 0;
+    core.grid = dim3((unsigned)mtiles, (unsigned)(ntiles * P.ksplit), (unsigned)gz);
+    if (!env_int("PETB200_TC_PINGPONG", 1) || P.ksplit > 1 || tiles <= ctx->sm_count || tiles > (1 << 30))
+        return;
+    const int nb_was = P.NB, nr_was = P.NR;
+    P.pp = 1;
+    while (smem_layout(P).total > budget && (P.NB > 2 || P.NR > 2)) // the drain warps' blocks take room from the rings
+        (P.NB > 2 && P.NB >= P.NR ? P.NB : P.NR)--;
+    if (smem_layout(P).total > budget) {
+        P.pp = 0, P.NB = nb_was, P.NR = nr_was;
+        return;
+    }
+    const long long per_cta = (tiles + ctx->sm_count - 1) / ctx->sm_count;
+    core.grid = dim3((unsigned)((tiles + per_cta - 1) / per_cta), 1, 1);
 }
 
 // The dynamic shared-memory attribute is per function, not per launch: raise it once to the device limit so that plans
@@ -1831,29 +1997,19 @@ static int raise_smem_limit(petb200_ctx *ctx) {
     if (attr_set)
         return PETB200_OK;
     const int lim = (int)std::min<size_t>(ctx->smem_optin, 227 * 1024);
-    cudaError_t e = cudaFuncSetAttribute(k_igemm<true, false, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_igemm<false, false, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_igemm<true, true, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_igemm<true, false, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_igemm<true, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_igemm<true, false, kMathBf16x3>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_igemm<true, true, kMathBf16x3>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_igemm<true, false, kMathTf32x3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_igemm<true, false, kMathBf16x3, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_igemm<true, false, kMathTf32x1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_igemm<true, true, kMathTf32x3, true, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_igemm<true, true, kMathTf32x3, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
+    const KernelFn kernels[] = {
+        k_igemm<false, kMathTf32x3>, k_igemm<false, kMathTf32x3, kNarrow>, k_igemm<false, kMathTf32x3, kWide>,
+        k_igemm<true, kMathTf32x3>, k_igemm<true, kMathTf32x3, kNarrow>, k_igemm<true, kMathTf32x3, kWide>,
+        k_igemm<false, kMathTf32x1>, k_igemm<false, kMathTf32x1, kNarrow>, k_igemm<false, kMathTf32x1, kWide>,
+        k_igemm<true, kMathTf32x1>, k_igemm<true, kMathTf32x1, kNarrow>, k_igemm<true, kMathTf32x1, kWide>,
+        k_igemm<false, kMathBf16x3>, k_igemm<false, kMathBf16x3, kNarrow>, k_igemm<false, kMathBf16x3, kWide>,
+        k_igemm<true, kMathBf16x3>, k_igemm<true, kMathBf16x3, kNarrow>, k_igemm<true, kMathBf16x3, kWide>,
+        k_igemm<true, kMathTf32x3, kNarrow, 1>, k_igemm<true, kMathTf32x3, kSingle, 2>, k_igemm<true, kMathTf32x3, kNarrow, 2>,
+        k_igemm<true, kMathTf32x3, kWide, 2>};
+    cudaError_t e = cudaSuccess;
+    for (auto k : kernels)
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, lim);
     if (e != cudaSuccess)
         return fail(ctx, PETB200_ERR_CUDA, "cudaFuncSetAttribute(%d bytes) failed: %s", lim, cudaGetErrorString(e));
     attr_set = true;
@@ -1930,9 +2086,8 @@ static int tc_configure(petb200_ctx *ctx, TcCore &core, const ConvGeom &g, int o
         // rows a tile touches: maximum over the tiles of one plane (in OUTPUT rows first)
         int RHo = 1;
         for (int tq = 0; tq < P.tpi; ++tq) {
-            int yl_lo, yl_hi;
-            tile_rows(P, tq * kTileM, std::min((tq + 1) * kTileM, P.Pw) - 1, P.ipt > 1, yl_lo, yl_hi);
-            RHo = std::max(RHo, yl_hi - yl_lo + 1);
+            const int q_hi = std::min((tq + 1) * kTileM, P.Pw) - 1; // (whole planes when a tile holds several)
+            RHo = std::max(RHo, P.ipt > 1 ? P.ohn : q_hi / P.own - tq * kTileM / P.own + 1);
         }
         P.RN = (g.OD == 1) ? P.ipt : 1;
         P.RD = ((g.OD == 1) ? 0 : (P.ipt - 1) * P.sd) + (g.T3[0] - 1) * g.dil[0] + 1;
@@ -1950,7 +2105,6 @@ static int tc_configure(petb200_ctx *ctx, TcCore &core, const ConvGeom &g, int o
         return fail(ctx, PETB200_ERR_UNSUPPORTED, "raw activation box %dx%dx%dx%d exceeds the TMA box limit", P.RN, P.RD, P.RH, P.RW);
     }
     const size_t budget = std::min<size_t>(ctx->smem_optin, 227 * 1024) - 1024; // alignment slack
-    core.a_tmem = core.single_pass || core.bf16 || env_int("PETB200_TC_A_TMEM", 1) != 0; // other variants exist for TS only
     const int forced_bc = force_bc > 0 ? force_bc : env_int("PETB200_TC_BC", 0);
     // Channels per chunk (32, or more for filters with few taps so that one raw tile still feeds several K stages) and
     // ring depths for a given tile width; false if not even one channel's raw tile fits.
@@ -1968,7 +2122,6 @@ static int tc_configure(petb200_ctx *ctx, TcCore &core, const ConvGeom &g, int o
             P.nchunks = (cpg + BC - 1) / BC;
             size_t raw = (size_t)P.RN * BC * P.RD * P.RH * P.RW * 4;
             P.raw_bytes = (int)((raw + 127) / 128 * 128);
-            P.NA = core.a_tmem ? 4 : 2;
             P.NB = 2;
             P.NR = 2;
             P.a_kmajor = 0;
@@ -1984,24 +2137,13 @@ static int tc_configure(petb200_ctx *ctx, TcCore &core, const ConvGeom &g, int o
                         P.flat_w = w, P.flat_rows = (int)(L / w);
                 shape_ok = P.flat_w != 0 && cpg % BC == 0 && P.RN <= 256;
             }
-            if (shape_ok && smem_layout(P, core.a_tmem).total <= budget) {
-                // deepen the rings while there is room: B first (it hides TMA latency), then A
-                for (bool grew = true; grew;) {
-                    grew = false;
-                    if (P.NB < kMaxNB) {
-                        P.NB++;
-                        if (smem_layout(P, core.a_tmem).total <= budget)
-                            grew = true;
-                        else
-                            P.NB--;
-                    }
-                    if (!core.a_tmem && P.NA < 3 && P.NB >= 3) {
-                        P.NA++;
-                        if (smem_layout(P, core.a_tmem).total <= budget)
-                            grew = true;
-                        else
-                            P.NA--;
-                    }
+            if (shape_ok && smem_layout(P).total <= budget) {
+                for (; P.NB < kMaxNB; P.NB++) { // deepen the filter ring while there is room
+                    P.NB++;
+                    const bool fits = smem_layout(P).total <= budget;
+                    P.NB--;
+                    if (!fits)
+                        break;
                 }
                 return true;
             }
@@ -2052,41 +2194,18 @@ static int tc_configure(petb200_ctx *ctx, TcCore &core, const ConvGeom &g, int o
     if (!have)
         return fail(ctx, PETB200_ERR_UNSUPPORTED, "raw activation tile does not fit shared memory");
     P = bestP;
-    // runs of consecutive channels (of one filter tap) per K stage, when the chunk size allows that kind of gather
-    P.gruns = P.BC % kStageK == 0 ? P.ke / kStageK : (P.BC == 16 ? P.ke / 16 : (P.BC == 8 ? P.ke / 8 : 0));
-    P.cstride = (P.gruns && env_int("PETB200_TC_TABLE", 0) == 0) ? P.RD * P.RH * P.RW : 0;
+    // eight consecutive K elements are channels of one filter tap: the cheap kind of gather
+    P.cstride = (P.BC % 8 == 0 && env_int("PETB200_TC_TABLE", 0) == 0) ? P.RD * P.RH * P.RW : 0;
     choose_flush(core);
-    if (flat && (!core.a_tmem || (long long)P.RN * P.BC * P.RD * P.RH * P.RW >= (1 << 24)))
-        return fail(ctx, PETB200_ERR_UNSUPPORTED, "flat raw tiles need the TS kernel variant");
+    if (flat && (long long)P.RN * P.BC * P.RD * P.RH * P.RW >= (1 << 24))
+        return fail(ctx, PETB200_ERR_UNSUPPORTED, "flat raw tile too large for the offset table");
     const int BN = P.BN;
-    if (core.a_tmem && BN > 256)
-        return fail(ctx, PETB200_ERR_INVALID, "TS variant supports BN <= 256");
     const int ntiles = (Fg + BN - 1) / BN;
-    // Persistent ping-pong mode (see IgemmParams::pp) where every SM would otherwise run several CTAs in sequence: narrow
-    // tiles (two accumulator regions must fit beside the A ring), no K split, no accumulator flush.
-    P.mtiles = mtiles;
-    P.pp = 0;
-    int grid_x = mtiles;
-    {
-        const int slots = std::max(1, ctx->sm_count / (ntiles * gz));
-        const int tiles_per_cta = (mtiles + slots - 1) / slots;
-        if (core.a_tmem && env_int("PETB200_TC_PINGPONG", 1) && P.ksplit == 1 && P.fl == 0 && BN <= 64 && tiles_per_cta >= 2) {
-            const int nb_was = P.NB;
-            P.pp = 1;
-            // (NA is 4 without a flush: two A slots per transform set)
-            while (smem_layout(P, true).total > budget && P.NB > 2)
-                P.NB--;
-            if (smem_layout(P, true).total > budget || P.NA != 4)
-                P.pp = 0, P.NB = nb_was;
-            else
-                grid_x = (mtiles + tiles_per_cta - 1) / tiles_per_cta;
-        }
-    }
-    core.smem = smem_layout(P, core.a_tmem).total + 1024;
+    choose_grid(ctx, core, mtiles, ntiles, gz, budget);
+    core.smem = smem_layout(P).total + 1024;
     core.y_elems = (z_is_batch ? (long long)images : (long long)n_img) * g.F * g.OD * g.OH * g.OW;
     if (z_is_batch)
         core.y_elems = (long long)images * ys_n;
-    core.grid = dim3((unsigned)grid_x, (unsigned)(ntiles * P.ksplit), (unsigned)gz);
     core.Ktot = (long long)P.nchunks * P.spc * P.ke;
     core.xd[0] = g.Wst;
     core.xd[1] = g.H;
@@ -2332,7 +2451,7 @@ int tc_set_wait_limit_ns(unsigned long long ns) {
 int tc_conv_row_pitch(void *h) { return ((TcConv *)h)->g.Wst; }
 const char *tc_conv_variant(void *h) {
     const TcCore &c = ((TcConv *)h)->full;
-    return c.single_pass ? "tc_1xtf32_ts" : (c.bf16 ? "tc_bf16x3_ts" : (c.a_tmem ? "tc_3xtf32_ts" : "tc_3xtf32_ss"));
+    return c.single_pass ? "tc_1xtf32_ts" : (c.bf16 ? "tc_bf16x3_ts" : "tc_3xtf32_ts");
 }
 
 // ---- matmul on the same kernel ------------------------------------------------------------------------------
@@ -2351,7 +2470,6 @@ static int tc_configure_kmajor(petb200_ctx *ctx, TcCore &core, int bs, int m, in
                                const long long *st) {
     IgemmParams &P = core.P;
     memset(&P, 0, sizeof P);
-    core.a_tmem = true;
     P.a_kmajor = 1;
     P.ke = core.bf16 ? 64 : kStageK;
     P.m_rows = m;
@@ -2365,7 +2483,6 @@ static int tc_configure_kmajor(petb200_ctx *ctx, TcCore &core, int bs, int m, in
     P.ys_n = st[4], P.ys_f = 1, P.ys_p = st[5];
     core.a_batch = st[0], core.a_row = st[1];
     P.has_bias = has_bias, P.act = act;
-    P.NA = 4;
     const size_t budget = std::min<size_t>(ctx->smem_optin, 227 * 1024) - 1024;
     P.NB = 2, P.NR = 2;
     // tile width and K split by the cycle model (before the rings are sized: a split takes shared memory)
@@ -2388,27 +2505,28 @@ static int tc_configure_kmajor(petb200_ctx *ctx, TcCore &core, int bs, int m, in
         P.BN = best_bn;
         P.ksplit = best_ks;
     }
-    if (smem_layout(P, true).total > budget)
+    if (smem_layout(P).total > budget)
         return fail(ctx, PETB200_ERR_UNSUPPORTED, "matmul tile does not fit shared memory");
     for (bool grew = true; grew;) { // deepen both rings alternately: every K stage needs one B tile and one raw tile
         grew = false;
         if (P.NB < kMaxNB) {
             P.NB++;
-            if (smem_layout(P, true).total <= budget)
+            if (smem_layout(P).total <= budget)
                 grew = true;
             else
                 P.NB--;
         }
         if (P.NR < kMaxNR) {
             P.NR++;
-            if (smem_layout(P, true).total <= budget)
+            if (smem_layout(P).total <= budget)
                 grew = true;
             else
                 P.NR--;
         }
     }
     choose_flush(core);
-    core.smem = smem_layout(P, true).total + 1024;
+    choose_grid(ctx, core, P.tpi, (n + P.BN - 1) / P.BN, bs, budget);
+    core.smem = smem_layout(P).total + 1024;
     core.Ktot = (long long)P.nchunks * P.ke;
     core.xd[0] = k, core.xd[1] = m, core.xd[2] = bs;
     std::vector<int> koff(P.ke, -1); // unused in this mode; the kernel still copies one stage worth of table
@@ -2416,7 +2534,6 @@ static int tc_configure_kmajor(petb200_ctx *ctx, TcCore &core, int bs, int m, in
         return fail(ctx, PETB200_ERR_NOMEM, "koff allocation failed");
     PETB200_CUDA(ctx, cudaMemcpy(core.koff.p, koff.data(), koff.size() * 4, cudaMemcpyHostToDevice));
     core.y_elems = (long long)bs * m * n;
-    core.grid = dim3((unsigned)P.tpi, (unsigned)(((n + P.BN - 1) / P.BN) * P.ksplit), (unsigned)bs);
     return raise_smem_limit(ctx);
 }
 
@@ -2488,7 +2605,7 @@ int tc_matmul_create(petb200_ctx *ctx, int bs, int m, int n, int k, int transA, 
 }
 // G2BMM on the tensor-core kernel (dilation 1): q [bs][n][m] is the row-major A operand, the keys k [bs][n][m] are packed like
 // a matmul's B operand ([bs*n rows][K]); a CTA column (blockIdx.y) is one 64-key piece of the 2w + 128 keys a row tile can
-// meet, and CTAs walk the row tiles in ping-pong mode.  `y` [bs][n][2w+1] is written by the banded epilogue.
+// meet, and CTAs walk the row tiles in persistent mode.  `y` [bs][n][2w+1] is written by the banded epilogue.
 int tc_g2bmm_create(petb200_ctx *ctx, int bs, int n, int m, int w, void **out) {
     if (ctx->cc_major != 10)
         return fail(ctx, PETB200_ERR_UNSUPPORTED, "tcgen05 kernels need compute capability 10.x");
@@ -2502,8 +2619,7 @@ int tc_g2bmm_create(petb200_ctx *ctx, int bs, int n, int m, int w, void **out) {
     core.ctx = ctx;
     IgemmParams &P = core.P;
     memset(&P, 0, sizeof P);
-    core.a_tmem = true;
-    P.a_kmajor = 1, P.ke = kStageK, P.m_rows = n, P.z_is_batch = 1, P.band_w = w;
+    P.a_kmajor = 1, P.ke = kStageK, P.m_rows = n, P.z_is_batch = 1, P.band_w = w, P.band_g2 = 1;
     P.OD = P.OH = 1, P.OW = n, P.ohn = 1, P.own = n, P.Pw = n, P.units = 1, P.ipt = 1, P.tpi = (n + kTileM - 1) / kTileM;
     P.sd = P.sh = P.sw = 1;
     P.cpg = m, P.Fg = n, P.BN = 64, P.ksplit = 1;
@@ -2511,12 +2627,12 @@ int tc_g2bmm_create(petb200_ctx *ctx, int bs, int n, int m, int w, void **out) {
     P.RN = P.RD = 1, P.RH = kTileM, P.RW = kStageK, P.raw_bytes = kAHalfBytes;
     P.ys_n = (long long)n * (2 * w + 1), P.ys_f = 1, P.ys_p = 2 * w + 1;
     core.a_batch = (long long)n * m, core.a_row = m;
-    P.NA = 4, P.a_col = 256, P.fl = 0, P.fl_regs = 0;
+    P.fl = 0;
     const int key_tiles = (2 * w + kTileM + P.BN - 1) / P.BN;
-    P.pp = 1, P.band_nt = key_tiles, P.mtiles = P.tpi * key_tiles;
+    P.pp = 1, P.ntiles = key_tiles, P.mtiles = P.tpi, P.tiles = P.tpi * key_tiles * bs;
     const size_t budget = std::min<size_t>(ctx->smem_optin, 227 * 1024) - 1024;
     P.NB = 2, P.NR = 2;
-    if (smem_layout(P, true).total > budget) {
+    if (smem_layout(P).total > budget) {
         delete t;
         return fail(ctx, PETB200_ERR_UNSUPPORTED, "g2bmm tile does not fit shared memory");
     }
@@ -2524,20 +2640,20 @@ int tc_g2bmm_create(petb200_ctx *ctx, int bs, int n, int m, int w, void **out) {
         grew = false;
         if (P.NB < kMaxNB) {
             P.NB++;
-            if (smem_layout(P, true).total <= budget)
+            if (smem_layout(P).total <= budget)
                 grew = true;
             else
                 P.NB--;
         }
         if (P.NR < kMaxNR) {
             P.NR++;
-            if (smem_layout(P, true).total <= budget)
+            if (smem_layout(P).total <= budget)
                 grew = true;
             else
                 P.NR--;
         }
     }
-    core.smem = smem_layout(P, true).total + 1024;
+    core.smem = smem_layout(P).total + 1024;
     core.Ktot = (long long)P.nchunks * P.ke;
     core.xd[0] = m, core.xd[1] = n, core.xd[2] = bs;
     std::vector<int> koff(P.ke, -1);
@@ -2546,9 +2662,7 @@ int tc_g2bmm_create(petb200_ctx *ctx, int bs, int n, int m, int w, void **out) {
         return fail(ctx, PETB200_ERR_NOMEM, "koff allocation failed");
     }
     cudaMemcpy(core.koff.p, koff.data(), koff.size() * 4, cudaMemcpyHostToDevice);
-    const int slots = std::max(1, ctx->sm_count / bs);
-    const int tiles_per_cta = (P.mtiles + slots - 1) / slots;
-    core.grid = dim3((unsigned)((P.mtiles + tiles_per_cta - 1) / tiles_per_cta), 1u, (unsigned)bs);
+    core.grid = dim3((unsigned)std::min(P.tiles, ctx->sm_count), 1u, 1u);
     core.y_elems = (long long)bs * n * (2 * w + 1);
     core.rows_b = bs * n;
     const size_t wbytes = (size_t)bs * n * core.Ktot * 4;
@@ -2573,8 +2687,8 @@ int tc_g2bmm_create(petb200_ctx *ctx, int bs, int n, int m, int w, void **out) {
 int tc_gbmml_create(petb200_ctx *ctx, int bs, int n, int m, int w, void **out) {
     if (ctx->cc_major != 10)
         return fail(ctx, PETB200_ERR_UNSUPPORTED, "tcgen05 kernels need compute capability 10.x");
-    if (m % 4 != 0 || m > 128 || w <= 0)
-        return fail(ctx, PETB200_ERR_UNSUPPORTED, "tensor-core gbmml needs m divisible by 4 and at most 128");
+    if (m % 4 != 0 || m > 128 || w < 3) // (w: see band_copy)
+        return fail(ctx, PETB200_ERR_UNSUPPORTED, "tensor-core gbmml needs m divisible by 4 and at most 128, and a width of 3 or more");
     auto *t = new TcMatmul();
     t->bs = bs, t->m = n, t->n = m, t->k = n, t->transB = 0;
     t->st[2] = (long long)n * m, t->st[3] = m; // v: batch stride, stride of a key row
@@ -2583,39 +2697,45 @@ int tc_gbmml_create(petb200_ctx *ctx, int bs, int n, int m, int w, void **out) {
     core.ctx = ctx;
     IgemmParams &P = core.P;
     memset(&P, 0, sizeof P);
-    core.a_tmem = true;
     P.a_kmajor = 1, P.ke = kStageK, P.m_rows = n, P.z_is_batch = 1, P.band_w = w;
     P.OD = P.OH = 1, P.OW = n, P.ohn = 1, P.own = n, P.Pw = n, P.units = 1, P.ipt = 1, P.tpi = (n + kTileM - 1) / kTileM;
     P.sd = P.sh = P.sw = 1;
     P.cpg = n, P.Fg = m, P.BN = m <= 32 ? 32 : (m <= 64 ? 64 : 128), P.ksplit = 1;
-    P.BC = P.ke, P.spc = 1, P.nchunks = (2 * w + kTileM + 3 + P.ke - 1) / P.ke; // K stages of one row tile's key window
-    P.RN = P.RD = 1, P.RH = kTileM, P.RW = kStageK, P.raw_bytes = 128; // no raw tiles
+    // a chunk is two K stages of a row tile's key window (whose start is rounded down to a multiple of 4)
+    P.BC = kBandKeys, P.spc = kBandStages, P.nchunks = (2 * w + kTileM + 3 + kBandKeys - 1) / kBandKeys;
+    P.RN = P.RD = 1, P.RH = kTileM, P.RW = kStageK, P.raw_bytes = kTileM * kBandPitch * 4;
+    P.band_words = (long long)bs * n * (2 * w + 1);
     P.ys_n = (long long)n * m, P.ys_f = 1, P.ys_p = m;
-    P.NA = 4, P.NB = 2, P.NR = 2;
-    P.mtiles = P.tpi;
+    P.NB = 2, P.NR = 2;
     const size_t budget = std::min<size_t>(ctx->smem_optin, 227 * 1024) - 1024;
+    if (smem_layout(P).total > budget) {
+        delete t;
+        return fail(ctx, PETB200_ERR_UNSUPPORTED, "gbmml tile does not fit shared memory");
+    }
     for (bool grew = true; grew;) {
         grew = false;
-        if (P.NB < kMaxNB) {
-            P.NB++;
-            if (smem_layout(P, true).total <= budget)
+        for (int *ring : {&P.NR, &P.NB}) {
+            if (*ring >= 4)
+                continue;
+            ++*ring;
+            if (smem_layout(P).total <= budget)
                 grew = true;
             else
-                P.NB--;
+                --*ring;
         }
     }
     choose_flush(core);
-    core.smem = smem_layout(P, true).total + 1024;
+    choose_grid(ctx, core, P.tpi, (m + P.BN - 1) / P.BN, bs, budget);
+    core.smem = smem_layout(P).total + 1024;
     core.Ktot = ((long long)n + P.ke - 1) / P.ke * P.ke; // the packed operand covers all keys; a tile reads its window of them
     core.xd[0] = kStageK, core.xd[1] = kTileM, core.xd[2] = 1; // (the activation map is not used: any valid extents)
     core.a_batch = kStageK * kTileM, core.a_row = kStageK;
-    std::vector<int> koff(P.ke, -1);
+    std::vector<int> koff(P.spc * P.ke, -1);
     if (core.koff.alloc(koff.size() * 4) != cudaSuccess) {
         delete t;
         return fail(ctx, PETB200_ERR_NOMEM, "koff allocation failed");
     }
     cudaMemcpy(core.koff.p, koff.data(), koff.size() * 4, cudaMemcpyHostToDevice);
-    core.grid = dim3((unsigned)P.tpi, (unsigned)((m + P.BN - 1) / P.BN), (unsigned)bs);
     core.y_elems = (long long)bs * n * m;
     core.rows_b = bs * m;
     const size_t wbytes = (size_t)bs * m * core.Ktot * 4;

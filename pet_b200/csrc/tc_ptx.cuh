@@ -55,16 +55,18 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
 __device__ unsigned long long g_mbar_wait_limit_ns = 2000000000ull;
 
 // Bounded wait: gives up after the limit above (or as soon as another thread of the CTA raised *abort), so a protocol
-// bug turns into an error status instead of a hung GPU.  Returns false on give-up.
+// bug turns into an error status instead of a hung GPU.  Returns false on give-up.  The spin loop is laid out away from the
+// caller's straight line (see the note on instruction fetch in igemm_tc.cu).
 __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
-    if (mbar_try_wait(bar, parity))
+    if (__builtin_expect(mbar_try_wait(bar, parity), 1))
         return true;
     if (*abort_flag)
         return false;
-    uint64_t t0 = globaltimer_ns();
+    const uint64_t t0 = globaltimer_ns();
     uint32_t spins = 0;
+#pragma unroll 1
     while (!mbar_try_wait(bar, parity)) {
-        if ((++spins & 0x3ff) == 0) {
+        if (__builtin_expect((++spins & 0x3ff) == 0, 0)) {
             if (*abort_flag)
                 return false;
             if (globaltimer_ns() - t0 > g_mbar_wait_limit_ns) {
@@ -74,6 +76,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
         }
     }
     return true;
+}
+
+// The same for a whole warp, which leaves with one answer: a lane may see its phase complete in the moment in which another sees
+// the abort flag, and the warp-wide tcgen05 instructions that follow need all of them.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag)) != 0;
 }
 
 // Barrier among a subset of the CTA's warps (id 1..15; id 0 is __syncthreads).
@@ -113,18 +121,21 @@ __device__ __forceinline__ float ld_dsmem_f32(uint32_t cluster_addr) {
     return v;
 }
 
-// ---- 4-byte asynchronous copies (for sources TMA cannot address) ---------------------------------------------------
-// Copies 4 bytes, or writes 4 zero bytes without reading the source when `valid` is false (the zeros are then tracked
-// by the same completion mechanism as the copies).
-__device__ __forceinline__ void cp_async_4_zfill(void *smem_dst, const void *gmem_src, bool valid) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src), "r"(valid ? 4 : 0)
-                 : "memory");
+// ---- 16-byte asynchronous copies (for sources TMA cannot address) ---------------------------------------------------
+__device__ __forceinline__ void cp_async_16(uint32_t smem_dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_dst), "l"(src) : "memory");
 }
 // The executing thread arrives on the barrier once all its earlier cp.async copies have completed; the arrival counts
 // against the barrier's expected count (noinc).
 __device__ __forceinline__ void cp_async_mbar_arrive_noinc(uint64_t *bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// ---- registers per thread of a warpgroup (all of its warps execute this; the shares of the block's groups must not add up to
+// more than the block was launched with) ------------------------------------------------------------------------------
+template <int N> __device__ __forceinline__ void reg_alloc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
+template <int N> __device__ __forceinline__ void reg_dealloc() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // ---- programmatic dependent launch ---------------------------------------------------------------------------------
 // launch_dependents: once every CTA of this grid has executed it (or exited), a following kernel launched with the
@@ -171,14 +182,7 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) { /
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// D[tmem] (+)= A[smem] * B[smem], TF32 inputs, fp32 accumulate; one thread issues.
-__device__ __forceinline__ void mma_tf32_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                 "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-                 ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-                 : "memory");
-}
-// D[tmem] (+)= A[tmem] * B[smem]
+// D[tmem] (+)= A[tmem] * B[smem], TF32 inputs, fp32 accumulate; one thread issues.
 __device__ __forceinline__ void mma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                  "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n\t}"
