@@ -274,7 +274,7 @@ __global__ void __launch_bounds__(256) k_rowmean(const float *__restrict__ x, fl
 }
 
 // Rows of at most 32 * NPL values: one warp per row keeps the row in registers, so the tensor is read once and written
-// once (8 bytes per element) and every exponential is evaluated once.  Same sums in the same order as k_softmax below.
+// once (8 bytes per element) and every exponential is evaluated once.
 template <int NPL>
 __global__ void __launch_bounds__(256) k_softmax_reg(const float *__restrict__ x, float *__restrict__ y, size_t rows, int cols) {
     pdl_prologue();
@@ -352,32 +352,10 @@ __global__ void __launch_bounds__(256) k_layernorm_reg(const float *__restrict__
     }
 }
 
-__global__ void __launch_bounds__(256) k_softmax(const float *__restrict__ x, float *__restrict__ y, size_t rows, int cols) {
-    pdl_prologue();
-    size_t warp = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) >> 5;
-    int lane = threadIdx.x & 31;
-    size_t nwarps = ((size_t)gridDim.x * blockDim.x) >> 5;
-    for (size_t r = warp; r < rows; r += nwarps) {
-        const float *xp = x + r * (size_t)cols;
-        float *yp = y + r * (size_t)cols;
-        float mx = -INFINITY;
-        for (int i = lane; i < cols; i += 32)
-            mx = fmaxf(mx, __ldg(xp + i));
-        mx = warp_max(mx);
-        float den = 0.f;
-        for (int i = lane; i < cols; i += 32)
-            den += expf(__ldg(xp + i) - mx);
-        den = warp_sum(den);
-        float inv = 1.f / den;
-        for (int i = lane; i < cols; i += 32)
-            yp[i] = expf(__ldg(xp + i) - mx) * inv;
-    }
-}
-
 // Softmax along an axis that is not the innermost one: x viewed as [outer, len, inner], normalised over `len`.  A 32 x 8
 // block owns 32 neighbouring `inner` positions of one `outer` index: threadIdx.x walks `inner` (every access of a warp is
 // one contiguous 128-byte piece of a row), the 8 values of threadIdx.y split `len`, and the maxima / sums of the 8 parts
-// meet in shared memory.  Per column the same arithmetic as k_softmax: max, sum of exp(x - max), scale.
+// meet in shared memory.  Per column the same arithmetic as for rows: max, sum of exp(x - max), scale.
 __global__ void __launch_bounds__(256) k_softmax_strided(const float *__restrict__ x, float *__restrict__ y, size_t outer, int len,
                                                          size_t inner) {
     pdl_prologue();
@@ -474,7 +452,43 @@ __device__ __forceinline__ float block_max(float v, float *red) {
     return t;
 }
 
-// One 256-thread block per row: used when there are too few rows to fill the GPU with one warp per row.
+// The same with one 256-thread block per row of at most 256 * NPL values: rows too long for a warp's registers, or too few rows to
+// fill the GPU with a warp each.  Bound by HBM: 8 bytes per element and the eight blocks of an SM keep about 64 KB of loads in
+// flight (10000 rows of 2001: 58.7 us = 2.7 TB/s when a warp walked its row three times).
+template <int NPL>
+__global__ void __launch_bounds__(256) k_softmax_block_reg(const float *__restrict__ x, float *__restrict__ y, size_t rows, int cols) {
+    pdl_prologue();
+    __shared__ float red[8];
+    for (size_t r = blockIdx.x; r < rows; r += gridDim.x) {
+        const float *xp = x + r * (size_t)cols;
+        float *yp = y + r * (size_t)cols;
+        float v[NPL];
+        float mx = -INFINITY;
+#pragma unroll
+        for (int i = 0; i < NPL; ++i) {
+            const int c = threadIdx.x + 256 * i;
+            v[i] = c < cols ? __ldg(xp + c) : -INFINITY;
+            mx = fmaxf(mx, v[i]);
+        }
+        mx = block_max(mx, red);
+        float den = 0.f;
+#pragma unroll
+        for (int i = 0; i < NPL; ++i) {
+            const int c = threadIdx.x + 256 * i;
+            v[i] = c < cols ? expf(v[i] - mx) : 0.f;
+            den += v[i];
+        }
+        const float inv = 1.f / block_sum(den, red);
+#pragma unroll
+        for (int i = 0; i < NPL; ++i) {
+            const int c = threadIdx.x + 256 * i;
+            if (c < cols)
+                yp[c] = v[i] * inv;
+        }
+    }
+}
+
+// Rows of more than 4096 values: three passes over the row, the second and third mostly out of the caches.
 __global__ void __launch_bounds__(256) k_softmax_block(const float *__restrict__ x, float *__restrict__ y, size_t rows, int cols) {
     pdl_prologue();
     __shared__ float red[8];
@@ -671,8 +685,17 @@ extern "C" int petb200_softmax_run(petb200_ctx *ctx, const float *x, float *y, s
         return fail(ctx, PETB200_ERR_INVALID, "softmax_run: bad arguments");
     if (!rows)
         return PETB200_OK;
-    if (cols >= 256 && rows <= (size_t)ctx->sm_count * 64) {
-        launch_pdl(k_softmax_block, (int)std::min<size_t>(rows, (size_t)ctx->sm_count * 8), 256, 0, (cudaStream_t)stream, x, y, rows, cols);
+    // A block per row for rows past a warp's registers, and where a warp per row would leave SMs without work (eight warps each).
+    if (cols > 1024 || (cols >= 256 && rows <= (size_t)ctx->sm_count * 8)) {
+        const int blocks = (int)std::min<size_t>(rows, (size_t)ctx->sm_count * 64);
+        if (cols <= 1024)
+            launch_pdl(k_softmax_block_reg<4>, blocks, 256, 0, (cudaStream_t)stream, x, y, rows, cols);
+        else if (cols <= 2048)
+            launch_pdl(k_softmax_block_reg<8>, blocks, 256, 0, (cudaStream_t)stream, x, y, rows, cols);
+        else if (cols <= 4096)
+            launch_pdl(k_softmax_block_reg<16>, blocks, 256, 0, (cudaStream_t)stream, x, y, rows, cols);
+        else
+            launch_pdl(k_softmax_block, blocks, 256, 0, (cudaStream_t)stream, x, y, rows, cols);
         return launched(ctx, "k_softmax_block");
     }
     const int grid = grid_for(ctx, rows, 8);
@@ -684,10 +707,8 @@ extern "C" int petb200_softmax_run(petb200_ctx *ctx, const float *x, float *y, s
         launch_pdl(k_softmax_reg<16>, grid, 256, 0, (cudaStream_t)stream, x, y, rows, cols);
     else if (cols <= 768)
         launch_pdl(k_softmax_reg<24>, grid, 256, 0, (cudaStream_t)stream, x, y, rows, cols);
-    else if (cols <= 1024)
-        launch_pdl(k_softmax_reg<32>, grid, 256, 0, (cudaStream_t)stream, x, y, rows, cols);
     else
-        launch_pdl(k_softmax, grid, 256, 0, (cudaStream_t)stream, x, y, rows, cols);
+        launch_pdl(k_softmax_reg<32>, grid, 256, 0, (cudaStream_t)stream, x, y, rows, cols);
     return launched(ctx, "k_softmax");
 }
 
