@@ -795,6 +795,7 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
     uint64_t *acc_ready = acc_full + 4; // a group of `fl` K stages has been accumulated: the main accumulator may be drained
     uint64_t *flushed = acc_full + 5;   // the four drain warps have drained it: the MMA warp may restart it
     uint64_t *acc_full1 = acc_full + 6; // persistent mode: the second accumulator region is complete
+    uint64_t *trash = acc_full + 9;     // takes the MMA thread's releases after it gave up
     uint64_t *acc_empty = acc_full + 7; // [2]: the drain warps have read accumulator region 0 / 1 out
 
     constexpr bool SPLIT = PASSES != kMathTf32x1; // hi/lo operands, two accumulators
@@ -832,6 +833,7 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
         ptx::mbar_init(acc_ready, 1);
         ptx::mbar_init(flushed, 4);
         ptx::mbar_init(acc_full1, 1);
+        ptx::mbar_init(trash, 1);
         ptx::mbar_init(acc_empty, 4);
         ptx::mbar_init(acc_empty + 1, 4);
         *abort_flag = 0;
@@ -1032,9 +1034,10 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
         // warps of an SM quarter share an instruction cache that the transform warps' unrolled code keeps flushing.  So: one
         // thread, ring positions as running values, the next stage's barriers polled before this stage's MMAs are issued,
         // and a plain stage that is one short straight line; everything rare (waits, group starts) sits outside it.
-        // A wait that gives up cuts the loops short (their bounds are running values), so that the common path has no test for
-        // it; nothing is issued or committed after it: releasing a filter slot whose bytes never came would let its producer
-        // arrive once more on a phase that expects no further arrival, which is a fault.
+        // A wait that gives up cuts the loops short (their bounds are running values) and sends the stage's releases to a barrier
+        // that nobody waits for, so that the common path has no test for it (one cost it 5 to 12 %).  The releases must not
+        // reach the filter slot: with bytes still missing from it, its producer would arrive once more on a phase that expects
+        // no further arrival, which is a fault.
         if (ptx::elect_one()) {
             const uint32_t idesc = BF ? ptx::idesc_bf16(kTileM, P.BN) : ptx::idesc_tf32(kTileM, P.BN);
             const uint32_t idesc_wide = BF ? ptx::idesc_bf16(kTileM, 2 * P.BN) : ptx::idesc_tf32(kTileM, 2 * P.BN);
@@ -1053,25 +1056,24 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
             uint32_t tmem_acc = tmem_base, tmem_small = tmem_base + BNu; // main and cross-term accumulators of the tile
             int tiles_left = ntl, stages_end = KS, left = 0; // tiles, end of the tile's K stages, stages left in the flush group
             bool ok = true;
-            auto give_up = [&]() {
-                ok = false;
-                tiles_left = stages_end = left = 0;
-            };
-            bool ready = false, next_ready = false; // the current / the next stage has been seen complete
             // Ring positions: slot, parity, and what they select.
             uint32_t sa = 0, sb = 0, pa = 0, pb = 0;
             uint64_t bhi = bdesc0;
+            uint64_t *release_a = a_empty, *release_b = b_empty;
+            auto give_up = [&]() {
+                ok = false;
+                tiles_left = stages_end = left = 0;
+                release_a = trash - sa, release_b = trash - sb;
+            };
+            bool ready = false, next_ready = false; // the current / the next stage has been seen complete
             auto wait_stage = [&]() {
                 if (__builtin_expect(!ready, 0)) {
                     const long long q0 = prof ? clock64() : 0;
-                    if (!ptx::mbar_wait(a_full + sa, pa, abort_flag) || !ptx::mbar_wait(b_full + sb, pb, abort_flag)) {
+                    if (!ptx::mbar_wait(a_full + sa, pa, abort_flag) || !ptx::mbar_wait(b_full + sb, pb, abort_flag))
                         give_up();
-                        return false;
-                    }
                     t_wa += prof ? clock64() - q0 : 0;
                 }
                 ptx::tc_fence_after();
-                return true;
             };
             struct Pos {
                 uint32_t sa, sb, pa, pb;
@@ -1085,8 +1087,8 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                 return n;
             };
             auto finish_stage = [&](const Pos &n) { // release the stage's slots, go on to the next
-                ptx::mma_commit(a_empty + sa);
-                ptx::mma_commit(b_empty + sb);
+                ptx::mma_commit(release_a + sa);
+                ptx::mma_commit(release_b + sb);
                 sa = n.sa, sb = n.sb, pa = n.pa, pb = n.pb;
                 bhi = bdesc0 + (uint64_t)(sb * 2u * b_half16);
                 ready = next_ready;
@@ -1095,8 +1097,7 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
             // accumulator after every MMA, a bias proportional to the accumulator's magnitude; keeping the small terms away
             // from the big sum removes most of those truncations from it.
             auto plain_stage = [&](uint32_t acc0) {
-                if (!wait_stage())
-                    return;
+                wait_stage();
                 const Pos n = next_pos();
                 // Is the next stage there?  Asked before this stage's MMAs and read after them: the answer travels while they
                 // are being issued.
@@ -1131,7 +1132,8 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
             // issued first, so the tensor pipe has work while the drain is in flight; if the stage after it is already there
             // (and belongs to the group), its eight as well.
             auto group_start = [&]() {
-                if (!wait_stage())
+                wait_stage();
+                if (!ok)
                     return;
                 const Pos n = next_pos();
                 cross_terms(sa, bhi);
@@ -1185,7 +1187,7 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
 #pragma unroll 1
                     for (; left > 0; --left, acc0 = 1u)
                         plain_stage(acc0);
-                    if (PP != kNarrow && g0 + FLm < stages_end) // fires once every MMA of the group has completed
+                    if (PP != kNarrow && g0 + FLm < stages_end) // (0 after a give-up) fires once every MMA of the group has completed
                         ptx::mma_commit(acc_ready);
                 }
                 if (ok)
