@@ -20,7 +20,8 @@ void tc_matmul_set_prof(void *h, long long *p);
 const char *tc_conv_variant(void *h);
 int tc_matmul_create(petb200_ctx *ctx, int bs, int m, int n, int k, int transA, int transB, int has_bias, int act, int passes,
                      const long long *strides, void **out, size_t *dev_bytes);
-int tc_matmul_native_a(void *h);
+long long tc_matmul_a_copy(void *h);
+int tc_matmul_prepare(void *h, const float *b, const float *a, float *a_copy, cudaStream_t s);
 void tc_matmul_destroy(void *h);
 int tc_matmul_pack_b(void *h, const float *b, cudaStream_t s);
 int tc_matmul_run(void *h, const float *a_t, const float *bias, const float *res, float *cmat, cudaStream_t s);
@@ -118,31 +119,6 @@ __global__ void __launch_bounds__(256) k_repitch(const float *__restrict__ x, fl
         const int col = (int)(i % wp);
         const long long row = i / wp;
         y[i] = col < w ? __ldg(x + row * w + col) : 0.f;
-    }
-}
-
-// [b][m][k] -> [b][k][mp]  (row pitch mp >= m, padding columns zero)
-__global__ void __launch_bounds__(256) k_transpose_a(const float *__restrict__ a, float *__restrict__ at, int bs, int m, int k, int mp) {
-    pdl_prologue();
-    __shared__ float tile[32][33];
-    const int tiles_k = (k + 31) / 32, tiles_m = (mp + 31) / 32;
-    const long long ntiles = (long long)bs * tiles_k * tiles_m;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        const int tk = (int)(t % tiles_k);
-        const int tm = (int)((t / tiles_k) % tiles_m);
-        const int bb = (int)(t / ((long long)tiles_k * tiles_m));
-        for (int r = ty; r < 32; r += 8) {
-            const int mm = tm * 32 + r, kk = tk * 32 + tx;
-            tile[r][tx] = (mm < m && kk < k) ? __ldg(a + ((long long)bb * m + mm) * k + kk) : 0.f;
-        }
-        __syncthreads();
-        for (int r = ty; r < 32; r += 8) {
-            const int kk = tk * 32 + r, mm = tm * 32 + tx;
-            if (kk < k && mm < mp)
-                at[((long long)bb * k + kk) * mp + mm] = tile[tx][r];
-        }
-        __syncthreads();
     }
 }
 
@@ -326,9 +302,8 @@ struct MatmulPlan : petb200_plan {
     int transA, transB, bs, m, n, k, has_bias, act;
     int algo = 0;
     void *tc = nullptr;
-    DevBuf at; // A re-laid as [b][k][m] when the caller's A is [b][m][k]
+    DevBuf at; // copy of A with rows that TMA can address, where the caller's are not
     const float *b_weight = nullptr; // set by matmul_set_weights
-    bool native_a = false;           // the kernel reads row-major A directly
     bool gemv = false;               // m <= 8: matrix-vector kernel
     bool strided = false;            // operands/result addressed through st[] (tensor-core kernel only)
     long long st[6] = {0, 0, 0, 0, 0, 0};
@@ -378,9 +353,8 @@ int make_matmul_plan(petb200_ctx *ctx, int transA, int transB, int b, int m, int
             pl->algo = PETB200_ALGO_TC_3XTF32;
             pl->kernel = tc_passes_for(algo) == 1 ? "tc_1xtf32_ts" : (tc_passes_for(algo) == 16 ? "tc_bf16x3_ts" : "tc_3xtf32_ts");
             pl->device_bytes = bytes;
-            pl->native_a = tc_matmul_native_a(pl->tc) != 0;
-            if (!pl->native_a && (!pl->transA || m % 4 != 0)) {
-                if (pl->at.alloc((size_t)b * ((m + 3) / 4 * 4) * k * 4) != cudaSuccess) {
+            if (const long long words = tc_matmul_a_copy(pl->tc)) {
+                if (pl->at.alloc((size_t)words * 4) != cudaSuccess) {
                     delete pl;
                     return fail(ctx, PETB200_ERR_NOMEM, "A re-layout scratch allocation failed");
                 }
@@ -418,28 +392,10 @@ int matmul_run(petb200_plan *plan, const float *a, const float *b, const float *
     if (pl->has_bias && !bias)
         return fail(ctx, PETB200_ERR_INVALID, "matmul run: plan was made with a bias but none was passed");
     if (pl->algo == PETB200_ALGO_TC_3XTF32) {
-        int rc = (b == pl->b_weight) ? PETB200_OK : tc_matmul_pack_b(pl->tc, b, s);
+        const float *at = pl->at.p ? (const float *)pl->at.p : a;
+        int rc = tc_matmul_prepare(pl->tc, b == pl->b_weight ? nullptr : b, pl->at.p ? a : nullptr, (float *)pl->at.p, s);
         if (rc)
             return rc;
-        const float *at = a;
-        const int mp = (pl->m + 3) / 4 * 4;
-        if (pl->native_a) {
-            // nothing to do: the kernel's K-major mode consumes A as it is
-        } else if (!pl->transA) {
-            long long tiles = (long long)pl->bs * ((pl->k + 31) / 32) * ((mp + 31) / 32);
-            launch_pdl(k_transpose_a, (int)std::min<long long>(tiles, (long long)ctx->sm_count * 8), 256, 0, s, a, (float *)pl->at.p, pl->bs, pl->m, pl->k, mp);
-            rc = launched(ctx, "k_transpose_a");
-            if (rc)
-                return rc;
-            at = (const float *)pl->at.p;
-        } else if (mp != pl->m) {
-            long long rows = (long long)pl->bs * pl->k;
-            launch_pdl(k_repitch, grid_for(ctx, rows * mp, 256), 256, 0, s, a, (float *)pl->at.p, rows, pl->m, mp);
-            rc = launched(ctx, "k_repitch");
-            if (rc)
-                return rc;
-            at = (const float *)pl->at.p;
-        }
         return tc_matmul_run(pl->tc, at, pl->has_bias ? bias : nullptr, res, c, s);
     }
     if (pl->gemv)

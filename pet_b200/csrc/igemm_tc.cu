@@ -152,10 +152,11 @@ __host__ __device__ inline SmemLayout smem_layout(const IgemmParams &P) {
     // own region: peers push into it while this CTA may still be in its main loop.
     L.split_off = (o + 127) & ~127u;
     o = L.split_off + (P.ksplit > 1 ? 512u * (uint32_t)P.BN + 1024u : 0u); // + each tile row's offset in y (-1: none)
-    // persistent mode: the drain warps' 32x32 transposition blocks need their own room (the B ring is never idle)
+    // Transposition blocks of the warps that store.  Persistent mode: the drain warps' own room (the B ring is never idle).
+    // Otherwise the eight transform warps use the B ring, unless it is too small (or the sums go through the cluster).
+    const bool in_ring = P.ksplit > 1 || (uint32_t)P.NB * 2 * (uint32_t)P.BN * 128 >= 8u * 4096u;
     L.stage_off = (o + 127) & ~127u;
-    o = L.stage_off + (P.pp ? 4u * 4096u : 0u);
-    L.bar_off = (o + 15) & ~15u;
+    L.bar_off = L.stage_off + (P.pp ? 4u * 4096u : (in_ring ? 0u : 8u * 4096u));
     L.total = L.bar_off + 384;
     return L;
 }
@@ -175,161 +176,6 @@ template <int ACT> __device__ __forceinline__ float act_fn(float v) {
     if (ACT == PETB200_ACT_GELU)
         return 0.5f * v * (1.f + erff(v * 0.70710678118654752440f));
     return v;
-}
-
-// Split-K, COLS (< 32) columns per CTA: the 32 columns in r[] belong to 32 / COLS consecutive CTAs of the cluster, starting
-// with `owner0`; each group goes to its owner's landing area [this rank][column][pixel] (this CTA's own group by a plain
-// shared-memory store).
-template <int COLS>
-__device__ __forceinline__ void push_groups(const uint32_t (&r)[32], uint32_t split_addr, int owner0, int me) {
-#pragma unroll
-    for (int g = 0; g < 32 / COLS; ++g) {
-        const int owner = owner0 + g;
-        if (owner == me) {
-#pragma unroll
-            for (int j = 0; j < COLS; ++j)
-                ptx::st_shared_f32(split_addr + (uint32_t)(j * kTileM) * 4u, __uint_as_float(r[g * COLS + j]));
-        } else {
-            const uint32_t remote = ptx::map_to_cta(split_addr, (uint32_t)owner);
-#pragma unroll
-            for (int j = 0; j < COLS; ++j)
-                ptx::st_dsmem_f32(remote + (uint32_t)(j * kTileM) * 4u, __uint_as_float(r[g * COLS + j]));
-        }
-    }
-}
-
-// TMEM accumulator rows -> (+bias, activation) -> global.  `yp` already points at this thread's pixel and the first
-// filter of the group; column j of the tile is filter f_tile0 + j.  The activation is a template parameter so that
-// the common no-activation case carries none of the transcendental code.
-template <int ACT, int PASSES>
-__device__ __forceinline__ void epilogue_store(uint32_t tacc, uint32_t tcross, int BN, int f_tile0, int Fg, bool valid, const float *bias,
-                                               const float *rp /*residual at this pixel, or null*/, float *yp, long long ys_f, bool vec_ok, float *stage, int nvalid_warp, float *ybase_warp,
-                                               const float *rbase_warp /*residual at the warp's first pixel, or null*/, int col0, int col1, uint32_t split_addr /*split-K: shared address of [this rank][0][this pixel]*/,
-                                               int split_shift /*log2(columns per CTA)*/) {
-    uint32_t r[32], nx[32], sm[32];
-    if (col0 >= col1)
-        return;
-    ptx::tmem_ld_32x32(tacc + (uint32_t)col0, nx);
-    if (PASSES != kMathTf32x1)
-        ptx::tmem_ld_32x32(tcross + (uint32_t)col0, sm);
-    for (int cc = col0; cc < col1; cc += 32) {
-        ptx::tmem_ld_wait();
-#pragma unroll
-        for (int j = 0; j < 32; ++j) // hi*hi sum + (lo*hi + hi*lo) sum, one rounded fp32 add
-            r[j] = PASSES != kMathTf32x1 ? __float_as_uint(__uint_as_float(nx[j]) + __uint_as_float(sm[j])) : nx[j];
-        if (cc + 32 < col1) { // in flight while this chunk is stored
-            ptx::tmem_ld_32x32(tacc + (uint32_t)(cc + 32), nx);
-            if (PASSES != kMathTf32x1)
-                ptx::tmem_ld_32x32(tcross + (uint32_t)(cc + 32), sm);
-        }
-        if (split_addr != 0u) {
-            // Split-K: column c of the tile is summed by CTA c / cols of the cluster.  Push this CTA's partial sum into
-            // that CTA's shared memory, slot [this rank][c % cols][pixel] (consecutive lanes = consecutive words).
-            if (split_shift >= 5) {
-                // at least 32 columns per CTA: the whole block has one owner — one address translation, and the block this
-                // CTA owns itself stays out of the cluster network
-                const int owner = cc >> split_shift, lc0 = cc & ((1 << split_shift) - 1);
-                const uint32_t local = split_addr + (uint32_t)(lc0 * kTileM) * 4u;
-                if (owner == (int)ptx::cluster_ctarank()) {
-#pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        ptx::st_shared_f32(local + (uint32_t)(j * kTileM) * 4u, __uint_as_float(r[j]));
-                } else {
-                    const uint32_t remote = ptx::map_to_cta(local, (uint32_t)owner);
-#pragma unroll
-                    for (int j = 0; j < 32; ++j)
-                        ptx::st_dsmem_f32(remote + (uint32_t)(j * kTileM) * 4u, __uint_as_float(r[j]));
-                }
-                continue;
-            }
-            if (split_shift == 4 || split_shift == 3) { // 16 or 8 columns per CTA: one translation per owner, not per column
-                const int me = (int)ptx::cluster_ctarank(), owner0 = cc >> split_shift;
-                if (split_shift == 4)
-                    push_groups<16>(r, split_addr, owner0, me);
-                else
-                    push_groups<8>(r, split_addr, owner0, me);
-                continue;
-            }
-#pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                const int col = cc + j, owner = col >> split_shift, lc = col & ((1 << split_shift) - 1);
-                ptx::st_dsmem_f32(ptx::map_to_cta(split_addr + (uint32_t)(lc * kTileM) * 4u, (uint32_t)owner), __uint_as_float(r[j]));
-            }
-            continue;
-        }
-        if (stage == nullptr && !valid)
-            continue;
-        const int f0 = f_tile0 + cc;
-        // bias / residual / activation: each behind ONE test per block (a test per column costs more than the sums)
-        if (bias != nullptr) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-                if (f0 + j < Fg)
-                    r[j] = __float_as_uint(__uint_as_float(r[j]) + __ldg(bias + f0 + j));
-        }
-        if (rp != nullptr && stage == nullptr) { // (only valid rows get here; the staged path adds the residual 16 bytes at a time)
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-                if (f0 + j < Fg)
-                    r[j] = __float_as_uint(__uint_as_float(r[j]) + __ldg(rp + (long long)(f0 + j) * ys_f));
-        }
-        if (ACT != PETB200_ACT_NONE && (stage == nullptr || rbase_warp == nullptr)) {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-                r[j] = __float_as_uint(act_fn<ACT>(__uint_as_float(r[j])));
-        }
-        if (stage != nullptr) {
-            // NCHW output, the warp's 32 pixels contiguous in memory: transpose the 32x32 block through shared memory so
-            // that every lane stores 16 bytes (4 pixels of one filter) instead of 4 — a quarter of the store instructions.
-            const int lane = threadIdx.x & 31;
-            __syncwarp();
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-                stage[j * 32 + lane] = __uint_as_float(r[j]);
-            __syncwarp();
-            const int px = (lane & 7) * 4, cq = lane >> 3;
-            const long long off = (long long)(f0 + cq) * ys_f + px; // from the warp's first pixel: filter f0 + cq, 4 filters apart per step
-            float *dst = ybase_warp + off;
-            const float *rsd = rbase_warp != nullptr ? rbase_warp + off : nullptr;
-            const float *src = stage + cq * 32 + px;
-            const int fmax = Fg - f0 - cq; // filters left from this lane's first one
-#pragma unroll
-            for (int i = 0; i < 8; ++i, dst += 4 * ys_f, src += 128) {
-                if (4 * i < fmax) {
-                    float4 v = *reinterpret_cast<const float4 *>(src);
-                    if (rsd != nullptr) { // y = act(sum + bias + residual): the residual's four pixels sit where y's will
-                        float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
-                        const float *rs = rsd + (long long)(4 * i) * ys_f;
-                        if (px + 3 < nvalid_warp) {
-                            q = __ldg(reinterpret_cast<const float4 *>(rs));
-                        } else {
-                            if (px < nvalid_warp) q.x = __ldg(rs);
-                            if (px + 1 < nvalid_warp) q.y = __ldg(rs + 1);
-                            if (px + 2 < nvalid_warp) q.z = __ldg(rs + 2);
-                        }
-                        v.x = act_fn<ACT>(v.x + q.x), v.y = act_fn<ACT>(v.y + q.y), v.z = act_fn<ACT>(v.z + q.z), v.w = act_fn<ACT>(v.w + q.w);
-                    }
-                    if (px + 3 < nvalid_warp) {
-                        *reinterpret_cast<float4 *>(dst) = v;
-                    } else {
-                        if (px < nvalid_warp) dst[0] = v.x;
-                        if (px + 1 < nvalid_warp) dst[1] = v.y;
-                        if (px + 2 < nvalid_warp) dst[2] = v.z;
-                    }
-                }
-            }
-        } else if (vec_ok) {
-#pragma unroll
-            for (int j = 0; j < 32; j += 4)
-                if (f0 + j < Fg)
-                    *reinterpret_cast<uint4 *>(yp + f0 + j) = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-                if (f0 + j < Fg)
-                    yp[(long long)(f0 + j) * ys_f] = __uint_as_float(r[j]);
-        }
-    }
 }
 
 // Banded product: the tile holds rows [128*bx, +128) x keys [128*bx - w + col_base, + BN) of q . k^T.  Entry (row pr, column c)
@@ -608,35 +454,25 @@ __device__ __forceinline__ void drain_add(float (&racc)[128], uint32_t tmain, ui
     }
 }
 
-__device__ __forceinline__ void act4(float4 &v, int act) {
-    if (act == PETB200_ACT_NONE)
-        return;
-    if (act == PETB200_ACT_RELU) {
-        v.x = fmaxf(v.x, 0.f), v.y = fmaxf(v.y, 0.f), v.z = fmaxf(v.z, 0.f), v.w = fmaxf(v.w, 0.f);
-        return;
-    }
-    v.x = apply_act(v.x, act), v.y = apply_act(v.y, act), v.z = apply_act(v.z, act), v.w = apply_act(v.w, act);
-}
-
-// Persistent mode: one 32-column block of a warp's 32 tile rows, sums in r (thread = row), to y through the warp's 4 KB block of
-// shared memory, so that every store instruction writes whole 16-byte pieces of consecutive addresses.
-//   kStorePixels  y's pixels are contiguous (NCHW): a lane stores four pixels of one filter;
-//   kStoreFilters y's filters are contiguous (row-major matmul, channels last): a lane stores four filters of one row;
-//   kStoreAny     anything else: a thread stores its own row, one element at a time.
-// The drain warps store a tile while the tensor core works on the next, which at 64 filters and few K stages lasts only two to
-// four thousand cycles, and a taken branch costs them 70 to 250 (see the MMA issuer): the common activations go out in
-// straight-line code, eight predicated loads and stores in flight; bias, residual and activation are applied on the way out,
-// once per 16 bytes.  (As a loop with tests per store a tile of 16 valid pixels took 15000 cycles.)
-enum { kStorePixels = 0, kStoreFilters = 1, kStoreAny = 2 };
+// One 32-column block of a warp's 32 tile rows, sums in r (thread = row), to y, through the warp's 4 KB block of shared memory where
+// that makes the stores coalesced:
+//   kStorePixels  pixels contiguous in y (NCHW), 16-byte aligned: a lane stores four pixels of one filter;
+//   kStoreFilters filters contiguous in y (row-major matmul, channels last), aligned: a lane stores four filters of one row;
+//   kStoreRows    the same off the 16-byte grid: a store instruction writes 32 filters of one row;
+//   kStoreAny     anything else: every thread stores its own row (for NCHW off the grid that is 32 pixels of one filter).
+// Straight-line code with predicated loads and stores: a tile's successor lasts only two to four thousand cycles at 64 filters,
+// and a taken branch costs 70 to 250 of them (see the MMA issuer; as a loop with tests per store a tile took 15000).  For the
+// same reason the long activations are a loop of their own over the block in shared memory, with bias and residual.
+enum { kStorePixels = 0, kStoreFilters = 1, kStoreRows = 2, kStoreAny = 3 };
 struct StoreJob {
     float *y;                // filter 0 of the group
     const float *bias, *res; // the same, or null
     long long ys_f, y_off, y_off0; // this row, the warp's first row
-    int mode, Fg, act, nvalid, lane;
+    int Fg, act, nvalid, lane;
     bool valid;
 };
 template <bool RES>
-__device__ __forceinline__ void store_pixels(const StoreJob &J, const float *stage, int f0) { // four pixels that are all valid per lane
+__device__ __forceinline__ void store_pixels(const StoreJob &J, const float *bias, const float *stage, int f0) { // four pixels that are all valid per lane
     const int px = (J.lane & 7) * 4, cq = J.lane >> 3, fmax = px + 4 <= J.nvalid ? J.Fg - f0 - cq : 0; // filters left from this lane's first one
     const long long off = J.y_off0 + (long long)(f0 + cq) * J.ys_f + px, step = 4 * J.ys_f;
     float4 v[8];
@@ -649,12 +485,12 @@ __device__ __forceinline__ void store_pixels(const StoreJob &J, const float *sta
     float b[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i)
-        b[i] = J.bias != nullptr && 4 * i < fmax ? __ldg(J.bias + f0 + cq + 4 * i) : 0.f;
+        b[i] = bias != nullptr && 4 * i < fmax ? __ldg(bias + f0 + cq + 4 * i) : 0.f;
     float *dst = J.y + off;
 #pragma unroll
     for (int i = 0; i < 8; ++i, dst += step) {
         float4 q = *reinterpret_cast<const float4 *>(stage + (cq + 4 * i) * 32 + px);
-        if (J.bias != nullptr)
+        if (bias != nullptr)
             q.x += b[i], q.y += b[i], q.z += b[i], q.w += b[i];
         if (RES) // y = act(sum + bias + residual): the residual's four pixels sit where y's will
             q.x += v[i].x, q.y += v[i].y, q.z += v[i].z, q.w += v[i].w;
@@ -664,107 +500,151 @@ __device__ __forceinline__ void store_pixels(const StoreJob &J, const float *sta
             *reinterpret_cast<float4 *>(dst) = q;
     }
 }
-__device__ __forceinline__ void store_block(const StoreJob &J, const float *r /*32 sums*/, float *stage, int f0) {
+// kStoreFilters / kStoreRows / kStoreAny; the block (filters, rows) lies in `stage`, for kStoreAny in r.  RES: with a residual (a test
+// per store would be a branch per store).
+template <bool RES>
+__device__ __forceinline__ void store_filters(const StoreJob &J, const float *bias, const float *stage, int f0) {
+    const int lane = J.lane, c = lane & 7, f = f0 + 4 * c;
+    const bool live = f < J.Fg, relu = J.act == PETB200_ACT_RELU; // (Fg % 4 == 0 in this mode)
+    float4 bv = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (bias != nullptr && live)
+        bv = make_float4(__ldg(bias + f), __ldg(bias + f + 1), __ldg(bias + f + 2), __ldg(bias + f + 3));
+    const long long yo = J.valid ? J.y_off : -1;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int row = 4 * i + (lane >> 3);
+        const long long off = __shfl_sync(0xffffffffu, yo, row);
+        const bool go = off >= 0 && live;
+        float4 v = *reinterpret_cast<const float4 *>(stage + row * 32 + ((c ^ (row & 7)) << 2));
+        v.x += bv.x, v.y += bv.y, v.z += bv.z, v.w += bv.w;
+        if (RES) {
+            const float4 q = go ? __ldg(reinterpret_cast<const float4 *>(J.res + off + f)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v.x += q.x, v.y += q.y, v.z += q.z, v.w += q.w;
+        }
+        if (relu)
+            v.x = fmaxf(v.x, 0.f), v.y = fmaxf(v.y, 0.f), v.z = fmaxf(v.z, 0.f), v.w = fmaxf(v.w, 0.f);
+        if (go)
+            *reinterpret_cast<float4 *>(J.y + off + f) = v;
+    }
+}
+template <bool RES>
+__device__ __forceinline__ void store_rows(const StoreJob &J, const float *bias, const float *stage, int f0) {
+    const int lane = J.lane, f = f0 + lane;
+    const bool live = f < J.Fg, relu = J.act == PETB200_ACT_RELU;
+    const float bv = bias != nullptr && live ? __ldg(bias + f) : 0.f;
+    const long long yo = J.valid ? J.y_off : -1;
+#pragma unroll
+    for (int row = 0; row < 32; ++row) {
+        const long long off = __shfl_sync(0xffffffffu, yo, row);
+        const bool go = off >= 0 && live;
+        float v = stage[row * 32 + (lane ^ row)] + bv;
+        if (RES)
+            v += go ? __ldg(J.res + off + f) : 0.f;
+        v = relu ? fmaxf(v, 0.f) : v;
+        if (go)
+            J.y[off + f] = v;
+    }
+}
+template <bool RES>
+__device__ __forceinline__ void store_any(const StoreJob &J, const float *bias, const float *r, int f0) {
+    const int nf = J.valid ? J.Fg - f0 : 0; // filters of this thread's row
+    const bool relu = J.act == PETB200_ACT_RELU;
+    const float bv = bias != nullptr && f0 + J.lane < J.Fg ? __ldg(bias + f0 + J.lane) : 0.f; // lane j holds filter j's
+    float *dst = J.y + J.y_off + (long long)f0 * J.ys_f;
+    const float *rs = RES ? J.res + J.y_off + (long long)f0 * J.ys_f : nullptr;
+#pragma unroll
+    for (int j = 0; j < 32; ++j, dst += J.ys_f) {
+        float v = r[j] + __shfl_sync(0xffffffffu, bv, j);
+        if (RES)
+            v += j < nf ? __ldg(rs + (long long)j * J.ys_f) : 0.f;
+        if (j < nf)
+            *dst = relu ? fmaxf(v, 0.f) : v;
+    }
+}
+// This thread's row through one of the long activations, four filters at a time, with bias and residual.
+__device__ __forceinline__ void activate_block(const StoreJob &J, float *r, float *stage, int f0) {
     const int lane = J.lane;
-    if (J.mode == kStorePixels && J.nvalid == 0)
-        return;
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+        stage[j * 32 + lane] = r[j];
+    const float *rp = J.res != nullptr && J.valid ? J.res + J.y_off + (long long)f0 * J.ys_f : nullptr;
+#pragma unroll 1
+    for (int j = 0; j < 32 && f0 + j < J.Fg; j += 4) {
+        float v[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            v[i] = stage[(j + i) * 32 + lane];
+            if (f0 + j + i < J.Fg) {
+                if (J.bias != nullptr)
+                    v[i] += __ldg(J.bias + f0 + j + i);
+                if (rp != nullptr)
+                    v[i] += __ldg(rp + (long long)(j + i) * J.ys_f);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            stage[(j + i) * 32 + lane] = apply_act(v[i], J.act);
+    }
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+        r[j] = stage[j * 32 + lane];
+    __syncwarp();
+}
+template <int MODE, bool RES>
+__device__ __forceinline__ void store_block(const StoreJob &J, float *r /*32 sums*/, float *stage, int f0) {
+    const int lane = J.lane;
     __syncwarp(); // the previous block has been read
-    if (J.mode == kStoreFilters) {
+    const float *bias = J.bias;
+    if (__builtin_expect(J.act > PETB200_ACT_RELU, 0)) {
+        activate_block(J, r, stage, f0);
+        bias = nullptr;
+        if (RES) { // the residual has been added
+            StoreJob R = J;
+            R.bias = R.res = nullptr, R.act = PETB200_ACT_NONE;
+            store_block<MODE, false>(R, r, stage, f0);
+            return;
+        }
+    }
+    if (MODE == kStorePixels) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+            stage[j * 32 + lane] = r[j];
+        __syncwarp();
+        store_pixels<RES>(J, bias, stage, f0);
+        if (__builtin_expect((J.nvalid & 3) != 0, 0)) { // the last one to three pixels of a ragged window are left
+            StoreJob R = J;
+            R.valid = J.valid && lane >= (J.nvalid & ~3);
+            store_any<RES>(R, bias, r, f0);
+        }
+    } else if (MODE == kStoreFilters) {
         // row r of the block at [r][32], 16-byte chunk c at c ^ (r & 7): conflict-free both ways
 #pragma unroll
         for (int c = 0; c < 8; ++c)
             *reinterpret_cast<float4 *>(stage + lane * 32 + ((c ^ (lane & 7)) << 2)) = make_float4(r[4 * c], r[4 * c + 1], r[4 * c + 2], r[4 * c + 3]);
         __syncwarp();
-        const int c = lane & 7, f = f0 + 4 * c;
-        const bool live = f < J.Fg; // (Fg % 4 == 0 in this mode)
-        float4 bv = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (J.bias != nullptr && live)
-            bv = make_float4(__ldg(J.bias + f), __ldg(J.bias + f + 1), __ldg(J.bias + f + 2), __ldg(J.bias + f + 3));
-        const long long yo = J.valid ? J.y_off : -1;
-        if (J.act <= PETB200_ACT_RELU) {
+        store_filters<RES>(J, bias, stage, f0);
+    } else if (MODE == kStoreRows) { // word c of row r at c ^ r
 #pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const int row = 4 * i + (lane >> 3);
-                const long long off = __shfl_sync(0xffffffffu, yo, row);
-                const bool go = off >= 0 && live;
-                float4 v = *reinterpret_cast<const float4 *>(stage + row * 32 + ((c ^ (row & 7)) << 2));
-                if (J.bias != nullptr)
-                    v.x += bv.x, v.y += bv.y, v.z += bv.z, v.w += bv.w;
-                if (J.res != nullptr && go) {
-                    const float4 q = __ldg(reinterpret_cast<const float4 *>(J.res + off + f));
-                    v.x += q.x, v.y += q.y, v.z += q.z, v.w += q.w;
-                }
-                if (J.act == PETB200_ACT_RELU)
-                    v.x = fmaxf(v.x, 0.f), v.y = fmaxf(v.y, 0.f), v.z = fmaxf(v.z, 0.f), v.w = fmaxf(v.w, 0.f);
-                if (go)
-                    *reinterpret_cast<float4 *>(J.y + off + f) = v;
-            }
-            return;
-        }
-#pragma unroll 1
-        for (int i = 0; i < 8; ++i) {
-            const int row = 4 * i + (lane >> 3);
-            const long long off = __shfl_sync(0xffffffffu, yo, row);
-            if (off >= 0 && live) {
-                float4 v = *reinterpret_cast<const float4 *>(stage + row * 32 + ((c ^ (row & 7)) << 2));
-                if (J.bias != nullptr)
-                    v.x += bv.x, v.y += bv.y, v.z += bv.z, v.w += bv.w;
-                if (J.res != nullptr) {
-                    const float4 q = __ldg(reinterpret_cast<const float4 *>(J.res + off + f));
-                    v.x += q.x, v.y += q.y, v.z += q.z, v.w += q.w;
-                }
-                act4(v, J.act);
-                *reinterpret_cast<float4 *>(J.y + off + f) = v;
-            }
-        }
-        return;
+        for (int j = 0; j < 32; ++j)
+            stage[lane * 32 + (j ^ lane)] = r[j];
+        __syncwarp();
+        store_rows<RES>(J, bias, stage, f0);
+    } else {
+        store_any<RES>(J, bias, r, f0);
     }
-#pragma unroll
-    for (int j = 0; j < 32; ++j)
-        stage[j * 32 + lane] = r[j];
-    __syncwarp();
-    if (J.mode == kStorePixels && J.act <= PETB200_ACT_RELU) {
-        if (J.res != nullptr)
-            store_pixels<true>(J, stage, f0);
-        else
-            store_pixels<false>(J, stage, f0);
-        if ((J.nvalid & 3) == 0 || lane < (J.nvalid & ~3)) // (only the last one to three pixels of a ragged window are left)
-            return;
-    }
-    if (J.mode == kStorePixels && J.act > PETB200_ACT_RELU) {
-        const int px = (lane & 7) * 4, cq = lane >> 3;
-        const int fmax = px + 4 <= J.nvalid ? J.Fg - f0 - cq : 0;
-        const long long off = J.y_off0 + (long long)(f0 + cq) * J.ys_f + px;
-#pragma unroll 1
-        for (int i = 0; 4 * i < fmax && i < 8; ++i) {
-            const long long o = off + (long long)(4 * i) * J.ys_f;
-            float4 v = *reinterpret_cast<const float4 *>(stage + (cq + 4 * i) * 32 + px);
-            if (J.bias != nullptr) {
-                const float bf = __ldg(J.bias + f0 + cq + 4 * i);
-                v.x += bf, v.y += bf, v.z += bf, v.w += bf;
-            }
-            if (J.res != nullptr) {
-                const float4 q = __ldg(reinterpret_cast<const float4 *>(J.res + o));
-                v.x += q.x, v.y += q.y, v.z += q.z, v.w += q.w;
-            }
-            act4(v, J.act);
-            *reinterpret_cast<float4 *>(J.y + o) = v;
-        }
-        if ((J.nvalid & 3) == 0 || lane < (J.nvalid & ~3))
-            return;
-    }
-    if (J.valid) {
-#pragma unroll 1
-        for (int j = 0; j < 32 && f0 + j < J.Fg; ++j) { // one element at a time: this lane's own row
-            float v = stage[j * 32 + lane];
-            const long long o = J.y_off + (long long)(f0 + j) * J.ys_f;
-            if (J.bias != nullptr)
-                v += __ldg(J.bias + f0 + j);
-            if (J.res != nullptr)
-                v += __ldg(J.res + o);
-            J.y[o] = apply_act(v, J.act);
-        }
-    }
+}
+// f(mode, with residual) as compile-time constants: the loops around store_block are instantiated per way of storing.
+template <typename F> __device__ __forceinline__ void with_store_mode(int mode, bool res, F &&f) {
+    const std::integral_constant<bool, true> yes;
+    const std::integral_constant<bool, false> no;
+    if (mode == kStorePixels)
+        res ? f(std::integral_constant<int, kStorePixels>(), yes) : f(std::integral_constant<int, kStorePixels>(), no);
+    else if (mode == kStoreFilters)
+        res ? f(std::integral_constant<int, kStoreFilters>(), yes) : f(std::integral_constant<int, kStoreFilters>(), no);
+    else if (mode == kStoreRows)
+        res ? f(std::integral_constant<int, kStoreRows>(), yes) : f(std::integral_constant<int, kStoreRows>(), no);
+    else
+        res ? f(std::integral_constant<int, kStoreAny>(), yes) : f(std::integral_constant<int, kStoreAny>(), no);
 }
 
 // BAND: 0 ordinary operands; 1 G2BMM (banded epilogue, key windows per tile; persistent row-major mode only); 2 GBMML (A operand
@@ -946,6 +826,11 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
         return P.ys_p == 1 && P.ipt == 1 && P.own == P.OW && P.ow0 == 0 && (plane_elems & 3) == 0 && (P.ys_n & 3) == 0 &&
                ((P.OH * P.OW) & 3) == 0 && (!P.wide || (P.OW & 3) == 0) && (P.ys_f & 3) == 0 && ((P.oh0 * P.OW) & 3) == 0 &&
                ((reinterpret_cast<uintptr_t>(P.y) | reinterpret_cast<uintptr_t>(P.res)) & 15) == 0;
+    };
+    auto store_mode = [&]() -> int {
+        const bool filters_run = (P.ys_f == 1) && ((P.ys_p & 3) == 0) && ((P.ys_n & 3) == 0) && ((P.Fg & 3) == 0) &&
+                                 (((reinterpret_cast<uintptr_t>(P.y) | reinterpret_cast<uintptr_t>(P.res)) & 15) == 0);
+        return pixel_runs() ? kStorePixels : (filters_run ? kStoreFilters : (P.ys_f == 1 ? kStoreRows : kStoreAny));
     };
     // split-K: this CTA reduces the channel chunks [c0, c1)
     const int c0 = (int)((long long)ksp * P.nchunks / P.ksplit), c1 = (int)((long long)(ksp + 1) * P.nchunks / P.ksplit);
@@ -1381,51 +1266,81 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
         long long t_epi0 = t_loop;
         if (!PP) {
             // ---------------- epilogue of the only tile ----------------
-            // Addresses and store mode first: the MMA warp is still working through the last stages, so this costs nothing.
-            const bool vec_ok = (P.ys_f == 1) && ((P.ys_p & 3) == 0) && ((P.ys_n & 3) == 0) && ((P.Fg & 3) == 0) &&
-                                ((reinterpret_cast<uintptr_t>(P.y) & 15) == 0);
-            const int f_tile0 = ntile * P.BN;
+            // Addresses and store mode first: the MMA thread is still working through the last stages, so this costs nothing.
+            // The two sets split the tile's columns.  Code that runs once per CTA comes out of a cold instruction cache, so its
+            // length is its cost: small loops.
+            const int per_set = P.BN / 2, col0 = tset * per_set, f_tile0 = ntile * P.BN;
             const long long f_glob0 = P.z_is_batch ? 0 : (long long)zb * P.Fg;
-            float *yp = P.y + y_off + f_glob0 * P.ys_f;
-            const float *bp = (P.has_bias && P.ksplit == 1) ? P.bias + f_glob0 : nullptr;
-            const float *rp = (P.res != nullptr && P.ksplit == 1) ? P.res + y_off + f_glob0 * P.ys_f : nullptr;
-            // split-K: partial sums go to the landing areas of the cluster's CTAs, summed after the role branches
-            const int split_cols = P.BN / P.ksplit, split_shift = 31 - __clz(split_cols);
-            const uint32_t split_addr =
-                P.ksplit > 1 ? ptx::smem_u32(sSplit) + (uint32_t)(((int)ptx::cluster_ctarank() * split_cols) * kTileM + p) * 4u : 0u;
-            float *stage = nullptr;
-            int nvalid_warp = 0;
-            const long long y_off0 = __shfl_sync(0xffffffffu, y_off, 0);
-            float *ybase_warp = yp - y_off + y_off0;
-            const float *rbase_warp = rp != nullptr ? rp - y_off + y_off0 : nullptr;
-            if (pixel_runs() && P.ksplit == 1) {
-                nvalid_warp = __popc(__ballot_sync(0xffffffffu, valid));
-                if (nvalid_warp > 0) // B stages are idle once the accumulator is complete
-                    stage = reinterpret_cast<float *>(sB) + (warp - kSetWarp) * 1024;
-                if ((uint32_t)(warp - kSetWarp + 1) * 4096u > (uint32_t)P.NB * (SPLIT ? 2u : 1u) * b_half)
-                    stage = nullptr; // not enough idle shared memory for this warp's block
-            }
-            // the two sets split the tile's columns (whole 32-column blocks)
-            const int nblk = P.BN / 32, half_blk = (nblk + 1) / 2;
-            const int col0 = tset == 0 ? 0 : half_blk * 32, col1 = tset == 0 ? half_blk * 32 : P.BN;
+            StoreJob J;
+            J.y = P.y + f_glob0 * P.ys_f;
+            J.bias = P.has_bias ? P.bias + f_glob0 : nullptr;
+            J.res = P.res != nullptr ? P.res + f_glob0 * P.ys_f : nullptr;
+            J.ys_f = P.ys_f, J.y_off = y_off, J.Fg = P.Fg, J.act = P.act, J.lane = lane, J.valid = valid;
+            J.nvalid = __popc(__ballot_sync(0xffffffffu, valid));
+            J.y_off0 = __shfl_sync(0xffffffffu, y_off, 0);
+            // a 4 KB block per warp: the filter ring is idle once the accumulator is complete (if it is large enough)
+            float *stage = reinterpret_cast<float *>(smem + (L.stage_off == L.bar_off ? L.b_off : L.stage_off)) + (warp - kSetWarp) * 1024;
             if (alive)
                 alive = ptx::mbar_wait_warp(acc_full, 0u, abort_flag);
             if (SPLIT && P.fl > 0) // the drain warps have written total + last group over the main accumulator
                 ptx::named_bar_sync(1, 384);
             t_epi0 = prof ? clock64() : 0;
-            if (alive) {
+            if (alive && P.ksplit > 1) {
+                // Split-K: column c of the tile is summed by CTA c / cols of the cluster.  Push this CTA's partial sum into that
+                // CTA's shared memory, slot [this rank][c % cols][pixel] (consecutive lanes = consecutive words).
                 ptx::tc_fence_after();
-#define PETB200_EPI(ACT_)                                                                                              \
-    epilogue_store<ACT_, PASSES>(t_row, t_row + (uint32_t)P.BN, P.BN, f_tile0, P.Fg, valid, bp, rp, yp, P.ys_f, vec_ok, stage, nvalid_warp, \
-                                 ybase_warp, rbase_warp, col0, col1, split_addr, split_shift)
-                switch (P.ksplit > 1 ? PETB200_ACT_NONE : P.act) {
-                case PETB200_ACT_RELU: PETB200_EPI(PETB200_ACT_RELU); break;
-                case PETB200_ACT_SIGMOID: PETB200_EPI(PETB200_ACT_SIGMOID); break;
-                case PETB200_ACT_TANH: PETB200_EPI(PETB200_ACT_TANH); break;
-                case PETB200_ACT_GELU: PETB200_EPI(PETB200_ACT_GELU); break;
-                default: PETB200_EPI(PETB200_ACT_NONE); break;
+                const int cols = P.BN / P.ksplit, shift = 31 - __clz(cols), me = (int)ptx::cluster_ctarank();
+                const uint32_t mine = ptx::smem_u32(sSplit) + (uint32_t)(me * cols * kTileM + p) * 4u;
+#pragma unroll 1
+                for (int c = col0; c < col0 + per_set; c += 8) {
+                    uint32_t v[8], x[8];
+                    ptx::tmem_ld_32x8(t_row + (uint32_t)c, v);
+                    if (SPLIT)
+                        ptx::tmem_ld_32x8(t_row + (uint32_t)(P.BN + c), x);
+                    ptx::tmem_ld_wait();
+                    if (cols >= 8) { // one owner: one address translation; the CTA's own block stays out of the cluster network
+                        const int owner = c >> shift;
+                        const uint32_t local = mine + (uint32_t)((c & (cols - 1)) * kTileM) * 4u;
+                        if (owner == me) {
+#pragma unroll
+                            for (int j = 0; j < 8; ++j)
+                                ptx::st_shared_f32(local + (uint32_t)(j * kTileM) * 4u, SPLIT ? __uint_as_float(v[j]) + __uint_as_float(x[j]) : __uint_as_float(v[j]));
+                        } else {
+                            const uint32_t remote = ptx::map_to_cta(local, (uint32_t)owner);
+#pragma unroll
+                            for (int j = 0; j < 8; ++j)
+                                ptx::st_dsmem_f32(remote + (uint32_t)(j * kTileM) * 4u, SPLIT ? __uint_as_float(v[j]) + __uint_as_float(x[j]) : __uint_as_float(v[j]));
+                        }
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const int col = c + j;
+                            ptx::st_dsmem_f32(ptx::map_to_cta(mine + (uint32_t)((col & (cols - 1)) * kTileM) * 4u, (uint32_t)(col >> shift)),
+                                              SPLIT ? __uint_as_float(v[j]) + __uint_as_float(x[j]) : __uint_as_float(v[j]));
+                        }
+                    }
                 }
-#undef PETB200_EPI
+            } else if (alive) {
+                ptx::tc_fence_after();
+                const int blocks = (P.BN / 32 + 1) / 2; // whole 32-column blocks per set
+                with_store_mode(store_mode(), J.res != nullptr, [&](auto mode_c, auto res_c) {
+#pragma unroll 1
+                for (int c = tset * blocks * 32; c < min(P.BN, (tset + 1) * blocks * 32); c += 32) {
+                    float r[32];
+#pragma unroll
+                    for (int h = 0; h < 32; h += 16) {
+                        uint32_t v[16], x[16];
+                        ptx::tmem_ld_32x16(t_row + (uint32_t)(c + h), v);
+                        if (SPLIT)
+                            ptx::tmem_ld_32x16(t_row + (uint32_t)(P.BN + c + h), x);
+                        ptx::tmem_ld_wait();
+#pragma unroll
+                        for (int j = 0; j < 16; ++j)
+                            r[h + j] = SPLIT ? __uint_as_float(v[j]) + __uint_as_float(x[j]) : __uint_as_float(v[j]);
+                    }
+                    store_block<decltype(mode_c)::value, decltype(res_c)::value>(J, r, stage, f_tile0 + c);
+                }
+                });
             }
         }
         if (prof_cta) { // lane 0 of the first warp of set 0
@@ -1462,10 +1377,10 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                     t_dw += cd1 - cd0, t_dd += clock64() - cd1;
             }
         } else if (PP || FL > 0) {
-            const bool filters_run = (P.ys_f == 1) && ((P.ys_p & 3) == 0) && ((P.ys_n & 3) == 0) && ((P.Fg & 3) == 0) &&
-                                     (((reinterpret_cast<uintptr_t>(P.y) | reinterpret_cast<uintptr_t>(P.res)) & 15) == 0);
-            const int store_mode = pixel_runs() ? kStorePixels : (filters_run ? kStoreFilters : kStoreAny);
             float *stage = reinterpret_cast<float *>(smem + L.stage_off) + quarter * 1024;
+            auto drain = [&](auto mode_c, auto res_c) {
+            constexpr int MODE = decltype(mode_c)::value;
+            constexpr bool RES = decltype(res_c)::value;
             for (int tl = 0; tl < ntl && alive; ++tl) {
                 const int reg = two_regions ? (tl & 1) : 0, use = two_regions ? (tl >> 1) : tl;
                 StoreJob J;
@@ -1477,7 +1392,7 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                     J.y = P.y + f_glob0 * P.ys_f;
                     J.bias = P.has_bias ? P.bias + f_glob0 : nullptr;
                     J.res = P.res != nullptr ? P.res + f_glob0 * P.ys_f : nullptr;
-                    J.ys_f = P.ys_f, J.mode = store_mode, J.Fg = P.Fg, J.act = P.act, J.lane = lane;
+                    J.ys_f = P.ys_f, J.Fg = P.Fg, J.act = P.act, J.lane = lane;
                     J.nvalid = __popc(__ballot_sync(0xffffffffu, J.valid));
                     J.y_off0 = __shfl_sync(0xffffffffu, J.y_off, 0);
                 }
@@ -1514,7 +1429,7 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                         }
                         if (c + 32 >= P.BN)
                             release();
-                        store_block(J, racc, stage, ntile * P.BN + c);
+                        store_block<MODE, RES>(J, racc, stage, ntile * P.BN + c);
                     }
                 } else {
                     // Groups in order, round-to-nearest adds; the MMA thread restarts the main accumulator once a group has been taken.
@@ -1556,7 +1471,7 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                         const long long cs0 = prof ? clock64() : 0;
 #pragma unroll 1
                         for (int c = 0; c < P.BN; c += 32) {
-                            store_block(J, racc, stage, ntile * P.BN + c);
+                            store_block<MODE, RES>(J, racc, stage, ntile * P.BN + c);
 #pragma unroll
                             for (int j = 0; j < 96; ++j) // the next block's sums move down
                                 racc[j] = racc[j + 32];
@@ -1565,6 +1480,11 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                     }
                 }
             }
+            };
+            if constexpr (PP == kSingle)
+                drain(std::integral_constant<int, kStoreAny>(), std::integral_constant<bool, false>()); // (stores nothing)
+            else
+                with_store_mode(store_mode(), P.res != nullptr, drain);
             if (!PP && FL > 0) // (also after a wait gave up: the transform sets wait here)
                 ptx::named_bar_sync(1, 384);
         }
@@ -1678,22 +1598,63 @@ __global__ void __launch_bounds__(256) k_pack_conv_w(const float *__restrict__ w
     }
 }
 
-template <bool BF>
-__global__ void __launch_bounds__(256) k_pack_mm_b(const float *__restrict__ b, void *__restrict__ hi,
-                                                   void *__restrict__ lo, int bs, int n, int k, int Kpad, int transB, int rna,
-                                                   long long sb_batch, long long sb_row, int BC, int Kc_pad) {
+// What a matmul needs before it can run, in one launch (bound by HBM: every operand read once, its copy written once).
+// Blocks [0, b_tiles): B[b][k][n] or [b][n][k] -> hi/lo [rows][Kpad], a tile of 32 rows x 32 packed positions per block; a [k][n]
+// tile is turned through shared memory, so that both sides move whole 128-byte lines (one thread per packed position read B
+// with a stride of n words: 35 us of the 76 us of a 4 x 500 x 1001 x 770 product).  The other blocks: rows of A copied to a
+// pitch that TMA can address (the padding is zero).
+struct PrepareArgs {
+    const float *b;
+    void *hi, *lo;
+    int bs, n, k, Kpad, rna, BC;
+    FastDiv by_kc_pad, by_tiles_k, by_tiles_n;
+    long long sb_batch, sb_row;
+    int b_tiles, tiles_k, tiles_n;
+    const float *a;
+    float *a_copy;
+    long long a_rows;
+    int a_w, a_pitch;
+};
+template <bool BF, bool TRANSB>
+__global__ void __launch_bounds__(256) k_prepare_mm(const PrepareArgs g) {
     pdl_prologue();
-    const long long total = (long long)bs * n * Kpad;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const int kp = (int)(i % Kpad); // packed position: chunk * Kc_pad + element of the chunk (BC of them, then padding)
-        const int ch = kp / Kc_pad, kc = kp - ch * Kc_pad, kk = ch * BC + kc;
-        const long long row = i / Kpad;
-        const int nn = (int)(row % n);
-        const int bb = (int)(row / n);
-        float v = 0.f;
-        if (kc < BC && kk < k)
-            v = transB ? __ldg(b + bb * sb_batch + nn * sb_row + kk) : __ldg(b + bb * sb_batch + kk * sb_row + nn);
-        store_split<BF>(hi, lo, i, v, rna);
+    __shared__ float tile[32][33];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if ((int)blockIdx.x >= g.b_tiles) { // rows of A, a warp each
+        const long long stride = (long long)(gridDim.x - g.b_tiles) * 8;
+        for (long long r = (long long)(blockIdx.x - g.b_tiles) * 8 + warp; r < g.a_rows; r += stride) {
+            const float *src = g.a + r * g.a_w;
+            float *dst = g.a_copy + r * g.a_pitch;
+#pragma unroll 8
+            for (int c = lane; c < g.a_pitch; c += 32)
+                dst[c] = c < g.a_w ? __ldg(src + c) : 0.f;
+        }
+        return;
+    }
+    const int rest = g.by_tiles_k.div((int)blockIdx.x), tk = (int)blockIdx.x - rest * g.tiles_k, bb = g.by_tiles_n.div(rest), tn = rest - bb * g.tiles_n;
+    const float *src = g.b + bb * g.sb_batch;
+    const int k0 = tk * 32, n0 = tn * 32;
+    // packed position -> row of B: chunk * Kc_pad + element of the chunk (BC of them, then padding; Kc_pad a multiple of 32)
+    const int ch = g.by_kc_pad.div(k0), kc0 = k0 - ch * (int)g.by_kc_pad.d, kk0 = ch * g.BC + kc0, kn = min(min(g.BC - kc0, g.k - kk0), 32);
+    if (TRANSB) {
+#pragma unroll
+        for (int i = 0; i < 32; i += 8) {
+            const int nn = n0 + warp + i;
+            const float v = lane < kn && nn < g.n ? __ldg(src + nn * g.sb_row + kk0 + lane) : 0.f;
+            if (nn < g.n)
+                store_split<BF>(g.hi, g.lo, ((long long)bb * g.n + nn) * g.Kpad + k0 + lane, v, g.rna);
+        }
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < 32; i += 8)
+        tile[warp + i][lane] = warp + i < kn && n0 + lane < g.n ? __ldg(src + (kk0 + warp + i) * g.sb_row + n0 + lane) : 0.f;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 32; i += 8) {
+        const int nn = n0 + warp + i;
+        if (nn < g.n)
+            store_split<BF>(g.hi, g.lo, ((long long)bb * g.n + nn) * g.Kpad + k0 + lane, tile[lane][warp + i], g.rna);
     }
 }
 
@@ -2464,7 +2425,9 @@ struct TcMatmul {
     long long st[6] = {0, 0, 0, 0, 0, 0};
     TcCore core;
     int bs, m, n, k, transB;
-    bool native_a = false; // A is consumed row-major as passed (no re-layout)
+    // A as passed is rows of `a_w` values that TMA cannot address: copied to a pitch of `a_pitch` first (0 rows: consumed as it is)
+    long long a_rows = 0;
+    int a_w = 0, a_pitch = 0;
 };
 
 // Row-major A ([b][m][k], k % 4 == 0): the kernel's K-major mode, no re-layout of A.
@@ -2557,13 +2520,18 @@ int tc_matmul_create(petb200_ctx *ctx, int bs, int m, int n, int k, int transA, 
     for (int i = 0; i < 6; ++i)
         t->st[i] = strides ? strides[i] : dense[i];
     int rc;
-    if (!transA && k % 4 == 0 && t->st[0] % 4 == 0 && t->st[1] % 4 == 0 && env_int("PETB200_TC_KMAJOR", 1)) {
+    if (!transA && k % 4 == 0 && t->st[0] % 4 == 0 && t->st[1] % 4 == 0) {
         rc = tc_configure_kmajor(ctx, t->core, bs, m, n, k, has_bias, act, t->st);
-        t->native_a = true;
+    } else if (!transA && !strides) { // rows of A off the 16-byte grid: the same on a copy with a pitch of whole 16-byte pieces
+        t->a_rows = (long long)bs * m, t->a_w = k, t->a_pitch = (k + 3) / 4 * 4;
+        const long long st[6] = {(long long)m * t->a_pitch, t->a_pitch, t->st[2], t->st[3], t->st[4], t->st[5]};
+        rc = tc_configure_kmajor(ctx, t->core, bs, m, n, t->a_pitch, has_bias, act, st);
     } else if (strides) {
         delete t;
         return fail(ctx, PETB200_ERR_UNSUPPORTED, "strided matmul operands need row-major A with k and the A strides multiples of 4");
     } else {
+        if (m % 4 != 0)
+            t->a_rows = (long long)bs * k, t->a_w = m, t->a_pitch = mp;
         ConvGeom g{};
         g.N = bs;
         g.C = k;
@@ -2616,7 +2584,6 @@ int tc_g2bmm_create(petb200_ctx *ctx, int bs, int n, int m, int w, void **out) {
     auto *t = new TcMatmul();
     t->bs = bs, t->m = n, t->n = n, t->k = m, t->transB = 1;
     t->st[2] = (long long)n * m, t->st[3] = m; // keys: batch and row strides
-    t->native_a = true;
     TcCore &core = t->core;
     core.ctx = ctx;
     IgemmParams &P = core.P;
@@ -2694,7 +2661,6 @@ int tc_gbmml_create(petb200_ctx *ctx, int bs, int n, int m, int w, void **out) {
     auto *t = new TcMatmul();
     t->bs = bs, t->m = n, t->n = m, t->k = n, t->transB = 0;
     t->st[2] = (long long)n * m, t->st[3] = m; // v: batch stride, stride of a key row
-    t->native_a = true;
     TcCore &core = t->core;
     core.ctx = ctx;
     IgemmParams &P = core.P;
@@ -2761,22 +2727,39 @@ int tc_gbmml_run(void *h, const float *p, float *y, cudaStream_t s) {
 }
 
 void tc_matmul_set_prof(void *h, long long *p) { ((TcMatmul *)h)->core.prof = p; }
-int tc_matmul_native_a(void *h) { return ((TcMatmul *)h)->native_a ? 1 : 0; }
+// Words of the copy of A that a call needs (0: A is consumed as it is).
+long long tc_matmul_a_copy(void *h) {
+    auto *t = (TcMatmul *)h;
+    return t->a_rows * t->a_pitch;
+}
 void tc_matmul_destroy(void *h) { delete (TcMatmul *)h; }
-int tc_matmul_pack_b(void *h, const float *b, cudaStream_t s) {
+// Packs B (null: it has been) and copies A to an addressable pitch (null: not needed), in one launch.
+int tc_matmul_prepare(void *h, const float *b, const float *a, float *a_copy, cudaStream_t s) {
     auto *t = (TcMatmul *)h;
     TcCore &c = t->core;
-    long long total = (long long)t->bs * t->n * c.Ktot;
-    int blocks = (int)std::min<long long>((total + 255) / 256, (long long)c.ctx->sm_count * 16);
+    PrepareArgs g{};
+    g.b = b, g.hi = c.whi.p, g.lo = c.wlo.p, g.bs = t->bs, g.n = t->n, g.k = t->k, g.Kpad = (int)c.Ktot, g.rna = c.single_pass;
+    g.BC = c.P.BC, g.sb_batch = t->st[2], g.sb_row = t->st[3];
+    g.tiles_k = g.Kpad / 32, g.tiles_n = (t->n + 31) / 32; // (Kpad is a multiple of 32)
+    g.by_kc_pad.set(c.P.spc * c.P.ke), g.by_tiles_k.set(g.tiles_k), g.by_tiles_n.set(g.tiles_n);
+    const long long tiles = b ? (long long)g.tiles_k * g.tiles_n * t->bs : 0;
+    if (tiles > (1 << 30))
+        return fail(c.ctx, PETB200_ERR_UNSUPPORTED, "matmul operand too large to pack in one launch");
+    g.b_tiles = (int)tiles;
+    g.a = a, g.a_copy = a_copy, g.a_rows = a ? t->a_rows : 0, g.a_w = t->a_w, g.a_pitch = t->a_pitch;
+    const long long a_blocks = std::min<long long>((g.a_rows + 7) / 8, (long long)c.ctx->sm_count * 8);
+    if (tiles + a_blocks == 0)
+        return PETB200_OK;
+    const dim3 grid((unsigned)(tiles + a_blocks));
     if (c.bf16)
-        launch_pdl(k_pack_mm_b<true>, blocks, 256, 0, s, b, c.whi.p, c.wlo.p, t->bs, t->n, t->k, (int)c.Ktot, t->transB, 0, t->st[2], t->st[3],
-                   c.P.BC, c.P.spc * c.P.ke);
+        launch_pdl(t->transB ? k_prepare_mm<true, true> : k_prepare_mm<true, false>, grid, 256, 0, s, g);
     else
-        launch_pdl(k_pack_mm_b<false>, blocks, 256, 0, s, b, c.whi.p, c.wlo.p, t->bs, t->n, t->k, (int)c.Ktot, t->transB, c.single_pass,
-                   t->st[2], t->st[3], c.P.BC, c.P.spc * c.P.ke);
-    c.weights_ready = true;
-    return launched(c.ctx, "k_pack_mm_b");
+        launch_pdl(t->transB ? k_prepare_mm<false, true> : k_prepare_mm<false, false>, grid, 256, 0, s, g);
+    if (b)
+        c.weights_ready = true;
+    return launched(c.ctx, "k_prepare_mm");
 }
+int tc_matmul_pack_b(void *h, const float *b, cudaStream_t s) { return tc_matmul_prepare(h, b, nullptr, nullptr, s); }
 int tc_matmul_run(void *h, const float *a_t, const float *bias, const float *res, float *cmat, cudaStream_t s) {
     auto *t = (TcMatmul *)h;
     return t->core.launch(a_t, bias, res, cmat, s);
