@@ -527,13 +527,33 @@ __device__ __forceinline__ void store_filters(const StoreJob &J, const float *bi
             *reinterpret_cast<float4 *>(J.y + off + f) = v;
     }
 }
+// Rows a constant pitch apart (a matmul's, or pixels of one image) take one pointer that moves down them, which is half the
+// instructions of an offset per row.
 template <bool RES>
 __device__ __forceinline__ void store_rows(const StoreJob &J, const float *bias, const float *stage, int f0) {
     const int lane = J.lane, f = f0 + lane;
     const bool live = f < J.Fg, relu = J.act == PETB200_ACT_RELU;
     const float bv = bias != nullptr && live ? __ldg(bias + f) : 0.f;
-    const long long yo = J.valid ? J.y_off : -1;
+    const long long pitch = __shfl_sync(0xffffffffu, J.y_off, 1) - J.y_off0;
+    if (__all_sync(0xffffffffu, J.valid == (lane < J.nvalid) && (!J.valid || J.y_off == J.y_off0 + lane * pitch))) {
+        const int rows = live ? J.nvalid : 0;
+        float *dst = J.y + J.y_off0 + f;
+        const float *rs = RES ? J.res + J.y_off0 + f : nullptr;
 #pragma unroll
+        for (int row = 0; row < 32; ++row, dst += pitch) {
+            float v = stage[row * 32 + (lane ^ row)] + bv;
+            if (RES) {
+                v += row < rows ? __ldg(rs) : 0.f;
+                rs += pitch;
+            }
+            v = relu ? fmaxf(v, 0.f) : v;
+            if (row < rows)
+                *dst = v;
+        }
+        return;
+    }
+    const long long yo = J.valid ? J.y_off : -1;
+#pragma unroll 1
     for (int row = 0; row < 32; ++row) {
         const long long off = __shfl_sync(0xffffffffu, yo, row);
         const bool go = off >= 0 && live;
