@@ -28,3 +28,63 @@ def test_matrix_vector_products_exact(ctx, m, trans_a, trans_b, n, k):
     got = ctx.matmul(dev(a), dev(w), trans_a, trans_b, bias=dev(bias), act="relu", residual=dev(res))
     ctx.sync_check()
     assert np.array_equal(got.cpu().numpy(), want)
+
+
+# Tensor-core matmul: k off the 16-byte grid (A re-pitched), n off it (rows stored one by one), one tile per CTA and several,
+# narrow tiles and wide ones with an accumulator flush (k > 768), tiles that end inside the last rows and columns
+@pytest.mark.parametrize("b,m,n,k", [(1, 33, 9, 31), (2, 129, 65, 70), (80, 130, 70, 33), (160, 128, 64, 34), (3, 1025, 129, 801), (4, 1921, 330, 773), (1, 257, 2047, 998)])
+@pytest.mark.parametrize("trans_a,trans_b", [(False, False), (False, True), (True, False)])
+def test_matmul_off_the_16_byte_grid(ctx, b, m, n, k, trans_a, trans_b):
+    rng = np.random.default_rng(m + n + k)
+    a = rng.integers(-2, 3, (b, k, m) if trans_a else (b, m, k)).astype(np.float32)
+    w = rng.integers(-2, 3, (b, n, k) if trans_b else (b, k, n)).astype(np.float32)
+    bias, res = rng.integers(-4, 5, n).astype(np.float32), rng.integers(-4, 5, (b, m, n)).astype(np.float32)
+    lin = torch.matmul(dev(a).double().transpose(1, 2) if trans_a else dev(a).double(), dev(w).double().transpose(1, 2) if trans_b else dev(w).double()) + dev(bias).double()
+    got = ctx.matmul(dev(a), dev(w), trans_a, trans_b, bias=dev(bias), act="relu", residual=dev(res))
+    assert np.array_equal(got.cpu().numpy(), torch.relu(lin + dev(res)).float().cpu().numpy())
+    got = ctx.matmul(dev(a), dev(w), trans_a, trans_b, bias=dev(bias), act="tanh")
+    ctx.sync_check()
+    assert rel_err(got.cpu().numpy(), torch.tanh(lin).cpu().numpy()) <= TOL
+
+
+# Several tiles per CTA: 16-byte runs of pixels that end inside a warp's 32 (10 x 14, 10 x 10), pixels off the 16-byte grid, two images in a
+# tile, filters that end inside a block; with and without a flush (c*9 > 768); each way of storing with and without a residual
+@pytest.mark.parametrize("n,c,h,w,f,act", [(300, 8, 13, 13, 70, "relu"), (170, 8, 16, 16, 64, "none"), (310, 5, 10, 10, 33, "relu"), (160, 90, 10, 14, 72, "relu"),
+                                           (320, 96, 7, 7, 130, "none"), (160, 6, 12, 18, 31, "sigmoid")])
+def test_conv_persistent_tiles_stores(ctx, n, c, h, w, f, act):
+    rng = np.random.default_rng(n + c)
+    x, wt = dev(rng.integers(-2, 3, (n, c, h, w)).astype(np.float32)), dev(rng.integers(-2, 3, (f, c, 3, 3)).astype(np.float32))
+    bias, res = dev(rng.integers(-4, 5, f).astype(np.float32)), dev(rng.integers(-4, 5, (n, f, h, w)).astype(np.float32))
+    lin = torch.nn.functional.conv2d(x.double().cpu(), wt.double().cpu(), bias.double().cpu(), padding=1)
+    fn = {"relu": torch.relu, "none": lambda v: v, "sigmoid": torch.sigmoid}[act]
+    for r in (None, res):
+        plan = ctx.conv2d_plan(x.shape, wt.shape, 1, 1, bias=True, act=act)
+        ctx.conv2d_set_weights(plan, wt)
+        got = ctx.conv2d_run(plan, x, bias, residual=r)
+        ctx.sync_check()
+        want = fn(lin if r is None else lin + r.double().cpu())
+        assert torch.equal(got.cpu(), want.float()) if act != "sigmoid" else rel_err(got.cpu().numpy(), want.numpy()) <= TOL
+
+
+# last register-resident rows of a warp, of a block, and the first row past them; fewer rows than a wave of blocks
+@pytest.mark.parametrize("cols", [1024, 1025, 1279, 2048, 2049, 4095, 4096, 4097])
+@pytest.mark.parametrize("rows", [1, 3, 700])
+def test_softmax_rows_by_length(ctx, oracle, rows, cols):
+    x = np.random.default_rng(cols).standard_normal((rows, cols)).astype(np.float32) * 4
+    x[0, cols - 1] = 40.0
+    got = ctx.softmax(dev(x))
+    ctx.sync_check()
+    assert rel_err(got.cpu().numpy(), oracle.softmax(x)) <= 1e-5
+
+
+# 2w+1 around a 16-byte piece, a K stage and more than a tile of keys; rows that end inside a tile; the first and last rows'
+# windows reach past the keys
+@pytest.mark.parametrize("b,n,m,w", [(1, 130, 64, 1), (2, 257, 32, 3), (3, 300, 64, 16), (1, 1000, 96, 130), (5, 129, 16, 200), (2, 2051, 64, 67)])
+def test_banded_products_by_width(ctx, oracle, b, n, m, w):
+    rng = np.random.default_rng(n + w)
+    q, k = (rng.integers(-2, 3, (b, n, m)).astype(np.float32) for _ in range(2))
+    p = rng.integers(-2, 3, (b, n, 2 * w + 1)).astype(np.float32)
+    scores, out = ctx.g2bmm(dev(q), dev(k), w), ctx.gbmml(dev(p), dev(k))
+    ctx.sync_check()
+    assert np.array_equal(scores.cpu().numpy(), oracle.g2bmm(q, k, w))
+    assert np.array_equal(out.cpu().numpy(), oracle.gbmml(p, k))
