@@ -22,11 +22,12 @@
 namespace petb200 {
 
 int tc_conv_create_view(petb200_ctx *ctx, int n, int c, int h, int w, int f, int r, int s, int pad_h, int pad_w, int ohn, int own,
-                        int ow_nominal, long long ys_n, long long ys_f, long long ys_p, int has_bias, int act, int passes, void **out,
+                        int ow_nominal, long long ys_n, long long ys_f, long long ys_p, int has_bias, int act, int passes, int beside, void **out,
                         size_t *dev_bytes);
 void tc_conv_destroy(void *h);
 int tc_conv_set_weights(void *h, const float *w, cudaStream_t s);
-int tc_conv_run(void *h, const float *x, const float *bias, const float *res, float *y, const int *win, cudaStream_t s);
+int tc_conv_run_part(void *h, const float *x, const float *bias, float *y, int link, cudaStream_t s);
+bool tc_conv_can_link(void *h);
 const char *tc_conv_variant(void *h);
 
 namespace {
@@ -118,11 +119,6 @@ struct Phase {
 
 struct ConvTransPlan : petb200_plan {
     std::vector<Phase *> phases; // non-empty: the phase decomposition is used instead of `conv`
-    // The phases write disjoint pixels of y and each fills only part of the GPU, so they run side by side: phase i goes to
-    // stream i % 4 (0 = the caller's), forked after the layout pass and joined before the call returns to the stream.
-    static constexpr int kSide = 3;
-    cudaStream_t side[kSide] = {nullptr, nullptr, nullptr};
-    cudaEvent_t ev_fork = nullptr, ev_join[kSide] = {nullptr, nullptr, nullptr};
     DevBuf xn;                   // x as NCHW for the phase convolutions
     int sh = 1, sw = 1;
     ExpandGeom g{};
@@ -135,14 +131,6 @@ struct ConvTransPlan : petb200_plan {
         delete conv;
         for (Phase *p : phases)
             delete p;
-        for (int i = 0; i < kSide; ++i) {
-            if (side[i])
-                cudaStreamDestroy(side[i]);
-            if (ev_join[i])
-                cudaEventDestroy(ev_join[i]);
-        }
-        if (ev_fork)
-            cudaEventDestroy(ev_fork);
     }
     int bench_launch(cudaStream_t s) override;
 };
@@ -183,11 +171,13 @@ int make_convtrans_plan(petb200_ctx *ctx, const int *a /*n,c,h,w,f,r,s,ph,pw,sh,
     pl->kernel = pl->conv->kernel;
     pl->device_bytes = pl->conv->device_bytes + xe_bytes + w_bytes;
     pl->sh = sh, pl->sw = sw;
-    // Phase decomposition: worth its sh*sw + 1 launches once the zero-inserted product is large (rough model from
-    // measurements on B200: the zero-inserted conv sustains ~100 TFLOP/s of issued work, a phase conv ~170 with a floor
-    // of ~8 us per launch).  Needs taps in every phase and a row stride of y that is a whole number of phase pixels.
+    // Phase decomposition: sh*sw + 1 launches, the phases side by side, of 1 / (sh*sw) of the zero-inserted product's work.
+    // Measured on B200: the zero-inserted path takes about 10 us plus its work at 100 TFLOP/s, the phases 8 us plus 2.2 us each
+    // (their launches) or their work at 120 TFLOP/s; 2 x 32 x 32 x 64 -> 32, 4 x 4 stride 2 lies on the line (19 and 15 us on the
+    // GPU, 22 and 24 us from call to call), 4 x 24 x 24 x 96 -> 48, 6 x 6 stride 3 takes 94 and 26 us.  Needs taps in every
+    // phase and a row stride of y that is a whole number of phase pixels.
     const double issued = 2.0 * n * c * (double)oh * ow * f * r * s;
-    const double us_inserted = issued / 100e6, us_phased = sh * sw * std::max(8.0, issued / (sh * sw) / 170e6);
+    const double us_inserted = 10.0 + issued / 100e6, us_phased = 8.0 + std::max(2.2 * sh * sw, issued / (sh * sw) / 120e6);
     const bool tc_algo = tc_is_tc_algo(algo);
     const char *env = getenv("PETB200_CONVTRANS_PHASES");
     const int want = env ? atoi(env) : -1; // 0 never, 1 whenever possible, unset: by size
@@ -211,7 +201,7 @@ int make_convtrans_plan(petb200_ctx *ctx, const int *a /*n,c,h,w,f,r,s,ph,pw,sh,
                 size_t bytes = 0;
                 int prc = tc_conv_create_view(ctx, n, f, h, w, c, ps->Ta, ps->Tb, -off_a, -off_b, Ua, Vb, (int)(((long long)sh * ow) / sw),
                                               (long long)oh * ow * c, 1, (long long)sw * c, has_bias, act,
-                                              tc_passes_for(algo), &ps->tc, &bytes);
+                                              tc_passes_for(algo), sh * sw, &ps->tc, &bytes);
                 if (prc != PETB200_OK || ps->wsub.alloc((size_t)c * f * ps->Ta * ps->Tb * 4) != cudaSuccess)
                     ok = false;
                 extra += bytes + ps->wsub.bytes;
@@ -224,7 +214,8 @@ int make_convtrans_plan(petb200_ctx *ctx, const int *a /*n,c,h,w,f,r,s,ph,pw,sh,
             pl->phases.clear();
             pl->xn.alloc(0);
         } else {
-            pl->device_bytes += extra + pl->xn.bytes;
+            pl->xe.alloc(0), pl->wflip.alloc(0); // (the zero-inserted path's)
+            pl->device_bytes += extra + pl->xn.bytes - xe_bytes - w_bytes;
             pl->kernel = tc_conv_variant(pl->phases.front()->tc);
         }
     }
@@ -237,13 +228,16 @@ int convtrans_set_weights(petb200_plan *plan, const float *w, cudaStream_t s) {
     if (!pl || !w)
         return PETB200_ERR_INVALID;
     petb200_ctx *ctx = pl->ctx;
-    const long long total = (long long)pl->c * pl->g.f * pl->r * pl->s;
-    const int blocks = (int)std::max<long long>(1, std::min<long long>((total + 255) / 256, (long long)ctx->sm_count * 16));
-    launch_pdl(k_convtrans_flip_w, blocks, 256, 0, s, w, (float *)pl->wflip.p, pl->r, pl->s, pl->g.f, pl->c, pl->ah, pl->aw);
-    int rc = launched(ctx, "k_convtrans_flip_w");
-    if (rc)
-        return rc;
-    rc = conv_set_weights(pl->conv, (const float *)pl->wflip.p, s);
+    int rc = PETB200_OK;
+    if (pl->phases.empty()) {
+        const long long total = (long long)pl->c * pl->g.f * pl->r * pl->s;
+        const int blocks = (int)std::max<long long>(1, std::min<long long>((total + 255) / 256, (long long)ctx->sm_count * 16));
+        launch_pdl(k_convtrans_flip_w, blocks, 256, 0, s, w, (float *)pl->wflip.p, pl->r, pl->s, pl->g.f, pl->c, pl->ah, pl->aw);
+        rc = launched(ctx, "k_convtrans_flip_w");
+        if (rc)
+            return rc;
+        rc = conv_set_weights(pl->conv, (const float *)pl->wflip.p, s);
+    }
     for (Phase *ps : pl->phases) {
         if (rc)
             break;
@@ -280,28 +274,15 @@ int convtrans_run(petb200_plan *plan, const float *x, const float *bias, float *
         int rc = launched(ctx, "k_convtrans_expand");
         if (rc)
             return rc;
-        const int nside = std::min<int>(ConvTransPlan::kSide, (int)pl->phases.size() - 1);
-        if (nside > 0 && !pl->ev_fork) {
-            PETB200_CUDA(ctx, cudaEventCreateWithFlags(&pl->ev_fork, cudaEventDisableTiming));
-            for (int i = 0; i < nside; ++i) {
-                PETB200_CUDA(ctx, cudaStreamCreateWithFlags(&pl->side[i], cudaStreamNonBlocking));
-                PETB200_CUDA(ctx, cudaEventCreateWithFlags(&pl->ev_join[i], cudaEventDisableTiming));
-            }
-        }
-        if (nside > 0) {
-            PETB200_CUDA(ctx, cudaEventRecord(pl->ev_fork, s));
-            for (int i = 0; i < nside; ++i)
-                PETB200_CUDA(ctx, cudaStreamWaitEvent(pl->side[i], pl->ev_fork, 0));
-        }
+        // The phases write disjoint pixels of y and each fills only part of the GPU, so they run side by side: a chain of launches
+        // in the caller's stream that wait for the layout pass but not for one another.  (Four streams, forked and joined with
+        // events, took 45 us for 8 x 32 x 32 x 128 -> 64, 4 x 4 stride 2.)
+        bool chain = pl->phases.size() > 1;
+        for (Phase *ps : pl->phases)
+            chain = chain && tc_conv_can_link(ps->tc);
         for (size_t i = 0; i < pl->phases.size() && rc == PETB200_OK; ++i) {
             Phase *ps = pl->phases[i];
-            const int lane = (int)(i % (size_t)(nside + 1));
-            rc = tc_conv_run(ps->tc, (const float *)pl->xn.p, bias, nullptr, y + ((size_t)ps->a * pl->ow + ps->b) * pl->c, nullptr,
-                             lane == 0 ? s : pl->side[lane - 1]);
-        }
-        for (int i = 0; i < nside; ++i) { // join even after a failed launch, so that a capture in progress stays well-formed
-            cudaEventRecord(pl->ev_join[i], pl->side[i]);
-            cudaStreamWaitEvent(s, pl->ev_join[i], 0);
+            rc = tc_conv_run_part(ps->tc, (const float *)pl->xn.p, bias, y + ((size_t)ps->a * pl->ow + ps->b) * pl->c, !chain ? 0 : (i == 0 ? 1 : 2), s);
         }
         return rc;
     }

@@ -84,7 +84,11 @@ struct FastDiv {
 #endif
 };
 
+// Launches in one stream that write disjoint parts of y and read only what was written before the first of them run side by side
+// under programmatic dependent launch (without it they run one after the other, which gives the same).
+enum { kLinkNone = 0, kLinkFirst = 1, kLinkNext = 2 };
 struct IgemmParams {
+    int link;               // position in such a chain
     FastDiv by_ntiles, by_mtiles, by_tpi, by_pw, by_od, by_own, by_ohn, by_row_tiles; // (made by set_divisors)
     int Pw, units;          // pixels of one output plane (one image, one depth slice); number of such planes
     int OD, OH, OW;         // full output extents (for addressing y)
@@ -673,6 +677,7 @@ template <bool A_KMAJOR, int PASSES, int PP = kSingle, int BAND = 0>
 __global__ void __launch_bounds__(kThreads, 1)
 k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_bhi,
         const __grid_constant__ CUtensorMap tmap_blo, const IgemmParams P) {
+    constexpr bool LINK = PP == kSingle && BAND == 0; // may be part of a chain of launches
     extern __shared__ uint8_t smem_raw[];
     long long *const prof = kTune ? P.prof : nullptr;
     // 1024-byte alignment for the swizzled operand tiles
@@ -755,8 +760,16 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
     const uint32_t tmem_base = *tmem_slot;
     // Everything above touched only this CTA's own state and the plan's constant table, so under programmatic dependent
     // launch it overlaps the tail of the preceding kernel; from here on the kernel reads what that kernel wrote.
-    ptx::grid_dep_launch_dependents();
-    ptx::grid_dep_wait();
+    // In a chain of launches that do not need one another's results (see `link`) the first lets its successor start only once
+    // the kernel before the chain has completed, and the others do not wait at all.
+    if (LINK && P.link == kLinkFirst) {
+        ptx::grid_dep_wait();
+        ptx::grid_dep_launch_dependents();
+    } else {
+        ptx::grid_dep_launch_dependents();
+        if (!LINK || P.link != kLinkNext)
+            ptx::grid_dep_wait();
+    }
     if (prof_cta)
         prof_cta[9] = (long long)ptx::globaltimer_ns();
 
@@ -1578,6 +1591,8 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
     __syncthreads();
     if (warp == 2)
         ptx::tmem_dealloc(tmem_base, kTmemCols);
+    if (LINK && P.link == kLinkNext) // whoever waits for this launch waits for the ones before it in the chain too
+        ptx::grid_dep_wait();
     if (prof_cta)
         prof_cta[11] = (long long)ptx::globaltimer_ns();
 }
@@ -1705,6 +1720,7 @@ static int env_int_early(const char *name, int dflt) {
 typedef void (*KernelFn)(CUtensorMap, CUtensorMap, CUtensorMap, IgemmParams);
 
 struct TcCore {
+    int beside = 1; // launches of this size that share the GPU (a split of K then only adds work)
     petb200_ctx *ctx = nullptr;
     IgemmParams P{};
     int single_pass = 0;
@@ -1803,12 +1819,13 @@ struct TcCore {
         }
         return PETB200_OK;
     }
-    int launch(const float *x, const float *bias, const float *res, float *y, cudaStream_t s) {
+    int launch(const float *x, const float *bias, const float *res, float *y, cudaStream_t s, int link = 0) {
         int rc = encode_x(x);
         if (rc)
             return rc;
         IgemmParams p = P;
         set_divisors(p);
+        p.link = link;
         p.bias = bias;
         p.res = res;
         p.y = y;
@@ -2153,7 +2170,7 @@ static int tc_configure(petb200_ctx *ctx, TcCore &core, const ConvGeom &g, int o
         P.ksplit = 1;
         if (!fit(bn))
             continue;
-        const long long base_ctas = (long long)mtiles * ((Fg + bn - 1) / bn) * gz;
+        const long long base_ctas = (long long)mtiles * ((Fg + bn - 1) / bn) * gz * core.beside;
         const int passes = core.single_pass ? 1 : 3;
         double cyc;
         const int ks = choose_ksplit(ctx->sm_count, base_ctas, P, passes, want_ks, &cyc);
@@ -2314,7 +2331,7 @@ int tc_conv_create(petb200_ctx *ctx, int nsp, const int *in_dims, int f, const i
 // with row = ow_nominal * pixel.  Used by the transposed convolution, whose sh*sw phases are such convolutions writing
 // every sh-th row and sw-th column of a channels-last tensor.
 int tc_conv_create_view(petb200_ctx *ctx, int n, int c, int h, int w, int f, int r, int s, int pad_h, int pad_w, int ohn, int own,
-                        int ow_nominal, long long ys_n, long long ys_f, long long ys_p, int has_bias, int act, int passes, void **out,
+                        int ow_nominal, long long ys_n, long long ys_f, long long ys_p, int has_bias, int act, int passes, int beside, void **out,
                         size_t *dev_bytes) {
     if (ctx->cc_major != 10)
         return fail(ctx, PETB200_ERR_UNSUPPORTED, "tcgen05 kernels need compute capability 10.x, device has %d.%d", ctx->cc_major, ctx->cc_minor);
@@ -2333,6 +2350,7 @@ int tc_conv_create_view(petb200_ctx *ctx, int n, int c, int h, int w, int f, int
     t->full.ctx = ctx;
     t->full.single_pass = passes == kMathTf32x1;
     t->full.bf16 = passes == kMathBf16x3;
+    t->full.beside = beside;
     t->ys[0] = ys_n, t->ys[1] = ys_f, t->ys[2] = ys_p;
     int rc = PETB200_ERR_UNSUPPORTED;
     if (w % 4 != 0)
@@ -2375,6 +2393,16 @@ int tc_conv_set_weights(void *h, const float *w, cudaStream_t s) {
                                                     c.single_pass);
     c.weights_ready = true;
     return launched(c.ctx, "k_pack_conv_w");
+}
+
+// One of several convolutions of the same x that fill disjoint parts of one tensor; link: its place in their chain of launches
+// (0: none), where tc_conv_can_link() holds for all of them.
+bool tc_conv_can_link(void *h) { return !((TcConv *)h)->full.P.pp; } // (persistent tiles fill the GPU by themselves)
+int tc_conv_run_part(void *h, const float *x, const float *bias, float *y, int link, cudaStream_t s) {
+    auto *t = (TcConv *)h;
+    if (!t->full.weights_ready)
+        return fail(t->full.ctx, PETB200_ERR_INVALID, "conv run before set_weights");
+    return t->full.launch(x, bias, nullptr, y, s, link);
 }
 
 int tc_conv_run(void *h, const float *x, const float *bias, const float *res, float *y, const int *win, cudaStream_t s) {

@@ -88,3 +88,19 @@ def test_banded_products_by_width(ctx, oracle, b, n, m, w):
     ctx.sync_check()
     assert np.array_equal(scores.cpu().numpy(), oracle.g2bmm(q, k, w))
     assert np.array_equal(out.cpu().numpy(), oracle.gbmml(p, k))
+
+
+# Phases side by side: with and without a K split, one launch per phase or persistent tiles (many images), calls back to back (the next
+# call's layout pass must wait for every phase), phases of different size
+@pytest.mark.parametrize("n,hw,f,c,k,s,pad", [(3, 9, 40, 33, 3, 2, 1), (16, 4, 512, 64, 4, 2, 1), (200, 16, 8, 64, 4, 2, 1), (2, 12, 96, 48, 5, 3, 1)])
+def test_convtrans_phases_back_to_back(ctx, oracle, monkeypatch, n, hw, f, c, k, s, pad):
+    monkeypatch.setenv("PETB200_CONVTRANS_PHASES", "1")
+    rng = np.random.default_rng(n + hw)
+    w = rng.integers(-2, 3, (k, k, f, c)).astype(np.float32)
+    xs = [rng.integers(-2, 3, (n, hw, hw, f)).astype(np.float32) for _ in range(3)]
+    plan = ctx.convtrans_plan((n, hw, hw, f), (k, k, f, c), pad, pad, s, s)
+    got = [ctx.convtrans_run(plan, x, dev(w) if i == 0 else None) for i, x in enumerate([dev(x) for x in xs])]
+    ctx.sync_check()
+    for g, x in zip(got, xs):
+        ref = torch.nn.functional.conv_transpose2d(dev(x).double().cpu().permute(0, 3, 1, 2), torch.from_numpy(w).double().permute(2, 3, 0, 1), stride=s, padding=pad)
+        assert np.array_equal(g.cpu().numpy(), ref.permute(0, 2, 3, 1).float().numpy())
