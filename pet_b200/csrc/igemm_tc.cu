@@ -636,9 +636,16 @@ __device__ __forceinline__ void store_block(const StoreJob &J, float *r /*32 sum
         __syncwarp();
         store_pixels<RES>(J, bias, stage, f0);
         if (__builtin_expect((J.nvalid & 3) != 0, 0)) { // the last one to three pixels of a ragged window are left
-            StoreJob R = J;
-            R.valid = J.valid && lane >= (J.nvalid & ~3);
-            store_any<RES>(R, bias, r, f0);
+            if (J.valid && lane >= (J.nvalid & ~3)) {
+                const long long off = J.y_off + (long long)f0 * J.ys_f;
+#pragma unroll 1
+                for (int j = 0; j < 32 && f0 + j < J.Fg; ++j) {
+                    float v = stage[j * 32 + lane] + (bias != nullptr ? __ldg(bias + f0 + j) : 0.f);
+                    if (RES)
+                        v += __ldg(J.res + off + j * J.ys_f);
+                    J.y[off + j * J.ys_f] = J.act == PETB200_ACT_RELU ? fmaxf(v, 0.f) : v;
+                }
+            }
         }
     } else if (MODE == kStoreFilters) {
         // row r of the block at [r][32], 16-byte chunk c at c ^ (r & 7): conflict-free both ways
