@@ -276,7 +276,7 @@ int convtrans_run(petb200_plan *plan, const float *x, const float *bias, float *
             return rc;
         // The phases write disjoint pixels of y and each fills only part of the GPU, so they run side by side: a chain of launches
         // in the caller's stream that wait for the layout pass but not for one another.  (Four streams, forked and joined with
-        // events, took 45 us for 8 x 32 x 32 x 128 -> 64, 4 x 4 stride 2.)
+        // events, took 45 us for 8 x 32 x 32 x 128 -> 64, 4 x 4 stride 2; this takes 27.)
         bool chain = pl->phases.size() > 1;
         for (Phase *ps : pl->phases)
             chain = chain && tc_conv_can_link(ps->tc);

@@ -532,7 +532,7 @@ __device__ __forceinline__ void store_filters(const StoreJob &J, const float *bi
     }
 }
 // Rows a constant pitch apart (a matmul's, or pixels of one image) take one pointer that moves down them, which is half the
-// instructions of an offset per row.
+// instructions of an offset per row (29 x 78 x 662 x 24: 24.6 -> 22 us, 4 x 500 x 1001 x 768: 19.6 -> 18.4 us).
 template <bool RES>
 __device__ __forceinline__ void store_rows(const StoreJob &J, const float *bias, const float *stage, int f0) {
     const int lane = J.lane, f = f0 + lane;
