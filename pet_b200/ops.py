@@ -14,8 +14,9 @@ from . import lib as L
 
 
 # The calls below sit in front of kernels of a few microseconds: plain integers instead of ctypes objects (every entry point
-# declares its argument types), and the stream handle without a torch.cuda.Stream object around it.
-_current_device, _raw_stream = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
+# declares its argument types), and the stream handle without a torch.cuda.Stream object around it.  torch has these two only
+# where it was built with CUDA; without them the module still imports (shapes, plans' arguments, the graph builders).
+_current_device, _raw_stream = getattr(torch._C, "_cuda_getDevice", None), getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
 def _ptr(t):
@@ -23,13 +24,14 @@ def _ptr(t):
 
 
 def _stream():
+    if _current_device is None or _raw_stream is None:
+        return torch.cuda.current_stream().cuda_stream  # (raises torch's own message where there is no CUDA)
     return _raw_stream(_current_device())
 
 
 def _f32(t):
     assert t.is_cuda and t.dtype is torch.float32, "device fp32 tensors only"
     return t.contiguous()
-
 
 
 def perm_spec(after):
