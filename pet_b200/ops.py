@@ -29,9 +29,15 @@ def _stream():
     return _raw_stream(_current_device())
 
 
+# Makes a dense copy of a view.  The caller keeps every copy in a variable until the call has been issued: one that is dropped
+# earlier gives its memory to the next copy, which is then written over it before the kernel has read it.
 def _f32(t):
     assert t.is_cuda and t.dtype is torch.float32, "device fp32 tensors only"
     return t.contiguous()
+
+
+def _opt(t):
+    return _f32(t) if t is not None else None
 
 
 def perm_spec(after):
@@ -106,27 +112,27 @@ class Context:
         return p
 
     def conv2d_set_weights(self, plan, w):
-        plan._w = _f32(w)  # keep alive: the CUDA-core path reads the caller's tensor
+        plan._w = _f32(w)  # kept with the plan: the CUDA-core path reads the caller's tensor in every run
         self.check(self.lib.petb200_conv2d_set_weights(plan.h, _ptr(plan._w), _stream()))
 
     def conv2d_run(self, plan, x, bias=None, out=None, residual=None):
         """y = act(conv(x) + bias [+ residual]); residual (shaped like y) folds a following Add into the epilogue."""
-        x = _f32(x)
+        x, bias = _f32(x), _opt(bias)
         y = out if out is not None else x.new_empty(plan.out_shape)
-        b = _ptr(_f32(bias) if bias is not None else None)
         if residual is not None:
             if tuple(residual.shape) != tuple(plan.out_shape):
                 raise L.PetError(L.ERR_INVALID, "residual must have the shape of the output")
-            self.check(self.lib.petb200_conv_run_residual(plan.h, _ptr(x), b, _ptr(_f32(residual)), _ptr(y), _stream()))
+            residual = _f32(residual)
+            self.check(self.lib.petb200_conv_run_residual(plan.h, _ptr(x), _ptr(bias), _ptr(residual), _ptr(y), _stream()))
         else:
-            self.check(self.lib.petb200_conv2d_run(plan.h, _ptr(x), b, _ptr(y), _stream()))
+            self.check(self.lib.petb200_conv2d_run(plan.h, _ptr(x), _ptr(bias), _ptr(y), _stream()))
         return y
 
     def conv2d_correct(self, plan, x, y, oh0, ohn, ow0=0, own=None, bias=None):
         """Recompute rows [oh0,oh0+ohn) x cols [ow0,ow0+own) of y from the ORIGINAL input x."""
         own = plan.out_shape[3] - ow0 if own is None else own
-        self.check(self.lib.petb200_conv2d_correct(plan.h, _ptr(_f32(x)), _ptr(bias), _ptr(y), oh0, ohn, ow0, own,
-                                                   _stream()))
+        x, bias = _f32(x), _opt(bias)
+        self.check(self.lib.petb200_conv2d_correct(plan.h, _ptr(x), _ptr(bias), _ptr(y), oh0, ohn, ow0, own, _stream()))
         return y
 
     def conv2d(self, x, w, ph, pw, sh=1, sw=1, dh=1, dw=1, bias=None, act="none", algo="auto", residual=None):
@@ -158,11 +164,12 @@ class Context:
             plan = self._plans[key] = self.conv3d_plan(x.shape, w.shape, pad, stride, dil, bias is not None, act, algo)
         plan._w = _f32(w)
         self.check(self.lib.petb200_conv3d_set_weights(plan.h, _ptr(plan._w), _stream()))
+        x, bias, residual = _f32(x), _opt(bias), _opt(residual)
         y = x.new_empty(plan.out_shape)
         if residual is not None:
-            self.check(self.lib.petb200_conv_run_residual(plan.h, _ptr(_f32(x)), _ptr(bias), _ptr(_f32(residual)), _ptr(y), _stream()))
+            self.check(self.lib.petb200_conv_run_residual(plan.h, _ptr(x), _ptr(bias), _ptr(residual), _ptr(y), _stream()))
         else:
-            self.check(self.lib.petb200_conv3d_run(plan.h, _ptr(_f32(x)), _ptr(bias), _ptr(y), _stream()))
+            self.check(self.lib.petb200_conv3d_run(plan.h, _ptr(x), _ptr(bias), _ptr(y), _stream()))
         return y
 
     # ---- transposed convolution, banded attention products -------------------------------------------------
@@ -187,9 +194,9 @@ class Context:
         if w is not None:
             plan._w = _f32(w)
             self.check(self.lib.petb200_convtrans_set_weights(plan.h, _ptr(plan._w), _stream()))
+        x, bias = _f32(x), _opt(bias)
         y = x.new_empty(plan.out_shape)
-        self.check(self.lib.petb200_convtrans_run(plan.h, _ptr(_f32(x)), _ptr(_f32(bias) if bias is not None else None),
-                                                  _ptr(y), _stream()))
+        self.check(self.lib.petb200_convtrans_run(plan.h, _ptr(x), _ptr(bias), _ptr(y), _stream()))
         return y
 
     def convtrans(self, x, w, ph, pw, sh=1, sw=1, dh=1, dw=1, oph=0, opw=0, bias=None, act="none", algo="auto"):
@@ -257,16 +264,15 @@ class Context:
         self.check(self.lib.petb200_matmul_set_weights(plan.h, _ptr(plan._b), _stream()))
 
     def matmul_run(self, plan, a, b, bias=None, out=None, residual=None):
+        a, b, bias = _f32(a), _opt(b), _opt(bias)
         c = out if out is not None else a.new_empty(plan.out_shape)
         if residual is not None:
             if tuple(residual.shape) != tuple(plan.out_shape):
                 raise L.PetError(L.ERR_INVALID, "residual must have the shape of the output")
-            self.check(self.lib.petb200_matmul_run_residual(plan.h, _ptr(_f32(a)), _ptr(_f32(b) if b is not None else None), _ptr(bias),
-                                                            _ptr(_f32(residual)),
-                                                            _ptr(c), _stream()))
+            residual = _f32(residual)
+            self.check(self.lib.petb200_matmul_run_residual(plan.h, _ptr(a), _ptr(b), _ptr(bias), _ptr(residual), _ptr(c), _stream()))
         else:
-            self.check(self.lib.petb200_matmul_run(plan.h, _ptr(_f32(a)), _ptr(_f32(b) if b is not None else None), _ptr(bias), _ptr(c),
-                                                   _stream()))
+            self.check(self.lib.petb200_matmul_run(plan.h, _ptr(a), _ptr(b), _ptr(bias), _ptr(c), _stream()))
         return c
 
     def matmul(self, a, b, transA=False, transB=False, bias=None, act="none", algo="auto", residual=None):
@@ -404,12 +410,11 @@ class Context:
         return y
 
     def batchnorm(self, x, scale, bias, mean, var, eps=1e-5):
-        x = _f32(x)
+        x, scale, bias, mean, var = (_f32(t) for t in (x, scale, bias, mean, var))
         y = torch.empty_like(x)
         inner = x[0, 0].numel()
-        self.check(self.lib.petb200_batchnorm_run(self.h, _ptr(x), _ptr(_f32(scale)), _ptr(_f32(bias)), _ptr(_f32(mean)),
-                                                  _ptr(_f32(var)), _ptr(y), x.shape[0], x.shape[1], inner, C.c_float(eps),
-                                                  _stream()))
+        self.check(self.lib.petb200_batchnorm_run(self.h, _ptr(x), _ptr(scale), _ptr(bias), _ptr(mean), _ptr(var), _ptr(y), x.shape[0],
+                                                  x.shape[1], inner, C.c_float(eps), _stream()))
         return y
 
     def _pool(self, kind, x, kh, kw, ph, pw, sh, sw):
@@ -497,7 +502,7 @@ class Context:
         return y
 
     def layernorm(self, x, gamma=None, beta=None, eps=1e-5):
-        x = _f32(x)
+        x, gamma, beta = _f32(x), _opt(gamma), _opt(beta)
         y = torch.empty_like(x)
         self.check(self.lib.petb200_layernorm_run(self.h, _ptr(x), _ptr(gamma), _ptr(beta), _ptr(y),
                                                   x.numel() // x.shape[-1], x.shape[-1], C.c_float(eps), _stream()))

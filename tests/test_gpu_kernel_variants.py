@@ -104,3 +104,18 @@ def test_convtrans_phases_back_to_back(ctx, oracle, monkeypatch, n, hw, f, c, k,
     for g, x in zip(got, xs):
         ref = torch.nn.functional.conv_transpose2d(dev(x).double().cpu().permute(0, 3, 1, 2), torch.from_numpy(w).double().permute(2, 3, 0, 1), stride=s, padding=pad)
         assert np.array_equal(g.cpu().numpy(), ref.permute(0, 2, 3, 1).float().numpy())
+
+
+# Operands that are views: each is copied, and the copies have sizes that the allocator could give the same memory
+def test_operands_that_are_views(ctx):
+    rng = np.random.default_rng(3)
+    ints = lambda *s: dev(rng.integers(-3, 4, s).astype(np.float32))
+    a, b, bias, res = ints(2, 64, 96).transpose(1, 2), ints(2, 96, 64).transpose(1, 2), ints(192)[::2], ints(2, 96, 96).transpose(1, 2)
+    assert torch.equal(ctx.matmul(a, b, bias=bias, residual=res).double(), a.double() @ b.double() + bias.double() + res.double())
+    x, r, w = ints(1, 8, 8, 8, 16).transpose(3, 4), ints(1, 8, 8, 8, 16).transpose(3, 4), ints(8, 8, 1, 1, 1)
+    want = torch.nn.functional.conv3d(x.double().cpu(), w.double().cpu(), bias[:8].double().cpu()) + r.double().cpu()
+    assert torch.equal(ctx.conv3d(x, w, (0, 0, 0), bias=bias[:8], residual=r).double().cpu(), want)
+    x, r, w = ints(1, 8, 8, 16).transpose(2, 3), ints(1, 8, 8, 16).transpose(2, 3), ints(8, 8, 1, 1)
+    want = torch.nn.functional.conv2d(x.double().cpu(), w.double().cpu(), bias[:8].double().cpu()) + r.double().cpu()
+    assert torch.equal(ctx.conv2d(x, w, 0, 0, bias=bias[:8], residual=r).double().cpu(), want)
+    ctx.sync_check()
