@@ -118,7 +118,9 @@ int petb200_matmul_plan(petb200_ctx *ctx, int transA, int transB, int b, int m, 
 int petb200_matmul_plan_strided(petb200_ctx *ctx, int transA, int transB, int b, int m, int n, int k, int has_bias, int act,
                                 int algo, const long long strides[6], petb200_plan **out);
 /* Declares B a weight: it is preprocessed once here (hoisted like the reference's weight-only operators,
- * ref: src/Graph/code_engine.cc:187-193) and petb200_matmul_run may then be called with b = NULL. */
+ * ref: src/Graph/code_engine.cc:187-193) and petb200_matmul_run may then be called with b = NULL.  The caller keeps B's
+ * memory valid meanwhile: kernels without a preprocessed operand read it in every run, and a plan that was called with
+ * another B in between preprocesses it again. */
 int petb200_matmul_set_weights(petb200_plan *plan, const float *b, petb200_stream stream);
 int petb200_matmul_run(petb200_plan *plan, const float *a, const float *b, const float *bias, float *c,
                        petb200_stream stream);

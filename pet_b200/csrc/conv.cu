@@ -304,6 +304,7 @@ struct MatmulPlan : petb200_plan {
     void *tc = nullptr;
     DevBuf at; // copy of A with rows that TMA can address, where the caller's are not
     const float *b_weight = nullptr; // set by matmul_set_weights
+    bool weight_packed = false;      // the plan's packed operand is that of b_weight, not of another B passed since
     bool gemv = false;               // m <= 8: matrix-vector kernel
     bool strided = false;            // operands/result addressed through st[] (tensor-core kernel only)
     long long st[6] = {0, 0, 0, 0, 0, 0};
@@ -393,9 +394,11 @@ int matmul_run(petb200_plan *plan, const float *a, const float *b, const float *
         return fail(ctx, PETB200_ERR_INVALID, "matmul run: plan was made with a bias but none was passed");
     if (pl->algo == PETB200_ALGO_TC_3XTF32) {
         const float *at = pl->at.p ? (const float *)pl->at.p : a;
-        int rc = tc_matmul_prepare(pl->tc, b == pl->b_weight ? nullptr : b, pl->at.p ? a : nullptr, (float *)pl->at.p, s);
+        const bool weight = b == pl->b_weight, ready = weight && pl->weight_packed;
+        int rc = tc_matmul_prepare(pl->tc, ready ? nullptr : b, pl->at.p ? a : nullptr, (float *)pl->at.p, s);
         if (rc)
             return rc;
+        pl->weight_packed = weight;
         return tc_matmul_run(pl->tc, at, pl->has_bias ? bias : nullptr, res, c, s);
     }
     if (pl->gemv)
@@ -411,9 +414,11 @@ int matmul_set_weights(petb200_plan *plan, const float *b, cudaStream_t s) {
     if (!pl || !b)
         return PETB200_ERR_INVALID;
     pl->b_weight = b;
+    int rc = PETB200_OK;
     if (pl->algo == PETB200_ALGO_TC_3XTF32)
-        return tc_matmul_pack_b(pl->tc, b, s);
-    return PETB200_OK;
+        rc = tc_matmul_pack_b(pl->tc, b, s);
+    pl->weight_packed = rc == PETB200_OK;
+    return rc;
 }
 
 int MatmulPlan::bench_launch(cudaStream_t s) {

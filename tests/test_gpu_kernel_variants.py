@@ -119,3 +119,15 @@ def test_operands_that_are_views(ctx):
     want = torch.nn.functional.conv2d(x.double().cpu(), w.double().cpu(), bias[:8].double().cpu()) + r.double().cpu()
     assert torch.equal(ctx.conv2d(x, w, 0, 0, bias=bias[:8], residual=r).double().cpu(), want)
     ctx.sync_check()
+
+
+# A plan with a declared weight that is given another B in between: the weight's packed operand has been overwritten and is made again
+@pytest.mark.parametrize("m,k", [(32, 64), (33, 70), (4, 64)])
+def test_matmul_weight_after_another_operand(ctx, m, k):
+    rng = np.random.default_rng(m + k)
+    a, w, other = (dev(rng.integers(-3, 4, s).astype(np.float32)) for s in ((1, m, k), (1, k, 40), (1, k, 40)))
+    plan = ctx.matmul_plan(a.shape, w.shape)
+    ctx.matmul_set_weights(plan, w)
+    for b in (None, other, None, w, other, w):
+        assert torch.equal(ctx.matmul_run(plan, a, b).double(), a.double() @ (w if b is None else b).double())
+    ctx.sync_check()
