@@ -61,3 +61,12 @@ def test_reference_arm_reports_the_same_config_as_the_gpu_arm():
     assert line["impl"] == "reference" and line["config"] == bench.config_for(1)
     assert line["cpu_baseline"]["kind"] in ("reference", "port") and line["cpu_baseline"]["cores"] >= 1
     assert abs(line["value"] * line["ms_per_step"] / 1000.0 - 1.0) < 1e-6   # one image per step: value = 1 / step time
+
+
+def test_reference_arm_runs_the_steps_it_is_asked_for():
+    out = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference", "--steps", "11", "--warmup", "0"],
+                         capture_output=True, text=True, timeout=600)
+    assert out.returncode == 0, out.stderr[-2000:]
+    line = json.loads([l for l in out.stdout.splitlines() if l.startswith("{")][0])
+    assert (line["steps"], line["warmup"]) == (11, 0)
+    assert (line["cpu_baseline"]["kind"] == "port") == ("restatement of the reference's host operators" in line["cpu_baseline"]["sample"])
