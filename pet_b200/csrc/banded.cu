@@ -301,17 +301,6 @@ static void *band_tc_plan(petb200_ctx *ctx, int kind, const void *a, const void 
     return plan;
 }
 
-// Tuning only: per-CTA counters of the tensor-core plans made so far (see IgemmParams::prof), null to stop.
-namespace petb200 {
-void tc_matmul_set_prof(void *h, long long *p);
-}
-extern "C" int petb200_debug_band_prof(petb200_ctx *ctx, long long *dev_counters) {
-    for (auto &e : ctx->band_tc)
-        if (e.plan)
-            tc_matmul_set_prof(e.plan, dev_counters);
-    return PETB200_OK;
-}
-
 // Argument order of the reference's launchers: _sg2bmm(q, k, y, bs, n, m, w, d), src/custom_ops.cu:6-9.
 extern "C" int petb200_g2bmm_run(petb200_ctx *ctx, const float *q, const float *k, float *y, int bs, int n, int m, int w, int d,
                                  petb200_stream stream) {

@@ -13,10 +13,8 @@ void tc_conv_destroy(void *h);
 int tc_conv_set_weights(void *h, const float *w, cudaStream_t s);
 int tc_conv_run(void *h, const float *x, const float *bias, const float *res, float *y, const int *win, cudaStream_t s);
 int tc_conv_row_pitch(void *h);
-void tc_conv_set_prof(void *h, long long *p);
 void tc_conv_set_starve(void *h, int on);
 int tc_set_wait_limit_ns(unsigned long long ns);
-void tc_matmul_set_prof(void *h, long long *p);
 const char *tc_conv_variant(void *h);
 int tc_matmul_create(petb200_ctx *ctx, int bs, int m, int n, int k, int transA, int transB, int has_bias, int act, int passes,
                      const long long *strides, void **out, size_t *dev_bytes);
@@ -442,21 +440,6 @@ int MatmulPlan::bench_launch(cudaStream_t s) {
 }
 
 } // namespace petb200
-
-// Tuning aid (not part of the public header): per-CTA cycle counters of the tensor-core conv kernel, 8 per CTA.
-extern "C" int petb200_debug_conv_prof(petb200_plan *plan, long long *dev_counters) {
-    if (auto *mp = dynamic_cast<petb200::MatmulPlan *>(plan)) {
-        if (!mp->tc)
-            return PETB200_ERR_INVALID;
-        petb200::tc_matmul_set_prof(mp->tc, dev_counters);
-        return PETB200_OK;
-    }
-    auto *pl = dynamic_cast<petb200::ConvPlan *>(plan);
-    if (!pl || !pl->tc)
-        return PETB200_ERR_INVALID;
-    petb200::tc_conv_set_prof(pl->tc, dev_counters);
-    return PETB200_OK;
-}
 
 // Test hooks for the give-up path of the tensor-core kernel's bounded waits (not part of the public header).
 // set_wait_limit: how long a wait on an mbarrier may last on the current device (default 2 s).  conv_starve: while on,

@@ -59,12 +59,6 @@ template <int PP> struct Regs {
                          drain = PP == kSingle ? 184 : (PP == kNarrow ? 152 : 200);
     static_assert(control + 2 * set + drain <= 512, "more registers than the block was launched with: setmaxnreg would wait forever");
 };
-constexpr int kProfSlots = 24; // tuning counters per CTA (see IgemmParams::prof)
-#ifdef PETB200_TUNE
-constexpr bool kTune = true; // a build of its own: the counters cost instructions in every role's inner loop
-#else
-constexpr bool kTune = false;
-#endif
 constexpr int kMaxNB = 6;
 constexpr int kMaxNR = 6;
 
@@ -125,7 +119,6 @@ struct IgemmParams {
     const float *res; // optional residual, laid out like y: y = act(sum + bias + res)
     float *y;
     int *status;
-    long long *prof; // optional per-CTA counters (kProfSlots per CTA), filled by builds with -DPETB200_TUNE only
     int pp;          // persistent mode: a one-dimensional grid of at most one CTA per SM walks all output tiles, CTA i tiles i,
                      // i + gridDim.x, ...
     int tiles, ntiles, mtiles; // persistent mode: all tiles, filter tiles (they vary fastest), pixel tiles
@@ -686,7 +679,6 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
         const __grid_constant__ CUtensorMap tmap_blo, const IgemmParams P) {
     constexpr bool LINK = PP == kSingle && BAND == 0; // may be part of a chain of launches
     extern __shared__ uint8_t smem_raw[];
-    long long *const prof = kTune ? P.prof : nullptr;
     // 1024-byte alignment for the swizzled operand tiles
     uint8_t *smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
     const SmemLayout L = smem_layout(P);
@@ -714,11 +706,6 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
     constexpr bool BF = PASSES == kMathBf16x3;
     constexpr int KE = BF ? 64 : 32;              // K elements per stage
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    long long *prof_cta = nullptr; // wall-clock marks of this CTA (entry, prologue done, epilogue done, exit), tuning only
-    if (prof && threadIdx.x == kSetWarp * 32) {
-        prof_cta = prof + ((size_t)(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * kProfSlots;
-        prof_cta[8] = (long long)ptx::globaltimer_ns();
-    }
     int ntile = PP ? 0 : (int)blockIdx.y / P.ksplit; // (persistent mode: set per tile by set_tile)
     const int ksp = PP ? 0 : (int)blockIdx.y - ntile * P.ksplit;
     int zb = PP ? 0 : (int)blockIdx.z;
@@ -777,8 +764,6 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
         if (!LINK || P.link != kLinkNext)
             ptx::grid_dep_wait();
     }
-    if (prof_cta)
-        prof_cta[9] = (long long)ptx::globaltimer_ns();
 
     // Tile origin in the input: first image, depth slice, row and (16-byte aligned) column of the raw box.  `bx` is the
     // pixel-tile index: blockIdx.x, or in persistent mode every gridDim.x-th tile from there.
@@ -975,8 +960,6 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
             };
             const uint64_t bdesc0 = ptx::smem_desc_k128(ptx::smem_u32(sB));
             const uint32_t b_half16 = b_half >> 4;
-            long long t_wa = 0, t_wf = 0;
-            const long long t_begin = prof ? clock64() : 0;
             const uint32_t BNu = (uint32_t)P.BN, a_col0 = tmem_base + kACol, NB = (uint32_t)P.NB;
             uint32_t tmem_acc = tmem_base, tmem_small = tmem_base + BNu; // main and cross-term accumulators of the tile
             int tiles_left = ntl, stages_end = KS, left = 0; // tiles, end of the tile's K stages, stages left in the flush group
@@ -993,10 +976,8 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
             bool ready = false, next_ready = false; // the current / the next stage has been seen complete
             auto wait_stage = [&]() {
                 if (__builtin_expect(!ready, 0)) {
-                    const long long q0 = prof ? clock64() : 0;
                     if (!ptx::mbar_wait(a_full + sa, pa, abort_flag) || !ptx::mbar_wait(b_full + sb, pb, abort_flag))
                         give_up();
-                    t_wa += prof ? clock64() - q0 : 0;
                 }
                 ptx::tc_fence_after();
             };
@@ -1068,12 +1049,10 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                     ptx::tc_fence_after();
                     cross_terms(n.sa, bdesc0 + (uint64_t)(n.sb * 2u * b_half16));
                 }
-                const long long q2 = prof ? clock64() : 0;
                 if (!ptx::mbar_wait(flushed, gpar, abort_flag)) {
                     give_up();
                     return;
                 }
-                t_wf += prof ? clock64() - q2 : 0;
                 gpar ^= 1u;
                 ptx::tc_fence_after();
                 main_terms(0u);
@@ -1095,12 +1074,10 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                     tmem_acc = tmem_base + (uint32_t)reg * 2u * BNu;
                     tmem_small = tmem_acc + BNu;
                     if (use >= 1) {
-                        const long long q3 = prof ? clock64() : 0;
                         if (!ptx::mbar_wait(acc_empty + reg, (uint32_t)((use - 1) & 1), abort_flag)) {
                             give_up();
                             break;
                         }
-                        t_wf += prof ? clock64() - q3 : 0;
                         ptx::tc_fence_after();
                     }
                 }
@@ -1118,10 +1095,6 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                 if (ok)
                     ptx::mma_commit((two_regions && (tl & 1)) ? acc_full1 : acc_full);
             }
-            if (prof) {
-                long long *pr = prof + ((size_t)(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * kProfSlots;
-                pr[0] = t_wa, pr[2] = clock64() - t_begin, pr[16] = t_wf;
-            }
         }
         __syncwarp();
     } else if (warp >= kSetWarp && warp < kDrainWarp) {
@@ -1136,8 +1109,6 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
         const int quarter = warp & 3;            // TMEM lane quarter this warp may access
         const int p = quarter * 32 + lane;       // pixel row inside the tile
         bool alive = true;
-        long long t_we = 0, t_wr = 0, t_g = 0, t_st = 0;
-        const long long t_begin = prof ? clock64() : 0;
         const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16);
         // This set's stages are number tset, tset + 2, ... of the CTA (all tiles in a row): `st` is the next one's index inside
         // the current chunk, `sa` / `pa` its A slot and the parity to wait for (first pass over the ring: every slot is free).
@@ -1195,10 +1166,7 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                         if (!alive)
                             break;
                     }
-                    const long long cr0 = prof ? clock64() : 0;
                     raw_ok = ptx::mbar_wait(raw_full + rb, prw, abort_flag) && raw_ok; // also by a set without a stage in this chunk
-                    if (prof)
-                        t_wr += clock64() - cr0;
                     const float *raw = reinterpret_cast<const float *>(sRaw + (size_t)rb * P.raw_bytes) + base_p;
                     for (; st < P.spc && alive; st += 2) {
                         const int *ko = sKoff + st * KE;
@@ -1209,7 +1177,6 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                         // registers on top of its slots in the ring.  (Announcing a stage only after the next one's gather,
                         // to hide the 200 to 250 cycles of the stores, was 8 % slower: the MMA thread starts later.)
                         uint32_t hi[32], lo[32];
-                        const long long cg0 = prof ? clock64() : 0;
                         if constexpr (MODE == kGatherBand) {
                             const int i = bx * kTileM + p, k0 = ((bx * kTileM - P.band_w) & ~3) + ((c0 + ch) * kBandStages + st) * kStageK;
                             const int j0 = k0 - i + P.band_w; // band column of the stage's first key
@@ -1255,7 +1222,6 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                                 split_words<PASSES>(v, hi + 8 * c, lo + 8 * c);
                             }
                         }
-                        const long long ce0 = prof ? clock64() : 0;
                         if (__builtin_expect(!__all_sync(0xffffffffu, slot_free && raw_ok), 0)) {
                             raw_ok = __all_sync(0xffffffffu, raw_ok) != 0;
                             alive = raw_ok && ptx::mbar_wait_warp(a_empty + sa, pa, abort_flag);
@@ -1263,15 +1229,12 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                                 break;
                         }
                         ptx::tc_fence_after();
-                        const long long cg1 = prof ? clock64() : 0;
                         const uint32_t t = t_row + kACol + sa * 64u;
                         ptx::tmem_st_32x32(t, hi);
                         if (SPLIT)
                             ptx::tmem_st_32x32(t + 32u, lo);
                         ptx::tmem_st_wait();
                         ptx::tc_fence_before();
-                        if (prof)
-                            t_we += cg1 - ce0, t_g += ce0 - cg0, t_st += clock64() - cg1;
                         __syncwarp();
                         if (lane == 0)
                             ptx::mbar_arrive(a_full + sa);
@@ -1302,8 +1265,6 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
         } else {
             transform(std::integral_constant<int, kGatherTable>());
         }
-        const long long t_loop = prof ? clock64() - t_begin : 0;
-        long long t_epi0 = t_loop;
         if (!PP) {
             // ---------------- epilogue of the only tile ----------------
             // Addresses and store mode first: the MMA thread is still working through the last stages, so this costs nothing.
@@ -1324,7 +1285,6 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                 alive = ptx::mbar_wait_warp(acc_full, 0u, abort_flag);
             if (SPLIT && P.fl > 0) // the drain warps have written total + last group over the main accumulator
                 ptx::named_bar_sync(1, 384);
-            t_epi0 = prof ? clock64() : 0;
             if (alive && P.ksplit > 1) {
                 // Split-K: column c of the tile is summed by CTA c / cols of the cluster.  Push this CTA's partial sum into that
                 // CTA's shared memory, slot [this rank][c % cols][pixel] (consecutive lanes = consecutive words).
@@ -1383,11 +1343,6 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                 });
             }
         }
-        if (prof_cta) { // lane 0 of the first warp of set 0
-            prof_cta[3] = t_we, prof_cta[4] = t_wr, prof_cta[5] = t_loop, prof_cta[6] = clock64() - t_epi0, prof_cta[7] = t_epi0 - t_begin;
-            prof_cta[10] = (long long)ptx::globaltimer_ns();
-            prof_cta[12] = t_g, prof_cta[13] = t_st;
-        }
     } else if (warp >= kDrainWarp) {
         // ---------------- drain warps: running totals of flushed accumulators; persistent mode: the epilogue ----------------
         ptx::reg_alloc<Regs<PP>::drain>();
@@ -1396,15 +1351,12 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
         const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16);
         bool alive = true;
         uint32_t gpar = 0; // parity of the next completed group
-        long long t_dw = 0, t_dd = 0, t_acc = 0, t_store = 0;
         if (BAND == 1) {
             for (int tl = 0; tl < ntl && alive; ++tl) {
                 set_tile((int)blockIdx.x + tl * (int)gridDim.x);
-                const long long cd0 = prof ? clock64() : 0;
                 alive = ptx::mbar_wait_warp((tl & 1) ? acc_full1 : acc_full, (uint32_t)((tl >> 1) & 1), abort_flag);
                 if (!alive)
                     break;
-                const long long cd1 = prof ? clock64() : 0;
                 ptx::tc_fence_after();
                 const uint32_t tacc = t_row + (uint32_t)((tl & 1) * 2 * P.BN);
                 epilogue_banded<PASSES>(tacc, tacc + (uint32_t)P.BN, 0, P.BN, ntile * P.BN, quarter * 32, bx, zb, P.m_rows, P.band_w, P.y,
@@ -1413,14 +1365,12 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                 __syncwarp();
                 if (lane == 0)
                     ptx::mbar_arrive(acc_empty + (tl & 1));
-                if (prof)
-                    t_dw += cd1 - cd0, t_dd += clock64() - cd1;
             }
         } else if (PP || FL > 0) {
             float *stage = reinterpret_cast<float *>(smem + L.stage_off) + quarter * 1024;
             auto drain = [&](auto mode_c, auto res_c) {
-            constexpr int MODE = decltype(mode_c)::value;
-            constexpr bool RES = decltype(res_c)::value;
+            [[maybe_unused]] constexpr int MODE = decltype(mode_c)::value; // (a single tile stores nothing here)
+            [[maybe_unused]] constexpr bool RES = decltype(res_c)::value;
             for (int tl = 0; tl < ntl && alive; ++tl) {
                 const int reg = two_regions ? (tl & 1) : 0, use = two_regions ? (tl >> 1) : tl;
                 StoreJob J;
@@ -1436,13 +1386,12 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                     J.nvalid = __popc(__ballot_sync(0xffffffffu, J.valid));
                     J.y_off0 = __shfl_sync(0xffffffffu, J.y_off, 0);
                 }
-                const uint32_t tmain = t_row + (uint32_t)(reg * 2 * P.BN), tcross = tmain + (uint32_t)P.BN;
+                const uint32_t tmain = t_row + (uint32_t)(reg * 2 * P.BN);
+                [[maybe_unused]] const uint32_t tcross = tmain + (uint32_t)P.BN;
                 float racc[PP == kNarrow ? 32 : 128]; // the sums of this thread's tile row (narrow: of the block being stored)
                 auto take_acc_full = [&]() {
-                    const long long c0 = prof ? clock64() : 0;
                     alive = ptx::mbar_wait_warp(reg ? acc_full1 : acc_full, (uint32_t)(use & 1), abort_flag);
                     ptx::tc_fence_after();
-                    t_acc += prof ? clock64() - c0 : 0;
                 };
                 auto release = [&]() { // the MMA thread may start the region's next tile
                     ptx::tc_fence_before();
@@ -1474,19 +1423,15 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                 } else {
                     // Groups in order, round-to-nearest adds; the MMA thread restarts the main accumulator once a group has been taken.
                     for (int g = 0; g + 1 < n_groups && alive; ++g, gpar ^= 1u) {
-                        const long long cd0 = prof ? clock64() : 0;
                         alive = ptx::mbar_wait_warp(acc_ready, gpar, abort_flag);
                         if (!alive)
                             break;
-                        const long long cd1 = prof ? clock64() : 0;
                         ptx::tc_fence_after();
                         drain_add<false>(racc, tmain, 0u, P.BN, g == 0);
                         ptx::tc_fence_before();
                         __syncwarp();
                         if (lane == 0)
                             ptx::mbar_arrive(flushed);
-                        if (prof)
-                            t_dw += cd1 - cd0, t_dd += clock64() - cd1;
                     }
                     if (alive)
                         take_acc_full();
@@ -1508,7 +1453,6 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                     } else {
                         drain_add<SPLIT>(racc, tmain, tcross, P.BN, n_groups == 1);
                         release();
-                        const long long cs0 = prof ? clock64() : 0;
 #pragma unroll 1
                         for (int c = 0; c < P.BN; c += 32) {
                             store_block<MODE, RES>(J, racc, stage, ntile * P.BN + c);
@@ -1516,7 +1460,6 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                             for (int j = 0; j < 96; ++j) // the next block's sums move down
                                 racc[j] = racc[j + 32];
                         }
-                        t_store += prof ? clock64() - cs0 : 0;
                     }
                 }
             }
@@ -1527,10 +1470,6 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
                 with_store_mode(store_mode(), P.res != nullptr, drain);
             if (!PP && FL > 0) // (also after a wait gave up: the transform sets wait here)
                 ptx::named_bar_sync(1, 384);
-        }
-        if (prof && threadIdx.x == kDrainWarp * 32) {
-            long long *pr = prof + ((size_t)(blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * kProfSlots;
-            pr[17] = t_dw, pr[18] = t_dd, pr[19] = t_acc, pr[21] = t_store;
         }
     }
 
@@ -1554,8 +1493,6 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
             }
         }
         ptx::cluster_sync_all(); // every CTA's pushes have landed; nothing touches a peer's memory after this
-        if (prof_cta)
-            prof_cta[14] = (long long)ptx::globaltimer_ns();
         if (warp >= kSetWarp && warp < kDrainWarp) {
             const int et = threadIdx.x - kSetWarp * 32;
             const long long y_off = sYoff[et & (kTileM - 1)];
@@ -1581,8 +1518,6 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
 #undef PETB200_RED
             }
         }
-        if (prof_cta)
-            prof_cta[15] = (long long)ptx::globaltimer_ns();
     }
 
     // ---------------- teardown ----------------
@@ -1600,8 +1535,6 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
         ptx::tmem_dealloc(tmem_base, kTmemCols);
     if (LINK && P.link == kLinkNext) // whoever waits for this launch waits for the ones before it in the chain too
         ptx::grid_dep_wait();
-    if (prof_cta)
-        prof_cta[11] = (long long)ptx::globaltimer_ns();
 }
 
 // -------------------------------------------------------------------------------------------------------------
@@ -1678,7 +1611,7 @@ __global__ void __launch_bounds__(256) k_prepare_mm(const PrepareArgs g) {
     const int k0 = tk * 32, n0 = tn * 32;
     // packed position -> row of B: chunk * Kc_pad + element of the chunk (BC of them, then padding; Kc_pad a multiple of 32)
     const int ch = g.by_kc_pad.div(k0), kc0 = k0 - ch * (int)g.by_kc_pad.d, kk0 = ch * g.BC + kc0, kn = min(min(g.BC - kc0, g.k - kk0), 32);
-    if (TRANSB) {
+    if constexpr (TRANSB) {
 #pragma unroll
         for (int i = 0; i < 32; i += 8) {
             const int nn = n0 + warp + i;
@@ -1686,17 +1619,17 @@ __global__ void __launch_bounds__(256) k_prepare_mm(const PrepareArgs g) {
             if (nn < g.n)
                 store_split<BF>(g.hi, g.lo, ((long long)bb * g.n + nn) * g.Kpad + k0 + lane, v, g.rna);
         }
-        return;
-    }
+    } else {
 #pragma unroll
-    for (int i = 0; i < 32; i += 8)
-        tile[warp + i][lane] = warp + i < kn && n0 + lane < g.n ? __ldg(src + (kk0 + warp + i) * g.sb_row + n0 + lane) : 0.f;
-    __syncthreads();
+        for (int i = 0; i < 32; i += 8)
+            tile[warp + i][lane] = warp + i < kn && n0 + lane < g.n ? __ldg(src + (kk0 + warp + i) * g.sb_row + n0 + lane) : 0.f;
+        __syncthreads();
 #pragma unroll
-    for (int i = 0; i < 32; i += 8) {
-        const int nn = n0 + warp + i;
-        if (nn < g.n)
-            store_split<BF>(g.hi, g.lo, ((long long)bb * g.n + nn) * g.Kpad + k0 + lane, tile[lane][warp + i], g.rna);
+        for (int i = 0; i < 32; i += 8) {
+            const int nn = n0 + warp + i;
+            if (nn < g.n)
+                store_split<BF>(g.hi, g.lo, ((long long)bb * g.n + nn) * g.Kpad + k0 + lane, tile[lane][warp + i], g.rna);
+        }
     }
 }
 
@@ -1744,7 +1677,6 @@ struct TcCore {
     CUtensorMap map_x{}, map_bhi{}, map_blo{};
     const void *map_x_ptr = nullptr;
     bool weights_ready = false;
-    long long *prof = nullptr;
     int starve = 0;
 
     KernelFn kernel() const {
@@ -1838,7 +1770,6 @@ struct TcCore {
         p.y = y;
         p.koff = (const int *)koff.p;
         p.status = ctx->d_status;
-        p.prof = prof;
         p.starve = starve;
         p.has_bias = (P.has_bias && bias) ? 1 : 0;
         KernelFn kern = kernel();
@@ -2461,7 +2392,6 @@ void tc_conv_out_dims(void *h, int *d5) {
     d5[3] = t->g.OH;
     d5[4] = t->g.OW;
 }
-void tc_conv_set_prof(void *h, long long *p) { ((TcConv *)h)->full.prof = p; }
 void tc_conv_set_starve(void *h, int on) { ((TcConv *)h)->full.starve = on; }
 int tc_set_wait_limit_ns(unsigned long long ns) {
     return cudaMemcpyToSymbol(ptx::g_mbar_wait_limit_ns, &ns, sizeof ns) == cudaSuccess ? PETB200_OK : PETB200_ERR_CUDA;
@@ -2781,7 +2711,6 @@ int tc_gbmml_run(void *h, const float *p, float *y, cudaStream_t s) {
     return t->core.launch(p, nullptr, nullptr, y, s); // (the activation map is encoded over p but never used by this mode)
 }
 
-void tc_matmul_set_prof(void *h, long long *p) { ((TcMatmul *)h)->core.prof = p; }
 // Words of the copy of A that a call needs (0: A is consumed as it is).
 long long tc_matmul_a_copy(void *h) {
     auto *t = (TcMatmul *)h;

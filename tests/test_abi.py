@@ -32,6 +32,19 @@ def test_library_builds_and_exports_every_declared_symbol():
     assert sorted(graph.GRAPH_SYMBOLS) == graph_names
 
 
+def test_entry_points_outside_the_headers_are_test_hooks():
+    """What the library defines beyond its headers is there for a test: an entry point that nothing calls is dead code."""
+    defined = set()
+    csrc = os.path.join(ROOT, "pet_b200", "csrc")
+    for f in os.listdir(csrc):
+        if f.endswith(".cu"):
+            defined |= set(re.findall(r'extern "C"[^;{(]*?\b(petb200_[a-z0-9_]+)\s*\(', open(os.path.join(csrc, f)).read()))
+    extra = defined - set(declared_symbols()) - set(declared_symbols("petb200_graph.h"))
+    here = os.path.join(ROOT, "tests")
+    tests = "".join(open(os.path.join(here, f)).read() for f in os.listdir(here) if f.endswith(".py"))
+    assert len(defined) >= 75 and not [n for n in extra if n not in tests]
+
+
 def test_status_strings_and_ctx_create_without_gpu():
     from pet_b200 import lib
     l = lib.load()
