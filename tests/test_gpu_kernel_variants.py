@@ -14,9 +14,11 @@ def dev(a):
     return torch.from_numpy(np.ascontiguousarray(a)).cuda()
 
 
-# n around a block of 128 (B as [k][n]) or 32 (B as [n][k]) columns; k below one warp pass, around a shared-memory tile of A
-# (512 / 1024 values) and past a split over a whole cluster; rows of B on and off the 16-byte grid
-@pytest.mark.parametrize("n,k", [(1, 1), (31, 69), (128, 8), (129, 511), (260, 1025), (33, 2052), (100, 9001), (4100, 640)])
+# n around a block of 128 (B as [k][n]) or 32 (B as [n][k]) columns; k below one warp pass, at a split over a whole cluster of eight
+# and, with that split, at slices of one shared-memory tile of A (512 values for m > 4, else 1024) and of one value more; rows of B
+# on and off the 16-byte grid
+@pytest.mark.parametrize("n,k", [(1, 1), (31, 69), (128, 8), (129, 511), (260, 1025), (33, 2052), (100, 9001), (4100, 640),
+                                 (100, 4096), (100, 4097), (100, 8192), (100, 8193)])
 @pytest.mark.parametrize("m,trans_a,trans_b", [(1, False, False), (1, False, True), (2, True, False), (3, False, True), (8, True, True), (8, False, False)])
 def test_matrix_vector_products_exact(ctx, m, trans_a, trans_b, n, k):
     rng = np.random.default_rng(n + k + m)
@@ -66,9 +68,10 @@ def test_conv_persistent_tiles_stores(ctx, n, c, h, w, f, act):
         assert torch.equal(got.cpu(), want.float()) if act != "sigmoid" else rel_err(got.cpu().numpy(), want.numpy()) <= TOL
 
 
-# last register-resident rows of a warp, of a block, and the first row past them; fewer rows than a wave of blocks
-@pytest.mark.parametrize("cols", [1024, 1025, 1279, 2048, 2049, 4095, 4096, 4097])
-@pytest.mark.parametrize("rows", [1, 3, 700])
+# last register-resident rows of a warp (enough of them for a warp each: 1300), of a block, and the first row past them; fewer rows
+# than a wave of blocks, and more than there are blocks (a block then takes several)
+@pytest.mark.parametrize("rows,cols", [(r, c) for c in (255, 256, 1024, 1025, 1279, 2048, 2049, 4095, 4096, 4097) for r in (1, 3, 700, 1300)] +
+                         [(9600, 1025), (9600, 4097)])
 def test_softmax_rows_by_length(ctx, oracle, rows, cols):
     x = np.random.default_rng(cols).standard_normal((rows, cols)).astype(np.float32) * 4
     x[0, cols - 1] = 40.0
