@@ -283,7 +283,7 @@ int petb200_matmul_splitk_noalloc(int transA, int transB, int b, int m, int n, i
  * Times `rounds` launches of a conv/matmul/layout plan after `warmup` launches on plan-owned scratch operands filled
  * with a fixed pattern, with CUDA events on the given stream; the counterpart of the loops in ConvOp::perf /
  * MatmulOp::perf (ref: src/Graph/operator.cc:416-467,770-812), which use wall clock around cudaDeviceSynchronize.
- * Returns milliseconds per launch through *ms. */
+ * A plan whose weights have been set is timed with them and keeps them.  Returns milliseconds per launch through *ms. */
 int petb200_plan_time(petb200_plan *plan, int rounds, int warmup, float *ms, petb200_stream stream);
 
 #ifdef __cplusplus

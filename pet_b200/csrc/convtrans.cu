@@ -308,15 +308,17 @@ int convtrans_out_dims(const petb200_plan *plan, int *nhwc) {
 int ConvTransPlan::bench_launch(cudaStream_t st) {
     if (!bx.p) {
         const size_t nx = (size_t)g.n * g.h * g.w * g.f, nw = (size_t)r * s * g.f * c, ny = (size_t)g.n * oh * ow * c;
-        if (bx.alloc(nx * 4) != cudaSuccess || bw.alloc(nw * 4) != cudaSuccess || by.alloc(ny * 4) != cudaSuccess ||
-            bb.alloc((size_t)c * 4) != cudaSuccess)
+        if (bx.alloc(nx * 4) != cudaSuccess || by.alloc(ny * 4) != cudaSuccess || bb.alloc((size_t)c * 4) != cudaSuccess ||
+            (!weights_ready && bw.alloc(nw * 4) != cudaSuccess))
             return fail(ctx, PETB200_ERR_NOMEM, "scratch allocation for timing failed");
         cudaMemsetAsync(bx.p, 0x3c, nx * 4, st); // 0x3c3c3c3c is 0.0115 as fp32
-        cudaMemsetAsync(bw.p, 0x3c, nw * 4, st);
         cudaMemsetAsync(bb.p, 0, (size_t)c * 4, st);
-        int rc = convtrans_set_weights(this, (const float *)bw.p, st);
-        if (rc)
-            return rc;
+        if (!weights_ready) { // (a plan that has its weights is timed with them and keeps them)
+            cudaMemsetAsync(bw.p, 0x3c, nw * 4, st);
+            int rc = convtrans_set_weights(this, (const float *)bw.p, st);
+            if (rc)
+                return rc;
+        }
     }
     return convtrans_run(this, (const float *)bx.p, has_bias ? (const float *)bb.p : nullptr, (float *)by.p, st);
 }

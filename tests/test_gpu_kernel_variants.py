@@ -134,3 +134,36 @@ def test_matmul_weight_after_another_operand(ctx, m, k):
     for b in (None, other, None, w, other, w):
         assert torch.equal(ctx.matmul_run(plan, a, b).double(), a.double() @ (w if b is None else b).double())
     ctx.sync_check()
+
+
+# Timing a plan or a graph leaves its weights as they are
+@pytest.mark.parametrize("algo", ["auto", "simt_fp32"])
+def test_timing_keeps_the_weights(ctx, algo, monkeypatch):
+    from pet_b200 import configs
+    from pet_b200.graph import Graph
+    x, w = torch.randn(2, 16, 12, 12, device="cuda"), torch.randn(24, 16, 3, 3, device="cuda")
+    plan = ctx.conv2d_plan(x.shape, w.shape, 1, 1, algo=algo)
+    ctx.conv2d_set_weights(plan, w)
+    before = ctx.conv2d_run(plan, x)
+    plan.time(rounds=2, warmup=1)
+    assert torch.equal(ctx.conv2d_run(plan, x), before)
+    for phases in ("0", "1"):
+        monkeypatch.setenv("PETB200_CONVTRANS_PHASES", phases)
+        wt = torch.randn(4, 4, 16, 8, device="cuda")
+        plan = ctx.convtrans_plan((2, 12, 12, 16), wt.shape, 1, 1, 2, 2, algo=algo)
+        xt = torch.randn(2, 12, 12, 16, device="cuda")
+        before = ctx.convtrans_run(plan, xt, wt)
+        plan.time(rounds=2, warmup=1)
+        assert torch.equal(ctx.convtrans_run(plan, xt), before)
+    graph = Graph(ctx)
+    b = configs.GraphBuilder(graph)
+    out = b.matmul(b.reshape(b.conv(b.input(x.cpu().numpy()), b.const(w.cpu().numpy()), 1, 1), [1, 2 * 24, 144]), b.const(np.ones((1, 144, 16), np.float32)))
+    graph.setOutputs([out])
+    graph.compile()
+    b.load()
+    graph.run()
+    before = graph.get_data(out).copy()
+    graph.perf(rounds=2, warmup=1)
+    graph.run()
+    assert np.array_equal(graph.get_data(out), before)
+    ctx.sync_check()
