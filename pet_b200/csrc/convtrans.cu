@@ -172,10 +172,14 @@ int make_convtrans_plan(petb200_ctx *ctx, const int *a /*n,c,h,w,f,r,s,ph,pw,sh,
     pl->device_bytes = pl->conv->device_bytes + xe_bytes + w_bytes;
     pl->sh = sh, pl->sw = sw;
     // Phase decomposition: sh*sw + 1 launches, the phases side by side, of 1 / (sh*sw) of the zero-inserted product's work.
-    // Measured on B200: the zero-inserted path takes about 10 us plus its work at 100 TFLOP/s, the phases 8 us plus 2.2 us each
-    // (their launches) or their work at 120 TFLOP/s; 2 x 32 x 32 x 64 -> 32, 4 x 4 stride 2 lies on the line (19 and 15 us on the
-    // GPU, 22 and 24 us from call to call), 4 x 24 x 24 x 96 -> 48, 6 x 6 stride 3 takes 94 and 26 us.  Needs taps in every
-    // phase and a row stride of y that is a whole number of phase pixels.
+    // The zero-inserted path is taken to last 10 us plus its work at 100 TFLOP/s, the phases 8 us plus 2.2 us each (their launches)
+    // or their work at 120 TFLOP/s: what both were measured to take from call to call.  On 80 shapes (filters of 2 and 4 and 5 at stride 2,
+    // 6 at stride 3, 8 at stride 4; 1 to 16 images of 8 x 8 to 64 x 64, 32 to 512 channels) the choice is within 5 % of the
+    // better path on 76, measured call to call, and on 69 inside a CUDA graph, where the phases' launches cost less; it never
+    // takes the phases where they lose.  Where it is wrong both are short: 4 x 32 x 32 x 64 -> 32, 2 x 2 stride 2, 24 us against 17;
+    // 1 x 32 x 32 x 64 -> 32, 5 x 5 stride 2, 25 against 17; on the line lies 2 x 32 x 32 x 64 -> 32, 4 x 4 stride 2, 19 against
+    // 18 (20 and 16 in a graph).  Far from it: 8 x 32 x 32 x 128 -> 64, 4 x 4 stride 2, 80 against 28.  Needs taps in every phase
+    // and a row stride of y that is a whole number of phase pixels.
     const double issued = 2.0 * n * c * (double)oh * ow * f * r * s;
     const double us_inserted = 10.0 + issued / 100e6, us_phased = 8.0 + std::max(2.2 * sh * sw, issued / (sh * sw) / 120e6);
     const bool tc_algo = tc_is_tc_algo(algo);
@@ -276,7 +280,7 @@ int convtrans_run(petb200_plan *plan, const float *x, const float *bias, float *
             return rc;
         // The phases write disjoint pixels of y and each fills only part of the GPU, so they run side by side: a chain of launches
         // in the caller's stream that wait for the layout pass but not for one another.  (Four streams, forked and joined with
-        // events, took 45 us for 8 x 32 x 32 x 128 -> 64, 4 x 4 stride 2; this takes 27.)
+        // events, took 45 us for 8 x 32 x 32 x 128 -> 64, 4 x 4 stride 2; this takes 28.)
         bool chain = pl->phases.size() > 1;
         for (Phase *ps : pl->phases)
             chain = chain && tc_conv_can_link(ps->tc);

@@ -2,28 +2,27 @@
 //
 //   D[pixel, filter] = sum_k A[pixel, k] * B[filter, k]            k = (channel chunk, tap, channel in chunk)
 //
-// One CTA computes a 128-pixel x BN-filter tile; the fp32 accumulator lives in tensor memory (TMEM).
-//   warp 0   : TMA producer for the packed weights: per 32-wide K stage one 2-D tile of B_hi and one of B_lo,
-//              straight into 128-byte-swizzled K-major shared memory.
-//   warp 2   : TMA producer for the RAW activation tile of one channel chunk (all taps share it): a 5-D box
-//              [images, channels, depth, rows, cols] of the NC(D)HW input, zero-filled outside the tensor, which
-//              is exactly the convolution's zero padding.  Box start along W is rounded down to 16 bytes.
-//   warps 3-6, 7-10: two transform sets taking alternate K stages.  Thread p owns pixel p of the tile: for every K stage it
-//              gathers its 32 values from the raw tile (fixed strides where the channel chunk allows, else through a
-//              precomputed offset table: tap shift, dilation, channel plane), splits each fp32
-//              into hi (top 19 bits) and lo = x - hi, and writes the two K-major operand tiles — into swizzled
-//              shared memory (SS variant) or directly into TMEM with tcgen05.st (TS variant, which leaves the
-//              shared-memory read port to B alone).  The same warps run the epilogue.
-//   warp 1   : issues, per K=8 step, the three products of 3xTF32 as two MMAs — A_hi x [B_hi;B_lo] (one MMA of width
-//              2*BN: the hi*hi sum and the hi*lo sum in adjacent accumulators) and A_lo x B_hi — and commits the stage
-//              release barriers.
-// Epilogue: tcgen05.ld -> +bias -> activation -> global stores, coalesced across the 32 pixels of a warp (conv)
-// or 128-bit per thread (row-major matmul output).
+// A tile is 128 pixels x BN filters (BN = 32, 64 or 128); a CTA computes one, or several in turn (persistent tiles).  The fp32
+// accumulators and the A operand live in tensor memory (TMEM).  Sixteen warps:
+//   0      TMA producer for the packed weights: per K stage (32 words of K) one 2-D tile of B_hi and one of B_lo, straight into
+//          128-byte-swizzled K-major shared memory.
+//   1      one thread issues, per K=8 step, the three products of 3xTF32 as two MMAs — A_hi x [B_hi;B_lo] (one MMA of width
+//          2*BN: the hi*hi sum and the hi*lo sum in adjacent accumulators) and A_lo x B_hi — and commits the stage release
+//          barriers.
+//   2      TMA producer for the RAW activation tile of one channel chunk (all taps share it): a 5-D box
+//          [images, channels, depth, rows, cols] of the NC(D)HW input, zero-filled outside the tensor, which is exactly the
+//          convolution's zero padding.  Box start along W is rounded down to 16 bytes.  (3 is idle.)
+//   4-7, 8-11  two transform sets taking alternate K stages.  Thread p owns pixel p of the tile: for every K stage it gathers its
+//          32 values from the raw tile (fixed strides where the channel chunk allows, else through a precomputed offset table:
+//          tap shift, dilation, channel plane), splits each fp32 into hi (top 19 bits) and lo = x - hi, and writes both to
+//          TMEM with tcgen05.st, which leaves the shared-memory read port to B alone.  With one tile per CTA they also store it.
+//   12-15  drain warps.  The tensor core truncates its fp32 accumulator after every MMA, so long K ranges empty the main
+//          accumulator every few stages into a running total that these warps hold.  With persistent tiles they store a finished
+//          tile (tcgen05.ld -> +bias -> activation -> global stores in the way the layout of y allows, see store_block) while
+//          the transform sets run on into the next.
 //
 // Variants (template parameters): 3xTF32 (default), one TF32 pass, error-compensated bf16 (64 K elements per stage, K = 16 per
-// MMA); persistent tiles (a CTA walks several pixel tiles, the transform sets run on into the next tile while the drain warps
-// store the last one).  Long K ranges drain the main accumulator into a
-// running total every few stages (the tensor core truncates its fp32 accumulator after every MMA).
+// MMA); one tile per CTA or persistent tiles; the banded products.
 // Split-K: the ksplit CTAs of one output tile form a thread-block cluster and exchange their partial sums through
 // distributed shared memory (pushes into the owner's landing area, one cluster barrier, reduction in rank order).
 // Every wait on an mbarrier is bounded (~2 s) and reports through a status word instead of hanging the GPU.
@@ -54,6 +53,9 @@ constexpr int kNA = 4; // A stages in TMEM: a transform set owns slots `set` and
 enum { kSingle = 0, kNarrow = 1, kWide = 2 };
 // Registers per thread of the four warp groups (512 in sum, what the block is launched with): drain warps that keep a row of 128
 // sums need 184 or more; in single-tile mode the transform sets also run the epilogue.
+// The compiler sees one limit for all roles (128 a thread) and spills in the persistent instantiations: 3xTF32 wide 76 bytes
+// stored / 176 loaded (convolutions), 64 / 152 (matmul), narrow 68 / 100 and 56 / 76, banded 20 / 28 .. 60 / 144, bf16 up to
+// 140 / 328; single-tile instantiations none.
 template <int PP> struct Regs {
     static constexpr int control = PP == kSingle ? 56 : 72, set = PP == kSingle ? 136 : (PP == kNarrow ? 144 : 120),
                          drain = PP == kSingle ? 184 : (PP == kNarrow ? 152 : 200);
@@ -1818,12 +1820,6 @@ static int env_int(const char *name, int dflt) {
     return v ? atoi(v) : dflt;
 }
 
-// Fills core.P (tiling, raw box, stage counts) for a window [oh0,ohn) x [ow0,own) of the output; returns
-// PETB200_ERR_UNSUPPORTED when the shape does not fit this kernel's constraints.
-// Rough cycle model of one launch, used to pick the tile width and the K split for problems that cannot fill the GPU
-// with 128-wide tiles.  Constants are measured on B200: a K stage costs its MMAs (N/2 cycles each, 12 per stage for
-// 3xTF32, 4 for one pass) or, if larger, the transform chain of the stage (~330 cycles with two warp sets); a CTA pays
-// ~3000 cycles before its first MMA and 1700 + 44*BN cycles of epilogue (split-K: the exchange through the cluster instead).
 // How many clusters of `ks` CTAs of this kernel (one CTA per SM) the device can hold at once: asked of the driver once
 // per size (clusters stay inside a GPC, which leaves some SMs of every GPC without a cluster).
 static int cluster_slots(int sm_count, int ks) {
@@ -1853,6 +1849,16 @@ static int cluster_slots(int sm_count, int ks) {
     return cached[ks];
 }
 
+// Rough cycle model of one launch, used to pick the tile width and the K split.  A K stage is charged its MMAs (N/2 cycles each,
+// 12 per stage for 3xTF32, 4 for one pass) or 520 cycles, a CTA 3000 cycles before its first MMA and 1700 + 44*BN of epilogue
+// (split-K: the exchange through the cluster instead), every wave of CTAs the sum.
+// These constants rank the choices; they don't predict times.  With persistent tiles, where start-up and epilogue hide, a 3xTF32
+// stage was measured to take about 1000 cycles at 128 filters (charged 768), 690 at 64 and 570 at 32 (charged 520).  Against the
+// fastest of all (width, split) pairs, forced one by one, on 44 shapes (every convolution of ResNet-18 at batch 1, 8 and 64 and
+// of ResNet3D-18, the 512-channel dilated one, the projections of an encoder of 768 at 128 and 384 rows), the choice is
+// within 2 % on 38.  The other six lose 6 to 34 % because 128-filter tiles, five times with K split in two, are preferred to unsplit
+// 64-filter ones: 64 -> 128 channels at stride 2 (batch 8: 15.7 us against 11.8; 1x1 at batch 64: 26.6 against 19.9; 3-D:
+// 29.4 against 26.5), 128 -> 128 at batch 8 (19.5 against 18.4), 384 rows of 768 -> 2304 and 3072 (15.4 against 12.5).
 static double est_cycles(int sm_count, long long base_ctas, int nchunks, int spc, int BN, int passes, int ks) {
     const double stage = std::max<double>((passes == 3 ? 12.0 : 4.0) * (BN / 2), 520.0);
     const long long stages = (long long)((nchunks + ks - 1) / ks) * spc;
@@ -1954,6 +1960,8 @@ static int raise_smem_limit(petb200_ctx *ctx) {
     return PETB200_OK;
 }
 
+// Fills core.P (tiling, raw box, stage counts) for a window [oh0,ohn) x [ow0,own) of the output; returns
+// PETB200_ERR_UNSUPPORTED when the shape does not fit this kernel's constraints.
 static int tc_configure(petb200_ctx *ctx, TcCore &core, const ConvGeom &g, int oh0, int ohn, int ow0, int own,
                         int z_is_batch, int images, long long ys_n, long long ys_f, long long ys_p, int has_bias, int act,
                         int force_bc = 0, int force_ksplit = 0, int force_bn = 0, int flat = 0, int max_ipt = 0) {
