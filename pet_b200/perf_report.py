@@ -133,6 +133,7 @@ def once_ops(ctx):
             ("rowmean 12544 cols", lambda: ctx.rowmean(x.view(64 * 64, 12544), 12544), 4 * x.numel()),
             ("softmax last axis 128 cols", lambda: ctx.softmax(r(12 * 512, 128, 128)), 8 * 12 * 512 * 128 * 128),
             ("softmax last axis 1000 cols", lambda: ctx.softmax(r(65536, 1000)), 8 * 65536 * 1000),
+            ("softmax last axis 2001 cols", lambda: ctx.softmax(r(40000, 2001)), 8 * 40000 * 2001),
             ("softmax axis 1 of [64,1000,784]", lambda: ctx.softmax(r(64, 1000, 784), 1), 8 * 64 * 1000 * 784),
             ("layernorm 768 cols", lambda: ctx.layernorm(r(65536, 768), r(768), r(768)), 8 * 65536 * 768),
             ("matmul m=1 (classifier head 512 -> 1000)", lambda: ctx.matmul(r(1, 1, 512), r(1, 512, 1000)), 4 * 512 * 1000),
