@@ -16,6 +16,7 @@ from . import lib as L
 # The calls below sit in front of kernels of a few microseconds: plain integers instead of ctypes objects (every entry point
 # declares its argument types), and the stream handle without a torch.cuda.Stream object around it.  torch has these two only
 # where it was built with CUDA; without them the module still imports (shapes, plans' arguments, the graph builders).
+_float32 = torch.float32
 _current_device, _raw_stream = getattr(torch._C, "_cuda_getDevice", None), getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
@@ -32,7 +33,7 @@ def _stream():
 # Makes a dense copy of a view.  The caller keeps every copy in a variable until the call has been issued: one that is dropped
 # earlier gives its memory to the next copy, which is then written over it before the kernel has read it.
 def _f32(t):
-    assert t.is_cuda and t.dtype is torch.float32, "device fp32 tensors only"
+    assert t.is_cuda and t.dtype is _float32, "device fp32 tensors only"
     return t.contiguous()
 
 
@@ -117,7 +118,9 @@ class Context:
 
     def conv2d_run(self, plan, x, bias=None, out=None, residual=None):
         """y = act(conv(x) + bias [+ residual]); residual (shaped like y) folds a following Add into the epilogue."""
-        x, bias = _f32(x), _opt(bias)
+        x = _f32(x)
+        if bias is not None:
+            bias = _f32(bias)
         y = out if out is not None else x.new_empty(plan.out_shape)
         if residual is not None:
             if tuple(residual.shape) != tuple(plan.out_shape):
@@ -264,15 +267,21 @@ class Context:
         self.check(self.lib.petb200_matmul_set_weights(plan.h, _ptr(plan._b), _stream()))
 
     def matmul_run(self, plan, a, b, bias=None, out=None, residual=None):
-        a, b, bias = _f32(a), _opt(b), _opt(bias)
+        a, pb, pbias = _f32(a), None, None
+        if b is not None:  # (spelled out: a helper's call per operand is 1 % of the smallest product's host time)
+            b = _f32(b)
+            pb = b.data_ptr()
+        if bias is not None:
+            bias = _f32(bias)
+            pbias = bias.data_ptr()
         c = out if out is not None else a.new_empty(plan.out_shape)
         if residual is not None:
             if tuple(residual.shape) != tuple(plan.out_shape):
                 raise L.PetError(L.ERR_INVALID, "residual must have the shape of the output")
             residual = _f32(residual)
-            self.check(self.lib.petb200_matmul_run_residual(plan.h, _ptr(a), _ptr(b), _ptr(bias), _ptr(residual), _ptr(c), _stream()))
+            self.check(self.lib.petb200_matmul_run_residual(plan.h, a.data_ptr(), pb, pbias, residual.data_ptr(), _ptr(c), _stream()))
         else:
-            self.check(self.lib.petb200_matmul_run(plan.h, _ptr(a), _ptr(b), _ptr(bias), _ptr(c), _stream()))
+            self.check(self.lib.petb200_matmul_run(plan.h, a.data_ptr(), pb, pbias, _ptr(c), _stream()))
         return c
 
     def matmul(self, a, b, transA=False, transB=False, bias=None, act="none", algo="auto", residual=None):
