@@ -16,6 +16,7 @@ int tc_conv_row_pitch(void *h);
 void tc_conv_set_starve(void *h, int on);
 int tc_set_wait_limit_ns(unsigned long long ns);
 const char *tc_conv_variant(void *h);
+const char *tc_matmul_variant(void *h);
 int tc_matmul_create(petb200_ctx *ctx, int bs, int m, int n, int k, int transA, int transB, int has_bias, int act, int passes,
                      const long long *strides, void **out, size_t *dev_bytes);
 long long tc_matmul_a_copy(void *h);
@@ -354,7 +355,7 @@ int make_matmul_plan(petb200_ctx *ctx, int transA, int transB, int b, int m, int
                               &pl->tc, &bytes);
         if (rc == PETB200_OK) {
             pl->algo = PETB200_ALGO_TC_3XTF32;
-            pl->kernel = tc_passes_for(algo) == 1 ? "tc_1xtf32_ts" : (tc_passes_for(algo) == 16 ? "tc_bf16x3_ts" : "tc_3xtf32_ts");
+            pl->kernel = tc_matmul_variant(pl->tc);
             pl->device_bytes = bytes;
             if (const long long words = tc_matmul_a_copy(pl->tc)) {
                 if (pl->at.alloc((size_t)words * 4) != cudaSuccess) {

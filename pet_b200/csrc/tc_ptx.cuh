@@ -189,9 +189,9 @@ __device__ __forceinline__ void mma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, ui
                  ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
                  : "memory");
 }
-// The same with 16-bit inputs (kind::f16; the instruction descriptor says bf16): K = 16 per instruction, two K elements
+// The same with 16-bit inputs (kind::f16; the instruction descriptor says fp16 or bf16): K = 16 per instruction, two K elements
 // per 32-bit TMEM column of A (lower index in the low half).
-__device__ __forceinline__ void mma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
                  ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate)
@@ -247,6 +247,20 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r
                    "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
                  : "memory");
 }
+__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&r)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+                 : "memory");
+}
+template <int N> __device__ __forceinline__ void tmem_st_words(uint32_t taddr, const uint32_t (&r)[N]) {
+    static_assert(N == 8 || N == 16 || N == 32, "widths of tcgen05.st that are used");
+    if constexpr (N == 8)
+        tmem_st_32x8(taddr, r);
+    else if constexpr (N == 16)
+        tmem_st_32x16(taddr, r);
+    else
+        tmem_st_32x32(taddr, r);
+}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t cvt_rna_tf32(float v) {
@@ -276,6 +290,35 @@ __host__ __device__ inline uint32_t idesc_tf32(int M, int N) {
 // kind::f16 with bf16 inputs (format code 1), fp32 accumulate, both operands K-major (K = 16 per instruction).
 __host__ __device__ inline uint32_t idesc_bf16(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+// The same with fp16 inputs (format code 0).
+__host__ __device__ inline uint32_t idesc_f16(int M, int N) {
+    return (1u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+// Two fp32 values rounded to nearest fp16 and packed, `a` in the low half; and back.
+__device__ __forceinline__ uint32_t pack_f16x2(float a, float b) {
+    uint32_t r;
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a)); // first source -> upper half
+    return r;
+}
+__device__ __forceinline__ float2 unpack_f16x2(uint32_t h) {
+    float2 v;
+    asm("{\n\t.reg .b16 l, u;\n\tmov.b32 {l, u}, %2;\n\tcvt.f32.f16 %0, l;\n\tcvt.f32.f16 %1, u;\n\t}" : "=f"(v.x), "=f"(v.y) : "r"(h));
+    return v;
+}
+// max(t, |a|, |b|) in one instruction (a NaN does not count).
+__device__ __forceinline__ float max3_abs(float t, float a, float b) {
+    float d;
+    asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(t), "f"(a), "f"(b));
+    return d;
+}
+// {(a - h.x) * s, (b - h.y) * s} for a power of two s, exact where a - h.x is: two instructions on pairs.
+__device__ __forceinline__ float2 scaled_diff_f32x2(float a, float b, float2 h, float s) {
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, p, n;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 p, {%6, %6};\n\tmov.b64 n, {%7, %7};\n\t"
+        "mul.rn.f32x2 x, x, p;\n\tfma.rn.f32x2 x, y, n, x;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "=f"(d.x), "=f"(d.y) : "f"(a), "f"(b), "f"(h.x), "f"(h.y), "f"(s), "f"(-s));
+    return d;
 }
 // Two fp32 values rounded to nearest bf16 and packed, `a` in the low half.
 __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {

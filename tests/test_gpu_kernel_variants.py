@@ -167,3 +167,83 @@ def test_timing_keeps_the_weights(ctx, algo, monkeypatch):
     graph.run()
     assert np.array_equal(graph.get_data(out), before)
     ctx.sync_check()
+
+
+# fp16 halves: hi and lo carry 22 bits of each operand (what is dropped is below 3 * 2^-22 of a product, and below 2^-22 of the
+# row's largest value for values that a half cannot hold as normal numbers); the tensor core truncates its sum after each of K / 16
+# MMAs, twice 2^-23 of it at most.  So |error| <= 2^-22 * ((4 + K / 8) * sum |x||w| + max |x| * sum |w|), elementwise.
+def _check_halves(got, x2, w2):
+    """x2 [rows, K], w2 [K, cols], float64; rows and filters of any magnitude."""
+    k = x2.shape[1]
+    fin = torch.isfinite(x2).all(1)
+    bound = 2.0 ** -22 * ((4 + k / 8) * (x2.abs() @ w2.abs()) + x2.abs().amax(1, keepdim=True) * w2.abs().sum(0, keepdim=True))
+    err = (got.double() - x2 @ w2).abs()
+    assert bool((err[fin] <= bound[fin] + 1e-37).all()), float((err[fin] / (bound[fin] + 1e-37)).max())
+    assert not bool(torch.isfinite(got[~fin]).any())
+
+
+def _outlandish(x2d, kind, gen):
+    """Rows (or filters) of magnitudes that a half cannot hold, beside ordinary ones."""
+    rows = x2d.shape[0]
+    pick = torch.randperm(rows, generator=gen)[: max(1, rows // 3)]
+    scale = {"ordinary": 1.0, "tiny": 1e-9, "huge": 1e7, "mixed": 10.0 ** torch.randint(-12, 13, (len(pick), 1), generator=gen).double()}[kind]
+    x2d[pick] = (x2d[pick].double() * scale).float()
+    if kind == "mixed":
+        x2d[pick[0]] = 0
+    return x2d
+
+
+# one stage and several, K remainders around a stage of 64 and a flush (K > 768), rows around a tile, one tile per CTA, several, K splits
+@pytest.mark.parametrize("b,m,n,k", [(1, 16, 32, 64), (1, 129, 65, 63), (2, 300, 130, 65), (1, 128, 96, 768), (1, 257, 129, 833), (3, 1000, 200, 260), (1, 64, 64, 4096),
+                                     (1, 5000, 300, 900)])
+@pytest.mark.parametrize("kind", ["ordinary", "tiny", "huge", "mixed"])
+@pytest.mark.parametrize("trans_b", [False, True])
+def test_matmul_of_halves_over_all_magnitudes(ctx, monkeypatch, b, m, n, k, kind, trans_b):
+    monkeypatch.setenv("PETB200_TC_MATH", "f16x3")
+    gen = torch.Generator().manual_seed(m + n + k)
+    a = _outlandish(torch.randn(b * m, k, generator=gen), kind, gen).reshape(b, m, k)
+    w = torch.stack([_outlandish(torch.randn(n, k, generator=gen), kind, gen) for _ in range(b)])
+    if kind == "ordinary":
+        a[0, m // 2, 0], a[0, 0, k - 1] = float("inf"), float("nan")
+    wd = (w if trans_b else w.transpose(1, 2).contiguous()).cuda()
+    plan = ctx.matmul_plan(tuple(a.shape), tuple(wd.shape), False, trans_b)
+    assert plan.kernel == "tc_3xtf32_f16_ts"
+    c = torch.empty(b, m, n, device="cuda")
+    for weights in (True, False):
+        if weights:
+            ctx.matmul_set_weights(plan, wd)
+        got = ctx.matmul_run(plan, a.cuda(), None if weights else wd.clone())
+        ctx.sync_check()
+        for i in range(b):
+            _check_halves(got[i].cpu(), a[i].double(), w[i].double().t())
+
+
+# the ways of gathering: chunks of 32 channels, of 8, the offset table, whole unpadded planes (odd widths); one tile per CTA, several (narrow
+# and, with a flush, wide), K split; a residual that is also the result's buffer must be added once
+@pytest.mark.parametrize("n,c,h,w,f,k,stride", [(1, 64, 20, 20, 64, 3, 1), (2, 24, 9, 12, 40, 3, 1), (3, 3, 20, 24, 33, 5, 2), (4, 10, 7, 7, 20, 3, 1), (1, 256, 14, 14, 64, 3, 1),
+                                                (40, 32, 32, 32, 64, 3, 1), (40, 96, 24, 24, 128, 3, 1), (30, 64, 28, 28, 130, 1, 2), (1, 7, 30, 150, 16, 3, 1)])
+@pytest.mark.parametrize("kind", ["ordinary", "tiny", "huge", "mixed"])
+def test_conv_of_halves_over_all_magnitudes(ctx, monkeypatch, n, c, h, w, f, k, stride, kind):
+    monkeypatch.setenv("PETB200_TC_MATH", "f16x3")
+    gen = torch.Generator().manual_seed(n + c + f)
+    x = _outlandish(torch.randn(n * h * w, c, generator=gen), kind, gen).reshape(n, h, w, c).permute(0, 3, 1, 2).contiguous()
+    wt = _outlandish(torch.randn(f, c * k * k, generator=gen), kind, gen).reshape(f, c, k, k)
+    if kind == "ordinary":
+        x[0, 0, h // 2, w // 2], x[-1, c - 1, 0, 0] = float("nan"), float("inf")
+    pad = k // 2
+    plan = ctx.conv2d_plan(tuple(x.shape), tuple(wt.shape), pad, pad, stride, stride)
+    assert plan.kernel == "tc_3xtf32_f16_ts"
+    ctx.conv2d_set_weights(plan, wt.cuda())
+    got = ctx.conv2d_run(plan, x.cuda())
+    ctx.sync_check()
+    oh, ow = plan.out_shape[2:]
+    cols = torch.nn.functional.unfold(x.double(), k, padding=pad, stride=stride)  # [n, c*k*k, L]
+    full = [(d + 2 * pad - k) // stride + 1 for d in (h, w)]
+    cols = cols.reshape(n, c * k * k, *full)[:, :, :oh, :ow].permute(0, 2, 3, 1).reshape(n * oh * ow, -1)
+    _check_halves(got.permute(0, 2, 3, 1).reshape(n * oh * ow, f).cpu(), cols, wt.reshape(f, -1).double().t())
+    if kind != "ordinary":
+        res = torch.ones_like(got)
+        y = ctx.conv2d_run(plan, x.cuda(), out=res, residual=res)
+        ctx.sync_check()
+        scale = got.abs().amax()
+        assert bool((y - (got + 1) <= 1e-6 * (scale + 1)).all()) and bool(((got + 1) - y <= 1e-6 * (scale + 1)).all())
