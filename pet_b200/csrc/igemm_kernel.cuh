@@ -1310,11 +1310,13 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
                         // memory: when the slot frees, only the two tcgen05.st remain, so a set is one stage ahead in
                         // registers on top of its slots in the ring.  (Announcing a stage only after the next one's gather,
                         // to hide the 200 to 250 cycles of the stores, was 8 % slower: the MMA thread starts later.)
-                        // A stage of halves is 64 elements: two rounds of the same code, 32 each (see split_words), the slot
-                        // awaited in the first.
+                        // A stage of halves is 64 elements: where they are gathered one by one, two rounds of the same code, 32 each
+                        // (see split_words), the slot awaited in the first; row-major rows are 16 reads, whose latencies
+                        // in two rounds made a stage 5 % longer (16 x 768 x 3072 on one tile row: 30.0 us, in one round 28.4).
+                        constexpr int kRounds = HALF && !A_KMAJOR ? 2 : 1, kParts = (HALF ? 2 : 1) / kRounds;
 #pragma unroll 1
-                        for (int half = 0; half < (HALF ? 2 : 1); ++half) {
-                        constexpr int kWords = HALF ? 16 : 32; // of hi and of lo in a round
+                        for (int round = 0; round < kRounds; ++round) {
+                        constexpr int kWords = 32 / kRounds; // of hi and of lo in a round
                         uint32_t hi[kWords], lo[kWords];
                         if constexpr (MODE == kGatherBand) {
                             const int i = bx * kTileM + p, k0 = ((bx * kTileM - P.band_w) & ~3) + ((c0 + ch) * kBandStages + st) * kStageK;
@@ -1329,6 +1331,9 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
                                 split_words<PASSES>(v, hi + 8 * c, lo + 8 * c, top);
                             }
                         } else {
+#pragma unroll
+                            for (int part = 0; part < kParts; ++part) {
+                            const int half = round + part;
                             const int *kh = ko + half * kStageK;
                             const uint8_t *krow = sRaw + (size_t)rb * P.raw_bytes + (size_t)p * 128 + half * kAHalfBytes; // (a stage's second tile follows the first)
                             const float *q = raw; // kGatherPlain: first element of the run
@@ -1359,10 +1364,11 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
                                     for (int i = 0; i < 16; ++i)
                                         v[i] *= factor;
                                 }
-                                split_words<PASSES>(v, hi + 8 * c, lo + 8 * c, top);
+                                split_words<PASSES>(v, hi + 16 * part + 8 * c, lo + 16 * part + 8 * c, top);
+                            }
                             }
                         }
-                        if (half == 0) {
+                        if (round == 0) {
                             if (__builtin_expect(!__all_sync(0xffffffffu, slot_free && raw_ok), 0)) {
                                 raw_ok = __all_sync(0xffffffffu, raw_ok) != 0;
                                 alive = raw_ok && ptx::mbar_wait_warp(a_empty + sa, pa, abort_flag);
@@ -1371,8 +1377,8 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
                             }
                             ptx::tc_fence_after();
                         }
-                        const uint32_t t = t_row + kACol + sa * 64u + half * 16u;
-                        if constexpr (HALF) {
+                        const uint32_t t = t_row + kACol + sa * 64u + round * 16u;
+                        if constexpr (kWords == 16) {
                             ptx::tmem_st_32x16(t, hi);
                             ptx::tmem_st_32x16(t + 32u, lo);
                         } else {

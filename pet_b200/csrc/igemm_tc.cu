@@ -514,43 +514,42 @@ static int cluster_slots(int sm_count, int ks) {
     return cached[ks];
 }
 
-// Rough cycle model of one launch, used to pick the tile width and the K split.  A K stage is charged its MMAs (N/2 cycles each,
-// 12 per stage for 3xTF32, 4 for one pass) or 520 cycles, a CTA 3000 cycles before its first MMA and 1700 + 44*BN of epilogue
-// (split-K: the exchange through the cluster instead), every wave of CTAs the sum.
-// These constants rank the choices; they don't predict times.  With persistent tiles, where start-up and epilogue hide, a 3xTF32
-// stage was measured to take about 1000 cycles at 128 filters (charged 768), 690 at 64 and 570 at 32 (charged 520).  Against the
-// fastest of all (width, split) pairs, forced one by one, on 44 shapes (every convolution of ResNet-18 at batch 1, 8 and 64 and
-// of ResNet3D-18, the 512-channel dilated one, the projections of an encoder of 768 at 128 and 384 rows), the choice is
-// within 2 % on 38.  The other six lose 6 to 34 % because 128-filter tiles, five times with K split in two, are preferred to unsplit
-// 64-filter ones: 64 -> 128 channels at stride 2 (batch 8: 15.7 us against 11.8; 1x1 at batch 64: 26.6 against 19.9; 3-D:
-// 29.4 against 26.5), 128 -> 128 at batch 8 (19.5 against 18.4), 384 rows of 768 -> 2304 and 3072 (15.4 against 12.5).
-static double est_cycles(int sm_count, long long base_ctas, int nchunks, int spc, int BN, int passes, int ks) {
-    const double stage = std::max<double>((passes == 3 ? 12.0 : 4.0) * (BN / 2), 520.0);
-    const long long stages = (long long)((nchunks + ks - 1) / ks) * spc;
-    // split-K: (ks-1)/ks of the 512*BN-byte tile crosses to other SMs at ~10 bytes per cycle, then barrier + local sums
-    const double per_cta = 3000.0 + (double)stages * stage + 1700.0 + (ks > 1 ? 1500.0 + 50.0 * BN * (ks - 1) / ks : 44.0 * BN);
+// Rough cycle model of one launch, used to pick the tile width and the K split.  All constants are measured on row-major products of
+// 16 to 1000 rows with every width and split forced in turn: start-up to the first MMA 6300; a K stage 570 / 655 / 890 at 32 /
+// 64 / 128 filters (3xTF32, 32 K) and 910 / 910 / 1045 (halves, 64 K); the epilogue of an unsplit tile 34 a filter; the exchange
+// through a cluster, reduction and stores together 2300 / 2500 / 8000 and 70 a filter of the CTA's share, which makes a split of a
+// 128-filter tile in two the dearest (12500).  Several unsplit tiles in turn hide start-up and epilogue (persistent tiles).
+// Against the fastest of all pairs on 57 shapes (these products, ResNet layers at batch 1 to 16): within 2 % on 54; the others lose
+// 4, 11 and 14 % (64 x 1000 x 256, a 200-channel 3x3 at 3 x 20 x 20, 16 x 3072 x 768).  The constants before lost up to 31 % on 12 of them.
+static double est_cycles(int sm_count, long long base_ctas, int nchunks, int spc, int BN, int math, int ks) {
+    const int w = BN <= 32 ? 0 : (BN <= 64 ? 1 : 2);
+    static const double tf32[3] = {570, 655, 890}, halves[3] = {910, 910, 1045}, exchange[3] = {2300, 2500, 8000};
+    const double stage = math == kMathTf32x1 ? 520.0 : (math == kMathTf32x3 ? tf32[w] : halves[w]), start = 6300.0;
+    const double stages = (double)((nchunks + ks - 1) / ks) * spc;
     const long long slots = cluster_slots(sm_count, ks);
     if (slots <= 0)
         return 1e30; // this cluster size cannot be launched here
-    const long long waves = (base_ctas + slots - 1) / slots;
-    return (double)waves * per_cta;
+    const double waves = (double)((base_ctas + slots - 1) / slots), epilogue = 34.0 * BN;
+    if (ks > 1)
+        return waves * (start + stages * stage + exchange[w] + 70.0 * BN / ks);
+    return start + waves * std::max(stages * stage, epilogue) + (waves - 1) * 1200.0 + epilogue;
 }
 // Split K over 1, 2, 4, 8 or 16 CTAs (a cluster; 16 is beyond the portable cluster size and allowed per function): the
 // split must divide the tile width and leave every CTA a chunk.
-static int choose_ksplit(int sm_count, long long base_ctas, const IgemmParams &P, int passes, int want, double *cycles) {
+static int choose_ksplit(int sm_count, long long base_ctas, const IgemmParams &P, int math, int want, double *cycles) {
     auto ok = [&](int ks) { return ks == 1 || (ks <= P.nchunks && P.BN % ks == 0); };
     int best = 1;
-    double best_c = est_cycles(sm_count, base_ctas, P.nchunks, P.spc, P.BN, passes, 1);
+    double best_c = est_cycles(sm_count, base_ctas, P.nchunks, P.spc, P.BN, math, 1);
     static const int ks_cap = std::min(16, std::max(1, env_int_early("PETB200_TC_KSPLIT_MAX", 16)));
     if (want > 0) {
         for (best = 16; best > 1 && !(best <= want && ok(best) && cluster_slots(sm_count, best) > 0); best /= 2) {
         }
-        best_c = est_cycles(sm_count, base_ctas, P.nchunks, P.spc, P.BN, passes, best);
+        best_c = est_cycles(sm_count, base_ctas, P.nchunks, P.spc, P.BN, math, best);
     } else {
         for (int ks = 2; ks <= ks_cap; ks *= 2) {
             if (!ok(ks))
                 continue;
-            const double c = est_cycles(sm_count, base_ctas, P.nchunks, P.spc, P.BN, passes, ks);
+            const double c = est_cycles(sm_count, base_ctas, P.nchunks, P.spc, P.BN, math, ks);
             if (c < best_c * 0.97) // a deeper split has to pay for itself
                 best = ks, best_c = c;
         }
@@ -786,9 +785,8 @@ static int tc_configure(petb200_ctx *ctx, TcCore &core, const ConvGeom &g, int o
         if (!fit(bn))
             continue;
         const long long base_ctas = (long long)mtiles * ((Fg + bn - 1) / bn) * gz * core.beside;
-        const int passes = core.math == kMathTf32x1 ? 1 : 3;
         double cyc;
-        const int ks = choose_ksplit(ctx->sm_count, base_ctas, P, passes, want_ks, &cyc);
+        const int ks = choose_ksplit(ctx->sm_count, base_ctas, P, core.math, want_ks, &cyc);
         if (ks > 1) { // the landing area takes shared memory from the rings (or even from the chunk size): fit again
             P.ksplit = ks;
             if (!fit(bn))
@@ -797,7 +795,7 @@ static int tc_configure(petb200_ctx *ctx, TcCore &core, const ConvGeom &g, int o
                 P.ksplit = 1;
                 if (!fit(bn))
                     continue;
-                cyc = est_cycles(ctx->sm_count, base_ctas, P.nchunks, P.spc, bn, passes, 1);
+                cyc = est_cycles(ctx->sm_count, base_ctas, P.nchunks, P.spc, bn, core.math, 1);
             }
         }
         if (!have || cyc < best_cycles * 0.97) { // prefer the wider tile unless the narrower one clearly wins
@@ -1147,7 +1145,7 @@ static int tc_configure_kmajor(petb200_ctx *ctx, TcCore &core, int bs, int m, in
                 continue;
             P.BN = bn;
             double cyc;
-            const int ks = choose_ksplit(ctx->sm_count, (long long)P.tpi * ((n + bn - 1) / bn) * bs, P, core.math == kMathTf32x1 ? 1 : 3,
+            const int ks = choose_ksplit(ctx->sm_count, (long long)P.tpi * ((n + bn - 1) / bn) * bs, P, core.math,
                                          env_int("PETB200_TC_KSPLIT", 0), &cyc);
             if (!best_bn || cyc < best * 0.97)
                 best = cyc, best_bn = bn, best_ks = ks;
