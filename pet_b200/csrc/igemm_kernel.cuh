@@ -55,8 +55,8 @@ constexpr int kNA = 4; // A stages in TMEM: a transform set owns slots `set` and
 enum { kSingle = 0, kNarrow = 1, kWide = 2 };
 // Registers per thread of the four warp groups (512 in sum, what the block is launched with): drain warps that keep a row of 128
 // sums need 184 or more; in single-tile mode the transform sets also run the epilogue.
-// The compiler sees one limit for all roles (128 a thread); the single-tile and narrow TF32 instances spill nothing, the others 8 to
-// 40 bytes stored / 24 to 130 loaded.
+// The compiler sees one limit for all roles (128 a thread): at most 48 bytes spilled / 190 loaded; the narrow TF32 instances and the
+// single-tile convolution spill nothing.
 template <int PP> struct Regs {
     static constexpr int control = PP == kSingle ? 56 : 72, set = PP == kSingle ? 136 : (PP == kNarrow ? 144 : 120),
                          drain = PP == kSingle ? 184 : (PP == kNarrow ? 152 : 200);
@@ -646,8 +646,8 @@ __device__ __forceinline__ void store_any(const StoreJob &J, const float *bias, 
 }
 // This thread's row through one of the long activations, with bias and residual.  One warp per SM quarter stores, so this is a chain of
 // latencies (shared memory, exponential, reciprocal): eight filters at a time, and the choice of activation outside the loop.
-// Four at a time with the choice inside, a 3x3 convolution of 18 x 16 x 24 x 24 to 216 filters in two groups took 37.5 us with a
-// sigmoid, 29.5 with GELU, 27.4 with tanh and 14 with none; now 36 (the division), 23.4 and 21.9.
+// Four at a time with the choice inside, a 3x3 convolution of 18 x 16 x 24 x 24 to 216 filters took 42.8 us with a sigmoid, 33.0 with
+// GELU, 30.8 with tanh and 15.2 with none; now 36.6 (its division), 24.6, 22.6 and 13.6.
 template <int ACT>
 __device__ __forceinline__ void activate_row(const StoreJob &J, float *stage, const float *rp, float bias, int f0) {
 #pragma unroll 1
@@ -685,21 +685,20 @@ __device__ __forceinline__ void activate_block(const StoreJob &J, float *r, floa
         r[j] = stage[j * 32 + lane];
     __syncwarp();
 }
-template <int MODE, bool RES>
+// LONG: with one of the long activations (RES is then false, activate_block adds a residual).  Its own instances: beside the others'
+// code it cost ResNet-18 at batch 64 5 %, whose layers have none of it.
+template <int MODE, bool RES, bool LONG>
 __device__ __forceinline__ void store_block(const StoreJob &J, float *r /*32 sums*/, float *stage, int f0) {
     const int lane = J.lane;
     __syncwarp(); // the previous block has been read
-    const float *bias = J.bias;
-    if (__builtin_expect(J.act > PETB200_ACT_RELU, 0)) {
+    if constexpr (LONG) {
         activate_block(J, r, stage, f0);
-        bias = nullptr;
-        if (RES) { // the residual has been added
-            StoreJob R = J;
-            R.bias = R.res = nullptr, R.act = PETB200_ACT_NONE;
-            store_block<MODE, false>(R, r, stage, f0);
-            return;
-        }
+        StoreJob R = J; // bias and residual have been added
+        R.bias = R.res = nullptr, R.act = PETB200_ACT_NONE;
+        store_block<MODE, false, false>(R, r, stage, f0);
+        return;
     }
+    const float *bias = J.bias;
     if (MODE == kStorePixels) {
 #pragma unroll
         for (int j = 0; j < 32; ++j)
@@ -735,18 +734,24 @@ __device__ __forceinline__ void store_block(const StoreJob &J, float *r /*32 sum
         store_any<RES>(J, bias, r, f0);
     }
 }
-// f(mode, with residual) as compile-time constants: the loops around store_block are instantiated per way of storing.
-template <typename F> __device__ __forceinline__ void with_store_mode(int mode, bool res, F &&f) {
+// f(mode, with residual, long activation) as compile-time constants: the loops around store_block are instantiated per way of storing.
+template <typename F> __device__ __forceinline__ void with_store_mode(int mode, bool res, int act, F &&f) {
     const std::integral_constant<bool, true> yes;
     const std::integral_constant<bool, false> no;
+    auto pick = [&](auto mode_c) {
+        if (__builtin_expect(act > PETB200_ACT_RELU, 0))
+            f(mode_c, no, yes);
+        else
+            res ? f(mode_c, yes, no) : f(mode_c, no, no);
+    };
     if (mode == kStorePixels)
-        res ? f(std::integral_constant<int, kStorePixels>(), yes) : f(std::integral_constant<int, kStorePixels>(), no);
+        pick(std::integral_constant<int, kStorePixels>());
     else if (mode == kStoreFilters)
-        res ? f(std::integral_constant<int, kStoreFilters>(), yes) : f(std::integral_constant<int, kStoreFilters>(), no);
+        pick(std::integral_constant<int, kStoreFilters>());
     else if (mode == kStoreRows)
-        res ? f(std::integral_constant<int, kStoreRows>(), yes) : f(std::integral_constant<int, kStoreRows>(), no);
+        pick(std::integral_constant<int, kStoreRows>());
     else
-        res ? f(std::integral_constant<int, kStoreAny>(), yes) : f(std::integral_constant<int, kStoreAny>(), no);
+        pick(std::integral_constant<int, kStoreAny>());
 }
 
 // A set of barriers (the last one is a word in each of the roles' slots, see the kernel).
@@ -1509,7 +1514,7 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
             } else if (alive) {
                 ptx::tc_fence_after();
                 const int blocks = (P.BN / 32 + 1) / 2; // whole 32-column blocks per set
-                with_store_mode(store_mode(), J.res != nullptr, [&](auto mode_c, auto res_c) {
+                with_store_mode(store_mode(), J.res != nullptr, P.act, [&](auto mode_c, auto res_c, auto long_c) {
 #pragma unroll 1
                 for (int c = tset * blocks * 32; c < min(P.BN, (tset + 1) * blocks * 32); c += 32) {
                     float r[32];
@@ -1526,7 +1531,7 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
                     }
                     if (REDO && (pass || factors))
                         unscale_block(r, unscale, P.fscale + (long long)zb * P.Fg, f_tile0 + c, P.Fg, factors, lane);
-                    store_block<decltype(mode_c)::value, decltype(res_c)::value>(J, r, stage, f_tile0 + c);
+                    store_block<decltype(mode_c)::value, decltype(res_c)::value, decltype(long_c)::value>(J, r, stage, f_tile0 + c);
                 }
                 });
             }
@@ -1558,7 +1563,7 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
             }
         } else if (PP || FL > 0) {
             float *stage = reinterpret_cast<float *>(smem + L.stage_off) + quarter * 1024;
-            auto drain = [&](auto mode_c, auto res_c) {
+            auto drain = [&](auto mode_c, auto res_c, [[maybe_unused]] auto long_c) {
             [[maybe_unused]] constexpr int MODE = decltype(mode_c)::value; // (a single tile stores nothing here)
             [[maybe_unused]] constexpr bool RES = decltype(res_c)::value;
             for (int tl = 0; tl < items && alive; ++tl) {
@@ -1622,7 +1627,7 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
                             release();
                         if (REDO && (pass || factors))
                             unscale_block(racc, unscale, P.fscale + (long long)zb * P.Fg, ntile * P.BN + c, P.Fg, factors, lane);
-                        store_block<MODE, RES>(J, racc, stage, ntile * P.BN + c);
+                        store_block<MODE, RES, decltype(long_c)::value>(J, racc, stage, ntile * P.BN + c);
                     }
                 } else {
                     // Groups in order, round-to-nearest adds; the MMA thread restarts the main accumulator once a group has been taken.
@@ -1667,7 +1672,7 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
                         for (int c = 0; c < P.BN; c += 32) {
                             if (REDO && (pass || factors))
                                 unscale_block(racc, unscale, P.fscale + (long long)zb * P.Fg, ntile * P.BN + c, P.Fg, factors, lane);
-                            store_block<MODE, RES>(J, racc, stage, ntile * P.BN + c);
+                            store_block<MODE, RES, decltype(long_c)::value>(J, racc, stage, ntile * P.BN + c);
 #pragma unroll
                             for (int j = 0; j < 96; ++j) // the next block's sums move down
                                 racc[j] = racc[j + 32];
@@ -1677,9 +1682,9 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
             }
             };
             if constexpr (PP == kSingle)
-                drain(std::integral_constant<int, kStoreAny>(), std::integral_constant<bool, false>()); // (stores nothing)
+                drain(std::integral_constant<int, kStoreAny>(), std::integral_constant<bool, false>(), std::integral_constant<bool, false>()); // (stores nothing)
             else
-                with_store_mode(store_mode(), P.res != nullptr, drain);
+                with_store_mode(store_mode(), P.res != nullptr, P.act, drain);
             if (!PP && FL > 0) // (also after a wait gave up: the transform sets wait here)
                 ptx::named_bar_sync(1, 384);
         }
