@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(256) k_tile_v4(const uint32_t *__restrict__ in
     constexpr int NI = VI ? kTileEPT / 4 : kTileEPT, NO = VO ? kTileEPT / 4 : kTileEPT;
     constexpr int WI = VI ? 4 : 1, WO = VO ? 4 : 1;
     int li[NI], lo[NO], ls[NI];
-    int svin = 0; // shared-memory stride of the input-contiguous digit
+    int sv1 = 0, sv2 = 0; // places in shared memory of the second and third word of a load, relative to the first
     {
         int sstride[kMaxTileDigits];
         int acc = 1;
@@ -345,8 +345,17 @@ __global__ void __launch_bounds__(256) k_tile_v4(const uint32_t *__restrict__ in
             }
 #pragma unroll
         for (int k = 0; k < kMaxTileDigits; ++k)
-            if (k == t.read_order[0])
-                svin = sstride[k];
+            if (k == t.read_order[0]) {
+                sv1 = sstride[k];
+                if (t.text[k] != 2)
+                    sv2 = 2 * sstride[k];
+            }
+        if (t.nt > 1) { // pairs of words: the third one is the next value of the second digit
+#pragma unroll
+            for (int k = 0; k < kMaxTileDigits; ++k)
+                if (k == t.read_order[1] && sv2 == 0)
+                    sv2 = sstride[k];
+        }
 #pragma unroll
         for (int u = 0; u < NO; ++u) {
             int rem = (threadIdx.x + u * 256) * WO, off_o = 0;
@@ -418,7 +427,7 @@ __global__ void __launch_bounds__(256) k_tile_v4(const uint32_t *__restrict__ in
             if ((threadIdx.x + u * 256) * WI < t.tile_elems) {
 #pragma unroll
                 for (int j = 0; j < WI; ++j) {
-                    const int sdx = ls[u] + j * svin;
+                    const int sdx = ls[u] + (j & 1) * sv1 + (j >> 1) * sv2;
                     tile[sdx + (sdx >> 5)] = v[WI * u + j];
                 }
             }
@@ -730,10 +739,13 @@ static int finalize_plan(petb200_ctx *ctx, LayoutPlan *pl, std::vector<Digit> di
             {
                 const bool whole_chunks = t.ck < 0 || t.chunk_ext % t.text[t.ck] == 0;
                 const int kin = t.read_order[0], kout = t.nt - 1;
-                bool vi = whole_chunks && t.tile_elems % 4 == 0 && t.tistr[kin] == 1 && t.text[kin] % 4 == 0 && t.m.ibase % 4 == 0;
+                // The input run may be two digits, an innermost pair and an even number of them (the interleave factor 2 of the
+                // space-to-batch rewrites): 16 x 512 x 64 x 64 55.7 -> 46.0 us, 0.74 -> 0.89 of the copy rate.
+                const int kin2 = t.nt > 1 && t.text[kin] == 2 && t.tistr[t.read_order[1]] == 2 && t.text[t.read_order[1]] % 2 == 0 ? t.read_order[1] : -1;
+                bool vi = whole_chunks && t.tile_elems % 4 == 0 && t.tistr[kin] == 1 && (t.text[kin] % 4 == 0 || kin2 >= 0) && t.m.ibase % 4 == 0;
                 bool vo = whole_chunks && t.tile_elems % 4 == 0 && t.tostr[kout] == 1 && t.text[kout] % 4 == 0 && t.m.obase % 4 == 0;
                 for (int q = 0; q < t.nt; ++q) {
-                    vi = vi && (q == kin || t.tistr[q] % 4 == 0);
+                    vi = vi && (q == kin || q == kin2 || t.tistr[q] % 4 == 0);
                     vo = vo && (q == kout || t.tostr[q] % 4 == 0);
                 }
                 for (int d = 0; d < t.m.nd; ++d) {

@@ -247,3 +247,21 @@ def test_conv_of_halves_over_all_magnitudes(ctx, monkeypatch, n, c, h, w, f, k, 
         ctx.sync_check()
         scale = got.abs().amax()
         assert bool((y - (got + 1) <= 1e-6 * (scale + 1)).all()) and bool(((got + 1) - y <= 1e-6 * (scale + 1)).all())
+
+
+# Tiled permutations whose input run is an innermost pair and a second digit (the interleave of the space-to-batch rewrites): runs of 4, of
+# 6 and 10 (off the 16-byte grid), around a tile's 64 words and beyond, channels around a tile; inputs off the 16-byte grid
+@pytest.mark.parametrize("shape", [(1, 3, 4, 4), (2, 5, 8, 8), (1, 33, 6, 10), (3, 7, 12, 64), (2, 40, 8, 68), (1, 64, 64, 132), (4, 512, 4, 16)])
+@pytest.mark.parametrize("shift", [0, 1, 4])
+def test_tiled_permutation_of_pairs(ctx, oracle, shape, shift):
+    from pet_b200.configs import SPACE_TO_BATCH
+    x = np.random.default_rng(shape[3]).standard_normal(shape).astype(np.float32)
+    buf = torch.empty(x.size + shift, device="cuda")
+    xd = buf[shift:].view(shape)
+    xd.copy_(torch.from_numpy(x))
+    want = x
+    for op in SPACE_TO_BATCH:
+        want = oracle.transpose(want, *op)
+    got = ctx.transpose_chain(xd, SPACE_TO_BATCH)
+    ctx.sync_check()
+    assert np.array_equal(got.cpu().numpy(), want)
