@@ -247,20 +247,6 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r
                    "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
                  : "memory");
 }
-__device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&r)[8]) {
-    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-                 : "memory");
-}
-template <int N> __device__ __forceinline__ void tmem_st_words(uint32_t taddr, const uint32_t (&r)[N]) {
-    static_assert(N == 8 || N == 16 || N == 32, "widths of tcgen05.st that are used");
-    if constexpr (N == 8)
-        tmem_st_32x8(taddr, r);
-    else if constexpr (N == 16)
-        tmem_st_32x16(taddr, r);
-    else
-        tmem_st_32x32(taddr, r);
-}
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t cvt_rna_tf32(float v) {
