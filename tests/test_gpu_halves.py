@@ -1,0 +1,119 @@
+"""GPU: products of fp16 halves on the tensor-core kernel: what holds for operands of any magnitude, in every family that runs on it
+and under capture."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def halves(monkeypatch):
+    monkeypatch.setenv("PETB200_TC_MATH", "f16x3")
+
+
+def _weights(shape, small, filter_dim, seed):
+    """Gaussian weights in which the filters `small` are too small for a half."""
+    w = torch.randn(shape, generator=torch.Generator().manual_seed(seed))
+    w.movedim(filter_dim, 0)[small] *= 1e-6
+    return w.cuda()
+
+
+def _captured(call):
+    """`call` captured into a CUDA graph, and what it returned there."""
+    call()  # (lazily made plans)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = call()
+    return graph, out
+
+
+def _replay(graph, out):
+    out.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    return out.clone()
+
+
+# A captured launch is replayed after its plan's operand has been packed again: with the same weights, with others whose small
+# filters are elsewhere, and with none small
+@pytest.mark.parametrize("kind", ["conv2d", "convtrans_phases", "convtrans", "matmul"])
+def test_captured_launch_after_a_new_packing(ctx, monkeypatch, kind):
+    if kind == "conv2d":
+        x, shape, fdim = torch.randn(2, 32, 12, 12, device="cuda"), (40, 32, 3, 3), 0
+        plan = ctx.conv2d_plan(x.shape, shape, 1, 1)
+        set_weights, run = lambda w: ctx.conv2d_set_weights(plan, w), lambda: ctx.conv2d_run(plan, x)
+    elif kind == "matmul":
+        x, shape, fdim = torch.randn(1, 70, 96, device="cuda"), (1, 96, 65), 2
+        plan = ctx.matmul_plan(x.shape, shape)
+        set_weights, run = lambda w: ctx.matmul_set_weights(plan, w), lambda: ctx.matmul_run(plan, x, None)
+    else:
+        monkeypatch.setenv("PETB200_CONVTRANS_PHASES", "1" if kind == "convtrans_phases" else "0")
+        x, shape, fdim = torch.randn(2, 8, 8, 32, device="cuda"), (4, 4, 32, 24), 3
+        plan = ctx.convtrans_plan(x.shape, shape, 1, 1, 2, 2)
+        set_weights, run = lambda w: ctx.convtrans_run(plan, x, w), lambda: ctx.convtrans_run(plan, x)
+    assert plan.kernel == "tc_3xtf32_f16_ts"
+    first = _weights(shape, [3, 7], fdim, 1)
+    set_weights(first)
+    graph, out = _captured(run)
+    for w in (first, _weights(shape, [5], fdim, 2), _weights(shape, [], fdim, 3), first):
+        set_weights(w)
+        assert torch.equal(run(), _replay(graph, out))
+    ctx.sync_check()
+
+
+# A declared weight packed again because another B came in between
+def test_captured_matmul_after_another_operand(ctx):
+    a, w, other = torch.randn(1, 70, 96, device="cuda"), _weights((1, 96, 65), [3, 7], 2, 1), _weights((1, 96, 65), [], 2, 2)
+    plan = ctx.matmul_plan(a.shape, w.shape)
+    ctx.matmul_set_weights(plan, w)
+    graph, out = _captured(lambda: ctx.matmul_run(plan, a, None))
+    want = ctx.matmul_run(plan, a, None)
+    ctx.matmul_run(plan, a, other)
+    assert torch.equal(ctx.matmul_run(plan, a, None), want) and torch.equal(_replay(graph, out), want)
+    ctx.sync_check()
+
+
+# The packing itself captured with the product, and other operands packed between two replays
+@pytest.mark.parametrize("kind", ["conv2d", "conv3d", "matmul", "matmul_trans_b"])
+def test_captured_packing_after_another(ctx, kind):
+    if kind.startswith("matmul"):
+        x, shape, fdim = torch.randn(3, 70, 96, device="cuda"), (3, 65, 96) if kind == "matmul_trans_b" else (3, 96, 65), 1 if kind == "matmul_trans_b" else 2
+        call = lambda w: ctx.matmul(x, w, False, kind == "matmul_trans_b")
+    elif kind == "conv2d":
+        x, shape, fdim = torch.randn(2, 32, 12, 12, device="cuda"), (40, 32, 3, 3), 0
+        call = lambda w: ctx.conv2d(x, w, 1, 1)
+    else:
+        x, shape, fdim = torch.randn(1, 16, 4, 8, 8, device="cuda"), (33, 16, 3, 3, 3), 0
+        call = lambda w: ctx.conv3d(x, w, (1, 1, 1))
+    w = _weights(shape, [3, 7], fdim, 1)
+    graph, out = _captured(lambda: call(w))
+    for i, new in enumerate((w, _weights(shape, [5], fdim, 2), _weights(shape, [], fdim, 3))):
+        w.copy_(new)  # what the captured packing reads
+        between = _weights(shape, [1] if i != 1 else [], fdim, 4 + i)
+        want = call(w)
+        call(between)
+        assert torch.equal(_replay(graph, out), want)
+    ctx.sync_check()
+
+
+# Operator by operator (the profiled run) and as one captured graph in turn: the same sums of a filter that is too small for a half
+def test_graph_runs_around_a_profiled_run(ctx):
+    from pet_b200 import configs
+    from pet_b200.graph import Graph
+    graph = Graph(ctx)
+    b = configs.GraphBuilder(graph)
+    x, w = np.random.default_rng(0).standard_normal((2, 32, 12, 12), np.float32), _weights((40, 32, 3, 3), [3, 7], 0, 1).cpu().numpy()
+    out = b.conv(b.input(x), b.const(w), 1, 1)
+    graph.setOutputs([out])
+    graph.compile()
+    b.load()
+    assert [k for _, k in graph.steps()] == ["tc_3xtf32_f16_ts"]
+    graph.run()
+    before = graph.get_data(out).copy()
+    graph.run_profiled(0, 1)
+    assert np.array_equal(graph.get_data(out), before)
+    graph.run()
+    assert np.array_equal(graph.get_data(out), before)
+    ctx.sync_check()
