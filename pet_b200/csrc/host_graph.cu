@@ -1076,6 +1076,7 @@ int petb200_graph::capture() {
         return rc;
     if (cudaStreamSynchronize(cap_stream) != cudaSuccess)
         return fail(PETB200_ERR_CUDA, "warm-up pass failed: %s", cudaGetErrorString(cudaGetLastError()));
+    hoisted_done = true; // (a profiled run between two replays packs nothing again)
     cudaGraph_t graph = nullptr;
     if (cudaStreamBeginCapture(cap_stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
         return fail(PETB200_ERR_CUDA, "begin capture failed");

@@ -396,3 +396,17 @@ def test_seam_transpose_pair_folds_into_the_conv_bit_for_bit(ctx, case):
         assert names == (["conv_seam_folded"] if fuse else ["transpose", "conv", "transpose"])
         outs.append(g.get_data(y))
     assert outs[0].shape == outs[1].shape and np.array_equal(outs[0], outs[1])
+
+
+# A profiled run after a captured one issues the replayed steps and packs no weight again
+def test_profiled_run_after_a_captured_one_packs_nothing(ctx):
+    from pet_b200 import configs
+    g, out, y = run_config(ctx, configs.bert_encoder, layers=1, seq=16, hidden=64, heads=2, ffn=128)
+    issued = []
+    for slot in range(2):
+        before = ctx.launches()
+        g.run_profiled(slot, 2)
+        issued.append(ctx.launches() - before)
+    ctx.sync_check()
+    assert issued[0] == issued[1]
+    assert np.array_equal(g.get_data(out), y)
