@@ -107,7 +107,7 @@ struct IgemmParams {
     int ke;                 // K elements per stage: 32 (TF32) or 64 (fp16 and bf16, two per 32-bit word)
     int f16;                // error-compensated fp16
     const float *fscale;    // fp16: what each packed filter has to be multiplied by (a power of two, mostly 1)
-    const uint32_t *factor_words; // two words that are equal if one of them is not 1 (see TcCore::factor_words)
+    const uint32_t *factor_word; // its halves are equal if one of them is not 1 (see TcCore::factor_word)
     int cpg, Fg, BN;        // channels per group, filters per group, tile N
     int z_is_batch;         // blockIdx.z: 0 = conv group, 1 = matmul batch
     int wide, row_tiles;    // wide mode: a tile is 128 consecutive pixels of ONE output row (rows wider than a tile)
@@ -945,15 +945,15 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
     };
     // fp16: has some filter of the packed operand a factor other than 1?  Asked by the warps that store before they have anything to
     // store; the answer is waited for where it is used.
-    [[maybe_unused]] auto ask_factors = [&]() -> uint2 {
-        uint2 words = make_uint2(0u, 1u);
+    [[maybe_unused]] auto ask_factors = [&]() -> uint32_t {
+        uint32_t word = 0;
         if (REDO)
-            asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(words.x), "=r"(words.y) : "l"(P.factor_words));
-        return words;
+            asm volatile("ld.global.u32 %0, [%1];" : "=r"(word) : "l"(P.factor_word));
+        return word;
     };
-    [[maybe_unused]] auto any_factor = [&](uint2 words) -> bool {
-        asm volatile("" : "+r"(words.x), "+r"(words.y));
-        return REDO && words.x == words.y;
+    [[maybe_unused]] auto any_factor = [&](uint32_t word) -> bool {
+        asm volatile("" : "+r"(word));
+        return REDO && (word >> 16) == (word & 0xffffu);
     };
     // split-K: this CTA reduces the channel chunks [c0, c1)
     const int c0 = (ksp * P.nchunks) >> P.ks_log, c1 = ((ksp + 1) * P.nchunks) >> P.ks_log;
@@ -1421,7 +1421,7 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
                 }
             }
         };
-        [[maybe_unused]] const uint2 factor_answer = !PP ? ask_factors() : make_uint2(0u, 1u);
+        [[maybe_unused]] const uint32_t factor_answer = !PP ? ask_factors() : 0u;
         auto transform_by_mode = [&](auto rescale_c) {
             if constexpr (BAND == 2) {
                 transform(std::integral_constant<int, kGatherBand>(), rescale_c);

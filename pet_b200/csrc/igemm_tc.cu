@@ -41,7 +41,7 @@ __device__ __forceinline__ uint32_t block_max_exponent(float top, float *warp_to
     return row_exponent(top);
 }
 __global__ void __launch_bounds__(256) k_filter_factors(const float *__restrict__ w, float *__restrict__ unscale, long long per_filter,
-                                                        uint32_t *words, uint32_t number) {
+                                                        uint16_t *numbers, uint16_t number) {
     __shared__ float tops[8];
     const float *row = w + blockIdx.x * per_filter;
     float top = 0.f;
@@ -51,9 +51,9 @@ __global__ void __launch_bounds__(256) k_filter_factors(const float *__restrict_
     if (threadIdx.x == 0) {
         unscale[blockIdx.x] = row_unscale(e);
         if (blockIdx.x == 0)
-            words[0] = number;
+            numbers[0] = number;
         if (row_out_of_range(e))
-            words[1] = number;
+            numbers[1] = number;
     }
 }
 
@@ -88,7 +88,7 @@ struct PrepareArgs {
     void *hi, *lo;
     int bs, n, k, Kpad, BC;
     float *unscale;          // fp16: what the sums of each packed row are multiplied by
-    uint32_t *words, number; // see TcCore::factor_words
+    uint16_t *numbers, number; // see TcCore::factor_word
     FastDiv by_kc_pad, by_tiles_k, by_tiles_n;
     long long sb_batch, sb_row;
     int b_tiles, tiles_k, tiles_n;
@@ -214,9 +214,9 @@ __global__ void __launch_bounds__(256) k_prepare_f16_kn(const PrepareArgs g) {
         if (rank == 0 && col_ok) {
             g.unscale[(long long)bb * g.n + n0 + lane] = row_unscale(e);
             if (blockIdx.x == 0 && lane == 0)
-                g.words[0] = g.number;
+                g.numbers[0] = g.number;
             if (row_out_of_range(e))
-                g.words[1] = g.number;
+                g.numbers[1] = g.number;
         }
     }
     if (g.split > 1)
@@ -278,9 +278,9 @@ __global__ void __launch_bounds__(256) k_prepare_f16_nk(const PrepareArgs g) {
     if (row_ok && u0 == 0 && lane == 0) {
         g.unscale[row] = row_unscale(e);
         if (row == 0)
-            g.words[0] = g.number;
+            g.numbers[0] = g.number;
         if (row_out_of_range(e))
-            g.words[1] = g.number;
+            g.numbers[1] = g.number;
     }
 #pragma unroll 4
     for (int u = u0; u < u1; u += step) {
@@ -329,16 +329,16 @@ struct TcCore {
     long long Ktot = 0;
     int rows_b = 0;
     DevBuf whi, wlo, koff;
-    // fp16: a factor per packed row of B, and behind them two words: the number of the last packing, and that of the last one which
-    // found a factor other than 1.  The kernel multiplies where they are equal.  Both are written by the packing and read by the
-    // product on the device: a launch that a CUDA graph holds is replayed after packings that came later than its capture.  (A
-    // packing that a graph repeats may find its own number in the second word from an earlier run: its sums are multiplied by
-    // ones.)  A plan that borrows another's operand has `packed_by` point there.
+    // fp16: a factor per packed row of B, and behind them a word of two halves: the number of the last packing (modulo 2^16), and that
+    // of the last one which found a factor other than 1.  The kernel multiplies where they are equal.  Both are written by the
+    // packing and read by the product on the device: a launch that a CUDA graph holds is replayed after packings that came later
+    // than its capture.  (An old number in the second half may come round again, or a graph repeat its own packing: the sums are
+    // then multiplied by ones.)  One word and not two: a second register kept through the transform loop cost 0.15 to 0.4 us a
+    // launch.  A plan that borrows another's operand has `packed_by` point there.
     DevBuf fscale_buf;
-    uint32_t packings = 0;
+    uint16_t packings = 0;
     const TcCore *packed_by = nullptr;
-    size_t factor_floats() const { return ((size_t)rows_b + 1) & ~(size_t)1; } // (the words are read as one of eight bytes)
-    uint32_t *factor_words() const { return (uint32_t *)fscale_buf.p + factor_floats(); }
+    uint32_t *factor_word() const { return (uint32_t *)fscale_buf.p + rows_b; }
     long long y_elems = 0;
     CUtensorMap map_x{}, map_bhi{}, map_blo{};
     const void *map_x_ptr = nullptr;
@@ -405,7 +405,7 @@ struct TcCore {
     }
     int alloc_b() { // the packed operand: rows_b rows of Ktot elements, hi and lo
         const size_t bytes = (size_t)rows_b * Ktot * (half() ? 2 : 4);
-        if (whi.alloc(bytes) != cudaSuccess || wlo.alloc(bytes) != cudaSuccess || (P.f16 && fscale_buf.alloc((factor_floats() + 2) * 4) != cudaSuccess))
+        if (whi.alloc(bytes) != cudaSuccess || wlo.alloc(bytes) != cudaSuccess || (P.f16 && fscale_buf.alloc((size_t)(rows_b + 1) * 4) != cudaSuccess))
             return fail(ctx, PETB200_ERR_NOMEM, "packed operand allocation (%zu bytes) failed", 2 * bytes);
         return encode_b();
     }
@@ -443,7 +443,7 @@ struct TcCore {
         p.koff = (const int *)koff.p;
         if (P.f16) {
             const TcCore *o = packed_by ? packed_by : this;
-            p.fscale = (const float *)o->fscale_buf.p, p.factor_words = o->factor_words();
+            p.fscale = (const float *)o->fscale_buf.p, p.factor_word = o->factor_word();
         }
         p.status = ctx->d_status;
         p.starve = starve;
@@ -1026,7 +1026,7 @@ int tc_conv_set_weights(void *h, const float *w, cudaStream_t s) {
     long long total = (long long)t->g.F * c.Ktot;
     int blocks = (int)std::min<long long>((total + 255) / 256, (long long)c.ctx->sm_count * 16);
     if (c.math == kMathF16x3)
-        k_filter_factors<<<t->g.F, 256, 0, s>>>(w, (float *)c.fscale_buf.p, (long long)cpg * T, c.factor_words(), ++c.packings);
+        k_filter_factors<<<t->g.F, 256, 0, s>>>(w, (float *)c.fscale_buf.p, (long long)cpg * T, (uint16_t *)c.factor_word(), ++c.packings);
     auto kern = c.math == kMathF16x3 ? k_pack_conv_w<kMathF16x3> : (c.math == kMathBf16x3 ? k_pack_conv_w<kMathBf16x3>
               : (c.math == kMathTf32x1 ? k_pack_conv_w<kMathTf32x1> : k_pack_conv_w<kMathTf32x3>));
     kern<<<blocks, 256, 0, s>>>(w, c.whi.p, c.wlo.p, t->g.F, cpg, T, c.P.BC, c.P.spc * c.P.ke, c.P.nchunks, (const float *)c.fscale_buf.p);
@@ -1422,7 +1422,7 @@ int tc_matmul_prepare(void *h, const float *b, const float *a, float *a_copy, cu
     PrepareArgs g{};
     g.b = b, g.hi = c.whi.p, g.lo = c.wlo.p, g.bs = t->bs, g.n = t->n, g.k = t->k, g.Kpad = (int)c.Ktot;
     if (f16)
-        g.unscale = (float *)c.fscale_buf.p, g.words = c.factor_words(), g.number = b ? ++c.packings : 0;
+        g.unscale = (float *)c.fscale_buf.p, g.numbers = (uint16_t *)c.factor_word(), g.number = b ? ++c.packings : (uint16_t)0;
     g.BC = c.P.BC, g.sb_batch = t->st[2], g.sb_row = t->st[3];
     g.tiles_k = g.Kpad / (f16 ? kPrepUnit : 32), g.tiles_n = (t->n + 31) / 32; // (Kpad is a multiple of the stage's K)
     g.by_kc_pad.set(c.P.spc * c.P.ke), g.by_tiles_k.set(g.tiles_k), g.by_tiles_n.set(g.tiles_n);
