@@ -258,6 +258,14 @@ __device__ __forceinline__ bool row_out_of_range(uint32_t e) { return (e - 1u < 
 __device__ __forceinline__ uint32_t row_scale_bits(uint32_t e) { return row_out_of_range(e) ? min(268u - e, 253u) : 127u; }
 __device__ __forceinline__ float row_scale(uint32_t e) { return __uint_as_float(row_scale_bits(e) << 23); }
 __device__ __forceinline__ float row_unscale(uint32_t e) { return __uint_as_float((254u - row_scale_bits(e)) << 23); }
+// A sum times the factors of its row and of its filter, each given as two powers of two of half its exponent: the product of two
+// whole factors may be infinite (a zero sum would become NaN) or zero where the sum's own result is neither.  (The first pass stores
+// rows in range only, whose factor is 1: there a sum is multiplied by its filter's alone.)
+__device__ __forceinline__ float2 factor_halves(float factor) {
+    const uint32_t e = __float_as_uint(factor) >> 23, h = (e + 127u) >> 1;
+    return make_float2(__uint_as_float(h << 23), __uint_as_float((e + 127u - h) << 23));
+}
+__device__ __forceinline__ float unscaled(float sum, float2 row, float2 filter) { return sum * (row.x * filter.x) * (row.y * filter.y); }
 
 // Operands of one tile row, eight 32-bit words at a time (a K stage is four such pieces: 32 TF32 values, or 64 halves in pairs),
 // split into hi/lo parts — TF32: hi = top 19 bits, lo = x - hi, one value per word; bf16: hi = bf16(x), lo = bf16(x - hi), two
@@ -526,12 +534,19 @@ struct StoreJob {
     int Fg, act, nvalid, lane;
     bool valid;
 };
-// fp16, rare: a block's sums times the factor of the row and those of the filters.
-__device__ __forceinline__ void unscale_block(float *r, float unscale, const float *fscale, int f0, int Fg, bool factors, int lane) {
+// fp16, rare: a block's sums times the factors of the filters and, in the second pass, that of the row.
+template <bool SECOND> __device__ __forceinline__ void unscale_block(float *r, float unscale, const float *fscale, int f0, int Fg, bool factors, int lane) {
     const float mine = factors && f0 + lane < Fg ? __ldg(fscale + f0 + lane) : 1.f;
+    if constexpr (SECOND) {
+        const float2 row = factor_halves(unscale), filter = factor_halves(mine);
 #pragma unroll
-    for (int j = 0; j < 32; ++j)
-        r[j] *= unscale * __shfl_sync(0xffffffffu, mine, j);
+        for (int j = 0; j < 32; ++j)
+            r[j] = unscaled(r[j], row, make_float2(__shfl_sync(0xffffffffu, filter.x, j), __shfl_sync(0xffffffffu, filter.y, j)));
+    } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+            r[j] *= __shfl_sync(0xffffffffu, mine, j);
+    }
 }
 template <bool RES>
 __device__ __forceinline__ void store_pixels(const StoreJob &J, const float *bias, const float *stage, int f0) { // four pixels that are all valid per lane
@@ -1485,8 +1500,10 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
                         sum[j] = join_sums<PASSES>(v[j], SPLIT ? x[j] : 0u);
                     if (REDO && (pass || factors)) {
 #pragma unroll
-                        for (int j = 0; j < 8; ++j)
-                            sum[j] *= unscale * (factors && f_tile0 + c + j < P.Fg ? __ldg(P.fscale + (long long)zb * P.Fg + f_tile0 + c + j) : 1.f);
+                        for (int j = 0; j < 8; ++j) {
+                            const float filter = factors && f_tile0 + c + j < P.Fg ? __ldg(P.fscale + (long long)zb * P.Fg + f_tile0 + c + j) : 1.f;
+                            sum[j] = SECOND ? unscaled(sum[j], factor_halves(unscale), factor_halves(filter)) : sum[j] * filter;
+                        }
                     }
                     if (cols >= 8) { // one owner: one address translation; the CTA's own block stays out of the cluster network
                         const int owner = c >> shift;
@@ -1529,7 +1546,7 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
                             r[h + j] = join_sums<PASSES>(v[j], SPLIT ? x[j] : 0u);
                     }
                     if (REDO && (pass || factors))
-                        unscale_block(r, unscale, P.fscale + (long long)zb * P.Fg, f_tile0 + c, P.Fg, factors, lane);
+                        unscale_block<SECOND>(r, unscale, P.fscale + (long long)zb * P.Fg, f_tile0 + c, P.Fg, factors, lane);
                     store_block<decltype(mode_c)::value, decltype(res_c)::value, decltype(long_c)::value>(J, r, stage, f_tile0 + c);
                 }
                 });
@@ -1625,7 +1642,7 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
                         if (c + 32 >= P.BN)
                             release();
                         if (REDO && (pass || factors))
-                            unscale_block(racc, unscale, P.fscale + (long long)zb * P.Fg, ntile * P.BN + c, P.Fg, factors, lane);
+                            unscale_block<SECOND>(racc, unscale, P.fscale + (long long)zb * P.Fg, ntile * P.BN + c, P.Fg, factors, lane);
                         store_block<MODE, RES, decltype(long_c)::value>(J, racc, stage, ntile * P.BN + c);
                     }
                 } else {
@@ -1670,7 +1687,7 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
 #pragma unroll 1
                         for (int c = 0; c < P.BN; c += 32) {
                             if (REDO && (pass || factors))
-                                unscale_block(racc, unscale, P.fscale + (long long)zb * P.Fg, ntile * P.BN + c, P.Fg, factors, lane);
+                                unscale_block<SECOND>(racc, unscale, P.fscale + (long long)zb * P.Fg, ntile * P.BN + c, P.Fg, factors, lane);
                             store_block<MODE, RES, decltype(long_c)::value>(J, racc, stage, ntile * P.BN + c);
 #pragma unroll
                             for (int j = 0; j < 96; ++j) // the next block's sums move down

@@ -117,3 +117,25 @@ def test_graph_runs_around_a_profiled_run(ctx):
     graph.run()
     assert np.array_equal(graph.get_data(out), before)
     ctx.sync_check()
+
+
+# Row and filter both so large (or small) that the product of their factors is no float, while the results are: zero sums of huge values that
+# meet zeros, sums of tiny values near the smallest normal number, huge rows with tiny filters and the other way round.  One tile per CTA,
+# several (narrow, wide), K split.
+@pytest.mark.parametrize("m,n,k", [(130, 40, 64), (5000, 60, 130), (5000, 200, 900), (64, 64, 2048)])
+@pytest.mark.parametrize("row,filt", [(2.0 ** 100, 2.0 ** 100), (2.0 ** -62, 2.0 ** -61), (2.0 ** 90, 2.0 ** -100), (2.0 ** -110, 2.0 ** 96)])
+def test_factors_of_row_and_filter_beyond_a_float(ctx, m, n, k, row, filt):
+    gen = torch.Generator().manual_seed(m + n)
+    a, w = torch.randn(m, k, generator=gen), torch.randn(k, n, generator=gen)
+    if row * filt > 2.0 ** 128:  # nothing huge meets anything but zero
+        a[:, k // 2:], w[:k // 2] = 0, 0
+    a, w = a * row, w * filt
+    plan = ctx.matmul_plan((1, m, k), (1, k, n))
+    assert plan.kernel == "tc_3xtf32_f16_ts"
+    ctx.matmul_set_weights(plan, w.cuda()[None])
+    got = ctx.matmul_run(plan, a.cuda()[None], None)[0].cpu().double()
+    ctx.sync_check()
+    a, w = a.double(), w.double()
+    # (3 * 2^-22 of each product dropped, K / 16 MMAs that each truncate a sum twice: see the tests over all magnitudes)
+    bound = 2.0 ** -22 * ((4 + k / 8) * (a.abs() @ w.abs()) + a.abs().amax(1, keepdim=True) * w.abs().sum(0, keepdim=True) * (row * filt <= 2.0 ** 128))
+    assert bool(((got - a @ w).abs() <= bound + 2.0 ** -149).all())
