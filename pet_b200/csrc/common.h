@@ -107,8 +107,8 @@ inline int launched(petb200_ctx *ctx, const char *what) {
 
 // ---- programmatic dependent launch ---------------------------------------------------------------------------------
 // Kernel families that run on the tensor-core kernel, and the arithmetic ("passes") each one asks of it: 3 = error-compensated
-// TF32, 1 = one TF32 product, 16 = error-compensated bf16, 17 = error-compensated fp16 (the precision of 3xTF32 at the rate of
-// 16-bit operands), 0 = 17 or 3, whichever is faster for the shape.  PETB200_ALGO_AUTO takes PETB200_TC_MATH from the environment
+// TF32, 1 = one TF32 product, 16 = error-compensated bf16, 17 = error-compensated fp16 (at the rate of 16-bit operands; no less
+// precise than 3xTF32 over 21 bits of range and more, see row_exponent), 0 = 17 or 3, whichever is faster for the shape.  PETB200_ALGO_AUTO takes PETB200_TC_MATH from the environment
 // ("3xtf32", "f16x3", "bf16x3"), else 0.
 inline bool tc_is_tc_algo(int algo) {
     return algo == PETB200_ALGO_AUTO || algo == PETB200_ALGO_TC_3XTF32 || algo == PETB200_ALGO_TC_1XTF32 || algo == PETB200_ALGO_TC_BF16X3;

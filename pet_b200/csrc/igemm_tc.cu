@@ -49,10 +49,10 @@ __global__ void __launch_bounds__(256) k_filter_factors(const float *__restrict_
         top = fmaxf(top, fabsf(__ldg(row + i)));
     const uint32_t e = block_max_exponent(top, tops);
     if (threadIdx.x == 0) {
-        unscale[blockIdx.x] = row_unscale(e);
+        unscale[blockIdx.x] = filter_unscale(e);
         if (blockIdx.x == 0)
             numbers[0] = number;
-        if (row_out_of_range(e))
+        if (filter_out_of_range(e))
             numbers[1] = number;
     }
 }
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(256) k_pack_conv_w(const float *__restrict__ w
         if (tap < T && c < cpg)
             v = __ldg(w + ((long long)f * cpg + c) * T + tap);
         if (MATH == kMathF16x3)
-            v *= 1.f / unscale[f]; // (a power of two)
+            v *= kFilterUnit / unscale[f]; // (a power of two)
         store_split<MATH>(hi, lo, i, v);
     }
 }
@@ -210,12 +210,12 @@ __global__ void __launch_bounds__(256) k_prepare_f16_kn(const PrepareArgs g) {
     }
     if (warp == 0) {
         const uint32_t e = row_exponent(top);
-        factor[lane] = row_scale(e);
+        factor[lane] = kFilterUnit / filter_unscale(e);
         if (rank == 0 && col_ok) {
-            g.unscale[(long long)bb * g.n + n0 + lane] = row_unscale(e);
+            g.unscale[(long long)bb * g.n + n0 + lane] = filter_unscale(e);
             if (blockIdx.x == 0 && lane == 0)
                 g.numbers[0] = g.number;
-            if (row_out_of_range(e))
+            if (filter_out_of_range(e))
                 g.numbers[1] = g.number;
         }
     }
@@ -274,12 +274,12 @@ __global__ void __launch_bounds__(256) k_prepare_f16_nk(const PrepareArgs g) {
             top = fmaxf(top, tops[i]);
     }
     const uint32_t e = row_exponent(top);
-    const float factor = row_scale(e);
+    const float factor = kFilterUnit / filter_unscale(e);
     if (row_ok && u0 == 0 && lane == 0) {
-        g.unscale[row] = row_unscale(e);
+        g.unscale[row] = filter_unscale(e);
         if (row == 0)
             g.numbers[0] = g.number;
-        if (row_out_of_range(e))
+        if (filter_out_of_range(e))
             g.numbers[1] = g.number;
     }
 #pragma unroll 4

@@ -298,12 +298,17 @@ __device__ __forceinline__ float max3_abs(float t, float a, float b) {
     asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(t), "f"(a), "f"(b));
     return d;
 }
-// {(a - h.x) * s, (b - h.y) * s} for a power of two s, exact where a - h.x is: two instructions on pairs.
-__device__ __forceinline__ float2 scaled_diff_f32x2(float a, float b, float2 h, float s) {
+__device__ __forceinline__ float2 mul_f32x2(float2 v, float s) {
     float2 d;
-    asm("{\n\t.reg .b64 x, y, p, n;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 p, {%6, %6};\n\tmov.b64 n, {%7, %7};\n\t"
-        "mul.rn.f32x2 x, x, p;\n\tfma.rn.f32x2 x, y, n, x;\n\tmov.b64 {%0, %1}, x;\n\t}"
-        : "=f"(d.x), "=f"(d.y) : "f"(a), "f"(b), "f"(h.x), "f"(h.y), "f"(s), "f"(-s));
+    asm("{\n\t.reg .b64 x, p;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 p, {%4, %4};\n\tmul.rn.f32x2 x, x, p;\n\tmov.b64 {%0, %1}, x;\n\t}"
+        : "=f"(d.x), "=f"(d.y) : "f"(v.x), "f"(v.y), "f"(s));
+    return d;
+}
+// {v.x - 2048 * lower half, v.y - 2048 * upper half}: fused multiply-adds that take the halves as they are (0xe800 is -2048).
+__device__ __forceinline__ float2 minus_2048_halves(float2 v, uint32_t h) {
+    float2 d;
+    asm("{\n\t.reg .b16 l, u, c;\n\tmov.b32 {l, u}, %2;\n\tmov.b16 c, 0xe800;\n\tfma.rn.f32.f16 %0, l, c, %3;\n\tfma.rn.f32.f16 %1, u, c, %4;\n\t}"
+        : "=f"(d.x), "=f"(d.y) : "r"(h), "f"(v.x), "f"(v.y));
     return d;
 }
 // Two fp32 values rounded to nearest bf16 and packed, `a` in the low half.

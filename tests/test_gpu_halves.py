@@ -139,3 +139,37 @@ def test_factors_of_row_and_filter_beyond_a_float(ctx, m, n, k, row, filt):
     # (3 * 2^-22 of each product dropped, K / 16 MMAs that each truncate a sum twice: see the tests over all magnitudes)
     bound = 2.0 ** -22 * ((4 + k / 8) * (a.abs() @ w.abs()) + a.abs().amax(1, keepdim=True) * w.abs().sum(0, keepdim=True) * (row * filt <= 2.0 ** 128))
     assert bool(((got - a @ w).abs() <= bound + 2.0 ** -149).all())
+
+
+# Values of very different size in one row or filter, the largest of which meet zeros: what is left of the small ones decides.  No less
+# precise than three products of TF32.
+@pytest.mark.parametrize("top,rest", [(1.0, 1.0), (1.0, 1e-6), (1.0, 1e-7), (1e-4, 1e-7), (200.0, 1e-6), (900.0, 1e-4), (0.02, 1e-6), (3e-3, 1e-7), (1e-9, 1e-15), (1e9, 1e3)])
+@pytest.mark.parametrize("where", ["rows", "filters"])
+@pytest.mark.parametrize("kind", ["matmul", "matmul_trans_b", "matmul_weight", "conv2d"])
+def test_mixed_magnitudes_no_less_precise_than_tf32(ctx, monkeypatch, kind, where, top, rest):
+    gen = torch.Generator().manual_seed(7)
+    m, n, k = 288, 64, 512
+    big, other = torch.randn(m if where == "rows" else n, k, generator=gen) * rest, torch.randn(n if where == "rows" else m, k, generator=gen)
+    big[:, 5], other[:, 5] = top, 0.0
+    x, w = ((big, other) if where == "rows" else (other, big))
+    want = x.double() @ w.double().t()
+
+    def product(math):
+        monkeypatch.setenv("PETB200_TC_MATH", math)
+        if kind == "conv2d":
+            xd, wd = x.t().reshape(1, k, 12, 24).contiguous().cuda(), w.reshape(n, k, 1, 1).cuda()
+            plan = ctx.conv2d_plan(xd.shape, wd.shape, 0, 0)
+            ctx.conv2d_set_weights(plan, wd)
+            got = ctx.conv2d_run(plan, xd).reshape(n, m).t()
+        else:
+            wd = (w if kind == "matmul_trans_b" else w.t().contiguous()).cuda()[None]
+            plan = ctx.matmul_plan((1, m, k), wd.shape, False, kind == "matmul_trans_b")
+            if kind == "matmul_weight":
+                ctx.matmul_set_weights(plan, wd)
+            got = ctx.matmul_run(plan, x.cuda()[None], None if kind == "matmul_weight" else wd)[0]
+        assert plan.kernel == ("tc_3xtf32_f16_ts" if math == "f16x3" else "tc_3xtf32_ts")
+        return float((got.cpu().double() - want).norm() / want.norm())
+
+    halves, tf32 = product("f16x3"), product("3xtf32")
+    ctx.sync_check()
+    assert halves <= tf32, (halves, tf32)
