@@ -42,7 +42,7 @@ enum {
      * times closer to the exact result.  What they leave out of a product x * w is at most 2^-21 |x w| + 2^-42 |w| + 2^-44 |x|
      * (3XTF32: 3 * 2^-20 |x w|, however small x or w are), so values below 2^-23 lose digits beside values of ordinary size.  Operands
      * of any scale are served: where the largest of an output's operands is outside [2^-12, 2^8), or a filter's (or column of B's)
-     * outside [2^-7, 2^6), they are scaled first; such rows make their tiles take two to four times as long. */
+     * outside [2^-7, 2^6), they are scaled first; such rows make a launch take two to three times as long. */
     PETB200_ALGO_AUTO = 0,
     PETB200_ALGO_TC_3XTF32 = 1, /* tcgen05 implicit GEMM, error-compensated TF32 (fp32-grade accuracy) */
     PETB200_ALGO_SIMT_FP32 = 2, /* CUDA-core FFMA, exact fp32 products */

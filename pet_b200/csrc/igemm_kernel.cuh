@@ -248,8 +248,10 @@ __device__ __forceinline__ void epilogue_banded(uint32_t tacc, uint32_t tcross, 
 // holds the probabilities of 4096 equal keys.)  Any other row would lose digits or overflow.  So the transform threads follow the
 // largest magnitude of what they split and leave its exponent beside every stage (a test for the tile's last stage would be a branch
 // per stage, which costs more); whoever stores 32 rows looks at theirs first and, if one is out of range, stores nothing and asks for a second
-// pass: the CTA's tiles once more, each twice in a row, the first time for the exponents and the second with rows out of range
-// multiplied by a power of two, which is taken out again when the sums are stored.  Only what the first pass left is stored.
+// pass: the CTA's tiles once more with rows out of range multiplied by a power of two, which is taken out again when the sums are
+// stored.  A CTA of more tiles than the exponents of kExpSlots tell has each twice in a row there, the first time for its exponents.
+// Only what the first pass left is stored.  (All rows at 1e-5, ordinary rows, 3xTF32: 384 x 3072 x 768 21 / 11 / 13 us, 64 images of
+// 128 x 28 x 28 through a 3x3 layer 175 / 59 / 82, the dilated 512-channel layer 111 / 52 / 78; with every tile twice 29, 238 and 172.)
 // A row in range has the factor 1 in both passes, so its result does not depend on its neighbours.  Filters get their factor
 // when they are packed, which costs nothing then, so theirs is 1 in [2^-7, 2^6) only.  Where the packing has seen another factor the
 // sums are multiplied before they are stored.
@@ -851,7 +853,7 @@ struct CtaPlace {
 };
 constexpr uint32_t kTmemCols = 512;
 
-// One pass over the CTA's tiles, by role.  fp16 may need a second, whose items are every tile twice (see row_exponent).
+// One pass over the CTA's tiles, by role.  fp16 may need a second, whose items may be every tile twice (see row_exponent).
 // BAND: 0 ordinary operands; 1 G2BMM (banded epilogue, key windows per tile; persistent row-major mode only); 2 GBMML (A operand
 // gathered from the band in global memory; row-major mode only).  Kernels of their own, so that the others carry none of it.
 template <bool A_KMAJOR, int PASSES, int PP, int BAND, bool SECOND>
@@ -991,7 +993,10 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
 
     if (!SECOND && warp < kSetWarp)
         ptx::reg_dealloc<Regs<PP>::control>();
-    auto tile_of = [&](int item) { return (int)blockIdx.x + (item >> pass) * (int)gridDim.x; };
+    // second pass: 1 where every tile is two items, the first for its exponents alone, the second for its sums
+    const int twice = SECOND && ntl > kExpSlots ? 1 : 0;
+    [[maybe_unused]] auto for_sums = [&](int item) -> bool { return !twice || (item & 1); };
+    auto tile_of = [&](int item) { return (int)blockIdx.x + (item >> twice) * (int)gridDim.x; };
     uint64_t *raw_full = bars, *raw_empty = bars + kMaxNR;
     uint64_t *b_full = bars + 2 * kMaxNR, *b_empty = b_full + kMaxNB; // up to kMaxNB stages
     uint64_t *a_full = b_empty + kMaxNB, *a_empty = a_full + 4;       // up to 4 stages
@@ -1002,12 +1007,12 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
     uint64_t *acc_empty = acc_full + 7; // [2]: the drain warps have read accumulator region 0 / 1 out
     uint64_t *trash = acc_full + 9;     // takes the MMA thread's releases after it gave up
     [[maybe_unused]] uint64_t *scanned = acc_full + 10; // second pass: both transform sets have recorded a tile's exponents
-    const int items = ntl << pass;
+    const int items = ntl << twice;
     // fp16: exponent of row `row` of a tile (one of a single stage was seen by one set alone; a pair's second item has its first's)
     [[maybe_unused]] auto exponent_of = [&](int item, int row) -> uint32_t {
-        if (SECOND)
+        if (twice)
             item &= ~1;
-        const volatile uint8_t *e = row_exps + ((item >> pass) & (kExpSlots - 1)) * 2 * kTileM + row;
+        const volatile uint8_t *e = row_exps + ((item >> twice) & (kExpSlots - 1)) * 2 * kTileM + row;
         return KS == 1 ? (uint32_t)e[(item & 1) * kTileM] : max((uint32_t)e[0], (uint32_t)e[kTileM]);
     };
     // Asked by a warp that stores 32 rows, one of them of exponent e: are they stored in this pass?
@@ -1249,8 +1254,7 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
                     if (PP != kNarrow && g0 + FLm < stages_end) // (0 after a give-up) fires once every MMA of the group has completed
                         ptx::mma_commit(acc_ready);
                 }
-                // (a single tile's second pass completes once, with its second item: the first is for the exponents alone)
-                if (ok && (!REDO || PP || tl + 1 == tiles_left))
+                if (ok)
                     ptx::mma_commit((two_regions && (tl & 1)) ? acc_full1 : acc_full);
             }
         }
@@ -1290,10 +1294,10 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
                 int base_p;
                 pixel_geom(p, valid, base_p, y_off);
                 float top = 0.f; // fp16: largest magnitude of this thread's operands
-                [[maybe_unused]] volatile uint8_t *my_exp = row_exps + (((tl >> pass) & (kExpSlots - 1)) * 2 + tset) * kTileM + p;
+                [[maybe_unused]] volatile uint8_t *my_exp = row_exps + (((tl >> twice) & (kExpSlots - 1)) * 2 + tset) * kTileM + p;
                 [[maybe_unused]] float factor = 1.f;
                 if constexpr (RESCALE) {
-                    if (tl & 1)
+                    if (for_sums(tl))
                         factor = row_scale(exponent_of(tl, p));
                 }
                 if (P.ksplit > 1 && tset == 0)
@@ -1423,7 +1427,7 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
                         }
                         if (!alive)
                             break;
-                        if (REDO && !(RESCALE && (tl & 1)))
+                        if (REDO && !(RESCALE && for_sums(tl)))
                             *my_exp = (uint8_t)row_exponent(top);
                         ptx::tmem_st_wait();
                         ptx::tc_fence_before();
@@ -1442,7 +1446,7 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
                     }
                 }
                 if constexpr (RESCALE) {
-                    if (!(tl & 1) && alive) { // the other set's exponents are needed too
+                    if (!for_sums(tl) && alive) { // the other set's exponents are needed too
                         __syncwarp();
                         if (lane == 0)
                             ptx::mbar_arrive(scanned);
@@ -1629,7 +1633,7 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
                 [[maybe_unused]] auto leave_out = [&]() { // fp16, once a tile is complete: not stored in this pass, or not by this item
                     const uint32_t e = exponent_of(tl, p);
                     unscale = row_unscale(e);
-                    return !store_now(e, J.valid) || (SECOND && !(tl & 1));
+                    return !store_now(e, J.valid) || !for_sums(tl);
                 };
                 if constexpr (PP == kNarrow) {
                     take_acc_full();
@@ -1673,8 +1677,6 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
                         if (lane == 0)
                             ptx::mbar_arrive(flushed);
                     }
-                    if (REDO && PP == kSingle && tl + 1 < items)
-                        continue; // (completes with the second item)
                     if (alive)
                         take_acc_full();
                     if (!alive)
@@ -1741,7 +1743,7 @@ k_igemm(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUte
     uint8_t *smem = smem_raw + ((1024u - (ptx::smem_u32(smem_raw) & 1023u)) & 1023u);
     const CtaSmem S(smem, P);
     const CtaPlace at(PP, P);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
     if (threadIdx.x == 0) {
         init_barriers(S.bars, BAND == 2 ? 256 : 1); // (GBMML: every transform thread)
         *S.abort_flag = 0;

@@ -173,3 +173,24 @@ def test_mixed_magnitudes_no_less_precise_than_tf32(ctx, monkeypatch, kind, wher
     halves, tf32 = product("f16x3"), product("3xtf32")
     ctx.sync_check()
     assert halves <= tf32, (halves, tf32)
+
+
+# Many tiles per CTA: with one row out of range a CTA repeats all of its tiles, those of more than eight twice in a row; narrow tiles, wide ones
+# with a flush, tiles of a single K stage (which one transform set sees alone)
+@pytest.mark.parametrize("m,n,k", [(148 * 128 * 8, 60, 130), (148 * 128 * 11 + 5, 60, 130), (148 * 128 * 9, 40, 50), (148 * 128 * 3, 40, 50), (20000, 1280, 800), (9000, 1280, 800)])
+@pytest.mark.parametrize("rows", ["some", "all"])
+def test_second_pass_of_many_tiles(ctx, m, n, k, rows):
+    gen = torch.Generator(device="cuda").manual_seed(m + k)
+    a, w = torch.randn(m, k, device="cuda", generator=gen), torch.randn(k, n, device="cuda", generator=gen)
+    a[:: 997 if rows == "some" else 1] *= 1e-9
+    a[5::1999] *= 1e7
+    w[:, 3] *= 1e-7
+    plan = ctx.matmul_plan((1, m, k), (1, k, n))
+    assert plan.kernel == "tc_3xtf32_f16_ts"
+    ctx.matmul_set_weights(plan, w[None])
+    got = ctx.matmul_run(plan, a[None], None)[0].double()
+    ctx.sync_check()
+    a, w = a.double(), w.double()
+    # (as in the tests over all magnitudes; the values of a row or filter are of one magnitude here)
+    bound = 2.0 ** -22 * ((4 + k / 8) * (a.abs() @ w.abs()) + a.abs().amax(1, keepdim=True) * w.abs().sum(0, keepdim=True))
+    assert bool(((got - a @ w).abs() <= bound).all())
