@@ -46,6 +46,8 @@ struct petb200_ctx {
     std::string err;
     int *d_status = nullptr; // device word kernels write when a bounded wait expires
     bool band_attr_set = false;   // the banded-product kernel's shared-memory limit was raised on this device
+    bool tc_attr_set = false;     // the same for the tensor-core kernel and its preparation
+    int cluster_slots[17] = {0};  // clusters of that many of its CTAs that the device holds (0: not asked yet)
     petb200::DevBuf band_scratch; // partial sums of a banded product split over its band columns (grown on demand)
     // Buffers band_scratch outgrew.  They stay allocated until the context goes: a CUDA graph captured while one of them
     // was current has its address baked into its kernel nodes and may still be replayed.

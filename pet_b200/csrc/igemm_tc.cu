@@ -496,11 +496,11 @@ static int env_int(const char *name, int dflt) {
 
 // How many clusters of `ks` CTAs of this kernel (one CTA per SM) the device can hold at once: asked of the driver once
 // per size (clusters stay inside a GPC, which leaves some SMs of every GPC without a cluster).
-static int cluster_slots(int sm_count, int ks) {
-    static int cached[17] = {0};
+static int cluster_slots(petb200_ctx *ctx, int ks) {
+    const int sm_count = ctx->sm_count;
     if (ks <= 1)
         return sm_count;
-    if (cached[ks] == 0) {
+    if (ctx->cluster_slots[ks] == 0) {
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(1, (unsigned)ks * 64, 1);
         cfg.blockDim = dim3(kThreads);
@@ -518,9 +518,9 @@ static int cluster_slots(int sm_count, int ks) {
             // what B200 was measured to hold; a cluster of 16 is only used where the driver itself says it fits
             n = ks > 8 ? -1 : std::max(1, (sm_count * (ks <= 2 ? 96 : 86) / 100) / ks);
         }
-        cached[ks] = n;
+        ctx->cluster_slots[ks] = n;
     }
-    return cached[ks];
+    return ctx->cluster_slots[ks];
 }
 
 // Rough cycle model of one launch, used to pick the tile width and the K split.  All constants are measured on row-major products of
@@ -530,12 +530,12 @@ static int cluster_slots(int sm_count, int ks) {
 // 128-filter tile in two the dearest (12500).  Several unsplit tiles in turn hide start-up and epilogue (persistent tiles).
 // Against the fastest of all pairs on 57 shapes (these products, ResNet layers at batch 1 to 16): within 2 % on 54; the others lose
 // 4, 11 and 14 % (64 x 1000 x 256, a 200-channel 3x3 at 3 x 20 x 20, 16 x 3072 x 768).  The constants before lost up to 31 % on 12 of them.
-static double est_cycles(int sm_count, long long base_ctas, int nchunks, int spc, int BN, int math, int ks) {
+static double est_cycles(petb200_ctx *ctx, long long base_ctas, int nchunks, int spc, int BN, int math, int ks) {
     const int w = BN <= 32 ? 0 : (BN <= 64 ? 1 : 2);
     static const double tf32[3] = {570, 655, 890}, halves[3] = {910, 910, 1045}, exchange[3] = {2300, 2500, 8000};
     const double stage = math == kMathTf32x1 ? 520.0 : (math == kMathTf32x3 ? tf32[w] : halves[w]), start = 6300.0;
     const double stages = (double)((nchunks + ks - 1) / ks) * spc;
-    const long long slots = cluster_slots(sm_count, ks);
+    const long long slots = cluster_slots(ctx, ks);
     if (slots <= 0)
         return 1e30; // this cluster size cannot be launched here
     const double waves = (double)((base_ctas + slots - 1) / slots), epilogue = 34.0 * BN;
@@ -545,20 +545,20 @@ static double est_cycles(int sm_count, long long base_ctas, int nchunks, int spc
 }
 // Split K over 1, 2, 4, 8 or 16 CTAs (a cluster; 16 is beyond the portable cluster size and allowed per function): the
 // split must divide the tile width and leave every CTA a chunk.
-static int choose_ksplit(int sm_count, long long base_ctas, const IgemmParams &P, int math, int want, double *cycles) {
+static int choose_ksplit(petb200_ctx *ctx, long long base_ctas, const IgemmParams &P, int math, int want, double *cycles) {
     auto ok = [&](int ks) { return ks == 1 || (ks <= P.nchunks && P.BN % ks == 0); };
     int best = 1;
-    double best_c = est_cycles(sm_count, base_ctas, P.nchunks, P.spc, P.BN, math, 1);
+    double best_c = est_cycles(ctx, base_ctas, P.nchunks, P.spc, P.BN, math, 1);
     static const int ks_cap = std::min(16, std::max(1, env_int_early("PETB200_TC_KSPLIT_MAX", 16)));
     if (want > 0) {
-        for (best = 16; best > 1 && !(best <= want && ok(best) && cluster_slots(sm_count, best) > 0); best /= 2) {
+        for (best = 16; best > 1 && !(best <= want && ok(best) && cluster_slots(ctx, best) > 0); best /= 2) {
         }
-        best_c = est_cycles(sm_count, base_ctas, P.nchunks, P.spc, P.BN, math, best);
+        best_c = est_cycles(ctx, base_ctas, P.nchunks, P.spc, P.BN, math, best);
     } else {
         for (int ks = 2; ks <= ks_cap; ks *= 2) {
             if (!ok(ks))
                 continue;
-            const double c = est_cycles(sm_count, base_ctas, P.nchunks, P.spc, P.BN, math, ks);
+            const double c = est_cycles(ctx, base_ctas, P.nchunks, P.spc, P.BN, math, ks);
             if (c < best_c * 0.97) // a deeper split has to pay for itself
                 best = ks, best_c = c;
         }
@@ -610,11 +610,10 @@ static void choose_grid(petb200_ctx *ctx, TcCore &core, int mtiles, int ntiles, 
     core.grid = dim3((unsigned)((tiles + per_cta - 1) / per_cta), 1, 1);
 }
 
-// The dynamic shared-memory attribute is per function, not per launch: raise it once to the device limit so that plans
-// with different needs can coexist.
+// The dynamic shared-memory attribute is per function and device, not per launch: each context raises it once to the device limit
+// so that plans with different needs can coexist.
 static int raise_smem_limit(petb200_ctx *ctx) {
-    static bool attr_set = false;
-    if (attr_set)
+    if (ctx->tc_attr_set)
         return PETB200_OK;
     const int lim = (int)std::min<size_t>(ctx->smem_optin, 227 * 1024);
     cudaError_t e = cudaSuccess;
@@ -632,7 +631,7 @@ static int raise_smem_limit(petb200_ctx *ctx) {
         e = cudaFuncSetAttribute(k_prepare_f16_kn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPrepSmem);
     if (e != cudaSuccess)
         return fail(ctx, PETB200_ERR_CUDA, "cudaFuncSetAttribute(%d bytes) failed: %s", lim, cudaGetErrorString(e));
-    attr_set = true;
+    ctx->tc_attr_set = true;
     return PETB200_OK;
 }
 
@@ -795,7 +794,7 @@ static int tc_configure(petb200_ctx *ctx, TcCore &core, const ConvGeom &g, int o
             continue;
         const long long base_ctas = (long long)mtiles * ((Fg + bn - 1) / bn) * gz * core.beside;
         double cyc;
-        const int ks = choose_ksplit(ctx->sm_count, base_ctas, P, core.math, want_ks, &cyc);
+        const int ks = choose_ksplit(ctx, base_ctas, P, core.math, want_ks, &cyc);
         if (ks > 1) { // the landing area takes shared memory from the rings (or even from the chunk size): fit again
             P.ksplit = ks;
             if (!fit(bn))
@@ -804,7 +803,7 @@ static int tc_configure(petb200_ctx *ctx, TcCore &core, const ConvGeom &g, int o
                 P.ksplit = 1;
                 if (!fit(bn))
                     continue;
-                cyc = est_cycles(ctx->sm_count, base_ctas, P.nchunks, P.spc, bn, core.math, 1);
+                cyc = est_cycles(ctx, base_ctas, P.nchunks, P.spc, bn, core.math, 1);
             }
         }
         if (!have || cyc < best_cycles * 0.97) { // prefer the wider tile unless the narrower one clearly wins
@@ -1154,7 +1153,7 @@ static int tc_configure_kmajor(petb200_ctx *ctx, TcCore &core, int bs, int m, in
                 continue;
             P.BN = bn;
             double cyc;
-            const int ks = choose_ksplit(ctx->sm_count, (long long)P.tpi * ((n + bn - 1) / bn) * bs, P, core.math,
+            const int ks = choose_ksplit(ctx, (long long)P.tpi * ((n + bn - 1) / bn) * bs, P, core.math,
                                          env_int("PETB200_TC_KSPLIT", 0), &cyc);
             if (!best_bn || cyc < best * 0.97)
                 best = cyc, best_bn = bn, best_ks = ks;

@@ -194,3 +194,27 @@ def test_second_pass_of_many_tiles(ctx, m, n, k, rows):
     # (as in the tests over all magnitudes; the values of a row or filter are of one magnitude here)
     bound = 2.0 ** -22 * ((4 + k / 8) * (a.abs() @ w.abs()) + a.abs().amax(1, keepdim=True) * w.abs().sum(0, keepdim=True))
     assert bool(((got - a @ w).abs() <= bound).all())
+
+
+# What a context asks of the device once (cluster sizes, shared-memory limits) is kept per context: contexts of several threads plan the same
+def test_contexts_of_two_threads(ctx):
+    import threading
+    from pet_b200.ops import Context
+    x, w = torch.randn(2, 64, 16, 16, device="cuda"), torch.randn(48, 64, 3, 3, device="cuda")
+    a, b = torch.randn(1, 16, 2048, device="cuda"), torch.randn(1, 2048, 96, device="cuda")
+    want, got = (ctx.conv2d(x, w, 1, 1), ctx.matmul(a, b)), {}
+    torch.cuda.synchronize()
+
+    def work(i):
+        own = Context(0)
+        got[i] = (own.conv2d(x, w, 1, 1), own.matmul(a, b))
+        own.sync_check()
+        own.close()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for i in range(2):
+        assert all(torch.equal(p, q) for p, q in zip(got[i], want))
