@@ -11,13 +11,9 @@ namespace petb200 {
 // weight packing: W[F][cpg][T] (conv) or B[b][k][n] / B[b][n][k] (matmul) -> hi/lo [rows][Ktot], K ordered as the
 // kernel consumes it: k = chunk*Kc_pad + tap*BC + ci, zero where there is no such element.
 // -------------------------------------------------------------------------------------------------------------
-// hi/lo parts of one packed value: TF32 (hi = top 19 bits, or rounded for a single pass) as fp32 words, or 16-bit halves
+// hi/lo parts of one packed value: TF32 (hi = top 19 bits, or rounded for a single pass) as fp32 words, or bf16
 template <int MATH> __device__ __forceinline__ void store_split(void *hi, void *lo, long long i, float v) {
-    if (MATH == kMathF16x3) {
-        const uint32_t h = ptx::pack_f16x2(v, 0.f) & 0xffffu;
-        reinterpret_cast<uint16_t *>(hi)[i] = (uint16_t)h;
-        reinterpret_cast<uint16_t *>(lo)[i] = (uint16_t)(ptx::pack_f16x2((v - ptx::unpack_f16x2(h).x) * kLoScale, 0.f) & 0xffffu);
-    } else if (MATH == kMathBf16x3) {
+    if (MATH == kMathBf16x3) {
         const uint32_t h = ptx::pack_bf16x2(v, 0.f) & 0xffffu;
         reinterpret_cast<uint16_t *>(hi)[i] = (uint16_t)h;
         reinterpret_cast<uint16_t *>(lo)[i] = (uint16_t)(ptx::pack_bf16x2(v - __uint_as_float(h << 16), 0.f) & 0xffffu);
@@ -28,39 +24,10 @@ template <int MATH> __device__ __forceinline__ void store_split(void *hi, void *
     }
 }
 
-// fp16: the factor of a filter whose largest magnitude has exponent e (see row_exponent), and what its sums are multiplied by.
-// Factors of conv filters [F][per_filter], one block each.
-__device__ __forceinline__ uint32_t block_max_exponent(float top, float *warp_tops /*[blockDim / 32]*/) {
-    for (int o = 16; o; o >>= 1)
-        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-    if ((threadIdx.x & 31) == 0)
-        warp_tops[threadIdx.x >> 5] = top;
-    __syncthreads();
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i)
-        top = fmaxf(top, warp_tops[i]);
-    return row_exponent(top);
-}
-__global__ void __launch_bounds__(256) k_filter_factors(const float *__restrict__ w, float *__restrict__ unscale, long long per_filter,
-                                                        uint16_t *numbers, uint16_t number) {
-    __shared__ float tops[8];
-    const float *row = w + blockIdx.x * per_filter;
-    float top = 0.f;
-    for (long long i = threadIdx.x; i < per_filter; i += 256)
-        top = fmaxf(top, fabsf(__ldg(row + i)));
-    const uint32_t e = block_max_exponent(top, tops);
-    if (threadIdx.x == 0) {
-        unscale[blockIdx.x] = filter_unscale(e);
-        if (blockIdx.x == 0)
-            numbers[0] = number;
-        if (filter_out_of_range(e))
-            numbers[1] = number;
-    }
-}
-
 template <int MATH>
 __global__ void __launch_bounds__(256) k_pack_conv_w(const float *__restrict__ w, void *__restrict__ hi,
                                                      void *__restrict__ lo, int F, int cpg, int T, int BC, int Kc_pad,
-                                                     int nchunks, const float *__restrict__ unscale) {
+                                                     int nchunks) {
     const long long Ktot = (long long)Kc_pad * nchunks;
     const long long total = (long long)F * Ktot;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -72,10 +39,62 @@ __global__ void __launch_bounds__(256) k_pack_conv_w(const float *__restrict__ w
         float v = 0.f;
         if (tap < T && c < cpg)
             v = __ldg(w + ((long long)f * cpg + c) * T + tap);
-        if (MATH == kMathF16x3)
-            v *= kFilterUnit / unscale[f]; // (a power of two)
         store_split<MATH>(hi, lo, i, v);
     }
+}
+
+// Two packed values of fp16, times the filter's factor and unit, in one word of hi and one of lo.
+__device__ __forceinline__ void store_halves(void *hi, void *lo, long long word, float a, float b, float factor) {
+    a *= factor, b *= factor;
+    const uint32_t h = ptx::pack_f16x2(a, b);
+    const float2 hf = ptx::unpack_f16x2(h);
+    reinterpret_cast<uint32_t *>(hi)[word] = h;
+    reinterpret_cast<uint32_t *>(lo)[word] = ptx::pack_f16x2((a - hf.x) * kLoScale, (b - hf.y) * kLoScale);
+}
+// fp16: a packed filter has a factor (see row_exponent), known only when all of it has been seen.  gridDim.y blocks share filter
+// blockIdx.x: each looks at all of it, the second time out of the caches, and packs its part.  (Factors in a launch of their own: 30
+// instead of 17 us for the weights of a 512-channel 3x3 layer, call to call, 15 instead of 12 for a 64-channel one.)
+struct PackFilters {
+    const float *w;
+    void *hi, *lo;
+    float *unscale;            // what the filter's sums are multiplied by
+    uint16_t *numbers, number; // see TcCore::factor_word
+    int cpg, T, BC, Ktot;
+    FastDiv by_kc_pad, by_bc;
+};
+__global__ void __launch_bounds__(256) k_pack_conv_f16(const PackFilters g) {
+    __shared__ float tops[8];
+    const int f = (int)blockIdx.x, lane = threadIdx.x & 31, per_filter = g.cpg * g.T;
+    const float *src = g.w + (long long)f * per_filter;
+    float top = 0.f;
+#pragma unroll 8
+    for (int i = threadIdx.x; i < per_filter; i += 256)
+        top = fmaxf(top, fabsf(__ldg(src + i)));
+    for (int o = 16; o; o >>= 1)
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+    if (lane == 0)
+        tops[threadIdx.x >> 5] = top;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+        top = fmaxf(top, tops[i]);
+    const uint32_t e = row_exponent(top);
+    const float factor = kFilterUnit / filter_unscale(e);
+    if (threadIdx.x == 0 && blockIdx.y == 0) {
+        g.unscale[f] = filter_unscale(e);
+        if (f == 0)
+            g.numbers[0] = g.number;
+        if (filter_out_of_range(e))
+            g.numbers[1] = g.number;
+    }
+    auto at = [&](int k) { // value at a packed position: 0 past the taps of a chunk or the channels of the filter
+        const int ch = g.by_kc_pad.div(k), kc = k - ch * (int)g.by_kc_pad.d, tap = g.by_bc.div(kc), c = ch * g.BC + kc - tap * g.BC;
+        return tap < g.T && c < g.cpg ? __ldg(src + c * g.T + tap) : 0.f;
+    };
+    const int words = g.Ktot / 2; // (a multiple of 32: whole stages of 64)
+#pragma unroll 4
+    for (int i = (int)blockIdx.y * 256 + threadIdx.x; i < words; i += (int)gridDim.y * 256)
+        store_halves(g.hi, g.lo, (long long)f * words + i, at(2 * i), at(2 * i + 1), factor);
 }
 
 // What a matmul needs before it can run, in one launch (bound by HBM: every operand read once, its copy written once).
@@ -151,13 +170,6 @@ __global__ void __launch_bounds__(256) k_prepare_mm(const PrepareArgs g) {
 // stay in shared memory (as many as there is room for, more are read again) while the columns' maxima meet through the cluster.
 constexpr int kPrepUnit = 64, kPrepKeep = 8, kPrepPitch = 33;
 constexpr size_t kPrepSmem = (size_t)kPrepKeep * kPrepUnit * kPrepPitch * 4;
-__device__ __forceinline__ void pack_pair(const PrepareArgs &g, long long word, float a, float b, float factor) {
-    a *= factor, b *= factor;
-    const uint32_t h = ptx::pack_f16x2(a, b);
-    const float2 hf = ptx::unpack_f16x2(h);
-    reinterpret_cast<uint32_t *>(g.hi)[word] = h;
-    reinterpret_cast<uint32_t *>(g.lo)[word] = ptx::pack_f16x2((a - hf.x) * kLoScale, (b - hf.y) * kLoScale);
-}
 // Unit u of the packed row: first row of B, number of rows.
 __device__ __forceinline__ void prep_unit(const PrepareArgs &g, int u, int &kk0, int &kn) {
     const int k0 = u * kPrepUnit, ch = g.by_kc_pad.div(k0), kc0 = k0 - ch * (int)g.by_kc_pad.d;
@@ -234,7 +246,7 @@ __global__ void __launch_bounds__(256) k_prepare_f16_kn(const PrepareArgs g) {
 #pragma unroll
         for (int c = warp; c < 32; c += 8)
             if (n0 + c < g.n)
-                pack_pair(g, (((long long)bb * g.n + n0 + c) * g.Kpad + u * kPrepUnit) / 2 + lane, tile[2 * lane * kPrepPitch + c],
+                store_halves(g.hi, g.lo, (((long long)bb * g.n + n0 + c) * g.Kpad + u * kPrepUnit) / 2 + lane, tile[2 * lane * kPrepPitch + c],
                           tile[(2 * lane + 1) * kPrepPitch + c], factor[c]);
     }
 }
@@ -286,7 +298,7 @@ __global__ void __launch_bounds__(256) k_prepare_f16_nk(const PrepareArgs g) {
     for (int u = u0; u < u1; u += step) {
         int kk0, kn;
         prep_unit(g, u, kk0, kn);
-        pack_pair(g, (row * g.Kpad + u * kPrepUnit) / 2 + lane, 2 * lane < kn ? __ldg(src + kk0 + 2 * lane) : 0.f,
+        store_halves(g.hi, g.lo, (row * g.Kpad + u * kPrepUnit) / 2 + lane, 2 * lane < kn ? __ldg(src + kk0 + 2 * lane) : 0.f,
                   2 * lane + 1 < kn ? __ldg(src + kk0 + 2 * lane + 1) : 0.f, factor);
     }
 }
@@ -329,6 +341,7 @@ struct TcCore {
     long long Ktot = 0;
     int rows_b = 0;
     DevBuf whi, wlo, koff;
+    std::vector<int> offsets; // what `koff` holds: made by the configuration (of which a plan may go through two), uploaded once
     // fp16: a factor per packed row of B, and behind them a word of two halves: the number of the last packing (modulo 2^16), and that
     // of the last one which found a factor other than 1.  The kernel multiplies where they are equal.  Both are written by the
     // packing and read by the product on the device: a launch that a CUDA graph holds is replayed after packings that came later
@@ -403,7 +416,15 @@ struct TcCore {
         map_x_ptr = x;
         return PETB200_OK;
     }
+    int upload_offsets() {
+        if (koff.alloc(offsets.size() * 4) != cudaSuccess)
+            return fail(ctx, PETB200_ERR_NOMEM, "koff allocation failed");
+        PETB200_CUDA(ctx, cudaMemcpy(koff.p, offsets.data(), offsets.size() * 4, cudaMemcpyHostToDevice));
+        return PETB200_OK;
+    }
     int alloc_b() { // the packed operand: rows_b rows of Ktot elements, hi and lo
+        if (int rc = upload_offsets())
+            return rc;
         const size_t bytes = (size_t)rows_b * Ktot * (half() ? 2 : 4);
         if (whi.alloc(bytes) != cudaSuccess || wlo.alloc(bytes) != cudaSuccess || (P.f16 && fscale_buf.alloc((size_t)(rows_b + 1) * 4) != cudaSuccess))
             return fail(ctx, PETB200_ERR_NOMEM, "packed operand allocation (%zu bytes) failed", 2 * bytes);
@@ -845,9 +866,7 @@ static int tc_configure(petb200_ctx *ctx, TcCore &core, const ConvGeom &g, int o
             koff[(size_t)tap * P.BC + ci] =
                 (ci * plane_d + t * g.dil[0] * plane_h + r * g.dil[1] * plane_w + s * g.dil[2]) | (flat ? tap << 24 : 0);
     }
-    if (core.koff.alloc(koff.size() * 4) != cudaSuccess)
-        return fail(ctx, PETB200_ERR_NOMEM, "koff allocation failed");
-    PETB200_CUDA(ctx, cudaMemcpy(core.koff.p, koff.data(), koff.size() * 4, cudaMemcpyHostToDevice));
+    core.offsets.swap(koff);
     return raise_smem_limit(ctx);
 }
 
@@ -1022,13 +1041,20 @@ int tc_conv_set_weights(void *h, const float *w, cudaStream_t s) {
     auto *t = (TcConv *)h;
     TcCore &c = t->full;
     const int cpg = t->g.C / t->g.groups, T = t->g.T3[0] * t->g.T3[1] * t->g.T3[2];
+    if (c.math == kMathF16x3) {
+        PackFilters g{};
+        g.w = w, g.hi = c.whi.p, g.lo = c.wlo.p, g.unscale = (float *)c.fscale_buf.p, g.numbers = (uint16_t *)c.factor_word(), g.number = ++c.packings;
+        g.cpg = cpg, g.T = T, g.BC = c.P.BC, g.Ktot = (int)c.Ktot;
+        g.by_kc_pad.set(c.P.spc * c.P.ke), g.by_bc.set(c.P.BC);
+        const int parts = std::max(1, std::min({8, 2 * c.ctx->sm_count / t->g.F, (int)((c.Ktot + 1023) / 1024)}));
+        k_pack_conv_f16<<<dim3((unsigned)t->g.F, (unsigned)parts), 256, 0, s>>>(g);
+        c.weights_ready = true;
+        return launched(c.ctx, "k_pack_conv_f16");
+    }
     long long total = (long long)t->g.F * c.Ktot;
     int blocks = (int)std::min<long long>((total + 255) / 256, (long long)c.ctx->sm_count * 16);
-    if (c.math == kMathF16x3)
-        k_filter_factors<<<t->g.F, 256, 0, s>>>(w, (float *)c.fscale_buf.p, (long long)cpg * T, (uint16_t *)c.factor_word(), ++c.packings);
-    auto kern = c.math == kMathF16x3 ? k_pack_conv_w<kMathF16x3> : (c.math == kMathBf16x3 ? k_pack_conv_w<kMathBf16x3>
-              : (c.math == kMathTf32x1 ? k_pack_conv_w<kMathTf32x1> : k_pack_conv_w<kMathTf32x3>));
-    kern<<<blocks, 256, 0, s>>>(w, c.whi.p, c.wlo.p, t->g.F, cpg, T, c.P.BC, c.P.spc * c.P.ke, c.P.nchunks, (const float *)c.fscale_buf.p);
+    auto kern = c.math == kMathBf16x3 ? k_pack_conv_w<kMathBf16x3> : (c.math == kMathTf32x1 ? k_pack_conv_w<kMathTf32x1> : k_pack_conv_w<kMathTf32x3>);
+    kern<<<blocks, 256, 0, s>>>(w, c.whi.p, c.wlo.p, t->g.F, cpg, T, c.P.BC, c.P.spc * c.P.ke, c.P.nchunks);
     c.weights_ready = true;
     return launched(c.ctx, "k_pack_conv_w");
 }
@@ -1072,6 +1098,8 @@ int tc_conv_run(void *h, const float *x, const float *bias, const float *res, fl
         }
         if (rc == PETB200_OK && (wc->P.BN != t->full.P.BN || wc->P.BC != t->full.P.BC || wc->Ktot != t->full.Ktot || wc->P.ksplit != t->full.P.ksplit))
             rc = fail(wc->ctx, PETB200_ERR_UNSUPPORTED, "window plan diverged from the full plan");
+        if (rc == PETB200_OK)
+            rc = wc->upload_offsets();
         if (rc) {
             delete wc;
             t->windows.erase(key);
@@ -1188,9 +1216,7 @@ static int tc_configure_kmajor(petb200_ctx *ctx, TcCore &core, int bs, int m, in
     core.Ktot = (long long)P.nchunks * P.ke;
     core.xd[0] = k, core.xd[1] = m, core.xd[2] = bs;
     std::vector<int> koff(P.ke, -1); // unused in this mode; the kernel still copies one stage worth of table
-    if (core.koff.alloc(koff.size() * 4) != cudaSuccess)
-        return fail(ctx, PETB200_ERR_NOMEM, "koff allocation failed");
-    PETB200_CUDA(ctx, cudaMemcpy(core.koff.p, koff.data(), koff.size() * 4, cudaMemcpyHostToDevice));
+    core.offsets.swap(koff);
     core.y_elems = (long long)bs * m * n;
     return raise_smem_limit(ctx);
 }
@@ -1311,12 +1337,7 @@ int tc_g2bmm_create(petb200_ctx *ctx, int bs, int n, int m, int w, void **out) {
     core.smem = smem_layout(P).total + 1024;
     core.Ktot = (long long)P.nchunks * P.ke;
     core.xd[0] = m, core.xd[1] = n, core.xd[2] = bs;
-    std::vector<int> koff(P.ke, -1);
-    if (core.koff.alloc(koff.size() * 4) != cudaSuccess) {
-        delete t;
-        return fail(ctx, PETB200_ERR_NOMEM, "koff allocation failed");
-    }
-    cudaMemcpy(core.koff.p, koff.data(), koff.size() * 4, cudaMemcpyHostToDevice);
+    core.offsets.assign(P.ke, -1);
     core.grid = dim3((unsigned)std::min(P.tiles, ctx->sm_count), 1u, 1u);
     core.y_elems = (long long)bs * n * (2 * w + 1);
     core.rows_b = bs * n;
@@ -1381,12 +1402,7 @@ int tc_gbmml_create(petb200_ctx *ctx, int bs, int n, int m, int w, void **out) {
     core.Ktot = ((long long)n + P.ke - 1) / P.ke * P.ke; // the packed operand covers all keys; a tile reads its window of them
     core.xd[0] = kStageK, core.xd[1] = kTileM, core.xd[2] = 1; // (the activation map is not used: any valid extents)
     core.a_batch = kStageK * kTileM, core.a_row = kStageK;
-    std::vector<int> koff(P.spc * P.ke, -1);
-    if (core.koff.alloc(koff.size() * 4) != cudaSuccess) {
-        delete t;
-        return fail(ctx, PETB200_ERR_NOMEM, "koff allocation failed");
-    }
-    cudaMemcpy(core.koff.p, koff.data(), koff.size() * 4, cudaMemcpyHostToDevice);
+    core.offsets.assign(P.spc * P.ke, -1);
     core.y_elems = (long long)bs * n * m;
     core.rows_b = bs * m;
     int rc = raise_smem_limit(ctx);
