@@ -836,6 +836,10 @@ static int tc_configure(petb200_ctx *ctx, TcCore &core, const ConvGeom &g, int o
     if (!have)
         return fail(ctx, PETB200_ERR_UNSUPPORTED, "raw activation tile does not fit shared memory");
     P = bestP;
+    // A group's last raw box then holds channels of the next group too.  They meet zero weights, but a row's largest value, which
+    // decides how its halves are scaled, would be looked for among them.
+    if (P.f16 && g.groups > 1 && cpg % P.BC != 0)
+        return fail(ctx, PETB200_ERR_UNSUPPORTED, "halves need whole channel chunks per group, got %d channels in chunks of %d", cpg, P.BC);
     // eight consecutive K elements are channels of one filter tap: the cheap kind of gather
     P.cstride = (P.BC % 8 == 0 && env_int("PETB200_TC_TABLE", 0) == 0) ? P.RD * P.RH * P.RW : 0;
     choose_flush(core);
@@ -885,16 +889,17 @@ static bool f16_pays(const petb200_ctx *ctx, const TcCore &core) {
     const long long tile = (long long)((P.nchunks + P.ksplit - 1) / P.ksplit) * P.spc * P.BN;
     return P.a_kmajor ? turns * tile >= 300 : tile >= 1600;
 }
-// Runs `configure` for the arithmetic that the caller asks for; kMathAuto: for TF32, and again for fp16 where that pays.
+// Runs `configure` for the arithmetic that the caller asks for; kMathAuto: for TF32, and again for fp16 where that pays.  What fp16
+// cannot serve stays with TF32.
 template <typename F> static int configure_for(petb200_ctx *ctx, TcCore &core, int math, F &&configure) {
     core.math = math == kMathAuto ? kMathTf32x3 : math;
     int rc = configure();
-    if (rc || math != kMathAuto || !f16_pays(ctx, core))
-        return rc;
-    core.math = kMathF16x3;
-    core.P = IgemmParams{};
-    rc = configure();
-    if (rc == PETB200_ERR_UNSUPPORTED) {
+    if (rc == PETB200_OK && math == kMathAuto && f16_pays(ctx, core)) {
+        core.math = kMathF16x3;
+        core.P = IgemmParams{};
+        rc = configure();
+    }
+    if (rc == PETB200_ERR_UNSUPPORTED && core.math == kMathF16x3) {
         core.math = kMathTf32x3;
         core.P = IgemmParams{};
         rc = configure();

@@ -218,3 +218,31 @@ def test_contexts_of_two_threads(ctx):
         t.join()
     for i in range(2):
         assert all(torch.equal(p, q) for p, q in zip(got[i], want))
+
+
+# What a product of halves, or three of TF32, may be off by: what the products leave out (2^-21 and 3 * 2^-20 of each), and the sum that the
+# tensor core truncates after each of K / 8 or fewer MMAs, twice 2^-23 of it at most for each of the two accumulators.
+def _within_bound(got, x2, w2):
+    """x2 [rows, K], w2 [K, cols], float64, the values of a row or filter of one magnitude."""
+    bound = 2.0 ** -22 * ((12 + x2.shape[1] / 4) * (x2.abs() @ w2.abs()) + x2.abs().amax(1, keepdim=True) * w2.abs().sum(0, keepdim=True))
+    return bool(((got.double() - x2 @ w2).abs() <= bound).all())
+
+
+# A group's rows are scaled by the group's own values: the last channels that are fetched with 48 or 40 of a group are its neighbour's
+@pytest.mark.parametrize("cpg,fg,groups,h,w,k", [(48, 64, 2, 12, 12, 3), (40, 48, 3, 10, 16, 3), (36, 33, 2, 9, 11, 3), (36, 33, 2, 90, 110, 1), (64, 64, 2, 12, 12, 3), (16, 40, 4, 8, 20, 3), (96, 130, 2, 30, 64, 1)])
+@pytest.mark.parametrize("scale", [1e-13, 1e-9, 1.0, 1e9])
+def test_groups_of_different_magnitude(ctx, cpg, fg, groups, h, w, k, scale):
+    gen = torch.Generator().manual_seed(cpg + fg)
+    x, wt = torch.randn(2, groups * cpg, h, w, generator=gen), torch.randn(groups * fg, cpg, k, k, generator=gen)
+    x[:, :cpg] *= scale
+    wt[fg + 3] *= 1e-7  # a filter of the second group has a factor
+    plan = ctx.conv2d_plan(x.shape, wt.shape, k // 2, k // 2)
+    ctx.conv2d_set_weights(plan, wt.cuda())
+    got = ctx.conv2d_run(plan, x.cuda()).cpu()
+    ctx.sync_check()
+    for g in range(groups):
+        cols = torch.nn.functional.unfold(x[:, g * cpg:(g + 1) * cpg].double(), k, padding=k // 2).transpose(1, 2).reshape(-1, cpg * k * k)
+        mine = got[:, g * fg:(g + 1) * fg].permute(0, 2, 3, 1).reshape(-1, fg)
+        assert _within_bound(mine, cols, wt[g * fg:(g + 1) * fg].reshape(fg, -1).double().t())
+    # (36 channels in planes of odd width are fetched whole, in chunks that divide the group)
+    assert plan.kernel == ("tc_3xtf32_ts" if cpg in (48, 40) else "tc_3xtf32_f16_ts")
