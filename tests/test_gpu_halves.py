@@ -228,6 +228,13 @@ def _within_bound(got, x2, w2):
     return bool(((got.double() - x2 @ w2).abs() <= bound).all())
 
 
+def _some_rows(shape, channel_dim, gen):
+    """Values of which some pixels are too small and some too large for halves."""
+    x = torch.randn(shape, generator=gen).movedim(channel_dim, -1)
+    scale = torch.tensor([1.0, 1.0, 1e-9, 1e7])[torch.randint(0, 4, x.shape[:-1], generator=gen)]
+    return (x * scale.unsqueeze(-1)).movedim(-1, channel_dim).contiguous()
+
+
 # A group's rows are scaled by the group's own values: the last channels that are fetched with 48 or 40 of a group are its neighbour's
 @pytest.mark.parametrize("cpg,fg,groups,h,w,k", [(48, 64, 2, 12, 12, 3), (40, 48, 3, 10, 16, 3), (36, 33, 2, 9, 11, 3), (36, 33, 2, 90, 110, 1), (64, 64, 2, 12, 12, 3), (16, 40, 4, 8, 20, 3), (96, 130, 2, 30, 64, 1)])
 @pytest.mark.parametrize("scale", [1e-13, 1e-9, 1.0, 1e9])
@@ -246,3 +253,97 @@ def test_groups_of_different_magnitude(ctx, cpg, fg, groups, h, w, k, scale):
         assert _within_bound(mine, cols, wt[g * fg:(g + 1) * fg].reshape(fg, -1).double().t())
     # (36 channels in planes of odd width are fetched whole, in chunks that divide the group)
     assert plan.kernel == ("tc_3xtf32_ts" if cpg in (48, 40) else "tc_3xtf32_f16_ts")
+
+
+# A correction window borrows its plan's packed filters and their factors; rows out of range are scaled as in the whole result
+@pytest.mark.parametrize("n,c,h,w,f,k,win", [(1, 64, 20, 20, 64, 3, (3, 5, 0, 20)), (3, 32, 16, 24, 130, 3, (0, 2, 7, 9)), (2, 96, 11, 13, 48, 3, (4, 7, 2, 11)), (40, 64, 28, 28, 128, 3, (26, 2, 0, 28)),
+                                             (1, 512, 14, 14, 64, 3, (1, 1, 1, 1)), (2, 3, 30, 150, 33, 5, (10, 9, 100, 50))])
+def test_windows_with_factors_bit_identical(ctx, n, c, h, w, f, k, win):
+    gen = torch.Generator().manual_seed(c + f)
+    x, wt = _some_rows((n, c, h, w), 1, gen).cuda(), _weights((f, c, k, k), [1, f - 1], 0, 5)
+    plan = ctx.conv2d_plan(x.shape, wt.shape, k // 2, k // 2)
+    assert plan.kernel == "tc_3xtf32_f16_ts"
+    ctx.conv2d_set_weights(plan, wt)
+    whole, part = ctx.conv2d_run(plan, x), torch.full(plan.out_shape, 7.0, device="cuda")
+    r0, rn, c0, cn = win
+    ctx.conv2d_correct(plan, x, part, r0, rn, c0, cn)
+    ctx.sync_check()
+    inside = (slice(None), slice(None), slice(r0, r0 + rn), slice(c0, c0 + cn))
+    assert torch.equal(part[inside], whole[inside])
+    part[inside] = 7.0
+    assert bool((part == 7.0).all())
+
+
+# Neighbouring pixels of different magnitude in one row of operands would leave the bound above no meaning: here a whole image is of one
+# magnitude.  One tile per CTA, several, K split.
+@pytest.mark.parametrize("n,c,d,hw,f", [(3, 16, 4, 8, 33), (3, 64, 4, 14, 64), (6, 64, 8, 28, 64), (3, 256, 2, 4, 128)])
+def test_conv3d_second_pass(ctx, n, c, d, hw, f):
+    gen = torch.Generator().manual_seed(c + f)
+    x, wt = torch.randn(n, c, d, hw, hw, generator=gen), _weights((f, c, 3, 3, 3), [2, f - 1], 0, 6)
+    x *= torch.tensor([1.0, 1e-9, 1e7])[torch.arange(n) % 3].reshape(-1, 1, 1, 1, 1)
+    plan = ctx.conv3d_plan(x.shape, wt.shape, (1, 1, 1))
+    assert plan.kernel == "tc_3xtf32_f16_ts"
+    got = ctx.conv3d(x.cuda(), wt, (1, 1, 1)).cpu()
+    ctx.sync_check()
+    pad = torch.nn.functional.pad(x, (1,) * 6)
+    cols = pad.unfold(2, 3, 1).unfold(3, 3, 1).unfold(4, 3, 1).permute(0, 2, 3, 4, 1, 5, 6, 7).reshape(-1, c * 27)
+    rows = torch.randperm(cols.shape[0], generator=gen)[:3000]
+    assert _within_bound(got.permute(0, 2, 3, 4, 1).reshape(-1, f)[rows], cols[rows].double(), wt.cpu().reshape(f, -1).double().t())
+
+
+# The phases of a transposed convolution are a chain of launches that fill every second row and column (channels last); with rows out of
+# range each makes its second pass
+@pytest.mark.parametrize("phases", ["1", "0"])
+@pytest.mark.parametrize("n,hw,f,c,k,act", [(3, 8, 32, 24, 4, "none"), (3, 16, 128, 64, 4, "none"), (3, 9, 40, 33, 4, "relu"), (12, 32, 64, 66, 4, "none"), (3, 4, 512, 64, 4, "none")])
+def test_convtrans_second_pass(ctx, monkeypatch, phases, n, hw, f, c, k, act):
+    monkeypatch.setenv("PETB200_CONVTRANS_PHASES", phases)
+    gen = torch.Generator().manual_seed(f + c)
+    x, wt, bias = torch.randn(n, hw, hw, f, generator=gen), _weights((k, k, f, c), [0, c - 1], 3, 8), torch.randn(c, generator=gen)
+    scale = torch.tensor([1.0, 1e-9, 1e7])[torch.arange(n) % 3].reshape(-1, 1, 1, 1)
+    x *= scale
+    plan = ctx.convtrans_plan(x.shape, wt.shape, 1, 1, 2, 2, bias=True, act=act)
+    assert plan.kernel == "tc_3xtf32_f16_ts"
+    got = ctx.convtrans_run(plan, x.cuda(), wt, bias.cuda()).cpu().double()
+    ctx.sync_check()
+    w4 = wt.cpu().permute(2, 3, 0, 1).double()  # [f, c, k, k]
+    exact = lambda a, b: torch.nn.functional.conv_transpose2d(a.double().permute(0, 3, 1, 2), b, stride=2, padding=1).permute(0, 2, 3, 1)
+    want = exact(x, w4) + bias.double()
+    want = want.clamp_min(0) if act == "relu" else want
+    bound = 2.0 ** -22 * (12 + f * k) * exact(x.abs(), w4.abs()) + 2.0 ** -22 * (want.abs() + bias.abs().double())
+    bound += 2.0 ** -22 * x.abs().amax((1, 2, 3)).double().reshape(-1, 1, 1, 1) * w4.abs().sum((0, 2, 3))
+    assert bool(((got - want).abs() <= bound).all())
+
+
+# Operands that are strided views, heads of [sequence, heads, width]: the same bits as on dense copies
+@pytest.mark.parametrize("seq,heads,d", [(128, 12, 64), (77, 3, 68), (384, 8, 128)])
+def test_strided_operands_second_pass(ctx, seq, heads, d):
+    gen = torch.Generator().manual_seed(seq)
+    q, v = _some_rows((seq, heads, d), 2, gen).cuda(), _some_rows((seq, heads, d), 2, gen).cuda()
+    plan = ctx.matmul_plan((heads, seq, d), (heads, seq, d), transB=True, strides=(d, heads * d, d, heads * d, seq * seq, seq))
+    assert plan.kernel == "tc_3xtf32_f16_ts"
+    out = torch.empty(heads, seq, seq, device="cuda")
+    ctx.matmul_run(plan, q, v, out=out)
+    qh, vh = q.permute(1, 0, 2).contiguous(), v.permute(1, 0, 2).contiguous()
+    assert torch.equal(out, ctx.matmul(qh, vh, transB=True))
+    ctx.sync_check()
+    for i in range(heads):
+        assert _within_bound(out[i].cpu(), qh[i].cpu().double(), vh[i].cpu().double().t())
+
+
+# Factors are taken out before bias, residual and activation.  (The activations agree with torch's to a few units in the last place, on
+# sums that are the same: 2^-20 of the value, or of 1 where the result is the small rest of larger terms.)
+@pytest.mark.parametrize("act", ["none", "relu", "sigmoid", "tanh", "gelu"])
+@pytest.mark.parametrize("n,c,hw,f", [(1, 64, 12, 40), (30, 64, 28, 72), (20, 128, 28, 128), (1, 512, 8, 64)])
+def test_epilogue_after_factors(ctx, act, n, c, hw, f):
+    gen = torch.Generator().manual_seed(c + f)
+    x, wt = _some_rows((n, c, hw, hw), 1, gen).cuda() * 0.05, _weights((f, c, 3, 3), [0, f - 1], 0, 9)
+    bias, res = torch.randn(f, generator=gen).cuda(), torch.randn(n, f, hw, hw, generator=gen).cuda()
+    plain, plan = ctx.conv2d_plan(x.shape, wt.shape, 1, 1), ctx.conv2d_plan(x.shape, wt.shape, 1, 1, bias=True, act=act)
+    assert plain.kernel == plan.kernel == "tc_3xtf32_f16_ts"
+    for p in (plain, plan):
+        ctx.conv2d_set_weights(p, wt)
+    sums = ctx.conv2d_run(plain, x) + bias.reshape(1, -1, 1, 1) + res
+    got = ctx.conv2d_run(plan, x, bias, residual=res)
+    ctx.sync_check()
+    want = {"none": lambda t: t, "relu": torch.relu, "sigmoid": torch.sigmoid, "tanh": torch.tanh, "gelu": torch.nn.functional.gelu}[act](sums)
+    assert bool(((got - want).abs() <= 2.0 ** -20 * torch.maximum(want.abs(), torch.ones_like(want))).all())
