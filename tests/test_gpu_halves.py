@@ -8,8 +8,9 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.fixture(autouse=True)
-def halves(monkeypatch):
+def halves(ctx, monkeypatch):
     monkeypatch.setenv("PETB200_TC_MATH", "f16x3")
+    monkeypatch.setattr(ctx, "_plans", {})  # none that another test made with another arithmetic
 
 
 def _weights(shape, small, filter_dim, seed):
