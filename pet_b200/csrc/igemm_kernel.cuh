@@ -685,7 +685,7 @@ __device__ __forceinline__ void store_any(const StoreJob &J, const float *bias, 
 template <int ACT>
 __device__ __forceinline__ void activate_row(const StoreJob &J, float *stage, const float *rp, float bias, int f0) {
 #pragma unroll 1
-    for (int j = 0; j < 32; j += 8) {
+    for (int j = 0; j < 32 && f0 + j < J.Fg; j += 8) {
         float v[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i)
