@@ -111,7 +111,7 @@ struct PrepareArgs {
     FastDiv by_kc_pad, by_tiles_k, by_tiles_n;
     long long sb_batch, sb_row;
     int b_tiles, tiles_k, tiles_n;
-    int split;              // fp16: CTAs per strip of columns (a cluster) or warps per row
+    int split;              // fp16: CTAs per strip of columns (a cluster) or warps per row, a power of two
     const float *a;
     float *a_copy;
     long long a_rows;
@@ -166,61 +166,72 @@ __global__ void __launch_bounds__(256) k_prepare_mm(const PrepareArgs g) {
 
 // The same for fp16, where a packed row (a column of B) has one factor, known only when all of it has been seen (row_exponent).
 // Both kernels read B once from memory and write each packed word once, 128 bytes per warp.
-// B[b][k][n]: the CTAs of a cluster share a strip of 32 columns, each a range of 64-position units of the packed row; the units
+// B[b][k][n]: the CTAs of a cluster share a strip of W columns, each a range of 64-position units of the packed row; the units
 // stay in shared memory (as many as there is room for, more are read again) while the columns' maxima meet through the cluster.
-constexpr int kPrepUnit = 64, kPrepKeep = 8, kPrepPitch = 33;
-constexpr size_t kPrepSmem = (size_t)kPrepKeep * kPrepUnit * kPrepPitch * 4;
+// W = 8 where strips of 32 would leave SMs idle (3 x 3960 x 36: 8.0 -> 5.0 us, the packing for TF32 takes 3.1).
+constexpr int kPrepUnit = 64, kPrepKeep = 8;
+template <int W> constexpr int kPrepPitch = W + 1;
+template <int W> constexpr int kPrepRoom = W == 32 ? kPrepKeep : 24; // units
+template <int W> constexpr size_t kPrepSmem = (size_t)kPrepRoom<W> * kPrepUnit *kPrepPitch<W> * 4;
 // Unit u of the packed row: first row of B, number of rows.
 __device__ __forceinline__ void prep_unit(const PrepareArgs &g, int u, int &kk0, int &kn) {
     const int k0 = u * kPrepUnit, ch = g.by_kc_pad.div(k0), kc0 = k0 - ch * (int)g.by_kc_pad.d;
     kk0 = ch * g.BC + kc0;
     kn = min(min(g.BC - kc0, g.k - kk0), kPrepUnit);
 }
-__global__ void __launch_bounds__(256) k_prepare_f16_kn(const PrepareArgs g) {
+template <int W> __global__ void __launch_bounds__(256) k_prepare_f16_kn(const PrepareArgs g) {
     pdl_prologue();
-    extern __shared__ float keep[]; // [unit][row][kPrepPitch]
-    __shared__ float tops[8][32], column_top[32], factor[32];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int kPitch = kPrepPitch<W>, kRoom = kPrepRoom<W>, kRows = 32 / W /*of a load*/, kLoads = kPrepUnit / (8 * kRows);
+    extern __shared__ float keep[]; // [unit][row][kPitch]
+    __shared__ float tops[8][32], column_top[W], factor[W];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, col = lane & (W - 1), row0 = warp * kRows + lane / W;
     if ((int)blockIdx.x >= g.b_tiles) {
         copy_a_rows(g, (int)blockIdx.x - g.b_tiles, (int)gridDim.x - g.b_tiles);
         return; // (whole clusters: b_tiles is a multiple of the cluster)
     }
-    const int rank = (int)blockIdx.x % g.split, strip = (int)blockIdx.x / g.split, bb = g.by_tiles_n.div(strip), n0 = (strip - bb * g.tiles_n) * 32;
+    const int rank = (int)blockIdx.x % g.split, strip = (int)blockIdx.x / g.split, bb = g.by_tiles_n.div(strip), n0 = (strip - bb * g.tiles_n) * W;
     const int u0 = rank * g.tiles_k / g.split, u1 = (rank + 1) * g.tiles_k / g.split;
-    const float *src = g.b + bb * g.sb_batch + n0 + lane;
-    const bool col_ok = n0 + lane < g.n;
+    const float *src = g.b + bb * g.sb_batch + n0 + col;
+    const bool col_ok = n0 + col < g.n;
     float top = 0.f;
     auto load = [&](int u, float *dst) { // 64 rows of the strip to shared memory
         int kk0, kn;
         prep_unit(g, u, kk0, kn);
-        float v[8];
+        float v[kLoads];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-            v[i] = col_ok && warp + 8 * i < kn ? __ldg(src + (kk0 + warp + 8 * i) * g.sb_row) : 0.f;
+        for (int i = 0; i < kLoads; ++i) {
+            const int r = row0 + 8 * kRows * i;
+            v[i] = col_ok && r < kn ? __ldg(src + (kk0 + r) * g.sb_row) : 0.f;
+        }
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < kLoads; ++i) {
             top = fmaxf(top, fabsf(v[i]));
-            dst[(warp + 8 * i) * kPrepPitch + lane] = v[i];
+            dst[(row0 + 8 * kRows * i) * kPitch + col] = v[i];
         }
     };
-#pragma unroll 2
+#pragma unroll (W == 32 ? 2 : 4)
     for (int u = u0; u < u1; ++u) // units beyond the room take turns in the last place: their maxima count, they are read again
-        load(u, keep + min(u - u0, kPrepKeep - 1) * kPrepUnit * kPrepPitch);
+        load(u, keep + min(u - u0, kRoom - 1) * kPrepUnit * kPitch);
+#pragma unroll
+    for (int o = W; o < 32; o *= 2)
+        top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
     tops[warp][lane] = top;
     __syncthreads();
     if (warp == 0) {
 #pragma unroll
         for (int i = 1; i < 8; ++i)
             top = fmaxf(top, tops[i][lane]);
-        column_top[lane] = top;
+        if (lane < W)
+            column_top[lane] = top;
     }
     if (g.split > 1) {
         ptx::cluster_sync_all();
         if (warp == 0)
             for (int r = 0; r < g.split; ++r)
-                top = fmaxf(top, ptx::ld_dsmem_f32(ptx::map_to_cta(ptx::smem_u32(column_top + lane), (uint32_t)r)));
+                top = fmaxf(top, ptx::ld_dsmem_f32(ptx::map_to_cta(ptx::smem_u32(column_top + col), (uint32_t)r)));
+        ptx::cluster_arrive(); // (waited for at the end: nobody leaves while its maxima are being read)
     }
-    if (warp == 0) {
+    if (warp == 0 && lane < W) {
         const uint32_t e = row_exponent(top);
         factor[lane] = kFilterUnit / filter_unscale(e);
         if (rank == 0 && col_ok) {
@@ -231,28 +242,29 @@ __global__ void __launch_bounds__(256) k_prepare_f16_kn(const PrepareArgs g) {
                 g.numbers[1] = g.number;
         }
     }
-    if (g.split > 1)
-        ptx::cluster_sync_all(); // (nobody leaves while its maxima are being read)
-    else
-        __syncthreads();
+    __syncthreads();
+#pragma unroll 2
     for (int u = u0; u < u1; ++u) {
-        const int slot = min(u - u0, kPrepKeep - 1);
-        const float *tile = keep + slot * kPrepUnit * kPrepPitch;
-        if (u1 - u0 > kPrepKeep && u - u0 >= kPrepKeep - 1) {
+        const int slot = min(u - u0, kRoom - 1);
+        const float *tile = keep + slot * kPrepUnit * kPitch;
+        if (u1 - u0 > kRoom && u - u0 >= kRoom - 1) {
             __syncthreads();
-            load(u, keep + slot * kPrepUnit * kPrepPitch);
+            load(u, keep + slot * kPrepUnit * kPitch);
             __syncthreads();
         }
 #pragma unroll
-        for (int c = warp; c < 32; c += 8)
+        for (int c = warp; c < W; c += 8)
             if (n0 + c < g.n)
-                store_halves(g.hi, g.lo, (((long long)bb * g.n + n0 + c) * g.Kpad + u * kPrepUnit) / 2 + lane, tile[2 * lane * kPrepPitch + c],
-                          tile[(2 * lane + 1) * kPrepPitch + c], factor[c]);
+                store_halves(g.hi, g.lo, (((long long)bb * g.n + n0 + c) * g.Kpad + u * kPrepUnit) / 2 + lane, tile[2 * lane * kPitch + c],
+                             tile[(2 * lane + 1) * kPitch + c], factor[c]);
     }
+    if (g.split > 1)
+        ptx::cluster_wait();
 }
-// B[b][n][k]: a packed row is a row of B; g.split warps share it (1, or the block's 8 where there are few rows), reading it a second
-// time out of the caches.
-__global__ void __launch_bounds__(256) k_prepare_f16_nk(const PrepareArgs g) {
+// B[b][n][k]: a packed row is a row of B; g.split warps share it.  A warp keeps its first KEEP units in registers, all loads in
+// flight at once; more are read a second time.  (All of them twice, a warp to a row where there were many rows: 29 x 140 rows of 3476 66 us,
+// now 27, 4096 of 4096 97, now 40, 4 x 1001 of 770 12.4, now 7.5; the packing for TF32 44, 50, 7.6.)
+template <int KEEP> __global__ void __launch_bounds__(256) k_prepare_f16_nk(const PrepareArgs g) {
     pdl_prologue();
     __shared__ float tops[8];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -260,30 +272,38 @@ __global__ void __launch_bounds__(256) k_prepare_f16_nk(const PrepareArgs g) {
         copy_a_rows(g, (int)blockIdx.x - g.b_tiles, (int)gridDim.x - g.b_tiles);
         return;
     }
-    const long long row = g.split > 1 ? blockIdx.x : (long long)blockIdx.x * 8 + warp;
+    const int step = g.split, u0 = warp & (step - 1); // (a power of two)
+    const long long row = (long long)blockIdx.x * (8 / step) + warp / step;
     const bool row_ok = row < (long long)g.bs * g.n;
-    const int step = g.split, u0 = g.split > 1 ? warp : 0, u1 = row_ok ? g.tiles_k : 0;
-    const int bb = (int)(row / g.n), nn = (int)(row - (long long)bb * g.n);
+    const int u1 = row_ok ? g.tiles_k : 0;
+    const int bb = row_ok ? (int)(row / g.n) : 0, nn = row_ok ? (int)(row - (long long)bb * g.n) : 0;
     const float *src = g.b + bb * g.sb_batch + nn * g.sb_row;
-    float top = 0.f;
-#pragma unroll 4
-    for (int u = u0; u < u1; u += step) {
+    auto take = [&](int u) {
         int kk0, kn;
         prep_unit(g, u, kk0, kn);
-        if (2 * lane < kn)
-            top = fmaxf(top, fabsf(__ldg(src + kk0 + 2 * lane)));
-        if (2 * lane + 1 < kn)
-            top = fmaxf(top, fabsf(__ldg(src + kk0 + 2 * lane + 1)));
+        return make_float2(2 * lane < kn ? __ldg(src + kk0 + 2 * lane) : 0.f, 2 * lane + 1 < kn ? __ldg(src + kk0 + 2 * lane + 1) : 0.f);
+    };
+    float2 v[KEEP];
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i)
+        v[i] = u0 + i * step < u1 ? take(u0 + i * step) : make_float2(0.f, 0.f);
+    float top = 0.f;
+#pragma unroll 4
+    for (int u = u0 + KEEP * step; u < u1; u += step) {
+        const float2 x = take(u);
+        top = ptx::max3_abs(top, x.x, x.y);
     }
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i)
+        top = ptx::max3_abs(top, v[i].x, v[i].y);
     for (int o = 16; o; o >>= 1)
         top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-    if (g.split > 1) {
+    if (step > 1) {
         if (lane == 0)
             tops[warp] = top;
         __syncthreads();
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-            top = fmaxf(top, tops[i]);
+        for (int i = 0; i < step; ++i)
+            top = fmaxf(top, tops[(warp & ~(step - 1)) + i]);
     }
     const uint32_t e = row_exponent(top);
     const float factor = kFilterUnit / filter_unscale(e);
@@ -294,13 +314,14 @@ __global__ void __launch_bounds__(256) k_prepare_f16_nk(const PrepareArgs g) {
         if (filter_out_of_range(e))
             g.numbers[1] = g.number;
     }
+    auto put = [&](int u, float2 x) { store_halves(g.hi, g.lo, (row * g.Kpad + u * kPrepUnit) / 2 + lane, x.x, x.y, factor); };
+#pragma unroll
+    for (int i = 0; i < KEEP; ++i)
+        if (u0 + i * step < u1)
+            put(u0 + i * step, v[i]);
 #pragma unroll 4
-    for (int u = u0; u < u1; u += step) {
-        int kk0, kn;
-        prep_unit(g, u, kk0, kn);
-        store_halves(g.hi, g.lo, (row * g.Kpad + u * kPrepUnit) / 2 + lane, 2 * lane < kn ? __ldg(src + kk0 + 2 * lane) : 0.f,
-                  2 * lane + 1 < kn ? __ldg(src + kk0 + 2 * lane + 1) : 0.f, factor);
-    }
+    for (int u = u0 + KEEP * step; u < u1; u += step)
+        put(u, take(u));
 }
 
 // -------------------------------------------------------------------------------------------------------------
@@ -649,7 +670,9 @@ static int raise_smem_limit(petb200_ctx *ctx) {
     }
     raise(igemm_band(1, kNarrow));
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_prepare_f16_kn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPrepSmem);
+        e = cudaFuncSetAttribute(k_prepare_f16_kn<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPrepSmem<32>);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_prepare_f16_kn<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPrepSmem<8>);
     if (e != cudaSuccess)
         return fail(ctx, PETB200_ERR_CUDA, "cudaFuncSetAttribute(%d bytes) failed: %s", lim, cudaGetErrorString(e));
     ctx->tc_attr_set = true;
@@ -1444,15 +1467,17 @@ int tc_matmul_prepare(void *h, const float *b, const float *a, float *a_copy, cu
     if (f16)
         g.unscale = (float *)c.fscale_buf.p, g.numbers = (uint16_t *)c.factor_word(), g.number = b ? ++c.packings : (uint16_t)0;
     g.BC = c.P.BC, g.sb_batch = t->st[2], g.sb_row = t->st[3];
-    g.tiles_k = g.Kpad / (f16 ? kPrepUnit : 32), g.tiles_n = (t->n + 31) / 32; // (Kpad is a multiple of the stage's K)
+    g.tiles_k = g.Kpad / (f16 ? kPrepUnit : 32); // (Kpad is a multiple of the stage's K)
+    const int width = f16 && (t->n + 31) / 32 * (long long)t->bs * std::min(8, g.tiles_k) < 2ll * c.ctx->sm_count ? 8 : 32; // of a strip of columns
+    g.tiles_n = (t->n + width - 1) / width;
     g.by_kc_pad.set(c.P.spc * c.P.ke), g.by_tiles_k.set(g.tiles_k), g.by_tiles_n.set(g.tiles_n);
     g.split = 1;
     const long long strips = (long long)g.tiles_n * t->bs, rows = (long long)t->n * t->bs;
     long long tiles = (long long)g.tiles_k * strips;
-    if (f16 && t->transB) {
-        if (rows < c.ctx->sm_count * 16ll && g.tiles_k >= 8)
-            g.split = 8;
-        tiles = g.split > 1 ? rows : (rows + 7) / 8;
+    if (f16 && t->transB) { // a row's units stay in registers, and there are sixteen warps for every SM
+        while (g.split < 8 && 2 * g.split <= g.tiles_k && (g.tiles_k > g.split * kPrepKeep || rows * g.split < 16ll * c.ctx->sm_count))
+            g.split *= 2;
+        tiles = (rows * g.split + 7) / 8;
     } else if (f16) { // a strip's units stay in shared memory, and there are two CTAs for every SM
         while (g.split < 8 && 2 * g.split <= g.tiles_k && (g.tiles_k > g.split * kPrepKeep || strips * g.split < 2ll * c.ctx->sm_count))
             g.split *= 2;
@@ -1469,7 +1494,8 @@ int tc_matmul_prepare(void *h, const float *b, const float *a, float *a_copy, cu
         return PETB200_OK;
     if (f16 && !t->transB) {
         a_blocks = (a_blocks + g.split - 1) / g.split * g.split; // whole clusters
-        const size_t smem = (size_t)std::min(kPrepKeep, (g.tiles_k + g.split - 1) / g.split) * kPrepUnit * kPrepPitch * 4;
+        const int units = (g.tiles_k + g.split - 1) / g.split;
+        const size_t smem = (size_t)(width == 32 ? std::min(kPrepRoom<32>, units) * kPrepPitch<32> : std::min(kPrepRoom<8>, units) * kPrepPitch<8>)*kPrepUnit * 4;
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)(tiles + a_blocks)), cfg.blockDim = dim3(256), cfg.dynamicSmemBytes = smem, cfg.stream = s;
         cudaLaunchAttribute attr[2] = {};
@@ -1478,14 +1504,14 @@ int tc_matmul_prepare(void *h, const float *b, const float *a, float *a_copy, cu
         attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
         attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.attrs = attr, cfg.numAttrs = pdl_enabled() ? 2 : 1;
-        (void)cudaLaunchKernelEx(&cfg, k_prepare_f16_kn, g); // (errors surface through launched())
+        (void)cudaLaunchKernelEx(&cfg, width == 32 ? k_prepare_f16_kn<32> : k_prepare_f16_kn<8>, g); // (errors surface through launched())
     } else {
         const dim3 grid((unsigned)(tiles + a_blocks));
         auto pick = [&](auto math) {
             constexpr int MATH = decltype(math)::value;
             return t->transB ? k_prepare_mm<MATH, true> : k_prepare_mm<MATH, false>;
         };
-        launch_pdl(f16 ? k_prepare_f16_nk : (c.math == kMathBf16x3 ? pick(std::integral_constant<int, kMathBf16x3>())
+        launch_pdl(f16 ? (g.tiles_k <= g.split ? k_prepare_f16_nk<1> : k_prepare_f16_nk<kPrepKeep>) : (c.math == kMathBf16x3 ? pick(std::integral_constant<int, kMathBf16x3>())
                      : (c.math == kMathTf32x1 ? pick(std::integral_constant<int, kMathTf32x1>()) : pick(std::integral_constant<int, kMathTf32x3>()))),
                    grid, 256, 0, s, g);
     }

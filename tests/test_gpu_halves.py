@@ -348,3 +348,20 @@ def test_epilogue_after_factors(ctx, act, n, c, hw, f):
     ctx.sync_check()
     want = {"none": lambda t: t, "relu": torch.relu, "sigmoid": torch.sigmoid, "tanh": torch.tanh, "gelu": torch.nn.functional.gelu}[act](sums)
     assert bool(((got - want).abs() <= 2.0 ** -20 * torch.maximum(want.abs(), torch.ones_like(want))).all())
+
+
+# Packing B: columns in strips of 32 or of 8 (few columns), rows of B by one warp or several; more units of K than have room in shared memory
+# or registers; one unit, remainders of a unit
+@pytest.mark.parametrize("b,n,k", [(1, 40, 20000), (1, 1300, 5000), (3, 9, 200), (2, 33, 64), (5, 8, 1000), (1, 1, 4100), (2, 2000, 70), (1, 600, 12300)])
+@pytest.mark.parametrize("trans_b", [False, True])
+def test_packing_of_halves(ctx, b, n, k, trans_b):
+    gen = torch.Generator().manual_seed(n + k)
+    a, w = torch.randn(b, 24, k, generator=gen), torch.randn(b, n, k, generator=gen)
+    w *= torch.tensor([1.0, 1.0, 1e-9, 1e9])[torch.randint(0, 4, (b, n, 1), generator=gen)]
+    wd = (w if trans_b else w.transpose(1, 2).contiguous()).cuda()
+    plan = ctx.matmul_plan(a.shape, wd.shape, False, trans_b)
+    assert plan.kernel == "tc_3xtf32_f16_ts"
+    got = ctx.matmul_run(plan, a.cuda(), wd).cpu()
+    ctx.sync_check()
+    for i in range(b):
+        assert _within_bound(got[i], a[i].double(), w[i].double().t())
