@@ -905,22 +905,34 @@ static int tc_configure(petb200_ctx *ctx, TcCore &core, const ConvGeom &g, int o
 //   channels 1.01), 0.95 at 1800, 0.88 at 2300, 0.65 to 0.8 from 4000 on (512 channels dilated: 74 -> 48 us);
 //   row-major products, times the tiles that a CTA takes in turn: 1.04 to 1.2 below 256, 0.8 to 1.1 at 256, 0.97 at 400 to 1000,
 //   0.9 at 2000, 0.7 at 8000 (4096 x 4096 x 512: 70 -> 50 us).
-static bool f16_pays(const petb200_ctx *ctx, const TcCore &core) {
-    const IgemmParams &P = core.P;
-    const long long ctas = (long long)core.grid.x * core.grid.y * core.grid.z;
-    const long long turns = P.pp ? (P.tiles + ctas - 1) / ctas : (ctas + ctx->sm_count - 1) / ctx->sm_count;
-    const long long tile = (long long)((P.nchunks + P.ksplit - 1) / P.ksplit) * P.spc * P.BN;
-    return P.a_kmajor ? turns * tile >= 300 : tile >= 1600;
+//   A stage of halves lasts about 1.6 times one of TF32, so none of this holds where K is mostly padding: 7 channels of 1x1 to a
+// chunk are one stage either way (46 us against 74), 72 values three stages or two (480 channels in chunks of 8, 36 us against 43).
+// And with one stage to a chunk a transform set waits for a raw tile of its own every time (144 channels in chunks of 4, 143 us
+// against 166).
+//   The B of a batched product is packed in every call as a rule (a weight has no batch), which for B[b][k][n] takes 1 to 4 us more
+// than for TF32: 37 x 423 x 608 x 76 (2432) 19.5 us against 21.5, 2 x 82 x 556 x 3052 (1152) 19 against 25; 4 x 500 x 770 x 1001 (3200)
+// 34.1 against 31.5.  `tf32`: the plan's parameters for TF32.
+static bool f16_pays(const petb200_ctx *ctx, const IgemmParams &tf32, const dim3 &grid, int batch) {
+    const long long ctas = (long long)grid.x * grid.y * grid.z;
+    const long long turns = tf32.pp ? (tf32.tiles + ctas - 1) / ctas : (ctas + ctx->sm_count - 1) / ctx->sm_count;
+    const long long tile = (long long)((tf32.nchunks + tf32.ksplit - 1) / tf32.ksplit) * tf32.spc * tf32.BN;
+    return tf32.a_kmajor ? turns * tile >= (batch > 1 ? 3000 : 300) : tile >= 1600;
+}
+static bool f16_fits(const IgemmParams &tf32, const IgemmParams &f16) {
+    return (tf32.a_kmajor || f16.spc > 1) && 5ll * f16.nchunks * f16.spc <= 3ll * tf32.nchunks * tf32.spc;
 }
 // Runs `configure` for the arithmetic that the caller asks for; kMathAuto: for TF32, and again for fp16 where that pays.  What fp16
 // cannot serve stays with TF32.
-template <typename F> static int configure_for(petb200_ctx *ctx, TcCore &core, int math, F &&configure) {
+template <typename F> static int configure_for(petb200_ctx *ctx, TcCore &core, int math, F &&configure, int batch = 1) {
     core.math = math == kMathAuto ? kMathTf32x3 : math;
     int rc = configure();
-    if (rc == PETB200_OK && math == kMathAuto && f16_pays(ctx, core)) {
+    if (rc == PETB200_OK && math == kMathAuto && f16_pays(ctx, core.P, core.grid, batch)) {
+        const IgemmParams tf32 = core.P;
         core.math = kMathF16x3;
         core.P = IgemmParams{};
         rc = configure();
+        if (rc == PETB200_OK && !f16_fits(tf32, core.P))
+            rc = PETB200_ERR_UNSUPPORTED;
     }
     if (rc == PETB200_ERR_UNSUPPORTED && core.math == kMathF16x3) {
         core.math = kMathTf32x3;
@@ -1266,11 +1278,11 @@ int tc_matmul_create(petb200_ctx *ctx, int bs, int m, int n, int k, int transA, 
         t->st[i] = strides ? strides[i] : dense[i];
     int rc;
     if (!transA && k % 4 == 0 && t->st[0] % 4 == 0 && t->st[1] % 4 == 0) {
-        rc = configure_for(ctx, t->core, passes, [&]() { return tc_configure_kmajor(ctx, t->core, bs, m, n, k, has_bias, act, t->st); });
+        rc = configure_for(ctx, t->core, passes, [&]() { return tc_configure_kmajor(ctx, t->core, bs, m, n, k, has_bias, act, t->st); }, bs);
     } else if (!transA && !strides) { // rows of A off the 16-byte grid: the same on a copy with a pitch of whole 16-byte pieces
         t->a_rows = (long long)bs * m, t->a_w = k, t->a_pitch = (k + 3) / 4 * 4;
         const long long st[6] = {(long long)m * t->a_pitch, t->a_pitch, t->st[2], t->st[3], t->st[4], t->st[5]};
-        rc = configure_for(ctx, t->core, passes, [&]() { return tc_configure_kmajor(ctx, t->core, bs, m, n, t->a_pitch, has_bias, act, st); });
+        rc = configure_for(ctx, t->core, passes, [&]() { return tc_configure_kmajor(ctx, t->core, bs, m, n, t->a_pitch, has_bias, act, st); }, bs);
     } else if (strides) {
         delete t;
         return fail(ctx, PETB200_ERR_UNSUPPORTED, "strided matmul operands need row-major A with k and the A strides multiples of 4");

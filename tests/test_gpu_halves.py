@@ -365,3 +365,14 @@ def test_packing_of_halves(ctx, b, n, k, trans_b):
     ctx.sync_check()
     for i in range(b):
         assert _within_bound(got[i], a[i].double(), w[i].double().t())
+
+
+# Left to itself a plan takes halves only where their stages are well filled and there is work enough: chunks of 1, 4 and 8 channels (planes
+# of odd width), K of 89; batched products of few stages, whose B is packed in every call
+@pytest.mark.parametrize("x,w,takes", [((2, 119, 66, 66), (23, 119, 1, 1), False), ((9, 144, 75, 75), (33, 144, 3, 3), False), ((3, 480, 43, 43), (64, 480, 3, 3), False),
+                                       ((1, 512, 64, 64), (512, 512, 3, 3), True), ((18, 120, 1088), (18, 1088, 232), False), ((1, 2000, 89), (1, 89, 2000), False),
+                                        ((1, 384, 768), (1, 768, 3072), True), ((4, 1000, 1024), (4, 1024, 1000), True)])
+def test_which_plans_take_halves(ctx, monkeypatch, x, w, takes):
+    monkeypatch.delenv("PETB200_TC_MATH")
+    plan = ctx.matmul_plan(x, w) if len(x) == 3 else ctx.conv2d_plan(x, w, w[2] // 2, w[2] // 2)
+    assert plan.kernel == ("tc_3xtf32_f16_ts" if takes else "tc_3xtf32_ts")
