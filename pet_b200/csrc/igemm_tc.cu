@@ -572,17 +572,22 @@ static int cluster_slots(petb200_ctx *ctx, int ks) {
 // 128-filter tile in two the dearest (12500).  Several unsplit tiles in turn hide start-up and epilogue (persistent tiles).
 // Against the fastest of all pairs on 57 shapes (these products, ResNet layers at batch 1 to 16): within 2 % on 54; the others lose
 // 4, 11 and 14 % (64 x 1000 x 256, a 200-channel 3x3 at 3 x 20 x 20, 16 x 3072 x 768).  The constants before lost up to 31 % on 12 of them.
-static double est_cycles(petb200_ctx *ctx, long long base_ctas, int nchunks, int spc, int BN, int math, int ks) {
-    const int w = BN <= 32 ? 0 : (BN <= 64 ? 1 : 2);
+//   A convolution whose stages each need a raw tile of their own takes 1000 a stage whatever its width (328 channels of 1x1 in chunks
+// of 8 to 511 filters: BN 64 26.4 us, BN 128 with K split in two 21.0). A long activation adds 85 a filter in persistent tiles, which
+// four warps store, 42 elsewhere, where eight do (768 x 89 x 873, three times, with GELU: 20.3 us in tiles of 64, 17.9 in 128).
+static double est_cycles(petb200_ctx *ctx, long long base_ctas, const IgemmParams &P, int math, int ks) {
+    const int BN = P.BN, w = BN <= 32 ? 0 : (BN <= 64 ? 1 : 2);
     static const double tf32[3] = {570, 655, 890}, halves[3] = {910, 910, 1045}, exchange[3] = {2300, 2500, 8000};
-    const double stage = math == kMathTf32x1 ? 520.0 : (math == kMathTf32x3 ? tf32[w] : halves[w]), start = 6300.0;
-    const double stages = (double)((nchunks + ks - 1) / ks) * spc;
+    const double mma = math == kMathTf32x1 ? 520.0 : (math == kMathTf32x3 ? tf32[w] : halves[w]), start = 6300.0;
+    const double gather = !P.a_kmajor && P.spc == 1 ? 1000.0 : 0.0;
+    const double stages = (double)((P.nchunks + ks - 1) / ks) * P.spc, stage = std::max(mma, gather);
     const long long slots = cluster_slots(ctx, ks);
     if (slots <= 0)
         return 1e30; // this cluster size cannot be launched here
-    const double waves = (double)((base_ctas + slots - 1) / slots), epilogue = 34.0 * BN;
+    const bool long_act = P.act > PETB200_ACT_RELU;
+    const double waves = (double)((base_ctas + slots - 1) / slots), epilogue = (34.0 + (!long_act ? 0.0 : (waves > 1 ? 85.0 : 42.0))) * BN;
     if (ks > 1)
-        return waves * (start + stages * stage + exchange[w] + 70.0 * BN / ks);
+        return waves * (start + stages * stage + exchange[w] + (70.0 + (long_act ? 42.0 : 0.0)) * BN / ks);
     return start + waves * std::max(stages * stage, epilogue) + (waves - 1) * 1200.0 + epilogue;
 }
 // Split K over 1, 2, 4, 8 or 16 CTAs (a cluster; 16 is beyond the portable cluster size and allowed per function): the
@@ -590,17 +595,17 @@ static double est_cycles(petb200_ctx *ctx, long long base_ctas, int nchunks, int
 static int choose_ksplit(petb200_ctx *ctx, long long base_ctas, const IgemmParams &P, int math, int want, double *cycles) {
     auto ok = [&](int ks) { return ks == 1 || (ks <= P.nchunks && P.BN % ks == 0); };
     int best = 1;
-    double best_c = est_cycles(ctx, base_ctas, P.nchunks, P.spc, P.BN, math, 1);
+    double best_c = est_cycles(ctx, base_ctas, P, math, 1);
     static const int ks_cap = std::min(16, std::max(1, env_int_early("PETB200_TC_KSPLIT_MAX", 16)));
     if (want > 0) {
         for (best = 16; best > 1 && !(best <= want && ok(best) && cluster_slots(ctx, best) > 0); best /= 2) {
         }
-        best_c = est_cycles(ctx, base_ctas, P.nchunks, P.spc, P.BN, math, best);
+        best_c = est_cycles(ctx, base_ctas, P, math, best);
     } else {
         for (int ks = 2; ks <= ks_cap; ks *= 2) {
             if (!ok(ks))
                 continue;
-            const double c = est_cycles(ctx, base_ctas, P.nchunks, P.spc, P.BN, math, ks);
+            const double c = est_cycles(ctx, base_ctas, P, math, ks);
             if (c < best_c * 0.97) // a deeper split has to pay for itself
                 best = ks, best_c = c;
         }
@@ -629,8 +634,8 @@ static void choose_flush(TcCore &core) {
                 core.math == kMathTf32x1 ? "1xtf32" : (core.math == kMathBf16x3 ? "bf16x3" : (core.math == kMathF16x3 ? "f16x3" : "3xtf32")));
 }
 
-// Persistent mode (see IgemmParams::pp) where some SM would otherwise run several CTAs in sequence: the start-up of a CTA (about
-// 3000 cycles to its first MMA) and its epilogue (2000 to 4000) hide behind the MMAs of its neighbour tiles.  Not with a K
+// Persistent mode (see IgemmParams::pp) where some SM would otherwise run several CTAs in sequence: the start-up of a CTA (see
+// est_cycles) and its epilogue hide behind the MMAs of its neighbour tiles.  Not with a K
 // split (a CTA's tile is then a cluster's).  Sets the grid.
 static void choose_grid(petb200_ctx *ctx, TcCore &core, int mtiles, int ntiles, int gz, size_t budget) {
     IgemmParams &P = core.P;
@@ -847,7 +852,7 @@ static int tc_configure(petb200_ctx *ctx, TcCore &core, const ConvGeom &g, int o
                 P.ksplit = 1;
                 if (!fit(bn))
                     continue;
-                cyc = est_cycles(ctx, base_ctas, P.nchunks, P.spc, bn, core.math, 1);
+                cyc = est_cycles(ctx, base_ctas, P, core.math, 1);
             }
         }
         if (!have || cyc < best_cycles * 0.97) { // prefer the wider tile unless the narrower one clearly wins
