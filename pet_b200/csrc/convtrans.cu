@@ -210,6 +210,8 @@ int make_convtrans_plan(petb200_ctx *ctx, const int *a /*n,c,h,w,f,r,s,ph,pw,sh,
                     ok = false;
                 extra += bytes + ps->wsub.bytes;
             }
+        // The one with the most taps first: launched last, it ran on alone (9 x 18 x 18 x 84 -> 176, 5 x 5 stride 2, 54 us).
+        std::stable_sort(pl->phases.begin(), pl->phases.end(), [](const Phase *p, const Phase *q) { return p->Ta * p->Tb > q->Ta * q->Tb; });
         if (ok && pl->xn.alloc((size_t)n * f * h * w * 4) != cudaSuccess)
             ok = false;
         if (!ok) { // keep the zero-insertion path
