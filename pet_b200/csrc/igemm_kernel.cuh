@@ -662,7 +662,7 @@ __device__ __forceinline__ void store_rows(const StoreJob &J, const float *bias,
             J.y[off + f] = v;
     }
 }
-template <bool RES>
+template <bool RES, int AHEAD /*values of the residual in flight*/>
 __device__ __forceinline__ void store_any(const StoreJob &J, const float *bias, const float *r, int f0) {
     const int nf = J.valid ? J.Fg - f0 : 0; // filters of this thread's row
     const bool relu = J.act == PETB200_ACT_RELU;
@@ -670,13 +670,13 @@ __device__ __forceinline__ void store_any(const StoreJob &J, const float *bias, 
     float *dst = J.y + J.y_off + (long long)f0 * J.ys_f;
     const float *rs = RES ? J.res + J.y_off + (long long)f0 * J.ys_f : nullptr;
 #pragma unroll
-    for (int j = 0; j < 32; j += 8) {
-        float q[8]; // eight loads in flight (one at a time: 46 x 116 x 19 x 19 to 299 filters 108 us, now 59)
+    for (int j = 0; j < 32; j += AHEAD) {
+        float q[AHEAD];
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < AHEAD; ++i)
             q[i] = RES && j + i < nf ? __ldg(rs + (long long)(j + i) * J.ys_f) : 0.f;
 #pragma unroll
-        for (int i = 0; i < 8; ++i, dst += J.ys_f) {
+        for (int i = 0; i < AHEAD; ++i, dst += J.ys_f) {
             float v = r[j + i] + __shfl_sync(0xffffffffu, bv, j + i);
             if (RES)
                 v += q[i];
@@ -728,7 +728,9 @@ __device__ __forceinline__ void activate_block(const StoreJob &J, float *r, floa
 }
 // LONG: with one of the long activations (RES is then false, activate_block adds a residual).  Its own instances: beside the others'
 // code it cost ResNet-18 at batch 64 5 %, whose layers have none of it.
-template <int MODE, bool RES, bool LONG>
+// AHEAD: 8 where the thread keeps a row of 128 sums (left to the compiler the loads were waited for one by one there: 46 x 116 x 19 x 19 to
+// 299 filters 108 us, now 59); elsewhere the compiler moves them up itself (eight: 2 x 16 x 63 x 63 to 142 filters 13.9 -> 15.9, 32: 16.5).
+template <int MODE, bool RES, bool LONG, int AHEAD>
 __device__ __forceinline__ void store_block(const StoreJob &J, float *r /*32 sums*/, float *stage, int f0) {
     const int lane = J.lane;
     __syncwarp(); // the previous block has been read
@@ -736,7 +738,7 @@ __device__ __forceinline__ void store_block(const StoreJob &J, float *r /*32 sum
         activate_block(J, r, stage, f0);
         StoreJob R = J; // bias and residual have been added
         R.bias = R.res = nullptr, R.act = PETB200_ACT_NONE;
-        store_block<MODE, false, false>(R, r, stage, f0);
+        store_block<MODE, false, false, AHEAD>(R, r, stage, f0);
         return;
     }
     const float *bias = J.bias;
@@ -772,7 +774,7 @@ __device__ __forceinline__ void store_block(const StoreJob &J, float *r /*32 sum
         __syncwarp();
         store_rows<RES>(J, bias, stage, f0);
     } else {
-        store_any<RES>(J, bias, r, f0);
+        store_any<RES, AHEAD>(J, bias, r, f0);
     }
 }
 // f(mode, with residual, long activation) as compile-time constants: the loops around store_block are instantiated per way of storing.
@@ -1576,7 +1578,7 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
                     }
                     if (REDO && (pass || factors))
                         unscale_block<SECOND>(r, unscale, P.fscale + (long long)zb * P.Fg, f_tile0 + c, P.Fg, factors, lane);
-                    store_block<decltype(mode_c)::value, decltype(res_c)::value, decltype(long_c)::value>(J, r, stage, f_tile0 + c);
+                    store_block<decltype(mode_c)::value, decltype(res_c)::value, decltype(long_c)::value, 1>(J, r, stage, f_tile0 + c);
                 }
                 });
             }
@@ -1672,7 +1674,7 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
                             release();
                         if (REDO && (pass || factors))
                             unscale_block<SECOND>(racc, unscale, P.fscale + (long long)zb * P.Fg, ntile * P.BN + c, P.Fg, factors, lane);
-                        store_block<MODE, RES, decltype(long_c)::value>(J, racc, stage, ntile * P.BN + c);
+                        store_block<MODE, RES, decltype(long_c)::value, PP == kNarrow ? 1 : 8>(J, racc, stage, ntile * P.BN + c);
                     }
                 } else {
                     // Groups in order, round-to-nearest adds; the MMA thread restarts the main accumulator once a group has been taken.
@@ -1715,7 +1717,7 @@ __device__ __forceinline__ void igemm_pass(const CUtensorMap &tmap_x, const CUte
                         for (int c = 0; c < P.BN; c += 32) {
                             if (REDO && (pass || factors))
                                 unscale_block<SECOND>(racc, unscale, P.fscale + (long long)zb * P.Fg, ntile * P.BN + c, P.Fg, factors, lane);
-                            store_block<MODE, RES, decltype(long_c)::value>(J, racc, stage, ntile * P.BN + c);
+                            store_block<MODE, RES, decltype(long_c)::value, PP == kNarrow ? 1 : 8>(J, racc, stage, ntile * P.BN + c);
 #pragma unroll
                             for (int j = 0; j < 96; ++j) // the next block's sums move down
                                 racc[j] = racc[j + 32];

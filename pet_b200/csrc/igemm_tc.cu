@@ -573,9 +573,11 @@ static int cluster_slots(petb200_ctx *ctx, int ks) {
 // Against the fastest of all pairs on 57 shapes (these products, ResNet layers at batch 1 to 16): within 2 % on 54; the others lose
 // 4, 11 and 14 % (64 x 1000 x 256, a 200-channel 3x3 at 3 x 20 x 20, 16 x 3072 x 768).  The constants before lost up to 31 % on 12 of them.
 //   A convolution whose stages each need a raw tile of their own takes 1000 a stage whatever its width (328 channels of 1x1 in chunks
-// of 8 to 511 filters: BN 64 26.4 us, BN 128 with K split in two 21.0). A long activation adds 85 a filter in persistent tiles, which
-// four warps store, 42 elsewhere, where eight do (768 x 89 x 873, three times, with GELU: 20.3 us in tiles of 64, 17.9 in 128).
-static double est_cycles(petb200_ctx *ctx, long long base_ctas, const IgemmParams &P, int math, int ks) {
+// of 8 to 511 filters: BN 64 26.4 us, BN 128 with K split in two 21.0). A long activation adds 42 a filter, twice that in persistent
+// tiles, which four warps store and not eight (768 x 89 x 873, three times, with GELU: 20.3 us in tiles of 64, 17.9 in 128).
+// A filter of a persistent tile's epilogue costs twice that of another's for the same reason (8 x 29 x 51 x 1454: 13.4 us in tiles of 32, 11.9
+// in 128).  `beside`: launches that share the GPU, none of which is persistent.
+static double est_cycles(petb200_ctx *ctx, long long ctas, const IgemmParams &P, int math, int ks, int beside) {
     const int BN = P.BN, w = BN <= 32 ? 0 : (BN <= 64 ? 1 : 2);
     static const double tf32[3] = {570, 655, 890}, halves[3] = {910, 910, 1045}, exchange[3] = {2300, 2500, 8000};
     const double mma = math == kMathTf32x1 ? 520.0 : (math == kMathTf32x3 ? tf32[w] : halves[w]), start = 6300.0;
@@ -585,27 +587,28 @@ static double est_cycles(petb200_ctx *ctx, long long base_ctas, const IgemmParam
     if (slots <= 0)
         return 1e30; // this cluster size cannot be launched here
     const bool long_act = P.act > PETB200_ACT_RELU;
-    const double waves = (double)((base_ctas + slots - 1) / slots), epilogue = (34.0 + (!long_act ? 0.0 : (waves > 1 ? 85.0 : 42.0))) * BN;
+    const double waves = (double)((ctas * beside + slots - 1) / slots), filters = (double)P.Fg / ((P.Fg + BN - 1) / BN);
+    const double epilogue = (34.0 + (long_act ? 42.0 : 0.0)) * filters * (waves > 1 && beside == 1 ? 2.0 : 1.0);
     if (ks > 1)
         return waves * (start + stages * stage + exchange[w] + (70.0 + (long_act ? 42.0 : 0.0)) * BN / ks);
     return start + waves * std::max(stages * stage, epilogue) + (waves - 1) * 1200.0 + epilogue;
 }
 // Split K over 1, 2, 4, 8 or 16 CTAs (a cluster; 16 is beyond the portable cluster size and allowed per function): the
 // split must divide the tile width and leave every CTA a chunk.
-static int choose_ksplit(petb200_ctx *ctx, long long base_ctas, const IgemmParams &P, int math, int want, double *cycles) {
+static int choose_ksplit(petb200_ctx *ctx, long long ctas, const IgemmParams &P, int math, int want, int beside, double *cycles) {
     auto ok = [&](int ks) { return ks == 1 || (ks <= P.nchunks && P.BN % ks == 0); };
     int best = 1;
-    double best_c = est_cycles(ctx, base_ctas, P, math, 1);
+    double best_c = est_cycles(ctx, ctas, P, math, 1, beside);
     static const int ks_cap = std::min(16, std::max(1, env_int_early("PETB200_TC_KSPLIT_MAX", 16)));
     if (want > 0) {
         for (best = 16; best > 1 && !(best <= want && ok(best) && cluster_slots(ctx, best) > 0); best /= 2) {
         }
-        best_c = est_cycles(ctx, base_ctas, P, math, best);
+        best_c = est_cycles(ctx, ctas, P, math, best, beside);
     } else {
         for (int ks = 2; ks <= ks_cap; ks *= 2) {
             if (!ok(ks))
                 continue;
-            const double c = est_cycles(ctx, base_ctas, P, math, ks);
+            const double c = est_cycles(ctx, ctas, P, math, ks, beside);
             if (c < best_c * 0.97) // a deeper split has to pay for itself
                 best = ks, best_c = c;
         }
@@ -841,9 +844,9 @@ static int tc_configure(petb200_ctx *ctx, TcCore &core, const ConvGeom &g, int o
         P.ksplit = 1;
         if (!fit(bn))
             continue;
-        const long long base_ctas = (long long)mtiles * ((Fg + bn - 1) / bn) * gz * core.beside;
+        const long long ctas = (long long)mtiles * ((Fg + bn - 1) / bn) * gz;
         double cyc;
-        const int ks = choose_ksplit(ctx, base_ctas, P, core.math, want_ks, &cyc);
+        const int ks = choose_ksplit(ctx, ctas, P, core.math, want_ks, core.beside, &cyc);
         if (ks > 1) { // the landing area takes shared memory from the rings (or even from the chunk size): fit again
             P.ksplit = ks;
             if (!fit(bn))
@@ -852,7 +855,7 @@ static int tc_configure(petb200_ctx *ctx, TcCore &core, const ConvGeom &g, int o
                 P.ksplit = 1;
                 if (!fit(bn))
                     continue;
-                cyc = est_cycles(ctx, base_ctas, P, core.math, 1);
+                cyc = est_cycles(ctx, ctas, P, core.math, 1, core.beside);
             }
         }
         if (!have || cyc < best_cycles * 0.97) { // prefer the wider tile unless the narrower one clearly wins
@@ -1227,7 +1230,7 @@ static int tc_configure_kmajor(petb200_ctx *ctx, TcCore &core, int bs, int m, in
             P.BN = bn;
             double cyc;
             const int ks = choose_ksplit(ctx, (long long)P.tpi * ((n + bn - 1) / bn) * bs, P, core.math,
-                                         env_int("PETB200_TC_KSPLIT", 0), &cyc);
+                                         env_int("PETB200_TC_KSPLIT", 0), 1, &cyc);
             if (!best_bn || cyc < best * 0.97)
                 best = cyc, best_bn = bn, best_ks = ks;
         }
