@@ -669,19 +669,30 @@ __device__ __forceinline__ void store_any(const StoreJob &J, const float *bias, 
     const float bv = bias != nullptr && f0 + J.lane < J.Fg ? __ldg(bias + f0 + J.lane) : 0.f; // lane j holds filter j's
     float *dst = J.y + J.y_off + (long long)f0 * J.ys_f;
     const float *rs = RES ? J.res + J.y_off + (long long)f0 * J.ys_f : nullptr;
+    if constexpr (AHEAD == 1) {
 #pragma unroll
-    for (int j = 0; j < 32; j += AHEAD) {
-        float q[AHEAD];
-#pragma unroll
-        for (int i = 0; i < AHEAD; ++i)
-            q[i] = RES && j + i < nf ? __ldg(rs + (long long)(j + i) * J.ys_f) : 0.f;
-#pragma unroll
-        for (int i = 0; i < AHEAD; ++i, dst += J.ys_f) {
-            float v = r[j + i] + __shfl_sync(0xffffffffu, bv, j + i);
+        for (int j = 0; j < 32; ++j, dst += J.ys_f) {
+            float v = r[j] + __shfl_sync(0xffffffffu, bv, j);
             if (RES)
-                v += q[i];
-            if (j + i < nf)
+                v += j < nf ? __ldg(rs + (long long)j * J.ys_f) : 0.f;
+            if (j < nf)
                 *dst = relu ? fmaxf(v, 0.f) : v;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < 32; j += AHEAD) {
+            float q[AHEAD];
+#pragma unroll
+            for (int i = 0; i < AHEAD; ++i)
+                q[i] = RES && j + i < nf ? __ldg(rs + (long long)(j + i) * J.ys_f) : 0.f;
+#pragma unroll
+            for (int i = 0; i < AHEAD; ++i, dst += J.ys_f) {
+                float v = r[j + i] + __shfl_sync(0xffffffffu, bv, j + i);
+                if (RES)
+                    v += q[i];
+                if (j + i < nf)
+                    *dst = relu ? fmaxf(v, 0.f) : v;
+            }
         }
     }
 }
