@@ -6,15 +6,15 @@
 // accumulators and the A operand live in tensor memory (TMEM).  Sixteen warps:
 //   0      TMA producer for the packed weights: per K stage (32 words of K) one 2-D tile of B_hi and one of B_lo, straight into
 //          128-byte-swizzled K-major shared memory.
-//   1      one thread issues, per K=8 step, the three products of 3xTF32 as two MMAs — A_hi x [B_hi;B_lo] (one MMA of width
+//   1      one thread issues, per K=8 step (K=16 of halves), the three products of 3xTF32 as two MMAs — A_hi x [B_hi;B_lo] (one MMA of width
 //          2*BN: the hi*hi sum and the hi*lo sum in adjacent accumulators) and A_lo x B_hi — and commits the stage release
 //          barriers.
 //   2      TMA producer for the RAW activation tile of one channel chunk (all taps share it): a 5-D box
 //          [images, channels, depth, rows, cols] of the NC(D)HW input, zero-filled outside the tensor, which is exactly the
 //          convolution's zero padding.  Box start along W is rounded down to 16 bytes.  (3 is idle.)
 //   4-7, 8-11  two transform sets taking alternate K stages.  Thread p owns pixel p of the tile: for every K stage it gathers its
-//          32 values from the raw tile (fixed strides where the channel chunk allows, else through a precomputed offset table:
-//          tap shift, dilation, channel plane), splits each fp32 into hi (top 19 bits) and lo = x - hi, and writes both to
+//          32 values (64 for halves) from the raw tile (fixed strides where the channel chunk allows, else through a precomputed offset table:
+//          tap shift, dilation, channel plane), splits each fp32 into hi (top 19 bits, or a half) and lo = x - hi, and writes both to
 //          TMEM with tcgen05.st, which leaves the shared-memory read port to B alone.  With one tile per CTA they also store it.
 //   12-15  drain warps.  The tensor core truncates its fp32 accumulator after every MMA, so long K ranges empty the main
 //          accumulator every few stages into a running total that these warps hold.  With persistent tiles they store a finished

@@ -1176,7 +1176,7 @@ int tc_set_wait_limit_ns(unsigned long long ns) {
     return PETB200_OK;
 }
 int tc_conv_row_pitch(void *h) { return ((TcConv *)h)->g.Wst; }
-// (fp16 halves carry TF32's significand: the family keeps its name)
+// (halves carry TF32's significand within their range, see row_exponent: the family keeps its name)
 static const char *tc_variant_name(int math) {
     return math == kMathTf32x1 ? "tc_1xtf32_ts" : (math == kMathBf16x3 ? "tc_bf16x3_ts" : (math == kMathF16x3 ? "tc_3xtf32_f16_ts" : "tc_3xtf32_ts"));
 }
